@@ -2409,7 +2409,7 @@ int lra_ctx_set_wait_limit(lra_ctx* ctx, int64_t ns) {
   }
   if (cudaSetDevice(ctx->device) != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess ||
       set_wait_limit_qr((uint64_t)ns) != cudaSuccess || set_wait_limit_dense((uint64_t)ns) != cudaSuccess ||
-      set_wait_limit_tc((uint64_t)ns) != cudaSuccess) {
+      set_wait_limit_tc((uint64_t)ns) != cudaSuccess || set_wait_limit_snorm((uint64_t)ns) != cudaSuccess) {
     ctx->last_error = cudaGetErrorString(cudaGetLastError());
     return LRA_ECUDA;
   }
@@ -3582,17 +3582,34 @@ int lra_curfact(lra_ctx* ctx, int dtype, int64_t m, int64_t n, const void* A, in
 namespace lra {
 namespace {
 
+// the start vector of a power iteration (n entries)
+template <typename T>
+T* snorm_start(lra_ctx* ctx, int64_t n, RandSrc& rs) {
+  T* x = ctx->arena.alloc_n<T>(std::max<int64_t>(n, 1));
+  if (rs.injected_gauss())
+    sketch_from_stream(ctx, rs.take_gauss_raw(n), n, x, false);
+  else
+    rs.gauss(n, x, false);
+  return x;
+}
+
+// the norm of a dense A (B null) or A - B
+template <typename T>
+double snorm_dense(lra_ctx* ctx, const lra_opts& o, int64_t m, int64_t n, const T* A, int64_t lda, const T* B,
+                   int64_t ldb, bool herm, RandSrc& rs) {
+  T* x = snorm_start<T>(ctx, n, rs);
+  // an empty matrix: zero after the first step, if one is taken
+  if (m <= 0 || n <= 0) return o.snorm_niter == 0 || o.atol >= 1 ? 1 : 0;
+  return snorm_power<T>(ctx, m, n, A, lda, B, ldb, herm, o.snorm_niter, o.atol, o.rtol, x);
+}
+
 // power iteration of src/snorm.jl:14-45 with the operator given as callbacks
 template <typename T, class FwdFn, class AdjFn>
 double snorm_loop(lra_ctx* ctx, const lra_opts& o, int64_t m, int64_t n, bool herm, RandSrc& rs, FwdFn fwd,
                   AdjFn adj) {
-  T* xn = ctx->arena.alloc_n<T>(std::max<int64_t>(n, 1));
+  T* xn = snorm_start<T>(ctx, n, rs);
   T* xm = ctx->arena.alloc_n<T>(std::max<int64_t>(m, 1));
   T* nrm = ctx->arena.alloc_n<T>(1);
-  if (rs.injected_gauss())
-    sketch_from_stream(ctx, rs.take_gauss_raw(n), n, xn, false);
-  else
-    rs.gauss(n, xn, false);
   auto norm = [&](const T* x, int64_t len) {
     col_norms(ctx, len, 1, x, std::max<int64_t>(len, 1), nrm);
     T h = 0;
@@ -3705,21 +3722,14 @@ int lra_snorm(lra_ctx* ctx, int dtype, int64_t m, int64_t n, const void* A, int6
       check_input(ctx, *opts, m, n, dA);
       const bool herm = hermitian < 0 ? (m == n && is_symmetric(ctx, n, dA.p, dA.ld)) : hermitian != 0;
       RandSrc rs(ctx, rand, opts->seed);
-      const bool lin = ctx->linop != nullptr;
+      if (!ctx->linop) {
+        *out = snorm_dense<T>(ctx, *opts, m, n, dA.p, dA.ld, (const T*)nullptr, 0, herm, rs);
+        return;
+      }
       *out = snorm_loop<T>(
           ctx, *opts, m, n, herm, rs,
-          [&](const T* x, T* y) {
-            if (lin)
-              linop_apply<T>(ctx, 'n', 1, x, std::max<int64_t>(n, 1), y, std::max<int64_t>(m, 1));
-            else
-              gemv<T>(ctx, 'n', m, n, T(1), dA.p, dA.ld, x, T(0), y);
-          },
-          [&](const T* y, T* x) {
-            if (lin)
-              linop_apply<T>(ctx, 'c', 1, y, std::max<int64_t>(m, 1), x, std::max<int64_t>(n, 1));
-            else
-              gemv<T>(ctx, 't', m, n, T(1), dA.p, dA.ld, y, T(0), x);
-          });
+          [&](const T* x, T* y) { linop_apply<T>(ctx, 'n', 1, x, std::max<int64_t>(n, 1), y, std::max<int64_t>(m, 1)); },
+          [&](const T* y, T* x) { linop_apply<T>(ctx, 'c', 1, y, std::max<int64_t>(m, 1), x, std::max<int64_t>(n, 1)); });
     });
   });
 }
@@ -3747,16 +3757,7 @@ int lra_snormdiff(lra_ctx* ctx, int dtype, int64_t m, int64_t n, const void* A, 
       DMat<T> dB = stage_in<T>(ctx, B, m, n, ldb);
       const bool herm = m == n && is_symmetric(ctx, n, dA.p, dA.ld) && is_symmetric(ctx, n, dB.p, dB.ld);
       RandSrc rs(ctx, rand, opts->seed);
-      *out = snorm_loop<T>(
-          ctx, *opts, m, n, herm, rs,
-          [&](const T* x, T* y) {
-            gemv<T>(ctx, 'n', m, n, T(1), dA.p, dA.ld, x, T(0), y);
-            gemv<T>(ctx, 'n', m, n, T(-1), dB.p, dB.ld, x, T(1), y);
-          },
-          [&](const T* y, T* x) {
-            gemv<T>(ctx, 't', m, n, T(1), dA.p, dA.ld, y, T(0), x);
-            gemv<T>(ctx, 't', m, n, T(-1), dB.p, dB.ld, y, T(1), x);
-          });
+      *out = snorm_dense<T>(ctx, *opts, m, n, dA.p, dA.ld, dB.p, dB.ld, herm, rs);
     });
   });
 }
@@ -3823,16 +3824,7 @@ int lra_snormdiff_id(lra_ctx* ctx, int dtype, char trans, int64_t m, int64_t n, 
       else if (N > k) set_zero(ctx, Fp + k * ldm, ldm * (N - k));
       scatter_cols(ctx, M, N, Fp, ldm, p, Fd, ldm);
       RandSrc rs(ctx, rand, opts->seed);
-      *out = snorm_loop<T>(
-          ctx, *opts, M, N, false, rs,
-          [&](const T* x, T* y) {
-            gemv<T>(ctx, 'n', M, N, T(1), Aop, ldm, x, T(0), y);
-            gemv<T>(ctx, 'n', M, N, T(-1), Fd, ldm, x, T(1), y);
-          },
-          [&](const T* y, T* x) {
-            gemv<T>(ctx, 't', M, N, T(1), Aop, ldm, y, T(0), x);
-            gemv<T>(ctx, 't', M, N, T(-1), Fd, ldm, y, T(1), x);
-          });
+      *out = snorm_dense<T>(ctx, *opts, M, N, Aop, ldm, Fd, ldm, false, rs);
     });
   });
 }

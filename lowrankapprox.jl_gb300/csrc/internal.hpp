@@ -428,6 +428,12 @@ template <typename T>
 void gemv(lra_ctx* ctx, char trans, int64_t m, int64_t n, T alpha, const T* A, int64_t lda,
           const T* x, T beta, T* y);
 
+// the power iteration of snorm on D = A, or A - B where B is given (x: the
+// start vector, n; overwritten), in one cooperative launch
+template <typename T>
+double snorm_power(lra_ctx* ctx, int64_t m, int64_t n, const T* A, int64_t lda, const T* B, int64_t ldb, bool herm,
+                   int64_t niter, double atol, double rtol, T* x);
+
 // kernel-launch accounting (every launcher calls this once per launch)
 inline void count_launch(lra_ctx* ctx, int n = 1) { ctx->launches += n; }
 void post_launch(lra_ctx* ctx, const char* name);
@@ -438,6 +444,7 @@ void post_launch(lra_ctx* ctx, const char* name);
 cudaError_t set_wait_limit_qr(uint64_t ns);
 cudaError_t set_wait_limit_dense(uint64_t ns);
 cudaError_t set_wait_limit_tc(uint64_t ns);
+cudaError_t set_wait_limit_snorm(uint64_t ns);
 int probe_grid_wait(lra_ctx* ctx, int* returned);
 
 // the tuning table: defaults, then the file named by LRA_TUNING or the
