@@ -213,7 +213,9 @@ int lra_ctx_stage_ms(const lra_ctx* ctx, double out[4]);
    parts of the tensor-core sketch, 0 as many as fill the SMs),
    "jacobi_jb" (FP32 Jacobi block columns 4, 8, 16, 32; 0 by size),
    "jacobi_cluster" (largest cluster of the in-cluster FP32 Jacobi, 2..16;
-   0 the largest schedulable, 1 never), "trsm_inv" (1: FP64 triangular
+   0 the largest schedulable, 1 never, -1 (default) the largest, except for
+   Float64 on the mixed path, whose FP32 sweeps run on Gram products),
+   "trsm_inv" (1: FP64 triangular
    solves on the tensor-core path by substitution instead of the
    unit-diagonal inverse), "gram_start" (cosine x 1e4 where the FP32 sweeps
    hand over to the Gram polish, 0 by order));

@@ -2409,7 +2409,8 @@ int lra_ctx_set_wait_limit(lra_ctx* ctx, int64_t ns) {
   }
   if (cudaSetDevice(ctx->device) != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess ||
       set_wait_limit_qr((uint64_t)ns) != cudaSuccess || set_wait_limit_dense((uint64_t)ns) != cudaSuccess ||
-      set_wait_limit_tc((uint64_t)ns) != cudaSuccess || set_wait_limit_snorm((uint64_t)ns) != cudaSuccess) {
+      set_wait_limit_tc((uint64_t)ns) != cudaSuccess || set_wait_limit_snorm((uint64_t)ns) != cudaSuccess ||
+      set_wait_limit_jg((uint64_t)ns) != cudaSuccess) {
     ctx->last_error = cudaGetErrorString(cudaGetLastError());
     return LRA_ECUDA;
   }
@@ -3337,7 +3338,7 @@ int lra_pheigfact(lra_ctx* ctx, int dtype, int64_t n, const void* A, int64_t lda
       add_diag(ctx, k, B, ldk, shift);
       T* Z = ctx->arena.alloc_n<T>((size_t)ldk * ldk);
       T* S = ctx->arena.alloc_n<T>(ldk);
-      jacobi_svd_fast<T>(ctx, k, B, ldk, Z, ldk, S);
+      jacobi_svd_fast<T>(ctx, k, B, ldk, Z, ldk, S, true);
       std::vector<T> hS(k);
       to_host(ctx, hS.data(), S, k);
       LRA_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -157,7 +157,8 @@ bool trace_on() {
 //   qr_sms <SMs a pivoted-QR launch may take; 0: all>
 //   tc_split <most K parts of the tensor-core sketch; 0: as many as fill the SMs>
 //   jacobi_jb <columns per FP32 Jacobi block: 4, 8, 16, 32; 0: by size>
-//   jacobi_cluster <largest cluster of the in-cluster FP32 Jacobi, 2..16; 0: largest schedulable; 1: off>
+//   jacobi_cluster <largest cluster of the in-cluster FP32 Jacobi, 2..16; 0: largest schedulable; 1: off;
+//     -1: the largest, but the Gram-product sweeps on the mixed path>
 //   trsm_inv <0: FP64 triangular solves on the tensor-core path by the explicit inverse; 1: substitution>
 //   gram_start <cosine x 1e4 where the FP32 Jacobi sweeps stop; 0: min(3e-2, 12 / n)>
 // lowrankapprox/autotune.py writes it from its sweeps; unknown keys and
@@ -173,7 +174,7 @@ static void tuning_defaults(lra_tuning* t) {
   t->qr_sms = 0;
   t->tc_split = 0;
   t->jacobi_jb = 0;
-  t->jacobi_cluster = 0;
+  t->jacobi_cluster = -1;
   t->trsm_inv = 0;
   t->gram_start = 0;
 }
@@ -220,7 +221,7 @@ bool set_tuning(lra_tuning* t, const char* key, int64_t index, int64_t value) {
     return true;
   }
   if (!std::strcmp(key, "jacobi_cluster")) {
-    if (value < 0 || value > 16) return false;
+    if (value < -1 || value > 16) return false;
     t->jacobi_cluster = (int)value;
     return true;
   }

@@ -1586,7 +1586,7 @@ void jacobi_svd(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t ldv, T
                  block ? " block" : "", (long long)n, sweeps, grid);
 }
 
-bool jacobi_svd_df(lra_ctx* ctx, int64_t n, double* X, int64_t ldx, double* V, int64_t ldv, double* S) {
+bool jacobi_svd_df(lra_ctx* ctx, int64_t n, double* X, int64_t ldx, double* V, int64_t ldv, double* S, bool clusters) {
   // 4-column blocks: the double-float rotations are issue-bound, so the work
   // is spread over as many SMs as the block pairs allow
   constexpr int JDF = 4;
@@ -1609,7 +1609,9 @@ bool jacobi_svd_df(lra_ctx* ctx, int64_t n, double* X, int64_t ldx, double* V, i
   P.S = S;
   // double-float resolves cosines down to a few units of 2^-46 sqrt(n)
   P.tol = std::max((double)Real<double>::eps * 2.0 * std::sqrt((double)n), 8.0 * std::ldexp(1.0, -46) * std::sqrt((double)n));
-  P.stop = std::sqrt(P.tol) * 0.1;  // quadratic convergence from the FP32 sweeps
+  // quadratic convergence from the FP32 sweeps; but not among columns of equal
+  // norms, whose rounding-level cosines no single sweep removes
+  P.stop = clusters ? 4.0 * P.tol : std::sqrt(P.tol) * 0.1;
   P.max_sweeps = 40;
   P.part = ctx->arena.alloc_n<double>(grid);
   P.bar = reinterpret_cast<GridBar*>(ctx->arena.alloc(sizeof(GridBar)));

@@ -86,7 +86,8 @@ struct lra_tuning {
   // columns per block of the FP32 block Jacobi (4, 8, 16, 32; 0: by size)
   int jacobi_jb;
   // largest cluster of the cluster-resident FP32 Jacobi (2..16; 0: the
-  // largest that can be scheduled; 1: never, the block-pair kernel instead)
+  // largest that can be scheduled; 1: never, the block-pair kernel instead;
+  // -1: the largest, but the mixed path's sweeps on Gram products)
   int jacobi_cluster;
   // FP64 triangular solves on the tensor-core path: 0 multiply by the
   // explicit inverse (k from 65 to 2048), 1 blocked substitution
@@ -330,12 +331,19 @@ std::vector<T> small_svd(lra_ctx* ctx, int64_t k, const T* Mm, T* U, T* V, T* S)
 template <typename T>
 std::vector<T> sort_desc(lra_ctx* ctx, int64_t k, T* S, T* U, T* V);
 
+// FP32 block Jacobi sweeps through Gram products (jacobi_gram.cu): X V
+// rotated until a sweep's largest cosine is at most `stop`; V is the identity
+// on entry, ld a multiple of 4, rows n .. ld zero.  False (nothing done) when
+// the shape does not fit
+bool jacobi_gram_sweeps(lra_ctx* ctx, int64_t n, float* X, float* V, int64_t ld, double stop);
 // Polish sweeps of the mixed-precision path in double-float (X and V
 // Float64 in and out, V overwritten); false when n does not fit.
-bool jacobi_svd_df(lra_ctx* ctx, int64_t n, double* X, int64_t ldx, double* V, int64_t ldv, double* S);
+// (clusters: to the last cosine, not by the quadratic stop)
+bool jacobi_svd_df(lra_ctx* ctx, int64_t n, double* X, int64_t ldx, double* V, int64_t ldv, double* S, bool clusters);
 // jacobi_svd for Float64 with the bulk of the sweeps in FP32 and FP64 polish
+// (shifted: the eigenproblem's B + s I, whose columns all have norms near s)
 template <typename T>
-void jacobi_svd_fast(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t ldv, T* S);
+void jacobi_svd_fast(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t ldv, T* S, bool shifted = false);
 
 // exact symmetry test of a square device matrix
 template <typename T>
@@ -445,6 +453,7 @@ cudaError_t set_wait_limit_qr(uint64_t ns);
 cudaError_t set_wait_limit_dense(uint64_t ns);
 cudaError_t set_wait_limit_tc(uint64_t ns);
 cudaError_t set_wait_limit_snorm(uint64_t ns);
+cudaError_t set_wait_limit_jg(uint64_t ns);
 int probe_grid_wait(lra_ctx* ctx, int* returned);
 
 // the tuning table: defaults, then the file named by LRA_TUNING or the

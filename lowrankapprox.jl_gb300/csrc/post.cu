@@ -527,7 +527,7 @@ bool gram_polish(lra_ctx* ctx, int64_t n, double* X, int64_t ldx, double* Wacc, 
 }
 
 template <typename T>
-void jacobi_svd_fast(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t ldv, T* S) {
+void jacobi_svd_fast(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t ldv, T* S, bool shifted) {
   if (sizeof(T) != 8 || n < 64) {
     jacobi_svd<T>(ctx, n, X, ldx, V, ldv, S);
     return;
@@ -573,14 +573,30 @@ void jacobi_svd_fast(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t l
   float* X32 = ctx->arena.alloc_n<float>((size_t)ld32 * n);
   float* V32 = ctx->arena.alloc_n<float>((size_t)ld32 * n);
   float* S32 = ctx->arena.alloc_n<float>(n);
-  cast<T, float>(ctx, n, n, X, ldx, X32, ld32, scale);
   // the Gram polish converges quadratically from cosines of a few 1e-3 (the
   // FP32 sweeps stop there); the pairwise FP64 sweeps want them near 1e-6
   // (neighbouring singular values of a smooth spectrum of n are ~1/n apart
   // relative to each other, and the simultaneous rotations converge only
   // from cosines below that gap: the start level falls with n)
   const double start = ctx->tuning.gram_start > 0 ? 1e-4 * ctx->tuning.gram_start : std::min(kGramStart, 12.0 / (double)n);
-  jacobi_svd<float>(ctx, n, X32, ld32, V32, ld32, S32, true, df_polish ? start : 0.0);
+  // Gram-product sweeps (jacobi_gram.cu) at every order they take (64 on): 3.5
+  // -> 2.3 ms against the in-cluster kernel at n = 363, 70 -> 26 ms against the
+  // block-pair kernel at n = 1803; the tuning keys of those two ask for them
+  // instead.  A shifted eigenproblem stays with the column rotations: its norms
+  // lie together, the pairwise sweeps have to finish it, and they start
+  // better from those (31.6 against 32.0 ms for a 1500 pheigfact).
+  bool swept = false;
+  if (df_polish && !shifted && ctx->tuning.jacobi_cluster < 0 && ctx->tuning.jacobi_jb == 0) {
+    set_zero(ctx, X32, ld32 * n);
+    set_zero(ctx, V32, ld32 * n);
+    cast<T, float>(ctx, n, n, X, ldx, X32, ld32, scale);
+    set_identity(ctx, n, n, V32, ld32);
+    swept = jacobi_gram_sweeps(ctx, n, X32, V32, ld32, start);
+  }
+  if (!swept) {
+    cast<T, float>(ctx, n, n, X, ldx, X32, ld32, scale);
+    jacobi_svd<float>(ctx, n, X32, ld32, V32, ld32, S32, true, df_polish ? start : 0.0);
+  }
   // 2. the rotation in FP64, re-orthonormalized by two Newton-Schulz steps
   //    W <- W (3 I - W'W) / 2: with |I - W'W| near 1e-6 from the FP32
   //    sweeps the error squares each step, to rounding level after two
@@ -611,7 +627,8 @@ void jacobi_svd_fast(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t l
       done = gram_polish(ctx, n, Xd, ldx, Yd, reinterpret_cast<double*>(S), tol, n > 1024 ? 8 : 5);
       if (!done) {
         double* Y2 = reinterpret_cast<double*>(W2);
-        done = jacobi_svd_df(ctx, n, Xd, ldx, Y2, n, reinterpret_cast<double*>(S));
+        // what the polish of an unshifted core leaves are clusters
+        done = jacobi_svd_df(ctx, n, Xd, ldx, Y2, n, reinterpret_cast<double*>(S), !shifted);
         if (!done) jacobi_svd<double>(ctx, n, Xd, ldx, Y2, n, reinterpret_cast<double*>(S), true);
         double* Gd = reinterpret_cast<double*>(G);
         gemm<double>(ctx, 'n', 'n', n, n, n, 1.0, Yd, n, Y2, n, 0.0, Gd, n);
@@ -625,7 +642,7 @@ void jacobi_svd_fast(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t l
   ctx->arena.release(mk);
 }
 
-template void jacobi_svd_fast<float>(lra_ctx*, int64_t, float*, int64_t, float*, int64_t, float*);
-template void jacobi_svd_fast<double>(lra_ctx*, int64_t, double*, int64_t, double*, int64_t, double*);
+template void jacobi_svd_fast<float>(lra_ctx*, int64_t, float*, int64_t, float*, int64_t, float*, bool);
+template void jacobi_svd_fast<double>(lra_ctx*, int64_t, double*, int64_t, double*, int64_t, double*, bool);
 
 }  // namespace lra
