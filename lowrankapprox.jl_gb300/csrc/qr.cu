@@ -19,6 +19,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <climits>
 #include <vector>
 #include <cstdio>
 #include <cstdlib>
@@ -882,151 +883,237 @@ struct QrDf {
 };
 
 
-template <int NT>
-__global__ void __launch_bounds__(NT) geqp3_df_kernel(QrParams<double> P, QrV2Extra X, QrDf D) {
-  __shared__ QrShared<double> sh;
-  __shared__ Df s_f;  // reflector scale / tau / beta in df form
-  __shared__ Df s_tau;
-  __shared__ Df s_beta;
-  extern __shared__ unsigned char qr_dyn[];
+// Sketches whose columns do not fit shared memory.  CTA b owns the columns
+// j = b mod G, a warp per column at a time; the columns stay in global memory
+// (L2, and L1 once a CTA's remaining rows fit there).
+//
+// Bound: the columns' traffic between L2 and the SMs, and the latency of the
+// step's serial parts.  The rank-1 update of a step is therefore deferred to
+// the next step's pass over the column, which updates each entry and adds it to
+// the new dot product at once: one read and one write of the column a pivot
+// (the two-pass form read it twice).  Until then the column's f is kept beside
+// its state, and its row c, which the norm downdate needs, is brought up to
+// date by itself; readers of the next pivot column apply its pending update as
+// they load it.  The pivot exchange is one 16-byte word per CTA (norm key,
+// column, stop flag, sequence number), polled by every CTA.  2056 x 2203, 1834
+// pivots: 21.2 us a pivot with separate passes and grid barriers, 15 us with this one
+// (38.7 -> 29 ms).
+struct QrXw {
+  ulonglong2* word;  // [2][G]
+  float2* f;         // [2][G] the candidate's pending f
+  float* prev;       // PG: [G][2][m] the previous reflector, each CTA its own
+};
+
+__device__ __forceinline__ void st_word(ulonglong2* p, unsigned long long x, unsigned long long y) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.release.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_word(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(v.x), "=l"(v.y)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+
+// PG: the previous reflector in global memory (sketches of more rows than two
+// reflectors fit shared memory)
+template <int NT, bool PG>
+__global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV2Extra X, QrDf D, QrXw E) {
   constexpr int NW = NT / 32;
+  constexpr int RB = 8;  // rows per lane of a register chunk; the next chunk is in flight meanwhile
+  __shared__ double s_redd[32];
+  __shared__ long long s_k[NW];
+  __shared__ int s_i[NW], s_fl[NW];
+  __shared__ Df s_alpha, s_f, s_tau, s_beta;
+  __shared__ double s_taud, s_betad;
+  __shared__ int s_pvt, s_stop, s_ok;
+  extern __shared__ unsigned char qr_dyn[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t gw = (int64_t)blockIdx.x * NW + wid;
-  const int64_t W = (int64_t)gridDim.x * NW;
-  const int64_t m = P.m, n = P.n, lda = P.lda;
-  auto ldown = [](const float* p) { return *p; };
+  const int G = (int)gridDim.x, cta = (int)blockIdx.x;
+  const int m = (int)P.m, n = (int)P.n;
+  const int64_t lda = P.lda;
   auto stamp = [&](int64_t c, int ph) {
-    if (D.stamps && blockIdx.x == 0 && threadIdx.x == 0 && c < P.kmax) D.stamps[c * 16 + ph] = globaltimer_ns();
+    if (D.stamps && cta == 0 && threadIdx.x == 0 && c < P.kmax) D.stamps[c * 16 + ph] = globaltimer_ns();
   };
   float* __restrict__ Bh = D.Bh;
   float* __restrict__ Bl = D.Bl;
   const double tol3z = sqrt(Real<double>::eps);
   const int64_t lastrk = m < n ? m : n;
-  const int64_t ncol = gw < n ? (n - 1 - gw) / W + 1 : 0;
-  const int64_t ncmax = (n + W - 1) / W;
-  const int nslot = (int)(ncmax * NW);
+  const int nslot = cta < n ? (n - 1 - cta) / G + 1 : 0;  // slot s: column cta + s G
+  // this step's reflector and the previous one's, entry of row i at [i]
   float* vh = reinterpret_cast<float*>(qr_dyn);
-  float* vl = vh + P.vcap;
-  Df* s_vn1 = reinterpret_cast<Df*>(vl + P.vcap);
-  Df* s_vn2 = s_vn1 + nslot;
-  Df* s_arc = s_vn2 + nslot;
-  unsigned char* s_st = reinterpret_cast<unsigned char*>(s_arc + nslot);
-  auto slot_col = [&](int s) -> int64_t {
-    return (int64_t)blockIdx.x * NW + (s % NW) + (int64_t)(s / NW) * W;
-  };
-  // warp 0 alone reduces the per-CTA candidates; one block barrier
-  __shared__ int s_lst;
-  auto reduce_pivot_key = [&](const int* lstp = nullptr) -> int64_t {
-    if (wid == 0) {
-      if (lane == 0 && lstp) s_lst = *((const volatile int*)lstp);
-      long long k = -2;
-      int64_t i = INT64_MAX;
-      for (int b = lane; b < gridDim.x; b += 32) key_merge(k, i, __ldcg(X.part_k + b), __ldcg(P.part_i + b));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const long long k2 = __shfl_xor_sync(0xffffffffu, k, o);
-        const int64_t i2 = __shfl_xor_sync(0xffffffffu, i, o);
-        key_merge(k, i, k2, i2);
-      }
-      if (lane == 0) sh.si[0] = i;
-    }
-    __syncthreads();
-    const int64_t r = sh.si[0];
-    return r;
-  };
-  auto publish = [&](long long k, int64_t i) {
+  float* vl = vh + m;
+  float* ph = PG ? E.prev + (size_t)cta * 2 * m : vl + m;
+  float* pl = ph + m;
+  const int ncap = (n + G - 1) / G;
+  Df* s_vn1 = reinterpret_cast<Df*>(PG ? vl + m : pl + m);
+  Df* s_vn2 = s_vn1 + ncap;
+  Df* s_arc = s_vn2 + ncap;  // row c of each column after step c
+  Df* s_fp = s_arc + ncap;   // f of the column's pending update (zero: none)
+  unsigned char* s_st = reinterpret_cast<unsigned char*>(s_fp + ncap);
+
+  // the CTA's candidate to all others, theirs back: the pivot (s_pvt) and the OR
+  // of the stop flags (s_stop); false when the wait gave up
+  unsigned seq = 0;
+  auto exchange = [&](long long k, int i, int fl) -> bool {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const long long k2 = __shfl_xor_sync(0xffffffffu, k, o);
-      const int64_t i2 = __shfl_xor_sync(0xffffffffu, i, o);
-      key_merge(k, i, k2, i2);
+      const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
+      if (k2 > k || (k2 == k && i2 < i)) {
+        k = k2;
+        i = i2;
+      }
+      fl |= __shfl_xor_sync(0xffffffffu, fl, o);
     }
-    __syncthreads();
     if (lane == 0) {
-      sh.sk[wid] = k;
-      sh.si[wid] = i;
+      s_k[wid] = k;
+      s_i[wid] = i;
+      s_fl[wid] = fl;
+    }
+    __syncthreads();  // (and every column write of this CTA is before the release below)
+    ++seq;
+    if (wid == 0) {
+      ulonglong2* wd = E.word + (seq & 1) * G;
+      k = lane < NW ? s_k[lane] : -2;
+      i = lane < NW ? s_i[lane] : INT_MAX;
+      fl = lane < NW ? s_fl[lane] : 0;
+      auto reduce = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const long long k2 = __shfl_xor_sync(0xffffffffu, k, o);
+          const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
+          if (k2 > k || (k2 == k && i2 < i)) {
+            k = k2;
+            i = i2;
+          }
+          fl |= __shfl_xor_sync(0xffffffffu, fl, o);
+        }
+      };
+      reduce();
+      if (lane == 0) {
+        const Df f = i < n ? s_fp[(i - cta) / G] : Df{0.f, 0.f};
+        __stcg(E.f + (seq & 1) * G + cta, make_float2(f.h, f.l));
+        __threadfence();
+        st_word(wd + cta, (unsigned long long)k,
+                ((unsigned long long)seq << 32) | ((unsigned long long)(fl ? 1u : 0u) << 31) | (unsigned)i);
+      }
+      bool ok = true;
+      k = -2;
+      i = INT_MAX;
+      fl = 0;
+      const uint64_t t0 = globaltimer_ns(), lim = wait_limit_ns();
+      for (int b = lane; b < G; b += 32) {
+        ulonglong2 w = ld_word(wd + b);
+        for (unsigned it = 1; ok && (unsigned)(w.y >> 32) != seq; ++it) {
+          w = ld_word(wd + b);
+          if (it & 15) continue;
+          if (*((volatile int*)&P.bar->err) != 0) {
+            ok = false;
+          } else if (globaltimer_ns() - t0 > lim) {
+            atomicCAS(&P.bar->err, 0, 4);
+            ok = false;
+          }
+        }
+        const long long kb = (long long)w.x;
+        const int ib = (int)(w.y & 0x7fffffffu);
+        if (kb > k || (kb == k && ib < i)) {
+          k = kb;
+          i = ib;
+        }
+        fl |= (int)(w.y >> 31) & 1;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      reduce();
+      __threadfence();
+      if (lane == 0) {
+        s_pvt = i;
+        s_stop = fl;
+        s_ok = ok ? 1 : 0;
+      }
     }
     __syncthreads();
-    if (wid == 0) {
-      long long k0 = lane < NW ? sh.sk[lane] : -2;
-      int64_t i0 = lane < NW ? sh.si[lane] : INT64_MAX;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const long long k2 = __shfl_xor_sync(0xffffffffu, k0, o);
-        const int64_t i2 = __shfl_xor_sync(0xffffffffu, i0, o);
-        key_merge(k0, i0, k2, i2);
-      }
-      if (lane == 0) {
-        X.part_k[blockIdx.x] = k0;
-        P.part_i[blockIdx.x] = i0;
-      }
-    }
-  };
-  // 2-norm of a column segment held as (h, l), by one warp, in FP64
-  auto warp_nrm2_df = [&](const float* h, const float* l, int64_t len) -> double {
-    double mx = 0;
-    for (int64_t i = lane; i < len; i += 32) mx = fmax(mx, fabs(df_val(__ldcg(h + i), __ldcg(l + i))));
-    mx = warp_max(mx);
-    if (mx == 0 || !isfinite(mx)) return mx;
-    const double sc = pow2_scale_inv(mx);
-    double acc = 0;
-    for (int64_t i = lane; i < len; i += 32) {
-      const double t = df_val(__ldcg(h + i), __ldcg(l + i)) * sc;
-      acc = fma(t, t, acc);
-    }
-    acc = warp_sum(acc);
-    return sqrt(acc) / sc;
+    return s_ok != 0;
   };
 
-  // ---- initial column norms (precomputed), ptol, first pivot ---------------
-  for (int s = threadIdx.x; s < nslot; s += NT) {
-    const int64_t j = slot_col(s);
-    s_st[s] = j < n ? ST_LIVE : 0;
-    const Df nr = (j < n && P.pivot) ? df_split(D.vn0[j]) : Df{0.f, 0.f};
-    s_vn1[s] = s_vn2[s] = nr;
-  }
-  __syncthreads();
+  // ---- initial column norms (precomputed), ptol, first pivot
   double lmax = 0;
   long long bk = -2;
-  int64_t bi = INT64_MAX;
-  for (int s = threadIdx.x; s < nslot; s += NT)
-    if (s_st[s] & ST_LIVE) {
-      lmax = fmax(lmax, D.vn0[slot_col(s)]);
-      key_merge(bk, bi, df_key(s_vn1[s]), slot_col(s));
+  int bi = INT_MAX;
+  for (int s = threadIdx.x; s < nslot; s += NT) {
+    const int j = cta + s * G;
+    s_st[s] = ST_LIVE;
+    const double v0 = D.vn0[j];
+    const Df nr = df_split(v0);
+    s_vn1[s] = s_vn2[s] = nr;
+    s_fp[s] = Df{0.f, 0.f};
+    lmax = fmax(lmax, v0);
+    const long long k = df_key(nr);
+    if (k > bk || (k == bk && j < bi)) {
+      bk = k;
+      bi = j;
     }
-  lmax = block_max(lmax, sh.red);
-  publish(bk, bi);
-  if (threadIdx.x == 0) P.part_d[blockIdx.x] = lmax;
+  }
+  lmax = block_max(lmax, s_redd);
+  if (threadIdx.x == 0) P.part_d[cta] = lmax;
   if (!grid_sync(P.bar)) return;
   double maxnrm = 0;
-  for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) maxnrm = fmax(maxnrm, __ldcg(P.part_d + b));
-  maxnrm = block_max(maxnrm, sh.red);
+  for (int b = threadIdx.x; b < G; b += NT) maxnrm = fmax(maxnrm, __ldcg(P.part_d + b));
+  maxnrm = block_max(maxnrm, s_redd);
   const double ptol = fmax(P.atol * *D.scale, P.rtol * maxnrm);
-  int64_t pvt = reduce_pivot_key();
+  if (!exchange(bk, bi, 0)) return;
 
   int64_t kres = P.kmax, nfac = 0;
   int64_t j = 0;
-  int par = 0;
   while (j < P.kmax) {
     const int64_t jb = min(P.nb, P.kmax - j);
-    int* lst = P.lsticc + par;
-    if (blockIdx.x == 0 && threadIdx.x == 0) P.lsticc[par ^ 1] = 0;
     int64_t kk = 0;
     bool stop_block = false;
     while (kk < jb && !stop_block) {
-      const int64_t c = j + kk;
-      if (!P.pivot) pvt = c;
+      const int c = (int)(j + kk);
+      const int pvt = s_pvt;
       stamp(c, 0);
-      // ---- every CTA: the reflector of column pvt, rows c..m-1 ---------------
-      const int64_t len = m - c - 1;
-      const float* ph = Bh + pvt * lda;
-      const float* pl = Bl + pvt * lda;
-      for (int64_t i = threadIdx.x; i < len; i += NT) {
-        vh[i] = __ldcg(ph + c + 1 + i);
-        vl[i] = __ldcg(pl + c + 1 + i);
+      const int len = m - c - 1, o1 = c + 1;
+      // ---- the pivot column, rows c .. m - 1, its pending update applied on the way
+      {
+        const float* ch = Bh + (int64_t)pvt * lda;
+        const float* cl = Bl + (int64_t)pvt * lda;
+        const float2 fr = __ldcg(E.f + (seq & 1) * G + pvt % G);
+        const Df fp{fr.x, fr.y};
+        for (int i = c + (int)threadIdx.x; i < m; i += NT) {
+          Df x{__ldcg(ch + i), __ldcg(cl + i)};
+          if (fp.h != 0.f) x = df_axpy_neg(x.h, x.l, fp, ph[i], pl[i]);
+          if (i == c) {
+            s_alpha = x;
+          } else {
+            vh[i] = x.h;
+            vl[i] = x.l;
+          }
+        }
       }
-      __shared__ Df s_alpha;
-      if (threadIdx.x == 0) s_alpha = Df{__ldcg(ph + c), __ldcg(pl + c)};
+      // the first chunk of this warp's first column, while the reflector is found
+      int sl = wid;
+      auto next = [&]() {
+        while (sl < nslot && ((s_st[sl] & ST_DONE) || cta + sl * G == pvt)) sl += NW;
+      };
+      next();
+      float xh[2][RB], xl[2][RB];
+      auto fetch = [&](const float* ah, const float* al, int b0, float (&h)[RB], float (&l)[RB]) {
+#pragma unroll
+        for (int q = 0; q < RB; ++q) {
+          const int i = b0 + lane + 32 * q;
+          h[q] = i < len ? ah[o1 + i] : 0.f;
+          l[q] = i < len ? al[o1 + i] : 0.f;
+        }
+      };
+      Df arc0{0.f, 0.f};
+      if (sl < nslot) {
+        const int64_t off = (int64_t)(cta + sl * G) * lda;
+        fetch(Bh + off, Bl + off, 0, xh[0], xl[0]);
+        arc0 = Df{Bh[off + c], Bl[off + c]};
+      }
       __syncthreads();
       stamp(c, 1);
       if (wid == 0) {
@@ -1037,7 +1124,8 @@ __global__ void __launch_bounds__(NT) geqp3_df_kernel(QrParams<double> P, QrV2Ex
         // 2^-970) cannot arise: a float pair holds nothing below 2^-149.
         const Df alpha = s_alpha;
         Df acc{0.f, 0.f};
-        for (int64_t i = lane; i < len; i += 32) df_fma_acc(acc, vh[i], vl[i], vh[i], vl[i]);
+#pragma unroll 4
+        for (int i = o1 + lane; i < m; i += 32) df_fma_acc(acc, vh[i], vl[i], vh[i], vl[i]);
         acc = quick_two_sum(acc.h, acc.l);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc = df_add(acc, df_shfl_xor(acc, o));
@@ -1049,8 +1137,8 @@ __global__ void __launch_bounds__(NT) geqp3_df_kernel(QrParams<double> P, QrV2Ex
           scal = df_div(Df{1.f, 0.f}, df_add(alpha, df_neg(beta)));
         }
         if (lane == 0) {
-          sh.tau = df_val(tau.h, tau.l);
-          sh.beta = df_val(beta.h, beta.l);
+          s_taud = df_val(tau.h, tau.l);
+          s_betad = df_val(beta.h, beta.l);
           s_f = scal;
           s_tau = tau;
           s_beta = beta;
@@ -1058,151 +1146,91 @@ __global__ void __launch_bounds__(NT) geqp3_df_kernel(QrParams<double> P, QrV2Ex
       }
       __syncthreads();
       stamp(c, 2);
-      const double tau = sh.tau;
+      const double tau = s_taud;
       if (tau != 0) {
         const Df sc = s_f;
-        for (int64_t i = threadIdx.x; i < len; i += NT) {
+        for (int i = o1 + (int)threadIdx.x; i < m; i += NT) {
           const Df y = df_mul(Df{vh[i], vl[i]}, sc);
           vh[i] = y.h;
           vl[i] = y.l;
         }
       }
       __syncthreads();
-      // the reflector goes back into column pvt only after the barrier that
-      // ends this step: other CTAs may still be reading the column until then
-      if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (cta == 0 && threadIdx.x == 0) {
         P.tau[c] = tau;
         X.piv[c] = pvt;
-        X.beta[c] = sh.beta;
+        X.beta[c] = s_betad;
       }
       stamp(c, 3);
       const Df tdf = s_tau;
-      // ---- each warp: apply H(c) to its live columns, two at a time -----------
-      // A warp's columns are read and written by that warp alone, so they
-      // are loaded through L1: a CTA's columns fit there for sketches of up
-      // to a few hundred rows, and a hit costs tens of cycles, not an L2
-      // round trip.  (The pivot column, written by another SM, is read
-      // around L1 above.)
-      auto dead = [&](int64_t t) {
-        return (s_st[t * NW + wid] & ST_DONE) || gw + t * W == pvt;
-      };
-      int64_t t = 0;
-      int pass = 0;
-      while (true) {
-        while (t < ncol && dead(t)) ++t;
-        if (t >= ncol) break;
-        const int64_t ta = t++;
-        while (t < ncol && dead(t)) ++t;
-        const bool two = t < ncol;
-        const int64_t tb = two ? t++ : ta;
-        const int64_t ja = gw + ta * W, jbb = gw + tb * W;
-        float* ah = Bh + ja * lda;
-        float* al = Bl + ja * lda;
-        float* bh = Bh + jbb * lda;
-        float* bl = Bl + jbb * lda;
-        const Df arca0{ldown(ah + c), ldown(al + c)};
-        const Df arcb0 = two ? Df{ldown(bh + c), ldown(bl + c)} : Df{0.f, 0.f};
-        Df sa{0.f, 0.f}, sb{0.f, 0.f};
-        float xah[QCH], xal[QCH], xbh[QCH], xbl[QCH];
-        const int64_t o = c + 1;
-        if (tau != 0) {
-          for (int64_t b0 = 0; b0 < len; b0 += 32 * QCH) {
-            const int64_t rem = len - b0;
+      // ---- each warp's live columns: the pending update and the dot product in
+      // one pass (each lane its rows in increasing order)
+      while (sl < nslot) {
+        const int cur = sl;
+        const int64_t off = (int64_t)(cta + cur * G) * lda;
+        float* ah = Bh + off;
+        float* al = Bl + off;
+        const Df fp = s_fp[cur];
+        const bool pend = fp.h != 0.f;
+        if (pend) arc0 = df_axpy_neg(arc0.h, arc0.l, fp, ph[c], pl[c]);
+        Df sa{0.f, 0.f};
+        auto use = [&](int b0, const float (&h)[RB], const float (&l)[RB]) {
 #pragma unroll
-            for (int q = 0; q < QCH; ++q) {
-              if (q % QG == 0 && 32 * q >= rem) break;
-              const int64_t i = b0 + lane + 32 * q;
-              const bool in = i < len;
-              xah[q] = in ? ldown(ah + o + i) : 0.f;
-              xal[q] = in ? ldown(al + o + i) : 0.f;
-              xbh[q] = (two && in) ? ldown(bh + o + i) : 0.f;
-              xbl[q] = (two && in) ? ldown(bl + o + i) : 0.f;
-            }
-#pragma unroll
-            for (int q = 0; q < QCH; ++q) {
-              if (q % QG == 0 && 32 * q >= rem) break;
-              const int64_t i = b0 + lane + 32 * q;
-              const float wh = i < len ? vh[i] : 0.f, wl = i < len ? vl[i] : 0.f;
-              df_fma_acc(sa, wh, wl, xah[q], xal[q]);
-              if (two) df_fma_acc(sb, wh, wl, xbh[q], xbl[q]);
+          for (int q = 0; q < RB; ++q) {
+            const int i = b0 + lane + 32 * q;
+            if (i < len) {
+              Df y{h[q], l[q]};
+              if (pend) {
+                y = df_axpy_neg(y.h, y.l, fp, ph[o1 + i], pl[o1 + i]);
+                ah[o1 + i] = y.h;
+                al[o1 + i] = y.l;
+              }
+              df_fma_acc(sa, vh[o1 + i], vl[o1 + i], y.h, y.l);
             }
           }
+        };
+        for (int b0 = 0; b0 < len; b0 += 64 * RB) {
+          fetch(ah, al, b0 + 32 * RB, xh[1], xl[1]);
+          use(b0, xh[0], xl[0]);
+          if (b0 + 32 * RB >= len) break;
+          fetch(ah, al, b0 + 64 * RB, xh[0], xl[0]);
+          use(b0 + 32 * RB, xh[1], xl[1]);
         }
-        if (pass < 2) stamp(c, 8 + 3 * pass);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          sa = df_add(sa, df_shfl_xor(sa, off));
-          sb = df_add(sb, df_shfl_xor(sb, off));
+        // the next column's first chunk, behind this one's reduction
+        sl += NW;
+        next();
+        const Df arcc = arc0;
+        if (sl < nslot) {
+          const int64_t of2 = (int64_t)(cta + sl * G) * lda;
+          fetch(Bh + of2, Bl + of2, 0, xh[0], xl[0]);
+          arc0 = Df{Bh[of2 + c], Bl[of2 + c]};
         }
-        const Df fa = df_mul(tdf, df_add(arca0, sa));
-        const Df fb = two ? df_mul(tdf, df_add(arcb0, sb)) : Df{0.f, 0.f};
-        if (pass < 2) stamp(c, 9 + 3 * pass);
-        const bool ua = fa.h != 0.f, ub = two && fb.h != 0.f;
-        if (ua || ub) {
-          for (int64_t b0 = 0; b0 < len; b0 += 32 * QCH) {
-            const int64_t rem = len - b0;
-            if (len > 32 * QCH) {
+        if (tau == 0) sa = Df{0.f, 0.f};
 #pragma unroll
-              for (int q = 0; q < QCH; ++q) {
-                if (q % QG == 0 && 32 * q >= rem) break;
-                const int64_t i = b0 + lane + 32 * q;
-                const bool in = i < len;
-                xah[q] = in ? ldown(ah + o + i) : 0.f;
-                xal[q] = in ? ldown(al + o + i) : 0.f;
-                xbh[q] = (two && in) ? ldown(bh + o + i) : 0.f;
-                xbl[q] = (two && in) ? ldown(bl + o + i) : 0.f;
-              }
-            }
-#pragma unroll
-            for (int q = 0; q < QCH; ++q) {
-              if (q % QG == 0 && 32 * q >= rem) break;
-              const int64_t i = b0 + lane + 32 * q;
-              if (i < len) {
-                const float wh = vh[i], wl = vl[i];
-                if (ua) {
-                  const Df y = df_axpy_neg(xah[q], xal[q], fa, wh, wl);
-                  ah[o + i] = y.h;
-                  al[o + i] = y.l;
-                }
-                if (ub) {
-                  const Df y = df_axpy_neg(xbh[q], xbl[q], fb, wh, wl);
-                  bh[o + i] = y.h;
-                  bl[o + i] = y.l;
-                }
-              }
-            }
-          }
-        }
-        if (pass < 2) stamp(c, 10 + 3 * pass);
-        ++pass;
+        for (int of = 16; of > 0; of >>= 1) sa = df_add(sa, df_shfl_xor(sa, of));
+        const Df fa = df_mul(tdf, df_add(arcc, sa));
         if (lane == 0) {
-          const Df arca = df_add(arca0, Df{-fa.h, -fa.l});
+          const Df arca = df_add(arcc, Df{-fa.h, -fa.l});
           ah[c] = arca.h;
           al[c] = arca.l;
-          s_arc[ta * NW + wid] = arca;
-          if (two) {
-            const Df arcb = df_add(arcb0, Df{-fb.h, -fb.l});
-            bh[c] = arcb.h;
-            bl[c] = arcb.l;
-            s_arc[tb * NW + wid] = arcb;
-          }
+          s_arc[cur] = arca;
+          s_fp[cur] = fa;
         }
       }
       __syncthreads();
       stamp(c, 4);
-      // ---- a thread per slot: norm downdate and the pivot candidate -----------
+      // ---- a thread per slot: norm downdate and the pivot candidate
       bk = -2;
-      bi = INT64_MAX;
+      bi = INT_MAX;
       int myflag = 0;
       for (int s = threadIdx.x; s < nslot; s += NT) {
         const unsigned char st = s_st[s];
-        if (!(st & ST_LIVE) || (st & ST_DONE)) continue;
-        const int64_t jj = slot_col(s);
+        if (st & ST_DONE) continue;
+        const int jj = cta + s * G;
         if (jj == pvt) {
           s_st[s] = st | ST_DONE;
           continue;
         }
-        if (!P.pivot) continue;
         Df v1 = s_vn1[s];
         if (c < lastrk - 1 && v1.h != 0.f) {
           // LAPACK's partial-norm downdate, in double-float
@@ -1220,74 +1248,125 @@ __global__ void __launch_bounds__(NT) geqp3_df_kernel(QrParams<double> P, QrV2Ex
             s_vn1[s] = v1;
           }
         }
-        key_merge(bk, bi, df_key(v1), jj);
+        const long long k = df_key(v1);
+        if (k > bk || (k == bk && jj < bi)) {
+          bk = k;
+          bi = jj;
+        }
       }
-      if (myflag) atomicAdd(lst, 1);
       stamp(c, 5);
-      publish(bk, bi);
+      if (!exchange(bk, bi, myflag)) return;
       stamp(c, 6);
-      if (!grid_sync(P.bar)) return;
-      stamp(c, 7);
-      if (blockIdx.x == 0) {
-        float* wh = Bh + pvt * lda;
-        float* wl = Bl + pvt * lda;
-        if (tau != 0)
-          for (int64_t i = threadIdx.x; i < len; i += NT) {
-            wh[c + 1 + i] = vh[i];
-            wl[c + 1 + i] = vl[i];
-          }
-        if (threadIdx.x == 0) {
+      // the finished pivot column, rows spread over the CTAs (all have read it)
+      {
+        float* wh = Bh + (int64_t)pvt * lda;
+        float* wl = Bl + (int64_t)pvt * lda;
+        const int r0 = o1 + (int)((int64_t)len * cta / G), r1 = o1 + (int)((int64_t)len * (cta + 1) / G);
+        for (int i = r0 + (int)threadIdx.x; i < r1; i += NT) {
+          wh[i] = vh[i];
+          wl[i] = vl[i];
+        }
+        if (cta == 0 && threadIdx.x == 0) {
           wh[c] = s_beta.h;
           wl[c] = s_beta.l;
         }
       }
-      pvt = reduce_pivot_key(lst);  // its block barrier also orders the writes above before vs is reloaded
-      stop_block = s_lst != 0;
+      if (PG)
+        for (int i = o1 + (int)threadIdx.x; i < m; i += NT) {
+          ph[i] = vh[i];
+          pl[i] = vl[i];
+        }
+      __syncthreads();
+      stamp(c, 7);
+      stop_block = s_stop != 0;
+      // this reflector becomes the pending one
+      if (!PG) {
+        float* t = ph;
+        ph = vh;
+        vh = t;
+        t = pl;
+        pl = vl;
+        vl = t;
+      }
       ++kk;
     }
-    const int64_t kb = kk;
-    const int64_t jn = j + kb;
+    const int64_t jn = j + kk;
     nfac = jn;
+    // a column's pending update, rows jn .. m - 1 (a warp, lane-strided from jn)
+    auto flush = [&](int s) {
+      const Df fp = s_fp[s];
+      if (fp.h == 0.f) return;
+      float* ah = Bh + (int64_t)(cta + s * G) * lda;
+      float* al = Bl + (int64_t)(cta + s * G) * lda;
+      for (int i = (int)jn + lane; i < m; i += 32) {
+        const Df y = df_axpy_neg(ah[i], al[i], fp, ph[i], pl[i]);
+        ah[i] = y.h;
+        al[i] = y.l;
+      }
+    };
     if (stop_block) {
-      for (int64_t t = 0; t < ncol; ++t) {
-        const int s = (int)(t * NW + wid);
+      // the flagged norms recomputed from their updated columns, in FP64
+      for (int s = wid; s < nslot; s += NW) {
         if (!(s_st[s] & ST_FLAG) || (s_st[s] & ST_DONE)) continue;
-        const int64_t jj = gw + t * W;
-        const Df v1 = df_split(warp_nrm2_df(Bh + jj * lda + jn, Bl + jj * lda + jn, m - jn));
+        flush(s);
+        const float* h = Bh + (int64_t)(cta + s * G) * lda + jn;
+        const float* l = Bl + (int64_t)(cta + s * G) * lda + jn;
+        const int ln = m - (int)jn;
+        double mx = 0;
+        for (int i = lane; i < ln; i += 32) mx = fmax(mx, fabs(df_val(h[i], l[i])));
+        mx = warp_max(mx);
+        double nr = mx;
+        if (mx != 0 && isfinite(mx)) {
+          const double sc = pow2_scale_inv(mx);
+          double acc = 0;
+          for (int i = lane; i < ln; i += 32) {
+            const double t = df_val(h[i], l[i]) * sc;
+            acc = fma(t, t, acc);
+          }
+          acc = warp_sum(acc);
+          nr = sqrt(acc) / sc;
+        }
         __syncwarp();
         if (lane == 0) {
-          s_vn1[s] = s_vn2[s] = v1;
+          s_vn1[s] = s_vn2[s] = df_split(nr);
+          s_fp[s] = Df{0.f, 0.f};
           s_st[s] = s_st[s] & (unsigned char)~ST_FLAG;
         }
       }
       __syncthreads();
       bk = -2;
-      bi = INT64_MAX;
+      bi = INT_MAX;
       for (int s = threadIdx.x; s < nslot; s += NT) {
-        const unsigned char st = s_st[s];
-        if (!(st & ST_LIVE) || (st & ST_DONE)) continue;
-        key_merge(bk, bi, df_key(s_vn1[s]), slot_col(s));
+        if (s_st[s] & ST_DONE) continue;
+        const long long k = df_key(s_vn1[s]);
+        const int jj = cta + s * G;
+        if (k > bk || (k == bk && jj < bi)) {
+          bk = k;
+          bi = jj;
+        }
       }
-      publish(bk, bi);
-      if (!grid_sync(P.bar)) return;
-      pvt = reduce_pivot_key();
+      if (!exchange(bk, bi, 0)) return;
     }
+    bool done = false;
     auto rdiag = [&](int64_t i) { return fabs(__ldcg(X.beta + i)); };
     if (rdiag(jn - 1) <= ptol) {
-      bool found = false;
       for (int64_t i = j; i < jn; ++i) {
         if (rdiag(i) <= ptol) {
           kres = i;
-          found = true;
+          done = true;
           break;
         }
       }
-      if (found) break;
+    }
+    if (done || jn >= P.kmax) {
+      // the columns that were not pivots, up to date below row jn
+      for (int s = wid; s < nslot; s += NW)
+        if (!(s_st[s] & ST_DONE)) flush(s);
+      break;
     }
     j = jn;
-    par ^= 1;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (cta == 0 && threadIdx.x == 0) {
     *P.k_out = kres;
     *X.nfac = nfac;
   }
@@ -2462,8 +2541,8 @@ static void print_qr_trace(lra_ctx* ctx, const unsigned long long* stamps, int64
       std::fprintf(stderr, "[lra] %s exchange: word spread %.2f us, last word to CTA 0 done %.2f us\n", kname,
                    spread / cnt / 1e3, after / cnt / 1e3);
   }
-  static const char* const glob[8] = {"vs-load", "reflector", "scale", "columns", "downdate", "publish", "barrier",
-                                      "write-back+pivot"};
+  static const char* const glob[8] = {"load", "reflector", "scale", "columns", "downdate", "exchange", "write-back",
+                                      "rest"};
   static const char* const sm[8] = {"stage-load", "dots+reflector", "-", "f+downdate+word",
                                     "stage+word", "deferred-update||exchange", "-", "rest"};
   const char* const* lab = smem ? sm : glob;
@@ -2488,12 +2567,6 @@ static void print_qr_trace(lra_ctx* ctx, const unsigned long long* stamps, int64
                  "word %.2f; flagged steps %lld\n",
                  kname, sub[0] / nsub / 1e3, sub[1] / nsub / 1e3, sub[2] / nsub / 1e3, sub[3] / nsub / 1e3,
                  sub[4] / nsub / 1e3, sub[5] / nsub / 1e3, (long long)nflag);
-  else if (nsub)
-    std::fprintf(stderr,
-                 "[lra] %s warp-0 passes (us): load+dots %.2f reduce+f %.2f update %.2f | load+dots %.2f "
-                 "reduce+f %.2f update %.2f\n",
-                 kname, sub[0] / nsub / 1e3, sub[1] / nsub / 1e3, sub[2] / nsub / 1e3, sub[3] / nsub / 1e3,
-                 sub[4] / nsub / 1e3, sub[5] / nsub / 1e3);
   if (cnt) {
     std::fprintf(stderr, "[lra] %s m=%lld n=%lld pivots=%lld us/pivot %.2f:", kname, (long long)m, (long long)n,
                  (long long)cnt, cyc / cnt / 1e3);
@@ -2981,7 +3054,7 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
   P.flag = ctx->arena.alloc_n<int>(n);
   P.part_v = ctx->arena.alloc_n<T>(grid);
   P.part_i = ctx->arena.alloc_n<int64_t>(grid);
-  P.part_d = ctx->arena.alloc_n<double>(grid);
+  P.part_d = ctx->arena.alloc_n<double>(std::max(grid, ctx->num_sms));
   int* small = ctx->arena.alloc_n<int>(8);
   P.lsticc = small;
   P.bar = reinterpret_cast<GridBar*>(ctx->arena.alloc(sizeof(GridBar)));
@@ -3054,7 +3127,14 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     iota_kernel<<<gi, 256, 0, ctx->stream>>>(n, col_at, pos);
     post_launch(ctx, "iota_kernel");
     // the mixed-precision path factors Float64 sketches in double-float
-    const bool dfq = sizeof(T) == 8 && ctx->gemm_tc && pivot;
+    // (two reflectors and four pairs per column in shared memory, one
+    // reflector when two do not fit; a million columns and more take the
+    // FP64 kernel, whose column state is smaller)
+    const int Gd = (int)std::min<int64_t>(qr_sm_cap(ctx), n);
+    const size_t cols_df = (size_t)((n + Gd - 1) / Gd) * 33;
+    const bool pg = (size_t)m * 16 + cols_df > 200 * 1024;
+    const size_t smem_df = (size_t)m * (pg ? 8 : 16) + cols_df;
+    const bool dfq = sizeof(T) == 8 && ctx->gemm_tc && pivot && smem_df <= 220 * 1024;
     if (dfq) {
       float* Bh = ctx->arena.alloc_n<float>((size_t)m * n);
       float* Bl = ctx->arena.alloc_n<float>((size_t)m * n);
@@ -3083,16 +3163,21 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
       // memory)
       const char* kname = "geqp3_df_kernel";
       {
-        raise_smem_limit(ctx, (const void*)geqp3_df_kernel<NT>);
+        const int G = Gd;
+        const void* fn = pg ? (const void*)geqp3_df_kernel<NT, true> : (const void*)geqp3_df_kernel<NT, false>;
+        raise_smem_limit(ctx, fn);
         // as much L1 as the shared memory leaves: the warps' columns live there
-        LRA_CUDA(cudaFuncSetAttribute(geqp3_df_kernel<NT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                      cudaSharedmemCarveoutMaxL1));
+        LRA_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1));
         int per_df = 0;
-        LRA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_df, geqp3_df_kernel<NT>, NT, smem2));
+        LRA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_df, fn, NT, smem_df));
         if (per_df < 1) fail(LRA_ECUDA, "geqp3 kernel cannot be resident");
-        void* args[] = {&Pd, &X, &D};
-        LRA_CUDA(cudaLaunchCooperativeKernel((const void*)geqp3_df_kernel<NT>, dim3(grid), dim3(NT), args, smem2,
-                                             ctx->stream));
+        QrXw E;
+        E.word = ctx->arena.alloc_n<ulonglong2>((size_t)2 * G);
+        E.f = ctx->arena.alloc_n<float2>((size_t)2 * G);
+        E.prev = pg ? ctx->arena.alloc_n<float>((size_t)G * 2 * m) : nullptr;
+        LRA_CUDA(cudaMemsetAsync(E.word, 0, (size_t)2 * G * sizeof(ulonglong2), ctx->stream));
+        void* args[] = {&Pd, &X, &D, &E};
+        LRA_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(NT), args, smem_df, ctx->stream));
       }
       post_launch(ctx, kname);
       if (D.stamps) print_qr_trace(ctx, D.stamps, P.kmax, m, n, kname, false, nullptr, 1);
