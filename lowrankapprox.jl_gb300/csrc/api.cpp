@@ -655,7 +655,10 @@ int sketchfact_steps(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, int
   int c;
   {
     Stage sq(ctx, 1);
-    c = geqp3_adap_steps<T>(ctx, cnt, st.data(), o.nb, o.atol, o.rtol, ks.data());
+    int likely = -1;
+    for (int i = 0; i < cnt && likely < 0; ++i)
+      if (st[(size_t)i].nt > rank_hint) likely = i;
+    c = geqp3_adap_steps<T>(ctx, cnt, st.data(), o.nb, o.atol, o.rtol, ks.data(), likely);
   }
   if (c < 0) {
     ctx->arena.release(base);

@@ -216,7 +216,8 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
 // next pivot; the factors (A, jpvt, tau) are written for the first such step
 // only.  k[i] is step i's rank (-1 for a step that a lower one stopped).
 // Returns the index of that first step, or -1 when every step's rank reached
-// its threshold (no factors written).
+// its threshold (no factors written).  `likely` is the step expected to reveal
+// the rank (-1: none in particular); it only decides how the CTAs are shared.
 template <typename T>
 struct QrStep {
   int64_t m, n;
@@ -232,7 +233,7 @@ template <typename T>
 int geqp3_steps_fit(lra_ctx* ctx, int count, const int64_t* m, int64_t n);
 template <typename T>
 int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* steps, int64_t nb, double atol, double rtol,
-                     int64_t* k);
+                     int64_t* k, int likely);
 
 template <typename T>
 int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_t* jpvt,

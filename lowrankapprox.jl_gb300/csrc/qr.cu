@@ -908,6 +908,18 @@ __device__ __forceinline__ void st_word(ulonglong2* p, unsigned long long x, uns
   asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.release.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
                : "memory");
 }
+__device__ __forceinline__ void st_word_relaxed(ulonglong2* p, unsigned long long x, unsigned long long y) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_word_acquire(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("{\n .reg .b128 t;\n ld.acquire.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(v.x), "=l"(v.y)
+               : "l"(p)
+               : "memory");
+  return v;
+}
 __device__ __forceinline__ ulonglong2 ld_word(const ulonglong2* p) {
   ulonglong2 v;
   asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
@@ -1378,24 +1390,22 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV
 // held as (h, l) float pairs, and applies every reflector to them there.
 // The only traffic between CTAs per pivot is one 64-bit word per CTA and
 // the winning candidate's column: each CTA stages its best candidate's
-// remaining rows in global memory, then publishes (norm key, column, stop
-// flag, sequence bit) as one word.  Readers poll the G words of the
-// exchange (one L2 round trip once they are written), take the argmax and
-// load the winner's staged rows; this replaces the grid barrier and the
-// separate read of the per-CTA partials.  Words and staged columns are
-// double-buffered by exchange parity, so a CTA that runs ahead never
-// overwrites what a slower CTA still reads, and the sequence bit tells
-// this exchange from the one two steps earlier.  The key keeps the 38
+// remaining rows in global memory, raises the exchange's maximum with its
+// word (norm key, column), and then arrives, counting its stop flag along.
+// Maximum and arrivals share 16 bytes, so the read that sees the last arrival
+// has the winner (a separate arrival counter cost a second L2 round trip, 0.7 us
+// of the 6.9 us a short pivot took; a fence of its own before the maximum 0.4
+// us); readers then load the winner's staged rows.  Slots rotate over four
+// exchanges and staged columns over two, so a CTA that runs ahead never
+// overwrites what a slower CTA still reads.  The key keeps the 38
 // leading bits of the double-float norm (relative resolution 2^-30, far
 // below the error of the downdated norms); ties go to the smaller column
 // index, as with xLAQPS's idamax.
 struct QrSm {
-  // the exchange, zeroed before the launch: exchange e's largest word in
-  // amax[(e % 4) * 16] and OR of stop flags in astop[(e % 4) * 32] (a 128-byte
-  // line each), and one arrival counter (G per exchange)
-  unsigned long long* amax;
-  unsigned* astop;
-  unsigned* arrive;
+  // the exchange, zeroed before the launch: exchange e in slot[(e % 4) * 8] (a
+  // 128-byte line each), its largest word in x, in y the arrivals (low half) and
+  // how many of them stop (high half): one 16-byte read takes all three
+  ulonglong2* slot;
   void* stage;               // [2][G][m] staged candidate columns (elements of the arithmetic)
   unsigned long long* pubt;  // LRA_TRACE: %globaltimer of each CTA's word per pivot, [kmax][G], or null
   // several adaptive steps factored by one launch: the lowest index of a
@@ -1407,11 +1417,12 @@ struct QrSm {
   int64_t nt = 0;
 };
 
-// the next four live slots s, s + step, ... of a warp (-1: absent); s moves on
-__device__ __forceinline__ int live_quad(const unsigned char* st, int nloc, int step, int& s, int (&q)[4]) {
+// the next GQ live slots s, s + step, ... of a warp (-1: absent); s moves on
+template <int GQ>
+__device__ __forceinline__ int live_group(const unsigned char* st, int nloc, int step, int& s, int (&q)[GQ]) {
   int cnt = 0;
 #pragma unroll
-  for (int g = 0; g < 4; ++g) {
+  for (int g = 0; g < GQ; ++g) {
     while (s < nloc && (st[s] & ST_DONE)) s += step;
     if (s < nloc) {
       q[g] = s;
@@ -1539,7 +1550,7 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
   constexpr int NCW = NW - 1;  // column warps
   __shared__ V s_part[NW];
   __shared__ unsigned long long s_w[NW];
-  __shared__ int s_fl[NW];
+  __shared__ unsigned long long s_cw;
   __shared__ V s_alpha, s_f, s_tau, s_beta;
   __shared__ double s_red[32];
   __shared__ unsigned long long s_win;
@@ -1575,44 +1586,42 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
     __syncthreads();
     if (b == 0 && threadIdx.x == 0 && c < P.kmax) D.stamps[c * 16 + ph] = globaltimer_ns();
   };
-  // the CTA's candidate: max of the warps' words (s_w) and OR of their
-  // stop flags (s_fl), into s_win / s_stop
-  auto cta_word = [&]() {
-    __syncthreads();
+  // the warp's largest word into s_w (the maximum of the high halves, then of
+  // the low halves among those)
+  auto warp_word = [&](unsigned long long w) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(w >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(w >> 32) == hi ? (unsigned)w : 0u);
+    if (lane == 0) s_w[wid] = ((unsigned long long)hi << 32) | lo;
+  };
+  // the CTA's candidate, the largest of the first nw warps' words: read by every
+  // thread when they are few (after a barrier that the caller has passed)
+  auto cta_word = [&](int nw) -> unsigned long long {
+    if (nw <= 4) {
+      unsigned long long w = s_w[0];
+      for (int q = 1; q < nw; ++q) w = s_w[q] > w ? s_w[q] : w;
+      return w;
+    }
     if (wid == 0) {
-      unsigned long long w0 = lane < NW ? s_w[lane] : 0ull;
-      int f0 = lane < NW ? s_fl[lane] : 0;
+      unsigned long long w0 = lane < nw ? s_w[lane] : 0ull;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long w2 = __shfl_xor_sync(0xffffffffu, w0, o);
         w0 = w2 > w0 ? w2 : w0;
-        f0 |= __shfl_xor_sync(0xffffffffu, f0, o);
       }
-      if (lane == 0) {
-        s_win = w0;
-        s_stop = f0;
-      }
+      if (lane == 0) s_cw = w0;
     }
     __syncthreads();
+    return s_cw;
   };
-  auto warp_word = [&](unsigned long long w, int fl) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long w2 = __shfl_xor_sync(0xffffffffu, w, o);
-      w = w2 > w ? w2 : w;
-      fl |= __shfl_xor_sync(0xffffffffu, fl, o);
-    }
-    if (lane == 0) {
-      s_w[wid] = w;
-      s_fl[wid] = fl;
-    }
-  };
+  const int ncw = min(NW, (nloc + 31) / 32);  // warps with columns in the thread-per-column loops
   // stage the CTA's candidate (rows r0..m-1) and publish its word for
   // exchange e; the candidate's deferred update (upd) is applied on the way.
   // The word goes out after every thread's staged rows.
-  auto publish = [&](unsigned e, int64_t r0, bool upd) {
+  // Returns the slot whose deferred update that applied (-1: none).
+  auto publish = [&](unsigned e, int64_t r0, bool upd, unsigned long long w, bool stop) -> int {
     const bool cancel = !GCOL && s_cancel;
-    const unsigned long long w = cancel ? XW_CANCEL : s_win;
+    if (cancel) w = XW_CANCEL;
+    int done = -1;
     if (!cancel && (w & XW_LOW)) {
       const int sc = (int)((int64_t)(XW_IDX - (w & XW_IDX)) - c0);
       E* col = C + (int64_t)sc * cs;
@@ -1624,30 +1633,33 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
           col[i * rs] = y;
           if (!GCOL) dst[i] = y;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) s_st[sc] |= ST_UPD;
+        done = sc;
       } else if (!GCOL) {
-        for (int64_t i = r0 + threadIdx.x; i < m; i += NT) dst[i] = col[i];
+        for (int64_t i = r0 + threadIdx.x; i < m; i += NT) dst[i] = col[i * rs];
       }
     }
     __syncthreads();
     if (!GCOL && threadIdx.x == 0) {
-      // the word into the exchange's maximum (and the stop flag into its
-      // OR), then the arrival, released after the staged rows
-      __threadfence();
       if (S.pubt && r0 >= 1 && r0 - 1 < P.kmax) S.pubt[(r0 - 1) * G + b] = globaltimer_ns();
-      const unsigned slot = e & 3;
-      if (w & XW_LOW) atomicMax(S.amax + slot * 16, w & XW_LOW);
-      if (!cancel && s_stop) atomicOr(S.astop + slot * 32, 1u);
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(S.arrive) : "memory");
+      // the word into the exchange's maximum, then the arrival, released after
+      // it and (through the block barrier) after every thread's staged rows
+      ulonglong2* sl = S.slot + (e & 3) * 8;
+      if (w & XW_LOW) atomicMax(&sl->x, w & XW_LOW);
+      const unsigned long long one = 1ull + ((!cancel && stop) ? 1ull << 32 : 0ull);
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&sl->y), "l"(one) : "memory");
     }
+    return done;
   };
   // wait for all G arrivals of exchange e (bounded): the winning word, its
   // CTA and the OR of the stop flags, in shared memory
-  auto collect = [&](unsigned e) -> bool {
+  auto collect = [&](unsigned e, unsigned long long own_w, bool own_stop) -> bool {
     if (GCOL) {
       // one CTA: its own candidate is the pivot
-      if (threadIdx.x == 0) s_owner = 0;
+      if (threadIdx.x == 0) {
+        s_owner = 0;
+        s_win = own_w;
+        s_stop = own_stop ? 1 : 0;
+      }
       __syncthreads();
       return true;
     }
@@ -1655,17 +1667,16 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
       // a lower step of the launch revealed its rank: this step stops at
       // the next exchange
       const int canc = S.success ? (*((volatile int*)S.success) < S.job ? 1 : 0) : 0;
-      // every CTA's arrival at exchange e (the counter grows by G per
-      // exchange), bounded
-      const unsigned target = (unsigned)G * (e + 1u);
+      // every CTA's arrival at exchange e, bounded; the read that sees the last
+      // one has the maximum with it (same 16 bytes, raised before the arrival)
+      ulonglong2* sl = S.slot + (e & 3) * 8;
       bool ok = true;
-      unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(S.arrive) : "memory");
-      if ((int)(v - target) < 0) {
+      ulonglong2 v = ld_word_acquire(sl);
+      if ((unsigned)v.y != (unsigned)G) {
         const uint64_t t0 = globaltimer_ns(), lim = wait_limit_ns();
         for (unsigned it = 1;; ++it) {
-          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(S.arrive) : "memory");
-          if ((int)(v - target) >= 0) break;
+          v = ld_word_acquire(sl);
+          if ((unsigned)v.y == (unsigned)G) break;
           // the error word and the clock every 16th poll
           if (it & 15) continue;
           if (*((volatile int*)&P.bar->err) != 0) {
@@ -1679,19 +1690,12 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
           }
         }
       }
-      const unsigned slot = e & 3;
-      unsigned long long best;
-      unsigned fl;
-      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(best) : "l"(S.amax + slot * 16) : "memory");
-      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(fl) : "l"(S.astop + slot * 32) : "memory");
+      const unsigned long long best = v.x;
+      const unsigned fl = (unsigned)(v.y >> 32);
       // every CTA has read exchange e - 1 (each read it before arriving at
       // e): its slot is cleared for exchange e + 3, before this CTA's next
       // arrival releases the clearing
-      if (b == 0 && ok) {
-        const unsigned prev = (e + 3) & 3;
-        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(S.amax + prev * 16), "l"(0ull) : "memory");
-        asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(S.astop + prev * 32), "r"(0u) : "memory");
-      }
+      if (b == 0 && ok) st_word_relaxed(S.slot + ((e + 3) & 3) * 8, 0ull, 0ull);
       // the winner's CTA: the one whose columns [n b / G, n (b + 1) / G)
       // hold the winning column
       const int64_t jw = (int64_t)(XW_IDX - (best & XW_IDX));
@@ -1709,7 +1713,14 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
     __syncthreads();
     return s_ok != 0;
   };
-  auto quad = [&](int& s, int (&q)[4]) { return live_quad(s_st, nloc, NCW, s, q); };
+  // the columns a warp takes at a time: four, so that a load of the reflector
+  // serves four and their reductions share shuffles; but two or one when the
+  // CTA has too few columns to give every column warp that many (15 columns in
+  // fours would leave eleven of the fifteen warps idle).  A column's sums do not
+  // depend on the others of its group.  F32 520 x 1103, 15 columns a CTA, 401
+  // pivots: 2.15 ms in fours, 1.83 one at a time; double-float 1032 x 1100, 600
+  // pivots: 8.4 and 4.8 ms.
+  const int per_warp = (nloc + NCW - 1) / NCW;
 
   if (threadIdx.x == 0) s_cancel = 0;
   // ---- the CTA's columns into shared memory (GCOL: the workspace is filled);
@@ -1733,11 +1744,14 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
   }
   lmax = block_max(lmax, s_red);
   if (!GCOL && threadIdx.x == 0) P.part_d[b] = lmax;
-  warp_word(cw, 0);
-  cta_word();
+  if (wid < ncw) warp_word(cw);
+  __syncthreads();
   unsigned e = 0;
-  publish(e, 0, false);
-  if (!collect(e)) return;
+  {
+    const unsigned long long w = cta_word(ncw);
+    publish(e, 0, false, w, false);
+    if (!collect(e, w, false)) return;
+  }
   double maxnrm = lmax;
   if (!GCOL) {
     maxnrm = 0;
@@ -1820,12 +1834,23 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
           const E* col = C + (int64_t)s * cs;
           s_x0[s] = col[c * rs];
           V d = A::zero();
-          // QSEQB rows loaded ahead, then added in row order
-          for (int64_t i0 = c + 1; i0 < m; i0 += QSEQB) {
+          // QSEQB rows loaded ahead, then added in row order (no masks in a whole
+          // chunk: a branch a row would keep the rows' products from overlapping)
+          int64_t i0 = c + 1;
+          for (; i0 + QSEQB <= m; i0 += QSEQB) {
+            E xb[QSEQB], vb[QSEQB];
+#pragma unroll
+            for (int r = 0; r < QSEQB; ++r) {
+              xb[r] = col[(i0 + r) * rs];
+              vb[r] = Vc[i0 + r];
+            }
+#pragma unroll
+            for (int r = 0; r < QSEQB; ++r) A::fma_acc(d, vb[r], xb[r]);
+          }
+          if (i0 < m) {
             E xb[QSEQB];
 #pragma unroll
-            for (int r = 0; r < QSEQB; ++r)
-              if (i0 + r < m) xb[r] = col[(i0 + r) * rs];
+            for (int r = 0; r < QSEQB; ++r) xb[r] = i0 + r < m ? col[(i0 + r) * rs] : A::ezero();
 #pragma unroll
             for (int r = 0; r < QSEQB; ++r)
               if (i0 + r < m) A::fma_acc(d, Vc[i0 + r], xb[r]);
@@ -1833,57 +1858,93 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
           s_dot[s] = A::norm(d);
         }
       } else if (len > 0) {
-        // ---- dot products x . a of the warp's live columns, four at a time
-        int s = wid - 1;
-        int q[4];
-        while (quad(s, q)) {
-          const E* cg[4];
+        // ---- dot products x . a of the warp's live columns, GQ at a time
+        auto dots = [&](auto gqc) {
+          constexpr int GQ = decltype(gqc)::value;
+          constexpr int R = GQ == 4 ? QRPL : 8;  // rows per lane loaded ahead
+          constexpr int LG = 32 / GQ;            // lanes that end with one column's total
+          int s = wid - 1;
+          int q[GQ];
+          while (live_group<GQ>(s_st, nloc, NCW, s, q)) {
+            const E* cg[GQ];
 #pragma unroll
-          for (int g = 0; g < 4; ++g) cg[g] = C + (int64_t)(q[g] >= 0 ? q[g] : q[0]) * cs;
-          // row c of the column, for the update that follows the dots
-          {
-            const int g = lane >> 3;
-            const int qg = g == 0 ? q[0] : g == 1 ? q[1] : g == 2 ? q[2] : q[3];
-            if ((lane & 7) == 0 && qg >= 0) s_x0[qg] = C[(int64_t)qg * cs + c * rs];
-          }
-          // QRPL rows per lane are loaded before they are used, so that a
-          // quad has 4 QRPL loads in flight (the global-memory form waits
-          // an L2 round trip per chunk); each lane still adds its rows in
-          // increasing order
-          V d[4] = {A::zero(), A::zero(), A::zero(), A::zero()};
-          for (int64_t b0 = c + 1; b0 < m; b0 += 32 * QRPL) {
-            E xv[QRPL], xc[4][QRPL];
+            for (int g = 0; g < GQ; ++g) cg[g] = C + (int64_t)(q[g] >= 0 ? q[g] : q[0]) * cs;
+            int qg = q[0];  // this lane's column once the sums are reduced
 #pragma unroll
-            for (int r = 0; r < QRPL; ++r) {
-              const int64_t i = b0 + lane + 32 * r;
-              const bool in = i < m;
-              xv[r] = in ? Vc[i] : A::ezero();
+            for (int g = 1; g < GQ; ++g) qg = lane / LG == g ? q[g] : qg;
+            // row c of the column, for the update that follows the dots
+            if (lane % LG == 0 && qg >= 0) s_x0[qg] = C[(int64_t)qg * cs + c * rs];
+            // R rows per lane are loaded before they are used, so that a
+            // group has GQ R loads in flight (the global-memory form waits
+            // an L2 round trip per chunk); each lane still adds its rows in
+            // increasing order
+            V d[GQ];
 #pragma unroll
-              for (int g = 0; g < 4; ++g) xc[g][r] = in ? cg[g][i * rs] : A::ezero();
+            for (int g = 0; g < GQ; ++g) d[g] = A::zero();
+            int64_t b0 = c + 1;
+            for (; b0 + 32 * R <= m; b0 += 32 * R) {  // whole chunks: no row to mask
+              E xv[R], xc[GQ][R];
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                const int64_t i = b0 + lane + 32 * r;
+                xv[r] = Vc[i];
+#pragma unroll
+                for (int g = 0; g < GQ; ++g) xc[g][r] = cg[g][i * rs];
+              }
+#pragma unroll
+              for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int g = 0; g < GQ; ++g) A::fma_acc(d[g], xv[r], xc[g][r]);
+            }
+            if (b0 < m) {
+              E xv[R], xc[GQ][R];
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                const int64_t i = b0 + lane + 32 * r;
+                const bool in = i < m;
+                xv[r] = in ? Vc[i] : A::ezero();
+#pragma unroll
+                for (int g = 0; g < GQ; ++g) xc[g][r] = in ? cg[g][i * rs] : A::ezero();
+              }
+#pragma unroll
+              for (int r = 0; r < R; ++r)
+                if (b0 + lane + 32 * r < m) {
+#pragma unroll
+                  for (int g = 0; g < GQ; ++g) A::fma_acc(d[g], xv[r], xc[g][r]);
+                }
             }
 #pragma unroll
-            for (int r = 0; r < QRPL; ++r)
-              if (b0 + lane + 32 * r < m) {
+            for (int g = 0; g < GQ; ++g) d[g] = A::norm(d[g]);
+            // transposed butterfly: a level that halves the columns a lane holds
+            // as it adds, then the rest; lanes LG g .. LG g + LG - 1 end with
+            // column g's total
+            V t;
+            if constexpr (GQ == 4) {
+              const bool up = lane & 16;
+              const V k0 = up ? d[2] : d[0], k1 = up ? d[3] : d[1];
+              const V e0 = A::add(k0, A::shfl_xor(up ? d[0] : d[2], 16));
+              const V e1 = A::add(k1, A::shfl_xor(up ? d[1] : d[3], 16));
+              const bool hi = lane & 8;
+              t = A::add(hi ? e1 : e0, A::shfl_xor(hi ? e0 : e1, 8));
+            } else if constexpr (GQ == 2) {
+              const bool up = lane & 16;
+              t = A::add(up ? d[1] : d[0], A::shfl_xor(up ? d[0] : d[1], 16));
+              t = A::add(t, A::shfl_xor(t, 8));
+            } else {
+              t = A::add(d[0], A::shfl_xor(d[0], 16));
+              t = A::add(t, A::shfl_xor(t, 8));
+            }
 #pragma unroll
-                for (int g = 0; g < 4; ++g) A::fma_acc(d[g], xv[r], xc[g][r]);
-              }
+            for (int o = 4; o > 0; o >>= 1) t = A::add(t, A::shfl_xor(t, o));
+            if (lane % LG == 0 && qg >= 0) s_dot[qg] = t;
           }
-#pragma unroll
-          for (int g = 0; g < 4; ++g) d[g] = A::norm(d[g]);
-          // transposed butterfly: after the 16- and 8-lane levels, lanes
-          // 8g..8g+7 hold column g's partial sums
-          const bool up = lane & 16;
-          const V k0 = up ? d[2] : d[0], k1 = up ? d[3] : d[1];
-          const V e0 = A::add(k0, A::shfl_xor(up ? d[0] : d[2], 16));
-          const V e1 = A::add(k1, A::shfl_xor(up ? d[1] : d[3], 16));
-          const bool hi = lane & 8;
-          V t = A::add(hi ? e1 : e0, A::shfl_xor(hi ? e0 : e1, 8));
-#pragma unroll
-          for (int o = 4; o > 0; o >>= 1) t = A::add(t, A::shfl_xor(t, o));
-          const int g = lane >> 3;
-          const int qg = g == 0 ? q[0] : g == 1 ? q[1] : g == 2 ? q[2] : q[3];
-          if ((lane & 7) == 0 && qg >= 0) s_dot[qg] = t;
-        }
+        };
+        if (per_warp >= 3)
+          dots(std::integral_constant<int, 4>{});
+        else if (per_warp == 2)
+          dots(std::integral_constant<int, 2>{});
+        else
+          dots(std::integral_constant<int, 1>{});
       }
       __syncthreads();
       stamp(c, 2);
@@ -1942,12 +2003,16 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
       }
       sub(9);
       sub(10);
+      if (wid < ncw) warp_word(ww);
       // ---- the flagged columns, a warp each: the deferred update of rows
       // c+1..m-1 now, then their norm in double-float at a power-of-two
       // scale that puts the largest entry in [1, 2) (lane-strided partial
       // sums and a butterfly, the same tree in both forms of the kernel)
-      if (__syncthreads_or(wfl)) {
+      const bool flagged = __syncthreads_or(wfl);
+      int ncand = ncw;
+      if (flagged) {
         sub(11);
+        if (wid < ncw) ww = s_w[wid];  // (its warp's largest)
         for (int s = wid; s < nloc; s += NW) {
           if (!(s_st[s] & ST_FLAG)) continue;
           E* col = C + (int64_t)s * cs;
@@ -1986,19 +2051,20 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
           const unsigned long long w = xw_pack<A>(nr, c0 + s);
           ww = w > ww ? w : ww;
         }
-        wfl = 1;
+        warp_word(ww);
+        ncand = NW;
+        __syncthreads();
       } else {
         sub(11);
       }
       sub(12);
-      warp_word(ww, wfl);
+      const unsigned long long wcand = cta_word(ncand);
       sub(13);
       const bool small = fabs(s_betad) <= ptol;
       if (small && first_small < 0) first_small = c;
       last_small = small;
-      cta_word();
       stamp(c, 4);
-      publish(e + 1, c + 1, true);
+      const int cand = publish(e + 1, c + 1, true, wcand, flagged);
       stamp(c, 5);
       ++e;
       // ---- warps 1..NW-1: the deferred updates, and the finished pivot column
@@ -2029,66 +2095,93 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
           }
         }
         // the rank-1 updates of rows c+1..m-1.  Shared-memory columns: a warp
-        // per four columns, QRPL rows per lane in registers.  Global columns
+        // per group of columns as above, rows in registers.  Global columns
         // (GCOL): a thread per column, whose rows stay in L1 between the
         // dot products and the update.
         if (!GCOL) {
-          int s = wid - 1;
-          int q[4];
-          while (quad(s, q)) {
-            V fq[4];
-            E* cg[4];
-            bool u[4];
+          // NU columns at once, whole chunks without masks, then the last rows
+          auto run = [&](auto nuc, E* const* pc, const V* pf) {
+            constexpr int NU = decltype(nuc)::value;
+            constexpr int R = NU >= 3 ? QRPL : 8;
+            int64_t b0 = c + 1;
+            for (; b0 + 32 * R <= m; b0 += 32 * R) {
+              E xv[R], xc[NU][R];
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              const int qh = q[h] >= 0 ? q[h] : q[0];
-              cg[h] = C + (int64_t)qh * cs;
-              fq[h] = s_fs[qh];
-              u[h] = q[h] >= 0 && A::hi(fq[h]) != 0.f && !(s_st[qh] & ST_UPD);
+              for (int r = 0; r < R; ++r) {
+                const int64_t i = b0 + lane + 32 * r;
+                xv[r] = Vc[i];
+#pragma unroll
+                for (int h = 0; h < NU; ++h) xc[h][r] = pc[h][i];
+              }
+#pragma unroll
+              for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int h = 0; h < NU; ++h) pc[h][b0 + lane + 32 * r] = A::axpy_neg(xc[h][r], pf[h], xv[r]);
             }
-            if (u[0] || u[1] || u[2] || u[3]) {
-              for (int64_t b0 = c + 1; b0 < m; b0 += 32 * QRPL) {
-                E xv[QRPL], xc[4][QRPL];
+            for (int64_t i = b0 + lane; i < m; i += 32) {
+              const E x = Vc[i];
 #pragma unroll
-                for (int r = 0; r < QRPL; ++r) {
-                  const int64_t i = b0 + lane + 32 * r;
-                  const bool in = i < m;
-                  xv[r] = in ? Vc[i] : A::ezero();
+              for (int h = 0; h < NU; ++h) pc[h][i] = A::axpy_neg(pc[h][i], pf[h], x);
+            }
+          };
+          auto updates = [&](auto gqc) {
+            constexpr int GQ = decltype(gqc)::value;
+            int s = wid - 1;
+            int q[GQ];
+            while (live_group<GQ>(s_st, nloc, NCW, s, q)) {
+              // the columns of the group that have an update, moved to the front
+              E* pc[GQ];
+              V pf[GQ];
+              int nu = 0;
 #pragma unroll
-                  for (int h = 0; h < 4; ++h) xc[h][r] = (in && u[h]) ? cg[h][i * rs] : A::ezero();
-                }
+              for (int h = 0; h < GQ; ++h) {
+                const int qh = q[h];
+                if (qh < 0 || qh == cand || (s_st[qh] & ST_UPD)) continue;
+                const V f = s_fs[qh];
+                if (A::hi(f) == 0.f) continue;
 #pragma unroll
-                for (int r = 0; r < QRPL; ++r) {
-                  const int64_t i = b0 + lane + 32 * r;
-                  if (i < m) {
-#pragma unroll
-                    for (int h = 0; h < 4; ++h)
-                      if (u[h]) cg[h][i * rs] = A::axpy_neg(xc[h][r], fq[h], xv[r]);
+                for (int k = 0; k <= h; ++k)
+                  if (k == nu) {
+                    pc[k] = C + (int64_t)qh * cs;
+                    pf[k] = f;
                   }
-                }
+                ++nu;
+              }
+              if (nu == 1) run(std::integral_constant<int, 1>{}, pc, pf);
+              if constexpr (GQ >= 2)
+                if (nu == 2) run(std::integral_constant<int, 2>{}, pc, pf);
+              if constexpr (GQ >= 4) {
+                if (nu == 3) run(std::integral_constant<int, 3>{}, pc, pf);
+                if (nu == 4) run(std::integral_constant<int, 4>{}, pc, pf);
               }
             }
-          }
+          };
+          if (per_warp >= 3)
+            updates(std::integral_constant<int, 4>{});
+          else if (per_warp == 2)
+            updates(std::integral_constant<int, 2>{});
+          else
+            updates(std::integral_constant<int, 1>{});
         }
         if (GCOL) {
           for (int sl = ct; sl < nloc; sl += NCT) {
-            if (s_st[sl] & (ST_DONE | ST_UPD)) continue;
+            if (sl == cand || (s_st[sl] & (ST_DONE | ST_UPD))) continue;
             const V fs = s_fs[sl];
             if (A::hi(fs) == 0.f) continue;
             E* col = C + (int64_t)sl * cs;
-            for (int64_t i0 = c + 1; i0 < m; i0 += QSEQB) {
+            int64_t i0 = c + 1;
+            for (; i0 + QSEQB <= m; i0 += QSEQB) {
               E xb[QSEQB];
 #pragma unroll
-              for (int r = 0; r < QSEQB; ++r)
-                if (i0 + r < m) xb[r] = col[(i0 + r) * rs];
+              for (int r = 0; r < QSEQB; ++r) xb[r] = col[(i0 + r) * rs];
 #pragma unroll
-              for (int r = 0; r < QSEQB; ++r)
-                if (i0 + r < m) col[(i0 + r) * rs] = A::axpy_neg(xb[r], fs, Vc[i0 + r]);
+              for (int r = 0; r < QSEQB; ++r) col[(i0 + r) * rs] = A::axpy_neg(xb[r], fs, Vc[i0 + r]);
             }
+            for (; i0 < m; ++i0) col[i0 * rs] = A::axpy_neg(col[i0 * rs], fs, Vc[i0]);
           }
         }
       }
-      if (!collect(e)) return;
+      if (!collect(e, wcand, flagged)) return;
       stamp(c, 6);
       stamp(c, 7);
       stop_block = s_stop != 0;
@@ -2862,7 +2955,7 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, int64_t m, int64_t n, T* A, int64_t ld
     post_launch(ctx, "f32_split_kernel");
   }
   QrSm& S = q.job.S;
-  S = QrSm{nullptr, nullptr, nullptr};
+  S = QrSm{nullptr, nullptr};
   if (trace_on()) {
     const int64_t km = std::max<int64_t>(P.kmax, 1);
     D.stamps = ctx->arena.alloc_n<unsigned long long>((size_t)16 * km);
@@ -2870,14 +2963,10 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, int64_t m, int64_t n, T* A, int64_t ld
     S.pubt = ctx->arena.alloc_n<unsigned long long>((size_t)G * km);
     LRA_CUDA(cudaMemsetAsync(S.pubt, 0, (size_t)G * km * 8, ctx->stream));
   }
-  // the exchange: 4 max words and 4 stop words a 128-byte line apart, and
-  // the arrival counter on a line of its own
-  unsigned char* xb = static_cast<unsigned char*>(ctx->arena.alloc(1152));
-  S.amax = reinterpret_cast<unsigned long long*>(xb);
-  S.astop = reinterpret_cast<unsigned*>(xb + 512);
-  S.arrive = reinterpret_cast<unsigned*>(xb + 1024);
+  // the exchange: four slots, a 128-byte line each
+  S.slot = ctx->arena.alloc_n<ulonglong2>(32);
   S.stage = ctx->arena.alloc_n<E>((size_t)2 * G * m);
-  LRA_CUDA(cudaMemsetAsync(xb, 0, 1152, ctx->stream));
+  LRA_CUDA(cudaMemsetAsync(S.slot, 0, 32 * sizeof(ulonglong2), ctx->stream));
   q.job.G = G;
   q.job.off = 0;
 }
@@ -2970,7 +3059,7 @@ int geqp3_steps_fit(lra_ctx* ctx, int count, const int64_t* m, int64_t n) {
 
 template <typename T>
 int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* st, int64_t nb, double atol, double rtol,
-                     int64_t* k) {
+                     int64_t* k, int likely) {
   using Ar = SmA<T>;
   if (count < 1 || count > kSmJobs) fail(LRA_EINVAL, "geqp3_adap_steps: %d steps", count);
   std::vector<int64_t> ms(count);
@@ -2981,12 +3070,19 @@ int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* st, int64_t nb, d
   if (geqp3_steps_fit<T>(ctx, count, ms.data(), st[0].n) < count) fail(LRA_EINVAL, "geqp3_adap_steps: no fit");
   const ArenaMark mark = ctx->arena.mark();
   const size_t cap = sm_capacity<Ar>(ctx);
-  // each step on the fewest CTAs that hold it; the rest to the last (the
-  // largest, with the most pivots)
+  // each step on the fewest CTAs that hold it; the rest to the step expected
+  // to reveal the rank (the launch ends with it), then from the last (the
+  // largest, with the most pivots) down
   std::vector<int> G(count);
-  int used = 0;
-  for (int i = 0; i < count; ++i) used += G[i] = sm_min_ctas<Ar>(cap, st[i].m, st[i].n);
-  G[count - 1] = std::min(sm_natural_ctas(ctx, st[count - 1].n), G[count - 1] + (qr_sm_cap(ctx) - used));
+  int spare = qr_sm_cap(ctx);
+  for (int i = 0; i < count; ++i) spare -= G[i] = sm_min_ctas<Ar>(cap, st[i].m, st[i].n);
+  auto widen = [&](int i) {
+    const int more = std::max(0, std::min(spare, sm_natural_ctas(ctx, st[i].n) - G[i]));
+    G[i] += more;
+    spare -= more;
+  };
+  if (likely >= 0 && likely < count) widen(likely);
+  for (int i = count - 1; i >= 0; --i) widen(i);
   int* success = ctx->arena.alloc_n<int>(1);
   LRA_CUDA(cudaMemsetAsync(success, 0x7f, sizeof(int), ctx->stream));
   std::vector<SmQr<T>> q(count);
@@ -3468,7 +3564,7 @@ template int64_t geqp3_adap_noalloc<double>(lra_ctx*, int64_t, int64_t, double*,
   template void orgqr<T>(lra_ctx*, int64_t, int64_t, T*, int64_t, const T*);                      \
   template void col_norms<T>(lra_ctx*, int64_t, int64_t, const T*, int64_t, T*);                  \
   template int geqp3_steps_fit<T>(lra_ctx*, int, const int64_t*, int64_t);                        \
-  template int geqp3_adap_steps<T>(lra_ctx*, int, const QrStep<T>*, int64_t, double, double, int64_t*);
+  template int geqp3_adap_steps<T>(lra_ctx*, int, const QrStep<T>*, int64_t, double, double, int64_t*, int);
 INST(float)
 INST(double)
 #undef INST
