@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <functional>
 #include <vector>
 #include <cstdio>
 #include <cstdlib>
@@ -2288,47 +2289,145 @@ struct DfPrepJob {
   unsigned long long* maxbits;  // 1, zeroed: max |B| as the bits of a double
 };
 
+// ---- conversions to pairs of floats -------------------------------------------
+// Bound: the FP64 unit, 64 cycles a warp instruction, if each entry's split and
+// square went through it (a dozen FP64 conversions, products and sums an entry).
+// The split of x 2^k is therefore done on the bits of x: h its 24 leading bits
+// rounded to even, l the rest rounded to a float, t = h + l as a double; one
+// FP64 multiply-add an entry remains, for the column's norm.  Same bits as
+// df_split.  160 sketches of 72 rows (108 MB): 1.05 -> 0.22 ms with the tile
+// below; an idfact_batched of 160: 20.7 -> 18.5 ms.
+__device__ __forceinline__ void df_split_pow2(double x, int k, double sc, float& h, float& l, double& t) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int ek = ((int)(b >> 52) & 0x7ff) + k;  // biased exponent of x 2^k
+  if (ek < 960 || ek > 1023) {
+    // zero, so small that l would be denormal, or not below 1
+    const Df d = df_split(x * sc);
+    h = d.h;
+    l = d.l;
+    t = df_val(d.h, d.l);
+    return;
+  }
+  const unsigned long long M = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+  unsigned q = (unsigned)(M >> 29);
+  const unsigned rem = (unsigned)M & 0x1fffffffu;
+  const unsigned up = (rem > 0x10000000u || (rem == 0x10000000u && (q & 1u))) ? 1u : 0u;
+  q += up;
+  const int r = (int)rem - (int)(up << 29);
+  const unsigned sg = (unsigned)(b >> 32) & 0x80000000u;
+  h = __uint_as_float(sg | (((unsigned)(ek - 897) << 23) + q));
+  const float lf = __int2float_rn(r);
+  l = r ? __uint_as_float((__float_as_uint(lf) + ((unsigned)(ek - 1075) << 23)) ^ sg) : 0.f;
+  const unsigned long long V = ((unsigned long long)q << 29) + (unsigned long long)(long long)__float2int_rn(lf);
+  t = __longlong_as_double((long long)(((unsigned long long)sg << 32) | (((unsigned long long)(ek - 1) << 52) + V)));
+}
+
+// sums over the lanes of four values: lanes 8g .. 8g + 7 get value g's, added in
+// warp_sum's order
+__device__ __forceinline__ double warp_sum4(const double (&d)[4], int lane) {
+  const bool up = lane & 16, hi = lane & 8;
+  const double e0 = (up ? d[2] : d[0]) + __shfl_xor_sync(0xffffffffu, up ? d[0] : d[2], 16);
+  const double e1 = (up ? d[3] : d[1]) + __shfl_xor_sync(0xffffffffu, up ? d[1] : d[3], 16);
+  double t = (hi ? e1 : e0) + __shfl_xor_sync(0xffffffffu, hi ? e0 : e1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+// below this sum of squares a column's norm is taken at its own scale
+constexpr double kNormSmall = 0x1p-900;
+
+// max |x| (NaN left out) as bits: integer maxima
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+  return b <= 0x7ff0000000000000ull ? b : 0ull;
+}
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long w) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(w >> 32));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(w >> 32) == hi ? (unsigned)w : 0u);
+  return ((unsigned long long)hi << 32) | lo;
+}
+
+// a column's norm at the scale of its largest entry (columns too small, zero or
+// with NaN), one warp
+template <class At>
+__device__ double small_norm(int64_t m, int lane, At at) {
+  double cm = 0;
+  for (int64_t i = lane; i < m; i += 32) cm = fmax(cm, fabs(at(i)));
+  cm = warp_max(cm);
+  if (!(cm > 0)) return 0;
+  const double s2 = pow2_scale_inv(cm);
+  double acc = 0;
+  for (int64_t i = lane; i < m; i += 32) {
+    const double t = at(i) * s2;
+    acc = fma(t, t, acc);
+  }
+  return sqrt(warp_sum(acc)) / s2;
+}
+
 // CTAs (matrix, part): max |B| of every part's columns into maxbits
 __global__ void __launch_bounds__(512) df_prep_max_kernel(const DfPrepJob* __restrict__ jobs) {
-  __shared__ double red[32];
   const DfPrepJob J = jobs[blockIdx.x];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double mx = 0;
+  unsigned long long mx = 0;
   for (int64_t j = (int64_t)blockIdx.y * nw + wid; j < J.n; j += (int64_t)gridDim.y * nw)
-    for (int64_t i = lane; i < J.m; i += 32) mx = fmax(mx, fabs(J.B[i + j * J.ldb]));
-  mx = block_max(mx, red);
-  if (threadIdx.x == 0 && mx > 0) atomicMax(J.maxbits, (unsigned long long)__double_as_longlong(mx));
+    for (int64_t i = lane; i < J.m; i += 32) mx = max(mx, abs_bits(J.B[i + j * J.ldb]));
+  mx = warp_max_bits(mx);
+  if (lane == 0 && mx > 0) atomicMax(J.maxbits, mx);
 }
 
 // CTAs (matrix, part): the scaled float pairs and each column's norm, a warp
-// per column
-__global__ void __launch_bounds__(512) df_prep_split_kernel(const DfPrepJob* __restrict__ jobs) {
+// per four columns; a row-major workspace is written through a shared tile of
+// 32 columns (a column's rows are a row of the workspace apart: 8-byte stores
+// into 32 different sectors otherwise)
+__global__ void __launch_bounds__(256) df_prep_split_kernel(const DfPrepJob* __restrict__ jobs) {
+  extern __shared__ float2 prep_tile[];
   const DfPrepJob J = jobs[blockIdx.x];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double mx = __longlong_as_double((long long)*J.maxbits);
   const double sc = mx > 0 ? ldexp(1.0, -(ilogb(mx) + 1)) : 1.0;
+  const int k = mx > 0 ? -(ilogb(mx) + 1) : 0;
   if (blockIdx.y == 0 && threadIdx.x == 0) *J.scale = sc;
-  for (int64_t j = (int64_t)blockIdx.y * nw + wid; j < J.n; j += (int64_t)gridDim.y * nw) {
-    float2* w = J.work + j * J.cs;
-    double cm = 0;
+  const bool rowmaj = J.rs != 1;
+  const int ts = (int)J.m + 1;
+  for (int64_t j0 = (int64_t)blockIdx.y * 32; j0 < J.n; j0 += (int64_t)gridDim.y * 32) {
+    const int64_t j = j0 + 4 * wid;
+    double acc[4] = {0, 0, 0, 0};
     for (int64_t i = lane; i < J.m; i += 32) {
-      const double x = J.B[i + j * J.ldb] * sc;
-      const Df d = df_split(x);
-      w[i * J.rs] = make_float2(d.h, d.l);
-      cm = fmax(cm, fabs(x));
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        if (j + g < J.n) {
+          float h, l;
+          double t;
+          df_split_pow2(J.B[i + (j + g) * J.ldb], k, sc, h, l, t);
+          if (rowmaj)
+            prep_tile[(4 * wid + g) * ts + i] = make_float2(h, l);
+          else
+            J.work[(j + g) * J.cs + i] = make_float2(h, l);
+          acc[g] = fma(t, t, acc[g]);
+        }
     }
-    cm = warp_max(cm);
-    double acc = 0;
-    if (cm > 0) {
-      const double s2 = pow2_scale_inv(cm);
-      for (int64_t i = lane; i < J.m; i += 32) {
-        const Df d = df_split(J.B[i + j * J.ldb] * sc);
-        const double t = df_val(d.h, d.l) * s2;
-        acc = fma(t, t, acc);
-      }
-      acc = sqrt(warp_sum(acc)) / s2;
+    const double a = warp_sum4(acc, lane);
+    const double v = sqrt(a);
+    const int g = lane >> 3;
+    if ((lane & 7) == 0 && j + g < J.n) J.vn0[j + g] = v;
+    for (unsigned odd = __ballot_sync(0xffffffffu, !(a >= kNormSmall) && (lane & 7) == 0 && j + g < J.n); odd;
+         odd &= odd - 1) {
+      const int64_t jj = j + ((__ffs(odd) - 1) >> 3);
+      const double* b = J.B + jj * J.ldb;
+      const double nr = small_norm(J.m, lane, [&](int64_t i) {
+        const Df d = df_split(b[i] * sc);
+        return df_val(d.h, d.l);
+      });
+      if (lane == 0) J.vn0[jj] = nr;
+      __syncwarp();
     }
-    if (lane == 0) J.vn0[j] = acc;
+    if (rowmaj) {
+      __syncthreads();
+      for (int64_t i = wid; i < J.m; i += 8)
+        if (j0 + lane < J.n) J.work[i * J.rs + (j0 + lane)] = prep_tile[lane * ts + i];
+      __syncthreads();
+    }
   }
 }
 
@@ -2343,9 +2442,10 @@ struct DfFinishJob {
   const int64_t* piv;
   const int64_t* nfac;
   int64_t* jpvt;
+  int* pos;  // n: the position of each column
 };
 
-__global__ void __launch_bounds__(512) df_finish_group_kernel(const DfFinishJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(512) df_finish_replay_kernel(const DfFinishJob* __restrict__ jobs) {
   extern __shared__ int fin_smem[];
   const DfFinishJob J = jobs[blockIdx.x];
   int* ca = fin_smem;        // column at position
@@ -2365,23 +2465,55 @@ __global__ void __launch_bounds__(512) df_finish_group_kernel(const DfFinishJob*
     }
   }
   __syncthreads();
-  const double inv = 1.0 / *J.scale;
-  for (int64_t j = threadIdx.x; j < J.n; j += blockDim.x) J.jpvt[j] = ca[j] + 1;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int64_t j = wid; j < J.n; j += nw) {
-    const float2* w = J.work + (int64_t)ca[j] * J.cs;
-    for (int64_t i = lane; i < J.m; i += 32) J.B[i + j * J.ldb] = df_val(w[i * J.rs].x, w[i * J.rs].y) * inv;
+  for (int64_t j = threadIdx.x; j < J.n; j += blockDim.x) {
+    J.jpvt[j] = ca[j] + 1;
+    J.pos[j] = ps[j];
   }
 }
 
-// max |B| as the bit pattern of a nonnegative double
-__global__ void df_absmax_kernel(int64_t m, int64_t n, const double* __restrict__ B, int64_t ldb,
-                                 unsigned long long* __restrict__ out) {
-  double mx = 0;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < m * n; t += (int64_t)gridDim.x * blockDim.x)
-    mx = fmax(mx, fabs(B[t % m + (t / m) * ldb]));
-  mx = warp_max(mx);
-  if ((threadIdx.x & 31) == 0 && mx > 0) atomicMax(out, (unsigned long long)__double_as_longlong(mx));
+// CTAs (matrix, part): the columns of the workspace to their positions in B,
+// 32 columns at a time; a row-major workspace is read through a shared tile
+__global__ void __launch_bounds__(256) df_finish_group_kernel(const DfFinishJob* __restrict__ jobs) {
+  extern __shared__ float2 fin_tile[];
+  const DfFinishJob J = jobs[blockIdx.x];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const double inv = 1.0 / *J.scale;
+  const bool rowmaj = J.rs != 1;
+  const int ts = (int)J.m + 1;
+  for (int64_t j0 = (int64_t)blockIdx.y * 32; j0 < J.n; j0 += (int64_t)gridDim.y * 32) {
+    if (rowmaj) {
+      __syncthreads();
+      for (int64_t i = wid; i < J.m; i += 8)
+        if (j0 + lane < J.n) fin_tile[lane * ts + i] = J.work[i * J.rs + (j0 + lane)];
+      __syncthreads();
+    }
+    for (int g = wid; g < 32 && j0 + g < J.n; g += 8) {
+      const float2* w = rowmaj ? fin_tile + g * ts : J.work + (j0 + g) * J.cs;
+      double* o = J.B + (int64_t)J.pos[j0 + g] * J.ldb;
+      for (int64_t i = lane; i < J.m; i += 32) o[i] = df_val(w[i].x, w[i].y) * inv;
+    }
+  }
+}
+// max |B| over an m x n matrix as the bits of a double, a warp per column
+template <typename T>
+__global__ void __launch_bounds__(256) absmax_cols_kernel(int64_t m, int64_t n, const T* __restrict__ B, int64_t ldb,
+                                                          unsigned long long* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  if constexpr (sizeof(T) == 8) {
+    unsigned long long mx = 0;
+    for (int64_t j = w0; j < n; j += nw)
+      for (int64_t i = lane; i < m; i += 32) mx = max(mx, abs_bits(B[i + j * ldb]));
+    mx = warp_max_bits(mx);
+    if (lane == 0 && mx > 0) atomicMax(out, mx);
+  } else {
+    float mx = 0;
+    for (int64_t j = w0; j < n; j += nw)
+      for (int64_t i = lane; i < m; i += 32) mx = fmaxf(mx, fabsf(B[i + j * ldb]));
+    mx = warp_max(mx);
+    if (lane == 0 && mx > 0) atomicMax(out, (unsigned long long)__double_as_longlong((double)mx));
+  }
 }
 
 // scale = 2^-E with max |B| in [2^(E-1), 2^E)
@@ -2390,34 +2522,40 @@ __global__ void df_scale_kernel(const unsigned long long* mx, double* scale) {
   *scale = m > 0 ? ldexp(1.0, -(ilogb(m) + 1)) : 1.0;
 }
 
-// (h, l) = split(B * scale); a warp per column also writes its norm
-__global__ void df_split_kernel(int64_t m, int64_t n, const double* __restrict__ B, int64_t ldb,
-                                const double* __restrict__ scale, float* __restrict__ Bh, float* __restrict__ Bl,
-                                int64_t ldh, double* __restrict__ vn0) {
+// (h, l) = split(B * scale) and each column's norm, a warp per four columns
+__global__ void __launch_bounds__(256) df_split_kernel(int64_t m, int64_t n, const double* __restrict__ B, int64_t ldb,
+                                                       const double* __restrict__ scale, float* __restrict__ Bh,
+                                                       float* __restrict__ Bl, int64_t ldh, double* __restrict__ vn0) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const double sc = *scale;
-  for (int64_t j = w0; j < n; j += nw) {
-    double mx = 0;
+  const int k = ilogb(sc);
+  for (int64_t j = 4 * w0; j < n; j += 4 * nw) {
+    double acc[4] = {0, 0, 0, 0};
     for (int64_t i = lane; i < m; i += 32) {
-      const double x = B[i + j * ldb] * sc;
-      const Df d = df_split(x);
-      Bh[i + j * ldh] = d.h;
-      Bl[i + j * ldh] = d.l;
-      mx = fmax(mx, fabs(x));
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        if (j + g < n) {
+          float h, l;
+          double t;
+          df_split_pow2(B[i + (j + g) * ldb], k, sc, h, l, t);
+          Bh[i + (j + g) * ldh] = h;
+          Bl[i + (j + g) * ldh] = l;
+          acc[g] = fma(t, t, acc[g]);
+        }
     }
-    mx = warp_max(mx);
-    double acc = 0;
-    if (mx > 0) {
-      const double s = pow2_scale_inv(mx);
-      for (int64_t i = lane; i < m; i += 32) {
-        const double t = df_val(Bh[i + j * ldh], Bl[i + j * ldh]) * s;
-        acc = fma(t, t, acc);
-      }
-      acc = sqrt(warp_sum(acc)) / s;
+    const double a = warp_sum4(acc, lane);
+    const double v = sqrt(a);
+    const int g = lane >> 3;
+    if ((lane & 7) == 0 && j + g < n) vn0[j + g] = v;
+    for (unsigned odd = __ballot_sync(0xffffffffu, !(a >= kNormSmall) && (lane & 7) == 0 && j + g < n); odd;
+         odd &= odd - 1) {
+      const int64_t jj = j + ((__ffs(odd) - 1) >> 3);
+      const double nr = small_norm(m, lane, [&](int64_t i) { return df_val(Bh[i + jj * ldh], Bl[i + jj * ldh]); });
+      if (lane == 0) vn0[jj] = nr;
+      __syncwarp();
     }
-    if (lane == 0) vn0[j] = acc;
   }
 }
 
@@ -2433,67 +2571,84 @@ __global__ void qr_step_of_kernel(int64_t n, const int64_t* __restrict__ piv, co
     for (int64_t c = threadIdx.x; c < nfac; c += blockDim.x) step_of[piv[c]] = c;
 }
 
-// B = (h + l) / scale, except the Householder vectors below the diagonal of
-// the pivot columns (rows below the step of column j), which carry no scale
-__global__ void df_join_kernel(int64_t m, int64_t n, const float* __restrict__ Bh, const float* __restrict__ Bl,
-                               int64_t ldh, const double* __restrict__ scale, double* __restrict__ B, int64_t ldb,
-                               const int64_t* __restrict__ step_of) {
+// B = (h + l) / scale in the pivoted column order (column j of B is column
+// jpvt[j] of the pairs), except the Householder vectors below the diagonal of
+// the pivot columns (rows below the step of the column), which carry no scale.
+// A warp per column.
+__global__ void __launch_bounds__(256) df_join_kernel(int64_t m, int64_t n, const float* __restrict__ Bh,
+                                                      const float* __restrict__ Bl, int64_t ldh,
+                                                      const double* __restrict__ scale, double* __restrict__ B,
+                                                      int64_t ldb, const int64_t* __restrict__ step_of,
+                                                      const int64_t* __restrict__ jpvt) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const double inv = 1.0 / *scale;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < m * n; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % m, j = t / m;
-    const double v = df_val(Bh[i + j * ldh], Bl[i + j * ldh]);
-    B[i + j * ldb] = i > step_of[j] ? v : v * inv;
+  for (int64_t j = w0; j < n; j += nw) {
+    const int64_t sj = jpvt[j] - 1, st = step_of[sj];
+    for (int64_t i = lane; i < m; i += 32) {
+      const double v = df_val(Bh[i + sj * ldh], Bl[i + sj * ldh]);
+      B[i + j * ldb] = i > st ? v : v * inv;
+    }
   }
 }
 
 // the Float32 sketch's conversions for the shared-memory QR: max |B| (as
 // the bits of a double, for df_scale_kernel), B * scale (exact: a power of
 // two) with each column's norm, and back
-__global__ void f32_absmax_kernel(int64_t m, int64_t n, const float* __restrict__ B, int64_t ldb,
-                                  unsigned long long* __restrict__ out) {
-  double mx = 0;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < m * n; t += (int64_t)gridDim.x * blockDim.x)
-    mx = fmax(mx, (double)fabsf(B[t % m + (t / m) * ldb]));
-  mx = warp_max(mx);
-  if ((threadIdx.x & 31) == 0 && mx > 0) atomicMax(out, (unsigned long long)__double_as_longlong(mx));
-}
-
-__global__ void f32_split_kernel(int64_t m, int64_t n, const float* __restrict__ B, int64_t ldb,
-                                 const double* __restrict__ scale, float* __restrict__ Bs, int64_t lds,
-                                 double* __restrict__ vn0) {
+__global__ void __launch_bounds__(256) f32_split_kernel(int64_t m, int64_t n, const float* __restrict__ B, int64_t ldb,
+                                                        const double* __restrict__ scale, float* __restrict__ Bs,
+                                                        int64_t lds, double* __restrict__ vn0) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const float sc = (float)*scale;
-  for (int64_t j = w0; j < n; j += nw) {
-    double mx = 0;
+  for (int64_t j = 4 * w0; j < n; j += 4 * nw) {
+    double acc[4] = {0, 0, 0, 0};
     for (int64_t i = lane; i < m; i += 32) {
-      const float x = B[i + j * ldb] * sc;
-      Bs[i + j * lds] = x;
-      mx = fmax(mx, (double)fabsf(x));
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        if (j + g < n) {
+          const float x = B[i + (j + g) * ldb] * sc;
+          Bs[i + (j + g) * lds] = x;
+          // (double)x of a normal x from its bits
+          const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xffu;
+          const double t = e != 0 && e != 0xffu
+                               ? __longlong_as_double((long long)(((unsigned long long)(b & 0x80000000u) << 32) |
+                                                                  ((unsigned long long)(e + 896u) << 52) |
+                                                                  ((unsigned long long)(b & 0x7fffffu) << 29)))
+                               : (double)x;
+          acc[g] = fma(t, t, acc[g]);
+        }
     }
-    mx = warp_max(mx);
-    double acc = 0;
-    if (mx > 0) {
-      const double s = pow2_scale_inv(mx);
-      for (int64_t i = lane; i < m; i += 32) {
-        const double t = (double)Bs[i + j * lds] * s;
-        acc = fma(t, t, acc);
-      }
-      acc = sqrt(warp_sum(acc)) / s;
+    const double a = warp_sum4(acc, lane);
+    const double v = sqrt(a);
+    const int g = lane >> 3;
+    if ((lane & 7) == 0 && j + g < n) vn0[j + g] = v;
+    for (unsigned odd = __ballot_sync(0xffffffffu, !(a >= kNormSmall) && (lane & 7) == 0 && j + g < n); odd;
+         odd &= odd - 1) {
+      const int64_t jj = j + ((__ffs(odd) - 1) >> 3);
+      const double nr = small_norm(m, lane, [&](int64_t i) { return (double)Bs[i + jj * lds]; });
+      if (lane == 0) vn0[jj] = nr;
+      __syncwarp();
     }
-    if (lane == 0) vn0[j] = acc;
   }
 }
 
-__global__ void f32_join_kernel(int64_t m, int64_t n, const float* __restrict__ Bs, int64_t lds,
-                                const double* __restrict__ scale, float* __restrict__ B, int64_t ldb,
-                                const int64_t* __restrict__ step_of) {
+__global__ void __launch_bounds__(256) f32_join_kernel(int64_t m, int64_t n, const float* __restrict__ Bs, int64_t lds,
+                                                       const double* __restrict__ scale, float* __restrict__ B,
+                                                       int64_t ldb, const int64_t* __restrict__ step_of,
+                                                       const int64_t* __restrict__ jpvt) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const float inv = (float)(1.0 / *scale);
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < m * n; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % m, j = t / m;
-    const float v = Bs[i + j * lds];
-    B[i + j * ldb] = i > step_of[j] ? v : v * inv;
+  for (int64_t j = w0; j < n; j += nw) {
+    const int64_t sj = jpvt[j] - 1, st = step_of[sj];
+    for (int64_t i = lane; i < m; i += 32) {
+      const float v = Bs[i + sj * lds];
+      B[i + j * ldb] = i > st ? v : v * inv;
+    }
   }
 }
 
@@ -2707,7 +2862,7 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
   std::vector<DfPrepJob> prep((size_t)count);
   std::vector<QrJob> qr((size_t)count);
   std::vector<DfFinishJob> fin((size_t)count);
-  size_t smem_qr = 0, smem_fin = 0;
+  size_t smem_qr = 0, smem_fin = 0, smem_tile = 0;
   unsigned long long* maxbits = ctx->arena.alloc_n<unsigned long long>((size_t)count);
   LRA_CUDA(cudaMemsetAsync(maxbits, 0, (size_t)count * sizeof(unsigned long long), ctx->stream));
   int64_t nmax = 1;
@@ -2746,7 +2901,9 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
     J.work = work;
     J.cs = cs;
     J.rs = rs;
-    fin[(size_t)t] = DfFinishJob{m, n, it.ldb, it.B, work, cs, rs, scale, J.X.piv, J.X.nfac, it.jpvt};
+    fin[(size_t)t] = DfFinishJob{m, n, it.ldb, it.B, work, cs, rs, scale, J.X.piv, J.X.nfac, it.jpvt,
+                                 ctx->arena.alloc_n<int>(n)};
+    if (rowmaj) smem_tile = std::max(smem_tile, (size_t)32 * (m + 1) * sizeof(float2));
     smem_qr = std::max(smem_qr, (size_t)m * sizeof(float2) + (size_t)n * (5 * 8 + 1));
     smem_fin = std::max(smem_fin, (size_t)2 * n * sizeof(int));
   }
@@ -2771,11 +2928,14 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
   if (tr)
     for (auto& e : ev) LRA_CUDA(cudaEventCreate(&e));
   if (tr) LRA_CUDA(cudaEventRecord(ev[0], ctx->stream));
+  // CTAs a matrix of the conversions, up to four tiles of 32 columns each
+  const unsigned tiles = (unsigned)std::max<int64_t>(1, (nmax + 127) / 128);
   {
     const unsigned parts = (unsigned)std::min<int64_t>(16, (nmax + 15) / 16);
     df_prep_max_kernel<<<dim3((unsigned)count, parts), 512, 0, ctx->stream>>>(dprep);
     post_launch(ctx, "df_prep_max_kernel");
-    df_prep_split_kernel<<<dim3((unsigned)count, parts), 512, 0, ctx->stream>>>(dprep);
+    raise_smem_limit(ctx, (const void*)df_prep_split_kernel);
+    df_prep_split_kernel<<<dim3((unsigned)count, tiles), 256, smem_tile, ctx->stream>>>(dprep);
     post_launch(ctx, "df_prep_split_kernel");
   }
   if (tr) LRA_CUDA(cudaEventRecord(ev[1], ctx->stream));
@@ -2784,8 +2944,11 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
   geqp3_df_group_kernel<NTG><<<grid, NTG, smem_qr, ctx->stream>>>(dqr, (int)count, next);
   post_launch(ctx, "geqp3_df_group_kernel");
   if (tr) LRA_CUDA(cudaEventRecord(ev[2], ctx->stream));
+  raise_smem_limit(ctx, (const void*)df_finish_replay_kernel);
+  df_finish_replay_kernel<<<(unsigned)count, 512, smem_fin, ctx->stream>>>(dfin);
+  post_launch(ctx, "df_finish_replay_kernel");
   raise_smem_limit(ctx, (const void*)df_finish_group_kernel);
-  df_finish_group_kernel<<<(unsigned)count, 512, smem_fin, ctx->stream>>>(dfin);
+  df_finish_group_kernel<<<dim3((unsigned)count, tiles), 256, smem_tile, ctx->stream>>>(dfin);
   post_launch(ctx, "df_finish_group_kernel");
   if (tr) {
     LRA_CUDA(cudaEventRecord(ev[3], ctx->stream));
@@ -2930,14 +3093,14 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, int64_t m, int64_t n, T* A, int64_t ld
   q.scale = ctx->arena.alloc_n<double>(1);
   unsigned long long* mx = ctx->arena.alloc_n<unsigned long long>(1);
   LRA_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned long long), ctx->stream));
-  q.gm = (unsigned)std::max<int64_t>(1, std::min<int64_t>((m * n + 255) / 256, ctx->num_sms * 8));
-  const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, ctx->num_sms * 8));
+  q.gm = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, ctx->num_sms * 8));
+  const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 31) / 32, ctx->num_sms * 8));
   QrDf& D = q.job.D;
   D = QrDf{nullptr, nullptr, vn0, q.scale, nullptr};
   if constexpr (sizeof(T) == 8) {
     const double* Bd = reinterpret_cast<const double*>(A);
-    df_absmax_kernel<<<q.gm, 256, 0, ctx->stream>>>(m, n, Bd, lda, mx);
-    post_launch(ctx, "df_absmax_kernel");
+    absmax_cols_kernel<double><<<q.gm, 256, 0, ctx->stream>>>(m, n, Bd, lda, mx);
+    post_launch(ctx, "absmax_cols_kernel");
     df_scale_kernel<<<1, 1, 0, ctx->stream>>>(mx, q.scale);
     post_launch(ctx, "df_scale_kernel");
     D.Bh = ctx->arena.alloc_n<float>((size_t)m * n);
@@ -2946,8 +3109,8 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, int64_t m, int64_t n, T* A, int64_t ld
     post_launch(ctx, "df_split_kernel");
   } else {
     const float* Bf = reinterpret_cast<const float*>(A);
-    f32_absmax_kernel<<<q.gm, 256, 0, ctx->stream>>>(m, n, Bf, lda, mx);
-    post_launch(ctx, "f32_absmax_kernel");
+    absmax_cols_kernel<float><<<q.gm, 256, 0, ctx->stream>>>(m, n, Bf, lda, mx);
+    post_launch(ctx, "absmax_cols_kernel");
     df_scale_kernel<<<1, 1, 0, ctx->stream>>>(mx, q.scale);
     post_launch(ctx, "df_scale_kernel");
     D.Bh = ctx->arena.alloc_n<float>((size_t)m * n);
@@ -3005,15 +3168,6 @@ void sm_finish(lra_ctx* ctx, SmQr<T>& q) {
   int64_t* step_of = ctx->arena.alloc_n<int64_t>(n);
   qr_step_of_kernel<<<1, 1024, 0, ctx->stream>>>(n, X.piv, X.nfac, step_of);
   post_launch(ctx, "qr_step_of_kernel");
-  if constexpr (sizeof(T) == 8) {
-    df_join_kernel<<<q.gm, 256, 0, ctx->stream>>>(m, n, D.Bh, D.Bl, m, q.scale, reinterpret_cast<double*>(q.A), q.lda,
-                                                  step_of);
-    post_launch(ctx, "df_join_kernel");
-  } else {
-    f32_join_kernel<<<q.gm, 256, 0, ctx->stream>>>(m, n, D.Bh, m, q.scale, reinterpret_cast<float*>(q.A), q.lda,
-                                                   step_of);
-    post_launch(ctx, "f32_join_kernel");
-  }
   if (n <= 24576) {
     const size_t rs = (size_t)2 * n * sizeof(int);
     raise_smem_limit(ctx, (const void*)geqp3_replay_smem_kernel);
@@ -3026,9 +3180,15 @@ void sm_finish(lra_ctx* ctx, SmQr<T>& q) {
   const unsigned gi = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, ctx->num_sms * 4));
   jpvt_kernel<<<gi, 256, 0, ctx->stream>>>(n, q.col_at, q.jpvt);
   post_launch(ctx, "jpvt_kernel");
-  T* tmp = ctx->arena.alloc_n<T>((size_t)m * n);
-  gather_cols(ctx, m, n, q.A, q.lda, q.jpvt, tmp, m);
-  copy_matrix(ctx, m, n, tmp, m, q.A, q.lda);
+  if constexpr (sizeof(T) == 8) {
+    df_join_kernel<<<q.gm, 256, 0, ctx->stream>>>(m, n, D.Bh, D.Bl, m, q.scale, reinterpret_cast<double*>(q.A), q.lda,
+                                                  step_of, q.jpvt);
+    post_launch(ctx, "df_join_kernel");
+  } else {
+    f32_join_kernel<<<q.gm, 256, 0, ctx->stream>>>(m, n, D.Bh, m, q.scale, reinterpret_cast<float*>(q.A), q.lda,
+                                                   step_of, q.jpvt);
+    post_launch(ctx, "f32_join_kernel");
+  }
 }
 
 // the shared-memory kernel applies to an m x n sketch of this type (the
@@ -3222,6 +3382,8 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     const unsigned gi = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, ctx->num_sms * 4));
     iota_kernel<<<gi, 256, 0, ctx->stream>>>(n, col_at, pos);
     post_launch(ctx, "iota_kernel");
+    int64_t* step_of = nullptr;
+    std::function<void()> join;  // the pairs back into A, in pivot order
     // the mixed-precision path factors Float64 sketches in double-float
     // (two reflectors and four pairs per column in shared memory, one
     // reflector when two do not fit; a million columns and more take the
@@ -3239,12 +3401,12 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
       unsigned long long* mx = ctx->arena.alloc_n<unsigned long long>(1);
       LRA_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned long long), ctx->stream));
       const double* Bd = reinterpret_cast<const double*>(A);
-      const unsigned gm = (unsigned)std::max<int64_t>(1, std::min<int64_t>((m * n + 255) / 256, ctx->num_sms * 8));
-      df_absmax_kernel<<<gm, 256, 0, ctx->stream>>>(m, n, Bd, lda, mx);
-      post_launch(ctx, "df_absmax_kernel");
+      const unsigned gm = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, ctx->num_sms * 8));
+      absmax_cols_kernel<double><<<gm, 256, 0, ctx->stream>>>(m, n, Bd, lda, mx);
+      post_launch(ctx, "absmax_cols_kernel");
       df_scale_kernel<<<1, 1, 0, ctx->stream>>>(mx, scale);
       post_launch(ctx, "df_scale_kernel");
-      const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, ctx->num_sms * 8));
+      const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 31) / 32, ctx->num_sms * 8));
       df_split_kernel<<<gs, 256, 0, ctx->stream>>>(m, n, Bd, lda, scale, Bh, Bl, m, vn0);
       post_launch(ctx, "df_split_kernel");
       QrDf D{Bh, Bl, vn0, scale, nullptr};
@@ -3277,12 +3439,14 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
       }
       post_launch(ctx, kname);
       if (D.stamps) print_qr_trace(ctx, D.stamps, P.kmax, m, n, kname, false, nullptr, 1);
-      int64_t* step_of = ctx->arena.alloc_n<int64_t>(n);
+      step_of = ctx->arena.alloc_n<int64_t>(n);
       qr_step_of_kernel<<<1, 1024, 0, ctx->stream>>>(n, X.piv, X.nfac, step_of);
       post_launch(ctx, "qr_step_of_kernel");
-      df_join_kernel<<<gm, 256, 0, ctx->stream>>>(m, n, Bh, Bl, m, scale, reinterpret_cast<double*>(A), lda,
-                                                  step_of);
-      post_launch(ctx, "df_join_kernel");
+      join = [=] {
+        df_join_kernel<<<gm, 256, 0, ctx->stream>>>(m, n, Bh, Bl, m, scale, reinterpret_cast<double*>(A), lda, step_of,
+                                                    jpvt);
+        post_launch(ctx, "df_join_kernel");
+      };
     } else {
       void* args[] = {&P, &X};
       LRA_CUDA(cudaLaunchCooperativeKernel((const void*)geqp3_v2_kernel<T, NT>, dim3(grid), dim3(NT), args,
@@ -3303,7 +3467,9 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     }
     jpvt_kernel<<<gi, 256, 0, ctx->stream>>>(n, col_at, jpvt);
     post_launch(ctx, "jpvt_kernel");
-    if (pivot) {
+    if (join) {
+      join();
+    } else if (pivot) {
       T* tmp = ctx->arena.alloc_n<T>((size_t)m * n);
       gather_cols(ctx, m, n, A, lda, jpvt, tmp, m);
       copy_matrix(ctx, m, n, tmp, m, A, lda);
