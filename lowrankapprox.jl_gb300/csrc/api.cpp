@@ -248,6 +248,20 @@ struct RandSrc {
     }
   }
 
+  // the next n lattice draws as a source for tc_sketch
+  SketchSrc lattice_src(int64_t n, bool right) {
+    SketchSrc s;
+    s.right = right ? 1 : 0;
+    if (injected_gauss()) {
+      s.g = take_gauss_raw(n);
+    } else {
+      s.seed = seed;
+      s.base = ctx->rng_counter;
+      ctx->rng_counter += (uint64_t)(n + 1) / 2;
+    }
+    return s;
+  }
+
   template <typename T>
   void signs(int64_t n, T* d) {
     if (n <= 0) return;
@@ -436,28 +450,28 @@ void make_sketch(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, int64_t
   const char tA = trans == 'c' ? 't' : 'n';
   switch (o.sketch) {
     case LRA_SKETCH_RANDN: {
-      const bool tc = use_tc(o, dtype) && tc_sketch_supported(order, M, N);
-      T* S = ctx->arena.alloc_n<T>((size_t)order * M);
-      if (right_layout) {
+      // the products with op(A): a GEMM, or the operator's own product for
+      // a matrix-free input (sketch_randn_* with A a LinOp, src/linop.jl)
+      const bool lin = ctx->linop != nullptr;
+      const bool tc = !lin && use_tc(o, dtype) && tc_sketch_supported(order, M, N);
+      T* S = tc ? nullptr : ctx->arena.alloc_n<T>((size_t)order * M);
+      if (tc) {
+        TcSplit local;
+        if (!split) split = &local;
+        if (split->ns == 0) tc_split<T>(ctx, trans, M, N, A, lda, dtype == LRA_F64 ? 6 : 3, split);
+        const SketchSrc src = rs.lattice_src(order * M, right_layout);
+        tc_sketch<T>(ctx, *split, 1, &src, &order, B, order);
+      } else if (right_layout) {
         T* Sr = ctx->arena.alloc_n<T>((size_t)order * M);
         rs.gauss(order * M, Sr, o.precision == LRA_PREC_MIXED);
         transpose(ctx, M, order, Sr, std::max<int64_t>(M, 1), S, std::max<int64_t>(order, 1));
       } else {
         rs.gauss(order * M, S, o.precision == LRA_PREC_MIXED);
       }
-      // the products with op(A): a GEMM, or the operator's own product for
-      // a matrix-free input (sketch_randn_* with A a LinOp, src/linop.jl)
-      const bool lin = ctx->linop != nullptr;
-      if (lin) {
+      if (lin)
         linop_rmul<T>(ctx, trans, order, M, N, S, order, B, order);
-      } else if (tc) {
-        TcSplit local;
-        if (!split) split = &local;
-        if (split->ns == 0) tc_split<T>(ctx, trans, M, N, A, lda, dtype == LRA_F64 ? 6 : 3, split);
-        tc_sketch<T>(ctx, *split, order, S, B, order);
-      } else {
+      else if (!tc)
         gemm<T>(ctx, 'n', tA, order, N, M, T(1), S, order, A, lda, T(0), B, order);
-      }
       if (o.sketch_randn_niter > 0) {
         const bool herm = (M == N) && is_symmetric(ctx, M, A, lda);
         T* Bq = ctx->arena.alloc_n<T>((size_t)order * M);
@@ -596,8 +610,12 @@ int sketchfact_steps(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, int
   if (cnt < 2) return 0;
   std::vector<QrStep<T>> st;
   std::vector<RandSrc::Pos> after;
+  // plain Gaussian sketches on the tensor cores: all steps' as one product, their
+  // rows stacked (the byte slices are read once instead of once a step)
+  const bool stack = split && o.sketch == LRA_SKETCH_RANDN && o.sketch_randn_niter == 0;
   {
     Stage sg(ctx, 0);
+    std::vector<SketchSrc> src;
     for (int i = 0; i < cnt; ++i) {
       const int64_t order = orders[(size_t)i];
       const int64_t l = std::min(order, N);
@@ -606,14 +624,17 @@ int sketchfact_steps(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, int
       q.m = order;
       q.n = N;
       q.lda = std::max<int64_t>(order, 1);
-      q.A = ctx->arena.alloc_n<T>((size_t)q.lda * N);
+      q.A = stack ? nullptr : ctx->arena.alloc_n<T>((size_t)q.lda * N);
       q.jpvt = ctx->arena.alloc_n<int64_t>(N);
       q.tau = ctx->arena.alloc_n<T>(std::max<int64_t>(l, 1));
       q.kmax = kmax;
       q.nt = nts[(size_t)i];
       const RandSrc::Pos before = rs.pos();
       try {
-        make_sketch<T>(ctx, o, trans, M, N, A, lda, order, rs, q.A, dtype, split);
+        if (stack)
+          src.push_back(rs.lattice_src(order * M, false));
+        else
+          make_sketch<T>(ctx, o, trans, M, N, A, lda, order, rs, q.A, dtype, split);
       } catch (const Error& e) {
         // an injected stream too short for a step drawn ahead: the launch
         // ends before it (the step-by-step loop meets the same error only if
@@ -625,6 +646,17 @@ int sketchfact_steps(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, int
       }
       st.push_back(q);
       after.push_back(rs.pos());
+    }
+    if (stack) {
+      int64_t total = 0;
+      for (int i = 0; i < cnt; ++i) total += orders[(size_t)i];
+      T* Bs = ctx->arena.alloc_n<T>((size_t)total * N);
+      tc_sketch<T>(ctx, *split, cnt, src.data(), orders.data(), Bs, total);
+      for (QrStep<T>& q : st) {
+        q.A = Bs;
+        q.lda = total;
+        Bs += q.m;
+      }
     }
   }
   if (cnt < 2) {
@@ -1113,40 +1145,6 @@ bool grouped_batch_ok(lra_ctx* ctx, int64_t count, const lra_matdesc* mats, cons
   return true;
 }
 
-// The per-matrix launches of a batch (staging, byte slices, sketches) are
-// small; they are spread over the context's side streams so that several run
-// at once.  fan_out makes the side streams wait for the work issued so far on
-// the main stream, fan_in makes the main stream wait for the side streams.
-void fan_out(lra_ctx* ctx) {
-  for (int i = 0; i < lra_ctx::kAux; ++i)
-    if (!ctx->aux[i]) LRA_CUDA(cudaStreamCreateWithFlags(&ctx->aux[i], cudaStreamNonBlocking));
-  for (cudaEvent_t& e : ctx->aux_ev)
-    if (!e) LRA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  LRA_CUDA(cudaEventRecord(ctx->aux_ev[lra_ctx::kAux], ctx->stream));
-  for (int i = 0; i < lra_ctx::kAux; ++i) LRA_CUDA(cudaStreamWaitEvent(ctx->aux[i], ctx->aux_ev[lra_ctx::kAux], 0));
-}
-
-void fan_in(lra_ctx* ctx) {
-  for (int i = 0; i < lra_ctx::kAux; ++i) {
-    LRA_CUDA(cudaEventRecord(ctx->aux_ev[i], ctx->aux[i]));
-    LRA_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->aux_ev[i], 0));
-  }
-}
-
-// runs fn with ctx->stream switched to side stream i (mod the count)
-template <typename Fn>
-void on_side(lra_ctx* ctx, int64_t i, Fn&& fn) {
-  cudaStream_t main = ctx->stream;
-  ctx->stream = ctx->aux[i % lra_ctx::kAux];
-  try {
-    fn();
-  } catch (...) {
-    ctx->stream = main;
-    throw;
-  }
-  ctx->stream = main;
-}
-
 void idfact_batched_grouped(lra_ctx* ctx, int64_t count, const lra_matdesc* mats, const lra_opts& oin,
                             lra_id** outs) {
   lra_opts o = oin;
@@ -1187,18 +1185,15 @@ void idfact_batched_grouped(lra_ctx* ctx, int64_t count, const lra_matdesc* mats
     std::vector<TcSplit> split((size_t)cn);
     int* flags = ctx->arena.alloc_n<int>((size_t)cn);
     LRA_CUDA(cudaMemsetAsync(flags, 0, (size_t)cn * sizeof(int), ctx->stream));
-    fan_out(ctx);
+    std::vector<SplitItem> sit((size_t)cn);
     for (int64_t i = 0; i < cn; ++i) {
       const lra_matdesc& d = mats[c0 + i];
-      on_side(ctx, i, [&] {
-        dA[(size_t)i] = stage_in<double>(ctx, d.A, d.m, d.n, d.lda);
-        if (o.check_finite) all_finite_async(ctx, d.m, d.n, dA[(size_t)i].p, dA[(size_t)i].ld, flags + i);
-        tc_split<double>(ctx, 'n', d.m, d.n, dA[(size_t)i].p, dA[(size_t)i].ld, 6, &split[(size_t)i]);
-      });
+      dA[(size_t)i] = stage_in<double>(ctx, d.A, d.m, d.n, d.lda);
+      sit[(size_t)i] = SplitItem{dA[(size_t)i].p, d.m, d.n, dA[(size_t)i].ld};
     }
-    fan_in(ctx);
+    tc_split_batch(ctx, cn, sit.data(), split.data(), flags);
     tmark(0);
-    {
+    if (o.check_finite) {
       std::vector<int> hf((size_t)cn);
       LRA_CUDA(cudaMemcpyAsync(hf.data(), flags, (size_t)cn * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       LRA_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1217,17 +1212,19 @@ void idfact_batched_grouped(lra_ctx* ctx, int64_t count, const lra_matdesc* mats
     std::vector<St> st((size_t)cn);
     for (auto& s : st) s.nt = adaptive ? o.nb : o.rank;
     int64_t* kdev = ctx->arena.alloc_n<int64_t>((size_t)cn);
-    int* errs = ctx->arena.alloc_n<int>((size_t)cn);
+    int* errs = ctx->arena.alloc_n<int>(1);
     for (int round = 0;; ++round) {
       if (round > 62) fail(LRA_EINVAL, "adaptive sketch did not terminate");
       std::vector<int64_t> act;
       for (int64_t i = 0; i < cn; ++i)
         if (!st[(size_t)i].done) act.push_back(i);
       if (act.empty()) break;
-      LRA_CUDA(cudaMemsetAsync(errs, 0, (size_t)cn * sizeof(int), ctx->stream));
+      LRA_CUDA(cudaMemsetAsync(errs, 0, sizeof(int), ctx->stream));
       std::vector<DfBatchItem> items;
+      std::vector<SketchItem> sk;
       items.reserve(act.size());
-      fan_out(ctx);
+      sk.reserve(act.size());
+      int64_t order = 0;  // the same for all: their thresholds double together
       for (const int64_t i : act) {
         St& s = st[(size_t)i];
         const lra_matdesc& d = mats[c0 + i];
@@ -1238,31 +1235,27 @@ void idfact_batched_grouped(lra_ctx* ctx, int64_t count, const lra_matdesc* mats
         s.B = ctx->arena.alloc_n<double>((size_t)s.order * d.n);
         s.jpvt = ctx->arena.alloc_n<int64_t>((size_t)d.n);
         s.tau = ctx->arena.alloc_n<double>((size_t)std::max<int64_t>(l, 1));
-        // S stays allocated until the chunk ends: the sketches run on several streams
-        double* S = ctx->arena.alloc_n<double>((size_t)s.order * d.m);
+        order = s.order;
         ctx->rng_counter = s.ctr;
-        on_side(ctx, i, [&] {
-          RandSrc rs(ctx, nullptr, o.seed);
-          rs.gauss(s.order * d.m, S, true);
-          tc_sketch<double>(ctx, split[(size_t)i], s.order, S, s.B, s.order, errs + i);
-        });
+        RandSrc rs(ctx, nullptr, o.seed);
+        sk.push_back(SketchItem{&split[(size_t)i], rs.lattice_src(s.order * d.m, false), s.B, s.order});
         s.ctr = ctx->rng_counter;
         items.push_back(DfBatchItem{s.order, d.n, s.order, kmax, s.B, s.jpvt, s.tau});
       }
-      fan_in(ctx);
+      tc_sketch_batch(ctx, (int64_t)sk.size(), sk.data(), order, errs);
       std::vector<int64_t> map(act.begin(), act.end());
       tmark(1);
       // the batch writes k of item t to kdev[t]
       geqp3_df_batch(ctx, (int64_t)items.size(), items.data(), o.nb, o.atol, o.rtol, kdev);
       tmark(2);
       std::vector<int64_t> hk(items.size());
-      std::vector<int> he((size_t)cn);
+      int he = 0;
       LRA_CUDA(cudaMemcpyAsync(hk.data(), kdev, hk.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-      LRA_CUDA(cudaMemcpyAsync(he.data(), errs, (size_t)cn * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      LRA_CUDA(cudaMemcpyAsync(&he, errs, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       LRA_CUDA(cudaStreamSynchronize(ctx->stream));
+      if (he) fail(LRA_ETIMEDOUT, "tc_sketch: a bounded wait timed out");
       for (size_t t = 0; t < map.size(); ++t) {
         St& s = st[(size_t)map[t]];
-        if (he[(size_t)map[t]]) fail(LRA_ETIMEDOUT, "tc_sketch: a bounded wait timed out");
         s.k = hk[t];
         s.nsteps = round + 1;
         if (!adaptive || s.k < s.nt)
@@ -2366,14 +2359,6 @@ void lra_ctx_destroy(lra_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
-  for (int i = 0; i < lra_ctx::kAux; ++i) {
-    if (ctx->aux[i]) {
-      cudaStreamSynchronize(ctx->aux[i]);
-      cudaStreamDestroy(ctx->aux[i]);
-    }
-  }
-  for (cudaEvent_t e : ctx->aux_ev)
-    if (e) cudaEventDestroy(e);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   if (ctx->dev_err) cudaFree(ctx->dev_err);
   delete ctx;

@@ -121,10 +121,6 @@ struct lra_ctx {
   // pinned host staging (grown on demand)
   void* pinned = nullptr;
   size_t pinned_cap = 0;
-  // side streams of the batched path and their join events (made on first use)
-  static constexpr int kAux = 8;
-  cudaStream_t aux[kAux] = {};
-  cudaEvent_t aux_ev[kAux + 1] = {};
   // the operator of a matrix-free call (lra_*_linop) while it runs, else null
   const lra_linop* linop = nullptr;
   lra_tuning tuning{};
@@ -154,11 +150,32 @@ bool tc_sketch_supported(int64_t order, int64_t M, int64_t N);
 template <typename T>
 void tc_split(lra_ctx* ctx, char trans, int64_t M, int64_t N, const T* A, int64_t lda, int ns,
               TcSplit* out, bool balanced = false);
-// B (order x N, ldb) = S op(A) on tcgen05 tensor cores; S is order x M
-// (ld = order) with entries on the 1/32 lattice.
+// where a sketch's lattice draws come from: an injected stream on the device, or
+// (g null) the generator of `seed` at counter `base`; `right`: drawn in the
+// layout of a right sketch (M x order), used transposed
+struct SketchSrc {
+  const double* g = nullptr;
+  uint64_t seed = 0, base = 0;
+  int right = 0;
+};
+// B (sum of rows[i] x N, ldb) = S op(A) on tcgen05 tensor cores, S the nsrc
+// sketches stacked (rows[i] x M each, entries on the 1/32 lattice).
 template <typename T>
-void tc_sketch(lra_ctx* ctx, const TcSplit& sp, int64_t order, const T* S, T* B, int64_t ldb,
-               int* err_slot = nullptr);
+void tc_sketch(lra_ctx* ctx, const TcSplit& sp, int nsrc, const SketchSrc* src, const int64_t* rows, T* B, int64_t ldb);
+
+// the same for a batch of Float64 matrices, grouped launches (lra_idfact_batched)
+struct SplitItem {
+  const double* A;
+  int64_t K, N, lda;
+};
+struct SketchItem {
+  const TcSplit* sp;
+  SketchSrc src;
+  double* B;
+  int64_t ldb;
+};
+void tc_split_batch(lra_ctx* ctx, int64_t count, const SplitItem* items, TcSplit* out, int* bad);
+void tc_sketch_batch(lra_ctx* ctx, int64_t count, const SketchItem* items, int64_t order, int* err);
 
 // Raises a kernel's dynamic shared memory limit to the most the device
 // allows beside its static shared memory.  Always the same value per kernel:

@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "draws.cuh"
 #include "internal.hpp"
 
 namespace lra {
@@ -109,43 +110,14 @@ __global__ void zero_lower_kernel(int64_t m, int64_t n, T* A, int64_t lda) {
   }
 }
 
-__device__ __forceinline__ double lattice(double g) {
-  double r = rint(g * 32.0);
-  r = fmin(127.0, fmax(-127.0, r));
-  return r * (1.0 / 32.0);
-}
-
-// the same rounding in FP32 (exact: the lattice values are k / 32, |k| <= 127)
-__device__ __forceinline__ float lattice_f(float g) {
-  const float r = fminf(127.0f, fmaxf(-127.0f, rintf(g * 32.0f)));
-  return r * 0.03125f;
-}
-
 template <typename T>
 __global__ void from_stream_kernel(const double* __restrict__ g, int64_t n, T* __restrict__ out,
                                    int lat) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x) {
     const double v = g[t];
-    out[t] = (T)(lat ? lattice(v) : v);
+    out[t] = lat ? (T)((float)lattice_int(v) * 0.03125f) : (T)v;
   }
-}
-
-// Philox-4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11), own implementation.
-struct U4 {
-  unsigned x, y, z, w;
-};
-__device__ __forceinline__ U4 philox(U4 c, unsigned k0, unsigned k1) {
-  const unsigned M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const unsigned hi0 = __umulhi(M0, c.x), lo0 = M0 * c.x;
-    const unsigned hi1 = __umulhi(M1, c.z), lo1 = M1 * c.z;
-    c = U4{hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0};
-    k0 += W0;
-    k1 += W1;
-  }
-  return c;
 }
 
 template <typename T>
@@ -155,16 +127,9 @@ __global__ void philox_kernel(uint64_t seed, uint64_t base, int64_t n, T* __rest
        t += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t ctr = base + (uint64_t)t;
     U4 r = philox(U4{(unsigned)ctr, (unsigned)(ctr >> 32), 0x6c72u, 0x61u}, k0, k1);
-    // Box-Muller on two uniforms in (0, 1], in FP32: the draws are rounded
-    // to the 1/32 lattice, far coarser than FP32's resolution, and FP64
-    // transcendentals are slow on this part
-    const float u1 = ((float)r.x + 1.0f) * 2.3283064365386963e-10f;
-    const float u2 = ((float)r.y + 0.5f) * 2.3283064365386963e-10f;
-    const float rad = sqrtf(-2.0f * logf(u1));
-    float s, c;
-    sincospif(2.0f * u2, &s, &c);
-    out[2 * t] = (T)lattice_f(rad * c);
-    if (2 * t + 1 < n) out[2 * t + 1] = (T)lattice_f(rad * s);
+    const float2 g = philox_gauss(r);
+    out[2 * t] = (T)lattice_f(g.x);
+    if (2 * t + 1 < n) out[2 * t + 1] = (T)lattice_f(g.y);
   }
 }
 

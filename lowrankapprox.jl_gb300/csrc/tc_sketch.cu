@@ -35,8 +35,10 @@
 #include <atomic>
 #include <cfloat>
 #include <cstring>
+#include <vector>
 
 #include "common.cuh"
+#include "draws.cuh"
 #include "internal.hpp"
 
 namespace lra {
@@ -57,6 +59,7 @@ template <int TN>
 struct TcTile {
   static constexpr int S_BYTES = TN * KBLK * 2;  // 4, 8 or 12 KB (1024 multiples)
   static constexpr int COLS = TN / 2;            // sketch rows per drain thread
+  // (128 rows a CTA only with up to four accumulators)
   static constexpr uint32_t TMEM_COLS = 5 * TN <= 256 ? 256u : 512u;
   static_assert(S_BYTES % 1024 == 0 && COLS % 16 == 0 && TN % 16 == 0, "tile N");
 };
@@ -204,10 +207,11 @@ __device__ __forceinline__ void tc_fence_after() {
 }
 
 // ---- the sketch kernel ----------------------------------------------------------
+// one tile: columns n_tile of op(A), sketch rows l_tile, K blocks kb0 .. kb0 + nkb
 template <int TILE_N>
-__global__ void __launch_bounds__(NTHREADS, 1)
-    tc_sketch_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmS,
-                     TcParams P) {
+__device__ __forceinline__ void tc_sketch_body(const CUtensorMap* tmA, const CUtensorMap* tmS, const TcParams& P,
+                                               const int64_t n_tile, const int64_t l_tile, const int kb0,
+                                               const int nkb) {
   constexpr int S_BYTES = TcTile<TILE_N>::S_BYTES;
   constexpr int COLS = TcTile<TILE_N>::COLS;
   constexpr uint32_t TMEM_COLS = TcTile<TILE_N>::TMEM_COLS;
@@ -226,13 +230,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t ntl = (P.L + TILE_N - 1) / TILE_N;
-  const int64_t n_tile = blockIdx.x / ntl, l_tile = blockIdx.x % ntl;
-  // this CTA's K blocks [kb0, kb0 + nkb): whole 512-long chunks, so that
-  // every chunk is rounded as without the split
-  const int nkb_all = (int)((P.K + KBLK - 1) / KBLK);
-  const int kb0 = (int)blockIdx.y * P.kc_per * CHUNK_KB;
-  const int nkb = min(nkb_all - kb0, P.kc_per * CHUNK_KB);
   const int nchunks = (nkb + CHUNK_KB - 1) / CHUNK_KB;
   const int n_exact = ns < MAX_EXACT ? ns : MAX_EXACT;
   const bool has_tail = ns > MAX_EXACT;
@@ -271,9 +268,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         ++issued;
         unsigned char* st = stages + s * stage_bytes;
         mbar_expect_tx(full + s, (uint32_t)stage_bytes);
-        tma_load_2d(st, &tmS, (kb0 + kb) * KBLK, (int)(l_tile * TILE_N), full + s);
+        tma_load_2d(st, tmS, (kb0 + kb) * KBLK, (int)(l_tile * TILE_N), full + s);
         for (int q = 0; q < ns; ++q)
-          tma_load_3d(st + S_BYTES + q * TILE_BYTES, &tmA, (kb0 + kb) * KBLK, (int)(n_tile * TILE_M), q, full + s);
+          tma_load_3d(st + S_BYTES + q * TILE_BYTES, tmA, (kb0 + kb) * KBLK, (int)(n_tile * TILE_M), q, full + s);
       }
       // no copy may still be landing in shared memory when the CTA exits
       int dummy = 0;
@@ -395,6 +392,38 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
+}
+
+template <int TILE_N>
+__global__ void __launch_bounds__(NTHREADS, 1)
+    tc_sketch_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmS,
+                     const __grid_constant__ TcParams P) {
+  const int64_t ntl = (P.L + TILE_N - 1) / TILE_N;
+  // this CTA's K blocks [kb0, kb0 + nkb): whole 512-long chunks, so that
+  // every chunk is rounded as without the split
+  const int nkb_all = (int)((P.K + KBLK - 1) / KBLK);
+  const int kb0 = (int)blockIdx.y * P.kc_per * CHUNK_KB;
+  tc_sketch_body<TILE_N>(&tmA, &tmS, P, blockIdx.x / ntl, blockIdx.x % ntl, kb0,
+                         min(nkb_all - kb0, P.kc_per * CHUNK_KB));
+}
+
+// a batch's sketches in one launch: CTA t takes tile[t] = (matrix, column tile,
+// row tile), the longest K first; the maps and parameters of matrix i at maps[2 i]
+// (planes), maps[2 i + 1] (draws) and params[i]
+template <int TILE_N>
+__global__ void __launch_bounds__(NTHREADS, 1)
+    tc_sketch_group_kernel(const CUtensorMap* __restrict__ maps, const TcParams* __restrict__ params,
+                           const int3* __restrict__ tile) {
+  const int3 t = tile[blockIdx.x];
+  const CUtensorMap* tmA = maps + 2 * t.x;
+  const CUtensorMap* tmS = tmA + 1;
+  if (threadIdx.x == 0) {
+    // the maps were written to global memory by a copy before this launch
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmA) : "memory");
+    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmS) : "memory");
+  }
+  const TcParams P = params[t.x];
+  tc_sketch_body<TILE_N>(tmA, tmS, P, t.y, t.z, 0, (int)((P.K + KBLK - 1) / KBLK));
 }
 
 // the split-K sketch's sums W (exact int64) scaled into B, as the unsplit
@@ -548,16 +577,90 @@ __device__ __forceinline__ void write_slices(long long F, int ns, int n_exact, i
   }
 }
 
+// A warp per column run of 128 rows, four consecutive rows a lane, so that every
+// plane is written in 8-byte pieces, 256 contiguous bytes a warp (2-byte stores
+// with a division per entry for its place ran at 2.1 TB/s: 1.29 ms for 65536 x
+// 4096 Float32, 0.82 ms this way)
 template <typename T>
-__global__ void split_n_kernel(int64_t K, int64_t N, const T* __restrict__ A, int64_t lda, const int* __restrict__ e,
-                               int ns, int n_exact, int W, __nv_bfloat16* __restrict__ S, int64_t Kp) {
-  const int64_t total = Kp * N;
-  const int64_t plane = Kp * N;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t % Kp, j = t / Kp;
-    const long long F = i < K ? fixed_point(A[i + j * lda], e[j], W) : 0;
-    write_slices<T>(F, ns, n_exact, W, S + i + j * Kp, plane);
+__device__ __forceinline__ void split_n_run(int64_t K, int64_t N, const T* __restrict__ A, int64_t lda,
+                                            const int* __restrict__ e, int ns, int n_exact, int W,
+                                            __nv_bfloat16* __restrict__ S, int64_t Kp, int64_t j, int64_t run, int lane) {
+  const int64_t plane = Kp * N, i = run * 128 + 4 * lane;
+  if (i >= Kp) return;
+  const T* a = A + j * lda + i;
+  T x[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) x[q] = i + q < K ? a[q] : T(0);
+  const int ej = e[j];
+  __nv_bfloat16 d[4][MAX_SLICES];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) write_slices<T>(i + q < K ? fixed_point(x[q], ej, W) : 0, ns, n_exact, W, d[q], 1);
+  __nv_bfloat16* o = S + i + j * Kp;
+#pragma unroll
+  for (int p = 0; p < MAX_SLICES; ++p) {
+    if (p >= ns) break;
+    ushort4 v;
+    v.x = __bfloat16_as_ushort(d[0][p]);
+    v.y = __bfloat16_as_ushort(d[1][p]);
+    v.z = __bfloat16_as_ushort(d[2][p]);
+    v.w = __bfloat16_as_ushort(d[3][p]);
+    *reinterpret_cast<ushort4*>(o + p * plane) = v;  // (Kp is a multiple of 8)
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) split_n_kernel(int64_t K, int64_t N, const T* __restrict__ A, int64_t lda,
+                                                      const int* __restrict__ e, int ns, int n_exact, int W,
+                                                      __nv_bfloat16* __restrict__ S, int64_t Kp) {
+  const int lane = threadIdx.x & 31;
+  const int64_t runs = (Kp + 127) / 128;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < runs * N; u += nw)
+    split_n_run(K, N, A, lda, e, ns, n_exact, W, S, Kp, u / runs, u % runs, lane);
+}
+
+// ---- the same for a batch: CTAs (matrix, part)
+struct SplitJob {
+  int64_t K, N, lda, Kp;
+  const double* A;
+  int* e;
+  __nv_bfloat16* S;
+  int* bad;  // set when an entry is NaN or infinite
+};
+
+__global__ void __launch_bounds__(256) colexp_group_kernel(const SplitJob* __restrict__ jobs) {
+  const SplitJob J = jobs[blockIdx.x];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int64_t j = (int64_t)blockIdx.y * 8 + wid; j < J.N; j += (int64_t)gridDim.y * 8) {
+    const double* a = J.A + j * J.lda;
+    unsigned long long mx = 0;
+    int64_t i = lane;
+    for (; i + 96 < J.K; i += 128) {
+      unsigned long long v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = abs_bits(a[i + 32 * q]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) mx = v[q] > mx ? v[q] : mx;
+    }
+    for (; i < J.K; i += 32) {
+      const unsigned long long v = abs_bits(a[i]);
+      mx = v > mx ? v : mx;
+    }
+    mx = warp_max_bits(mx);
+    if (lane == 0) {
+      const int e = colexp_of(bits_value(mx));
+      J.e[j] = e;
+      if (e >= kNonFinite) *J.bad = 1;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) split_group_kernel(const SplitJob* __restrict__ jobs, int ns, int n_exact, int W) {
+  const SplitJob J = jobs[blockIdx.x];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t runs = (J.Kp + 127) / 128;
+  for (int64_t u = (int64_t)blockIdx.y * 8 + wid; u < runs * J.N; u += (int64_t)gridDim.y * 8)
+    split_n_run(J.K, J.N, J.A, J.lda, J.e, ns, n_exact, W, J.S, J.Kp, u / runs, u % runs, lane);
 }
 
 // op(A) = A^T through 32 x 32 shared-memory tiles
@@ -585,25 +688,93 @@ __global__ void split_c_kernel(int64_t K, int64_t N, const T* __restrict__ A, in
   }
 }
 
-// St (Kp x Lp, K-major: St[i + r Kp]) = 32 S(r, i) in BF16, zero padded
-template <typename T>
-__global__ void sketch_t_kernel(int64_t L, int64_t K, const T* __restrict__ S, int64_t Lp, int64_t Kp,
-                                __nv_bfloat16* __restrict__ St) {
-  __shared__ T tile[32][33];
-  const int64_t tr = (Lp + 31) / 32, tk = (Kp + 31) / 32;
-  for (int64_t t = blockIdx.x; t < tr * tk; t += gridDim.x) {
-    const int64_t r0 = (t % tr) * 32, i0 = (t / tr) * 32;
-    for (int c = threadIdx.y; c < 32; c += blockDim.y) {
-      const int64_t r = r0 + threadIdx.x, i = i0 + c;  // S(r, i) contiguous in r
-      tile[c][threadIdx.x] = (r < L && i < K) ? S[r + i * L] : T(0);
+// Rows [r0, r0 + L) of St (K-major: St[i + r Kp]) = 32 S(r, i) in BF16, straight
+// from the draws: S(r, i) is draw r + i L of the source (a left sketch's L x K
+// layout) or i + r K (`right`: a right sketch's K x L).  Tiles of 32 rows of S
+// x 64 of its columns through shared memory.  (Through an S in memory, read
+// back transposed, a 65536-row stream took 1.81 ms of a 16.8 ms call; 0.48 ms so.)
+__device__ __forceinline__ unsigned short bf16_small(float k) {  // an integer |k| <= 127
+  return (unsigned short)(__float_as_uint(k) >> 16);
+}
+
+__device__ void sketch_src_tile(const SketchSrc& src, int64_t L, int64_t K, int64_t Kp, __nv_bfloat16* __restrict__ St,
+                                int64_t r0, int64_t tr, int64_t tk, unsigned short (*tile)[66]) {
+  const int64_t rr = tr * 32, ii = tk * 64;
+  if (src.right) {
+    // draws along i: no transposition
+    for (int e = threadIdx.x; e < 32 * 32; e += 256) {
+      const int64_t r = rr + e / 32, i = ii + 2 * (e % 32);
+      if (r >= L || i >= Kp) continue;
+      unsigned short v[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        float k = 0.f;
+        if (i + q < K) {
+          const int64_t t = i + q + r * K;
+          if (src.g) {
+            k = (float)lattice_int(src.g[t]);
+          } else {
+            const float2 p = philox_pair(src.seed, src.base, t >> 1);
+            k = lattice_f((t & 1) ? p.y : p.x) * 32.0f;
+          }
+        }
+        v[q] = bf16_small(k);
+      }
+      *reinterpret_cast<ushort2*>(St + i + (r0 + r) * Kp) = make_ushort2(v[0], v[1]);
     }
-    __syncthreads();
-    for (int c = threadIdx.y; c < 32; c += blockDim.y) {
-      const int64_t i = i0 + threadIdx.x, r = r0 + c;
-      if (i < Kp && r < Lp) St[i + r * Kp] = __float2bfloat16_rn((float)(tile[threadIdx.x][c] * T(32)));
-    }
-    __syncthreads();
+    return;
   }
+  __syncthreads();
+  if (src.g) {
+    for (int e = threadIdx.x; e < 64 * 32; e += 256) {
+      const int r = e & 31, i = e >> 5;
+      const bool in = rr + r < L && ii + i < K;
+      tile[r][i] = bf16_small(in ? (float)lattice_int(src.g[rr + r + (ii + i) * L]) : 0.f);
+    }
+  } else {
+    // pairs of draws: column i's 32 rows touch at most 17
+    for (int e = threadIdx.x; e < 64 * 17; e += 256) {
+      const int i = e / 17;
+      const int64_t t0 = rr + (ii + i) * L;  // draw of row rr
+      const int64_t q = (t0 >> 1) + e % 17;
+      float2 p = make_float2(0.f, 0.f);
+      if (ii + i < K) p = philox_pair(src.seed, src.base, q);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int64_t r = 2 * q + h - t0;
+        if (r >= 0 && r < 32)
+          tile[r][i] = bf16_small(ii + i < K && rr + r < L ? lattice_f(h ? p.y : p.x) * 32.0f : 0.f);
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 32 * 32; e += 256) {
+    const int r = e >> 5, i = 2 * (e & 31);
+    if (rr + r < L && ii + i < Kp)
+      *reinterpret_cast<ushort2*>(St + ii + i + (r0 + rr + r) * Kp) = make_ushort2(tile[r][i], tile[r][i + 1]);
+  }
+}
+
+__global__ void __launch_bounds__(256) sketch_src_kernel(SketchSrc src, int64_t L, int64_t K, int64_t Kp,
+                                                         __nv_bfloat16* __restrict__ St, int64_t r0) {
+  __shared__ unsigned short tile[32][66];
+  const int64_t tr = (L + 31) / 32, tk = (Kp + 63) / 64;
+  for (int64_t t = blockIdx.x; t < tr * tk; t += gridDim.x)
+    sketch_src_tile(src, L, K, Kp, St, r0, t % tr, t / tr, tile);
+}
+
+struct SrcJob {
+  SketchSrc src;
+  int64_t L, K, Kp;
+  __nv_bfloat16* St;
+};
+
+__global__ void __launch_bounds__(256) sketch_src_group_kernel(const SrcJob* __restrict__ jobs) {
+  __shared__ unsigned short tile[32][66];
+  const SrcJob J = jobs[blockIdx.x];
+  const int64_t tr = (J.L + 31) / 32, tk = (J.Kp + 63) / 64;
+  for (int64_t t = blockIdx.y; t < tr * tk; t += gridDim.y)
+    sketch_src_tile(J.src, J.L, J.K, J.Kp, J.St, 0, t % tr, t / tr, tile);
 }
 
 // ---- FP64 GEMM from two-sided byte slices -------------------------------------------
@@ -884,7 +1055,7 @@ void tc_split(lra_ctx* ctx, char trans, int64_t M, int64_t N, const T* A, int64_
   } else {
     colexp_n_kernel<T><<<nblk(ctx, N, 8), 256, 0, ctx->stream>>>(M, N, A, lda, out->colexp);
     post_launch(ctx, "colexp_n_kernel");
-    split_n_kernel<T><<<nblk(ctx, Kp * N, 256), 256, 0, ctx->stream>>>(
+    split_n_kernel<T><<<nblk(ctx, (Kp + 127) / 128 * N * 32, 256), 256, 0, ctx->stream>>>(
         M, N, A, lda, out->colexp, ns, n_exact, W, static_cast<__nv_bfloat16*>(out->slices), Kp);
     post_launch(ctx, "split_n_kernel");
   }
@@ -899,19 +1070,27 @@ static int tuned_tile_n(const lra_ctx* ctx, bool f64, int64_t order) {
 }
 
 template <typename T>
-void tc_sketch(lra_ctx* ctx, const TcSplit& sp, int64_t order, const T* S, T* B, int64_t ldb, int* err_slot) {
+void tc_sketch(lra_ctx* ctx, const TcSplit& sp, int nsrc, const SketchSrc* src, const int64_t* rows, T* B, int64_t ldb) {
   const int64_t K = sp.K, N = sp.N, Kp = sp.Kp;
   const int ns = sp.ns;
-  const int TILE_N = tuned_tile_n(ctx, sizeof(T) == 8, order);
+  int64_t order = 0;
+  for (int i = 0; i < nsrc; ++i) order += rows[i];
+  int TILE_N = tuned_tile_n(ctx, sizeof(T) == 8, order);
+  // three planes (Float32) leave TMEM for 128 rows a CTA: a quarter less plane
+  // traffic into the SMs per row, the bound of this kernel, where that means
+  // fewer tiles
+  if (TILE_N == 96 && ns <= 3 && (order + 127) / 128 < (order + 95) / 96) TILE_N = 128;
   const int64_t Lp = (order + TILE_N - 1) / TILE_N * TILE_N;
   const ArenaMark mk = ctx->arena.mark();
   __nv_bfloat16* St = ctx->arena.alloc_n<__nv_bfloat16>((size_t)Kp * Lp);
-  {
-    const int64_t tiles = ((Lp + 31) / 32) * ((Kp + 31) / 32);
-    sketch_t_kernel<T><<<(unsigned)std::min<int64_t>(tiles, (int64_t)ctx->num_sms * 16), dim3(32, 8), 0,
-                         ctx->stream>>>(order, K, S, Lp, Kp, St);
-    post_launch(ctx, "sketch_t_kernel");
+  for (int64_t i = 0, r0 = 0; i < nsrc; r0 += rows[i], ++i) {
+    const int64_t tiles = ((rows[i] + 31) / 32) * ((Kp + 63) / 64);
+    sketch_src_kernel<<<(unsigned)std::min<int64_t>(tiles, (int64_t)ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+        src[i], rows[i], K, Kp, St, r0);
+    post_launch(ctx, "sketch_src_kernel");
   }
+  if (Lp > order)
+    LRA_CUDA(cudaMemsetAsync(St + Kp * order, 0, (size_t)Kp * (Lp - order) * sizeof(__nv_bfloat16), ctx->stream));
   CUtensorMap tmA, tmS;
   {
     cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)N, (cuuint64_t)ns};
@@ -925,11 +1104,8 @@ void tc_sketch(lra_ctx* ctx, const TcSplit& sp, int64_t order, const T* S, T* B,
     cuuint32_t box[2] = {KBLK, (cuuint32_t)TILE_N};
     make_map(&tmS, St, 2, dims, strides, box);
   }
-  int* err = err_slot;
-  if (!err) {
-    err = ctx->arena.alloc_n<int>(1);
-    LRA_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
-  }
+  int* err = ctx->arena.alloc_n<int>(1);
+  LRA_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
   TcParams P;
   P.K = K;
   P.ncols = N;
@@ -977,6 +1153,8 @@ void tc_sketch(lra_ctx* ctx, const TcSplit& sp, int64_t order, const T* S, T* B,
     launch(tc_sketch_kernel<32>);
   else if (TILE_N == 64)
     launch(tc_sketch_kernel<64>);
+  else if (TILE_N == 128)
+    launch(tc_sketch_kernel<128>);
   else
     launch(tc_sketch_kernel<96>);
   post_launch(ctx, "tc_sketch_kernel");
@@ -988,16 +1166,142 @@ void tc_sketch(lra_ctx* ctx, const TcSplit& sp, int64_t order, const T* S, T* B,
                                                          P.out_double);
     post_launch(ctx, "tc_sketch_finish_kernel");
   }
-  // a caller that passes err_slot checks it later (the batch, once per
-  // round) and releases the transposed sketch with its own arena mark: the
-  // batch issues sketches on several streams, so this memory may not be
-  // reused before they have all run
-  if (err_slot) return;
   int herr = 0;
   LRA_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   LRA_CUDA(cudaStreamSynchronize(ctx->stream));
   ctx->arena.release(mk);
   if (herr) fail(LRA_ETIMEDOUT, "tc_sketch: a bounded wait timed out");
+}
+
+// the byte slices of a batch of Float64 matrices in two launches; bad (count
+// ints, zeroed) marks those with a NaN or infinite entry
+void tc_split_batch(lra_ctx* ctx, int64_t count, const SplitItem* items, TcSplit* out, int* bad) {
+  constexpr int ns = MAX_SLICES;
+  std::vector<SplitJob> jobs((size_t)count);
+  int64_t nmax = 1, runs = 1;
+  for (int64_t t = 0; t < count; ++t) {
+    const SplitItem& it = items[t];
+    TcSplit& sp = out[t];
+    sp.K = it.K;
+    sp.N = it.N;
+    sp.Kp = (it.K + 7) / 8 * 8;
+    sp.ns = ns;
+    sp.trans = 'n';
+    sp.colexp = ctx->arena.alloc_n<int>(it.N);
+    sp.slices = ctx->arena.alloc_n<__nv_bfloat16>((size_t)ns * sp.Kp * it.N);
+    jobs[(size_t)t] = SplitJob{it.K, it.N, it.lda, sp.Kp, it.A, sp.colexp, static_cast<__nv_bfloat16*>(sp.slices), bad + t};
+    nmax = std::max(nmax, it.N);
+    runs = std::max(runs, (sp.Kp + 127) / 128 * it.N);
+  }
+  SplitJob* d = ctx->arena.alloc_n<SplitJob>((size_t)count);
+  LRA_CUDA(cudaMemcpyAsync(d, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice, ctx->stream));
+  // up to four columns (runs of 128 rows) a warp in the largest matrix
+  colexp_group_kernel<<<dim3((unsigned)count, (unsigned)std::max<int64_t>(1, (nmax + 31) / 32)), 256, 0, ctx->stream>>>(d);
+  post_launch(ctx, "colexp_group_kernel");
+  split_group_kernel<<<dim3((unsigned)count, (unsigned)std::max<int64_t>(1, std::min<int64_t>(1024, (runs + 31) / 32))), 256, 0,
+                       ctx->stream>>>(d, ns, MAX_EXACT, 8 * ns);
+  post_launch(ctx, "split_group_kernel");
+  // the host copy must outlive the upload
+  LRA_CUDA(cudaStreamSynchronize(ctx->stream));
+}
+
+// the sketches of a batch (one order for all), in two launches; err: one word,
+// zeroed, set when a bounded wait gave up
+void tc_sketch_batch(lra_ctx* ctx, int64_t count, const SketchItem* items, int64_t order, int* err) {
+  if (count <= 0) return;
+  const int TILE_N = tuned_tile_n(ctx, true, order);
+  const int64_t Lp = (order + TILE_N - 1) / TILE_N * TILE_N;
+  constexpr int ns = MAX_SLICES;
+  // the draws: one array when all start at the same place of the same stream
+  // (S(r, i) depends on r, i and the order alone), else one per matrix
+  bool same = true;
+  int64_t kmax = 8;
+  size_t words = 0;
+  for (int64_t t = 0; t < count; ++t) {
+    const SketchItem &a = items[t], &b = items[0];
+    same = same && !a.src.g && !b.src.g && a.src.seed == b.src.seed && a.src.base == b.src.base && !a.src.right;
+    kmax = std::max(kmax, a.sp->Kp);
+    words += (size_t)a.sp->Kp * Lp;
+  }
+  if (same) words = (size_t)kmax * Lp;
+  __nv_bfloat16* St = ctx->arena.alloc_n<__nv_bfloat16>(words);
+  LRA_CUDA(cudaMemsetAsync(St, 0, words * sizeof(__nv_bfloat16), ctx->stream));
+  std::vector<SrcJob> src;
+  std::vector<CUtensorMap> maps((size_t)2 * count);
+  std::vector<TcParams> par((size_t)count);
+  std::vector<int3> tile;
+  std::vector<int64_t> ord((size_t)count);
+  for (int64_t t = 0; t < count; ++t) ord[(size_t)t] = t;
+  std::stable_sort(ord.begin(), ord.end(), [&](int64_t a, int64_t b) { return items[a].sp->K > items[b].sp->K; });
+  if (same) src.push_back(SrcJob{items[0].src, order, kmax, kmax, St});
+  __nv_bfloat16* at = St;
+  for (int64_t t = 0; t < count; ++t) {
+    const TcSplit& sp = *items[t].sp;
+    __nv_bfloat16* my = same ? St : at;
+    const int64_t kp = same ? kmax : sp.Kp;
+    if (!same) {
+      src.push_back(SrcJob{items[t].src, order, sp.K, sp.Kp, at});
+      at += (size_t)sp.Kp * Lp;
+    }
+    {
+      cuuint64_t dims[3] = {(cuuint64_t)sp.Kp, (cuuint64_t)sp.N, (cuuint64_t)ns};
+      cuuint64_t strides[2] = {(cuuint64_t)sp.Kp * 2, (cuuint64_t)sp.Kp * sp.N * 2};
+      cuuint32_t box[3] = {KBLK, TILE_M, 1};
+      make_map(&maps[(size_t)2 * t], sp.slices, 3, dims, strides, box);
+    }
+    {
+      cuuint64_t dims[2] = {(cuuint64_t)kp, (cuuint64_t)Lp};
+      cuuint64_t strides[1] = {(cuuint64_t)kp * 2};
+      cuuint32_t box[2] = {KBLK, (cuuint32_t)TILE_N};
+      make_map(&maps[(size_t)2 * t + 1], my, 2, dims, strides, box);
+    }
+    TcParams& P = par[(size_t)t];
+    std::memset(&P, 0, sizeof P);
+    P.K = sp.K;
+    P.ncols = sp.N;
+    P.L = order;
+    P.ns = ns;
+    P.tshift = ((sp.K + 511) / 512 <= 64) ? 8 : 0;
+    P.colexp = sp.colexp;
+    P.B = items[t].B;
+    P.ldb = items[t].ldb;
+    P.out_double = 1;
+    P.err = err;
+  }
+  for (const int64_t t : ord)
+    for (int64_t nt = 0; nt < (items[t].sp->N + TILE_M - 1) / TILE_M; ++nt)
+      for (int64_t lt = 0; lt < Lp / TILE_N; ++lt) tile.push_back(make_int3((int)t, (int)nt, (int)lt));
+  const size_t stage_bytes = (size_t)TILE_N * KBLK * 2 + (size_t)ns * TILE_BYTES;
+  int smem_optin = 0;
+  LRA_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  const int nstage = (int)std::max<size_t>(2, std::min<size_t>(MAX_NSTAGE, ((size_t)smem_optin - 1024 - 256) / stage_bytes));
+  for (TcParams& P : par) P.nstage = nstage;
+  SrcJob* dsrc = ctx->arena.alloc_n<SrcJob>(src.size());
+  CUtensorMap* dmaps = ctx->arena.alloc_n<CUtensorMap>(maps.size());  // (256-byte aligned, 128 bytes each)
+  TcParams* dpar = ctx->arena.alloc_n<TcParams>(par.size());
+  int3* dtile = ctx->arena.alloc_n<int3>(tile.size());
+  LRA_CUDA(cudaMemcpyAsync(dsrc, src.data(), src.size() * sizeof(SrcJob), cudaMemcpyHostToDevice, ctx->stream));
+  LRA_CUDA(cudaMemcpyAsync(dmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, ctx->stream));
+  LRA_CUDA(cudaMemcpyAsync(dpar, par.data(), par.size() * sizeof(TcParams), cudaMemcpyHostToDevice, ctx->stream));
+  LRA_CUDA(cudaMemcpyAsync(dtile, tile.data(), tile.size() * sizeof(int3), cudaMemcpyHostToDevice, ctx->stream));
+  const int64_t src_tiles = (order + 31) / 32 * ((kmax + 63) / 64);
+  sketch_src_group_kernel<<<dim3((unsigned)src.size(), (unsigned)std::min<int64_t>(src_tiles, same ? 1024 : 32)), 256, 0,
+                            ctx->stream>>>(dsrc);
+  post_launch(ctx, "sketch_src_group_kernel");
+  const size_t smem = 1024 + (size_t)nstage * stage_bytes + 256;
+  auto launch = [&](auto kern) {
+    raise_smem_limit(ctx, (const void*)kern);
+    kern<<<(unsigned)tile.size(), NTHREADS, smem, ctx->stream>>>(dmaps, dpar, dtile);
+  };
+  if (TILE_N == 32)
+    launch(tc_sketch_group_kernel<32>);
+  else if (TILE_N == 64)
+    launch(tc_sketch_group_kernel<64>);
+  else
+    launch(tc_sketch_group_kernel<96>);
+  post_launch(ctx, "tc_sketch_group_kernel");
+  // the host copies must outlive the uploads
+  LRA_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 
 bool tc_gemm_worthwhile(int64_t m, int64_t n, int64_t k) {
@@ -1085,8 +1389,8 @@ void tc_gemm(lra_ctx* ctx, char ta, char tb, int64_t m, int64_t n, int64_t k, do
 
 template void tc_split<float>(lra_ctx*, char, int64_t, int64_t, const float*, int64_t, int, TcSplit*, bool);
 template void tc_split<double>(lra_ctx*, char, int64_t, int64_t, const double*, int64_t, int, TcSplit*, bool);
-template void tc_sketch<float>(lra_ctx*, const TcSplit&, int64_t, const float*, float*, int64_t, int*);
-template void tc_sketch<double>(lra_ctx*, const TcSplit&, int64_t, const double*, double*, int64_t, int*);
+template void tc_sketch<float>(lra_ctx*, const TcSplit&, int, const SketchSrc*, const int64_t*, float*, int64_t);
+template void tc_sketch<double>(lra_ctx*, const TcSplit&, int, const SketchSrc*, const int64_t*, double*, int64_t);
 
 cudaError_t set_wait_limit_tc(uint64_t ns) { return set_unit_wait_limit(ns); }
 
