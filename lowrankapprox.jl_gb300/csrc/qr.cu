@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <climits>
 #include <functional>
+#include <numeric>
 #include <vector>
 #include <cstdio>
 #include <cstdlib>
@@ -1517,6 +1518,11 @@ struct QrArithF32 {
   __device__ static unsigned long long key38(V v) { return v > 0.f ? (unsigned long long)__float_as_uint(v) << 6 : 0ull; }
 };
 
+// the column stride in shared memory: odd, so that a thread per column (short
+// columns) reads a row from 32 different banks (16-way conflicts at 40 and 72 rows
+// otherwise: 5.0 against 1.7 us of dot products at 72 rows, 338 columns a CTA)
+__host__ __device__ constexpr int64_t sm_stride(int64_t m) { return m | 1; }
+
 template <class A>
 __device__ __forceinline__ unsigned long long xw_pack(typename A::V v, int64_t j) {
   return (A::key38(v) << 24) | (XW_IDX - (unsigned long long)j);
@@ -1569,8 +1575,8 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
   // element (row i, slot s) at C[s cs + i rs]: column-major in shared
   // memory; the workspace of GCOL may be row-major (coalesced thread-per-
   // column access)
-  const int64_t cs = GCOL ? gcs : m, rs = GCOL ? grs : 1;
-  V* s_vn1 = reinterpret_cast<V*>(GCOL ? Vc + m : C + ncap * m);
+  const int64_t cs = GCOL ? gcs : sm_stride(m), rs = GCOL ? grs : 1;
+  V* s_vn1 = reinterpret_cast<V*>(GCOL ? Vc + m : C + ncap * cs);
   V* s_vn2 = s_vn1 + ncap;
   V* s_dot = s_vn2 + ncap;
   V* s_fs = s_dot + ncap;  // f scal of each column for the deferred update
@@ -1730,7 +1736,7 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
     for (int s = wid; s < nloc; s += NW) {
       const float* ph = Bh + (c0 + s) * lda;
       const float* pl = Bl ? Bl + (c0 + s) * lda : nullptr;
-      for (int64_t i = lane; i < m; i += 32) C[s * m + i] = A::from_planes(ph, pl, i);
+      for (int64_t i = lane; i < m; i += 32) C[s * cs + i] = A::from_planes(ph, pl, i);
     }
   double lmax = 0;
   unsigned long long cw = 0;
@@ -2014,43 +2020,81 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
       if (flagged) {
         sub(11);
         if (wid < ncw) ww = s_w[wid];  // (its warp's largest)
-        for (int s = wid; s < nloc; s += NW) {
-          if (!(s_st[s] & ST_FLAG)) continue;
-          E* col = C + (int64_t)s * cs;
-          const V fs = s_fs[s];
-          const bool upd = A::hi(fs) != 0.f;
-          float mx = 0.f;
+        // Four neighbouring columns a warp at a time: their chains of reductions
+        // overlap and share shuffles (one at a time, 40 flagged columns a warp took
+        // 19 us of a step).
+        for (int base = 4 * wid; base < nloc; base += 4 * NW) {
+          int q[4];
+          bool any = false;
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            q[g] = base + g < nloc && (s_st[base + g] & ST_FLAG) ? base + g : -1;
+            any |= q[g] >= 0;
+          }
+          if (!any) continue;
+          V fs[4];
+          float mx[4];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            fs[g] = q[g] >= 0 ? s_fs[q[g]] : A::zero();
+            mx[g] = 0.f;
+          }
           for (int64_t i = c + 1 + lane; i < m; i += 32) {
-            E y = col[i * rs];
-            if (upd) {
-              y = A::axpy_neg(y, fs, Vc[i]);
-              col[i * rs] = y;
-            }
-            mx = fmaxf(mx, fabsf(A::ehi(y)));
-          }
+            const E v = Vc[i];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-          V nr = A::from_float(mx);
-          if (mx > 0.f && isfinite(mx)) {
-            const int ex = ilogbf(mx);
-            const float sc = ldexpf(1.f, -ex);
-            V acc = A::zero();
-            for (int64_t i = c + 1 + lane; i < m; i += 32) {
-              const E x = A::escale(col[i * rs], sc);
-              A::fma_acc(acc, x, x);
-            }
-            acc = A::norm(acc);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc = A::add(acc, A::shfl_xor(acc, o));
-            nr = A::ldexp_(A::sqrt_(acc), ex);
+            for (int g = 0; g < 4; ++g)
+              if (q[g] >= 0) {
+                E* p = C + (int64_t)q[g] * cs + i * rs;
+                E y = *p;
+                if (A::hi(fs[g]) != 0.f) {
+                  y = A::axpy_neg(y, fs[g], v);
+                  *p = y;
+                }
+                mx[g] = fmaxf(mx[g], fabsf(A::ehi(y)));
+              }
           }
+          int ex[4];
+          float sc[4];
+          V acc[4];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            // (nonnegative floats order like their bits)
+            mx[g] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx[g])));
+            const bool on = mx[g] > 0.f && isfinite(mx[g]);
+            ex[g] = on ? ilogbf(mx[g]) : 0;
+            sc[g] = on ? ldexpf(1.f, -ex[g]) : 0.f;
+            acc[g] = A::zero();
+          }
+          for (int64_t i = c + 1 + lane; i < m; i += 32)
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+              if (sc[g] != 0.f) {
+                const E x = A::escale(C[(int64_t)q[g] * cs + i * rs], sc[g]);
+                A::fma_acc(acc[g], x, x);
+              }
+#pragma unroll
+          for (int g = 0; g < 4; ++g) acc[g] = A::norm(acc[g]);
+          // the transposed butterfly of the dot products: the tree of one column's
+          // own butterfly
+          const bool up = lane & 16, hi = lane & 8;
+          const V e0 = A::add(up ? acc[2] : acc[0], A::shfl_xor(up ? acc[0] : acc[2], 16));
+          const V e1 = A::add(up ? acc[3] : acc[1], A::shfl_xor(up ? acc[1] : acc[3], 16));
+          V t = A::add(hi ? e1 : e0, A::shfl_xor(hi ? e0 : e1, 8));
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) t = A::add(t, A::shfl_xor(t, o));
+          const int g = lane >> 3;
+          const int qg = g == 0 ? q[0] : g == 1 ? q[1] : g == 2 ? q[2] : q[3];
+          const float mg = g == 0 ? mx[0] : g == 1 ? mx[1] : g == 2 ? mx[2] : mx[3];
+          const float sg = g == 0 ? sc[0] : g == 1 ? sc[1] : g == 2 ? sc[2] : sc[3];
+          const int eg = g == 0 ? ex[0] : g == 1 ? ex[1] : g == 2 ? ex[2] : ex[3];
+          const V nr = sg != 0.f ? A::ldexp_(A::sqrt_(t), eg) : A::from_float(mg);
           __syncwarp();
-          if (lane == 0) {
-            s_vn1[s] = s_vn2[s] = nr;
-            s_st[s] = (unsigned char)((s_st[s] & ~ST_FLAG) | ST_UPD);
+          if ((lane & 7) == 0 && qg >= 0) {
+            s_vn1[qg] = s_vn2[qg] = nr;
+            s_st[qg] = (unsigned char)((s_st[qg] & ~ST_FLAG) | ST_UPD);
+            const unsigned long long w = xw_pack<A>(nr, c0 + qg);
+            ww = w > ww ? w : ww;
           }
-          const unsigned long long w = xw_pack<A>(nr, c0 + s);
-          ww = w > ww ? w : ww;
         }
         warp_word(ww);
         ncand = NW;
@@ -2097,9 +2141,11 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
         }
         // the rank-1 updates of rows c+1..m-1.  Shared-memory columns: a warp
         // per group of columns as above, rows in registers.  Global columns
-        // (GCOL): a thread per column, whose rows stay in L1 between the
-        // dot products and the update.
-        if (!GCOL) {
+        // (GCOL), and many short ones: a thread per column (its rows stay in L1
+        // between the dot products and the update; a warp's lanes run out of
+        // rows).
+        const bool seq_upd = GCOL || (len <= P.seq_len && nloc >= 64);
+        if (!seq_upd) {
           // NU columns at once, whole chunks without masks, then the last rows
           auto run = [&](auto nuc, E* const* pc, const V* pf) {
             constexpr int NU = decltype(nuc)::value;
@@ -2164,7 +2210,7 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
           else
             updates(std::integral_constant<int, 1>{});
         }
-        if (GCOL) {
+        if (seq_upd) {
           for (int sl = ct; sl < nloc; sl += NCT) {
             if (sl == cand || (s_st[sl] & (ST_DONE | ST_UPD))) continue;
             const V fs = s_fs[sl];
@@ -2203,7 +2249,7 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
     if (s_st[s] & ST_DONE) continue;
     float* ph = Bh + (c0 + s) * lda;
     float* pl = Bl ? Bl + (c0 + s) * lda : nullptr;
-    for (int64_t i = lane; i < m; i += 32) A::to_planes(C[(int64_t)s * m + i], ph, pl, i);
+    for (int64_t i = lane; i < m; i += 32) A::to_planes(C[(int64_t)s * cs + i], ph, pl, i);
   }
   if (b == 0 && threadIdx.x == 0) {
     *P.k_out = kres;
@@ -2275,6 +2321,34 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_group_kernel(const QrJob* __re
   }
 }
 
+// A batch's sketches that fit shared memory: each is factored by a gang of G CTAs
+// that hold its columns (as in the shared-memory kernel, the same bits), and each
+// CTA works through a list of (sketch, its rank in the gang).  The lists keep
+// one global order, so the earliest unfinished sketch always has its whole gang
+// at it, and no gang can wait for another.  A CTA alone with a sketch in global
+// memory took 79 us a pivot at 72 x 2025, and the largest sketch bounded the
+// launch: 5.1 ms for the two rounds of a batch of 160, 3.3 ms in gangs (6.2 and 8.5 ms
+// with gangs twice and four times the size).
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) geqp3_df_gang_kernel(const SmJob<QrArithDf>* __restrict__ jobs,
+                                                              const int* __restrict__ start,
+                                                              const int2* __restrict__ list) {
+  extern __shared__ unsigned char qr_dyn[];
+  __shared__ __align__(16) unsigned char s_jb[sizeof(SmJob<QrArithDf>)];
+  for (int e = start[blockIdx.x]; e < start[blockIdx.x + 1]; ++e) {
+    const int2 w = list[e];
+    __syncthreads();
+    {
+      const unsigned* src = reinterpret_cast<const unsigned*>(jobs + w.x);
+      unsigned* dst = reinterpret_cast<unsigned*>(s_jb);
+      for (int i = threadIdx.x; i < (int)(sizeof(SmJob<QrArithDf>) / 4); i += NT) dst[i] = src[i];
+    }
+    __syncthreads();
+    const SmJob<QrArithDf>& job = *reinterpret_cast<const SmJob<QrArithDf>*>(s_jb);
+    geqp3_df_body<QrArithDf, NT, false>(job.P, job.X, job.D, job.S, job.G, w.y, nullptr, 0, 0, qr_dyn);
+  }
+}
+
 // ---- the batch's conversions ---------------------------------------------------
 // prep: max |B| (its power-of-two scale as df_scale_kernel), the scaled
 // float pairs into the workspace and each column's norm as df_split_kernel
@@ -2287,6 +2361,7 @@ struct DfPrepJob {
   double* vn0;                 // n
   double* scale;               // 1
   unsigned long long* maxbits;  // 1, zeroed: max |B| as the bits of a double
+  float *Bh, *Bl;              // the pairs as planes (ld m) instead of the workspace, or null
 };
 
 // ---- conversions to pairs of floats -------------------------------------------
@@ -2400,7 +2475,10 @@ __global__ void __launch_bounds__(256) df_prep_split_kernel(const DfPrepJob* __r
           float h, l;
           double t;
           df_split_pow2(J.B[i + (j + g) * J.ldb], k, sc, h, l, t);
-          if (rowmaj)
+          if (J.Bh) {
+            J.Bh[(j + g) * J.m + i] = h;
+            J.Bl[(j + g) * J.m + i] = l;
+          } else if (rowmaj)
             prep_tile[(4 * wid + g) * ts + i] = make_float2(h, l);
           else
             J.work[(j + g) * J.cs + i] = make_float2(h, l);
@@ -2443,6 +2521,7 @@ struct DfFinishJob {
   const int64_t* nfac;
   int64_t* jpvt;
   int* pos;  // n: the position of each column
+  const float *Bh, *Bl;  // the pairs as planes (ld m), or null: the workspace
 };
 
 __global__ void __launch_bounds__(512) df_finish_replay_kernel(const DfFinishJob* __restrict__ jobs) {
@@ -2488,8 +2567,13 @@ __global__ void __launch_bounds__(256) df_finish_group_kernel(const DfFinishJob*
       __syncthreads();
     }
     for (int g = wid; g < 32 && j0 + g < J.n; g += 8) {
-      const float2* w = rowmaj ? fin_tile + g * ts : J.work + (j0 + g) * J.cs;
       double* o = J.B + (int64_t)J.pos[j0 + g] * J.ldb;
+      if (J.Bh) {
+        const float *h = J.Bh + (j0 + g) * J.m, *l = J.Bl + (j0 + g) * J.m;
+        for (int64_t i = lane; i < J.m; i += 32) o[i] = df_val(h[i], l[i]) * inv;
+        continue;
+      }
+      const float2* w = rowmaj ? fin_tile + g * ts : J.work + (j0 + g) * J.cs;
       for (int64_t i = lane; i < J.m; i += 32) o[i] = df_val(w[i].x, w[i].y) * inv;
     }
   }
@@ -2831,6 +2915,13 @@ static void print_qr_trace(lra_ctx* ctx, const unsigned long long* stamps, int64
 // launch each for the conversion, the factorization (a CTA per matrix,
 // largest first) and the replay into column order.  Each matrix comes out
 // as geqp3_adap leaves it when its shared-memory kernel runs, bit for bit.
+template <class A>
+size_t sm_smem(int64_t m, int64_t ncap);
+template <class A>
+int sm_min_ctas(size_t cap, int64_t m, int64_t n);
+static int qr_sm_cap(const lra_ctx* ctx);
+static int sm_natural_ctas(lra_ctx* ctx, int64_t n);
+
 bool geqp3_df_batch_fits(lra_ctx* ctx, int64_t m, int64_t n) {
   constexpr int NTG = 512;
   if (m < 1 || n < 1 || n >= (int64_t)XW_IDX || m > 20480) return false;
@@ -2863,6 +2954,33 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
   std::vector<QrJob> qr((size_t)count);
   std::vector<DfFinishJob> fin((size_t)count);
   size_t smem_qr = 0, smem_fin = 0, smem_tile = 0;
+  // gangs of CTAs that hold the sketches in shared memory, unless one is too
+  // large for a gang of 16
+  raise_smem_limit(ctx, (const void*)geqp3_df_gang_kernel<NTG>);
+  cudaFuncAttributes fg;
+  LRA_CUDA(cudaFuncGetAttributes(&fg, geqp3_df_gang_kernel<NTG>));
+  const size_t cap = (size_t)fg.maxDynamicSharedSizeBytes;
+  bool gang = qr_smem_enabled();
+  std::vector<int> G((size_t)count, 1);
+  int64_t sum_g = 0;
+  for (int64_t t = 0; t < count && gang; ++t) {
+    const DfBatchItem& it = items[ord[(size_t)t]];
+    sum_g += G[(size_t)t] = sm_min_ctas<QrArithDf>(cap, it.m, it.n);
+    gang = G[(size_t)t] > 0 && G[(size_t)t] <= std::min(16, qr_sm_cap(ctx));
+  }
+  if (gang) {
+    // a batch too small for the SMs: wider gangs
+    const int64_t wide = std::max<int64_t>(1, qr_sm_cap(ctx) / sum_g);
+    for (int64_t t = 0; t < count; ++t)
+      G[(size_t)t] = (int)std::max<int64_t>(
+          G[(size_t)t], std::min<int64_t>(G[(size_t)t] * wide, sm_natural_ctas(ctx, items[ord[(size_t)t]].n)));
+  }
+  std::vector<SmJob<QrArithDf>> sm(gang ? (size_t)count : 0);
+  size_t smem_gang = 0;
+  GridBar* bar = reinterpret_cast<GridBar*>(ctx->arena.alloc(sizeof(GridBar)));
+  LRA_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), ctx->stream));
+  ulonglong2* slots = gang ? ctx->arena.alloc_n<ulonglong2>((size_t)32 * count) : nullptr;
+  if (gang) LRA_CUDA(cudaMemsetAsync(slots, 0, (size_t)32 * count * sizeof(ulonglong2), ctx->stream));
   unsigned long long* maxbits = ctx->arena.alloc_n<unsigned long long>((size_t)count);
   LRA_CUDA(cudaMemsetAsync(maxbits, 0, (size_t)count * sizeof(unsigned long long), ctx->stream));
   int64_t nmax = 1;
@@ -2877,9 +2995,11 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
     double* scale = ctx->arena.alloc_n<double>(1);
     // row-major when every step sums its columns row by row (a thread per
     // column reads a row of the workspace coalesced), else column-major
-    const bool rowmaj = m - 1 <= ctx->tuning.qr_seq_len;
+    const bool rowmaj = !gang && m - 1 <= ctx->tuning.qr_seq_len;
     const int64_t cs = rowmaj ? 1 : m, rs = rowmaj ? n : 1;
-    prep[(size_t)t] = DfPrepJob{m, n, it.ldb, it.B, work, cs, rs, vn0, scale, maxbits + t};
+    float* Bh = gang ? reinterpret_cast<float*>(work) : nullptr;
+    float* Bl = gang ? Bh + (size_t)m * n : nullptr;
+    prep[(size_t)t] = DfPrepJob{m, n, it.ldb, it.B, work, cs, rs, vn0, scale, maxbits + t, Bh, Bl};
     QrJob& J = qr[(size_t)t];
     std::memset(&J, 0, sizeof J);
     J.P.m = m;
@@ -2902,7 +3022,22 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
     J.cs = cs;
     J.rs = rs;
     fin[(size_t)t] = DfFinishJob{m, n, it.ldb, it.B, work, cs, rs, scale, J.X.piv, J.X.nfac, it.jpvt,
-                                 ctx->arena.alloc_n<int>(n)};
+                                 ctx->arena.alloc_n<int>(n), Bh, Bl};
+    if (gang) {
+      SmJob<QrArithDf>& S = sm[(size_t)t];
+      std::memset(&S, 0, sizeof S);
+      S.P = J.P;
+      S.P.bar = bar;
+      S.P.part_d = ctx->arena.alloc_n<double>((size_t)G[(size_t)t]);
+      S.X = J.X;
+      S.D = J.D;
+      S.D.Bh = Bh;
+      S.D.Bl = Bl;
+      S.S.slot = slots + 32 * t;
+      S.S.stage = ctx->arena.alloc_n<float2>((size_t)2 * G[(size_t)t] * m);
+      S.G = G[(size_t)t];
+      smem_gang = std::max(smem_gang, sm_smem<QrArithDf>(m, (n + S.G - 1) / S.G));
+    }
     if (rowmaj) smem_tile = std::max(smem_tile, (size_t)32 * (m + 1) * sizeof(float2));
     smem_qr = std::max(smem_qr, (size_t)m * sizeof(float2) + (size_t)n * (5 * 8 + 1));
     smem_fin = std::max(smem_fin, (size_t)2 * n * sizeof(int));
@@ -2914,6 +3049,42 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
     stamps = ctx->arena.alloc_n<unsigned long long>((size_t)16 * km);
     LRA_CUDA(cudaMemsetAsync(stamps, 0, (size_t)16 * km * 8, ctx->stream));
     qr[0].D.stamps = stamps;
+    if (gang) sm[0].D.stamps = stamps;
+  }
+  // the CTAs' lists: each sketch, largest first, to the CTAs that are free first
+  std::vector<int> start;
+  std::vector<int2> list;
+  SmJob<QrArithDf>* dsm = nullptr;
+  int* dstart = nullptr;
+  int2* dlist = nullptr;
+  if (gang) {
+    const int nc = (int)std::min<int64_t>(qr_sm_cap(ctx), std::accumulate(G.begin(), G.end(), (int64_t)0));
+    std::vector<std::vector<int2>> per((size_t)nc);
+    std::vector<std::pair<double, int>> free_at((size_t)nc);
+    for (int c = 0; c < nc; ++c) free_at[(size_t)c] = {0.0, c};
+    for (int64_t t = 0; t < count; ++t) {
+      const DfBatchItem& it = items[ord[(size_t)t]];
+      const int g = G[(size_t)t];
+      std::partial_sort(free_at.begin(), free_at.begin() + g, free_at.end());
+      // a pivot: the fixed latency of its exchange and its columns' work
+      const double cost = (double)std::min(it.kmax, it.m) * (700.0 + (double)it.n / g * (1.0 + 0.02 * (double)it.m));
+      const double end = free_at[(size_t)g - 1].first + cost;
+      for (int b = 0; b < g; ++b) {
+        per[(size_t)free_at[(size_t)b].second].push_back(make_int2((int)t, b));
+        free_at[(size_t)b].first = end;
+      }
+    }
+    start.push_back(0);
+    for (const auto& v : per) {
+      list.insert(list.end(), v.begin(), v.end());
+      start.push_back((int)list.size());
+    }
+    dsm = ctx->arena.alloc_n<SmJob<QrArithDf>>((size_t)count);
+    dstart = ctx->arena.alloc_n<int>(start.size());
+    dlist = ctx->arena.alloc_n<int2>(list.size());
+    LRA_CUDA(cudaMemcpyAsync(dsm, sm.data(), sm.size() * sizeof(sm[0]), cudaMemcpyHostToDevice, ctx->stream));
+    LRA_CUDA(cudaMemcpyAsync(dstart, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    LRA_CUDA(cudaMemcpyAsync(dlist, list.data(), list.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
   }
   DfPrepJob* dprep = ctx->arena.alloc_n<DfPrepJob>((size_t)count);
   QrJob* dqr = ctx->arena.alloc_n<QrJob>((size_t)count);
@@ -2939,10 +3110,17 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
     post_launch(ctx, "df_prep_split_kernel");
   }
   if (tr) LRA_CUDA(cudaEventRecord(ev[1], ctx->stream));
-  raise_smem_limit(ctx, (const void*)geqp3_df_group_kernel<NTG>);
-  const int grid = (int)std::min<int64_t>(count, ctx->num_sms);
-  geqp3_df_group_kernel<NTG><<<grid, NTG, smem_qr, ctx->stream>>>(dqr, (int)count, next);
-  post_launch(ctx, "geqp3_df_group_kernel");
+  if (gang) {
+    void* args[] = {&dsm, &dstart, &dlist};
+    LRA_CUDA(cudaLaunchCooperativeKernel((const void*)geqp3_df_gang_kernel<NTG>, dim3((unsigned)start.size() - 1), dim3(NTG),
+                                         args, smem_gang, ctx->stream));
+    post_launch(ctx, "geqp3_df_gang_kernel");
+  } else {
+    raise_smem_limit(ctx, (const void*)geqp3_df_group_kernel<NTG>);
+    const int grid = (int)std::min<int64_t>(count, ctx->num_sms);
+    geqp3_df_group_kernel<NTG><<<grid, NTG, smem_qr, ctx->stream>>>(dqr, (int)count, next);
+    post_launch(ctx, "geqp3_df_group_kernel");
+  }
   if (tr) LRA_CUDA(cudaEventRecord(ev[2], ctx->stream));
   raise_smem_limit(ctx, (const void*)df_finish_replay_kernel);
   df_finish_replay_kernel<<<(unsigned)count, 512, smem_fin, ctx->stream>>>(dfin);
@@ -2964,11 +3142,14 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
     }
     std::fprintf(stderr, "[lra] geqp3_df_batch %lld sketches (%.1f MB, <= %lld pivots): prep %.3f ms qr %.3f ms finish %.3f ms\n",
                  (long long)count, 8e-6 * (double)mn, (long long)piv, a, b, c);
-    print_qr_trace(ctx, stamps, qr[0].P.kmax, qr[0].P.m, qr[0].P.n, "geqp3_df_group_kernel", true, nullptr, 1);
+    print_qr_trace(ctx, stamps, qr[0].P.kmax, qr[0].P.m, qr[0].P.n, gang ? "geqp3_df_gang_kernel" : "geqp3_df_group_kernel", true, nullptr, 1);
     for (auto& e : ev) cudaEventDestroy(e);
   }
   // the host copies of the job lists must outlive the asynchronous uploads
+  GridBar hb;
+  LRA_CUDA(cudaMemcpyAsync(&hb, bar, sizeof hb, cudaMemcpyDeviceToHost, ctx->stream));
   LRA_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (hb.err != 0) fail(LRA_ETIMEDOUT, "geqp3: a wait between CTAs timed out");
 }
 
 // ---- the shared-memory pivoted QR in phases ---------------------------------------
@@ -2988,7 +3169,7 @@ template <class A>
 size_t sm_smem(int64_t m, int64_t ncap) {
   using E = typename A::E;
   using V = typename A::V;
-  return (size_t)(m + ncap * m) * sizeof(E) + (size_t)ncap * (4 * sizeof(V) + sizeof(E) + 1);
+  return (size_t)(m + ncap * sm_stride(m)) * sizeof(E) + (size_t)ncap * (4 * sizeof(V) + sizeof(E) + 1);
 }
 
 template <class A>
@@ -3026,7 +3207,7 @@ int sm_min_ctas(size_t cap, int64_t m, int64_t n) {
   using E = typename A::E;
   using V = typename A::V;
   const size_t fixed = (size_t)m * sizeof(E);
-  const size_t per = (size_t)m * sizeof(E) + 4 * sizeof(V) + sizeof(E) + 1;
+  const size_t per = (size_t)sm_stride(m) * sizeof(E) + 4 * sizeof(V) + sizeof(E) + 1;
   if (cap < fixed + per) return 0;
   const int64_t ncap = (int64_t)((cap - fixed) / per);
   return (int)((n + ncap - 1) / ncap);
