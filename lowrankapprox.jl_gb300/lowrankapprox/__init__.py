@@ -14,6 +14,7 @@ Matrices are numpy arrays (host) or column-major torch CUDA tensors
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from dataclasses import dataclass
 
 import numpy as np
@@ -418,7 +419,7 @@ class _Mat:
     lin: object = None
 
 
-def _mat(A) -> _Mat:
+def _mat(A, wait=True) -> _Mat:
     if isinstance(A, LinearOperator):
         return _Mat(0, A.m, A.n, max(A.m, 1), A.c.dtype, A.np_dtype, A, A)
     if _is_torch(A):
@@ -431,14 +432,15 @@ def _mat(A) -> _Mat:
             raise ArgumentError(_ffi.LRA_EINVAL, "Float32, Float64, ComplexF32 or ComplexF64 matrix expected")
         if not A.is_cuda:
             return _mat(A.numpy())
-        # the library works on its own stream: what torch queued to make A
-        # must be done before the library reads it
-        torch.cuda.current_stream(A.device).synchronize()
         m, n = A.shape
-        if not (A.stride(0) == 1 and A.stride(1) >= max(1, m)):
+        s0, ld = A.stride()
+        if not (s0 == 1 and ld >= max(1, m)):
             A = A.t().contiguous().t()
+            ld = A.stride(1)
+        if wait:
+            _torch_wait([A])
         dt = tmap[A.dtype]
-        return _Mat(A.data_ptr(), m, n, max(A.stride(1), 1), dt, _NP_OF[dt], A)
+        return _Mat(A.data_ptr(), m, n, max(ld, 1), dt, _NP_OF[dt], A)
     A = np.asarray(A)
     if A.ndim != 2:
         raise DimensionMismatch(_ffi.LRA_EDIM, "matrix expected")
@@ -448,6 +450,16 @@ def _mat(A) -> _Mat:
     m, n = A.shape
     dt = _DT_OF[A.dtype]
     return _Mat(A.ctypes.data, m, n, max(m, 1), dt, A.dtype.type, A)
+
+
+def _torch_wait(keeps) -> None:
+    """The library works on its own stream: what torch queued to make its CUDA
+    inputs must be done before the library reads them (once a device)."""
+    devs = {A.device for A in keeps if _is_torch(A) and A.is_cuda}
+    if devs:
+        import torch
+        for dev in devs:
+            torch.cuda.current_stream(dev).synchronize()
 
 
 def _host(ptr, shape, dtype, order="F") -> np.ndarray:
@@ -475,12 +487,23 @@ class _Result:
 
 def _view(ptr, shape, dtype, owner, order="F") -> np.ndarray:
     """A numpy array on library result memory, kept alive by owner."""
-    count = int(np.prod(shape)) if len(shape) else 1
-    if count == 0 or not ptr:
-        return np.zeros(shape, dtype=dtype, order=order)
-    buf = (C.c_byte * (count * np.dtype(dtype).itemsize)).from_address(int(ptr) if not isinstance(ptr, int) else ptr)
-    buf._owner = owner
-    return np.frombuffer(buf, dtype=dtype, count=count).reshape(shape, order=order)
+    dt = _np_dtype(dtype)
+    if not ptr or 0 in shape:
+        return np.zeros(shape, dtype=dt, order=order)
+    # the array interface, which numpy reads at once and which makes the owner
+    # the array's base (a ctypes array type per size cost 7 us a view)
+    if len(shape) == 2:
+        strides = (dt.itemsize, dt.itemsize * shape[0]) if order == "F" else None
+    else:
+        strides = None
+    owner.__array_interface__ = {"version": 3, "data": (int(ptr), False), "shape": shape, "typestr": dt.str,
+                                 "strides": strides}
+    return np.asarray(owner)
+
+
+@functools.lru_cache(maxsize=None)
+def _np_dtype(t) -> np.dtype:
+    return np.dtype(t)
 
 
 def _iptr(p) -> int:
@@ -631,9 +654,10 @@ def idfact_batched(mats, opts: LRAOptions | None = None, rands=None, ctx: "Conte
     (lra_idfact_batched): their work overlaps on the device; each result is
     identical to an idfact call on that matrix."""
     ctx = ctx or default_context()
-    Ms = [_mat(A) for A in mats]
+    Ms = [_mat(A, wait=False) for A in mats]
     if not Ms:
         return []
+    _torch_wait([M.keep for M in Ms])
     if len({M.dtype for M in Ms}) != 1:
         raise ArgumentError(_ffi.LRA_EINVAL, "idfact_batched needs one element type")
     opts = opts or LRAOptions(Ms[0].np_dtype)
