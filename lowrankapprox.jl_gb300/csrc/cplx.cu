@@ -4,9 +4,8 @@
 // the pivoted QR keeps xLAQPS's pivot order, downdate and recompute trigger
 // and early block exit for ZLAQPS / CLAQPS (src/lapack.jl:117-139), its
 // reflectors are xLARFG's complex ones (beta real, tau complex), and every
-// transpose of the reference's A' is a conjugate transpose.  These are
-// straightforward SIMT kernels: the complex paths are correct and
-// complete, not tuned like the real ones.
+// transpose of the reference's A' is a conjugate transpose.  All are SIMT
+// kernels on the FP64 / FP32 units.
 
 #include <algorithm>
 #include <cfloat>
@@ -28,53 +27,106 @@ inline unsigned grid_for_c(lra_ctx* ctx, int64_t n, int t) {
 }
 
 // ---- GEMM: C = alpha op(A) op(B) + beta C, op 0 = n, 1 = t, 2 = c ------------------
+// Each entry is summed over k in order, whatever the tile.  ComplexF64: bound by
+// the FP64 units, 4 instructions of 64 cycles a term and a quarter of an SM, so
+// an entry a thread and small blocks (8 x 16 entries, a warp for each quarter),
+// which deal a sketch's few rows out evenly and pad none of them (orders are
+// 32 2^t + 8): tiles of 32 x 32 left 40 x 768 on 48 SMs.  (40 + 72 + 136) x 768,
+// K = 1024: 5.42 ms so, 1.43 now (the instructions alone: 1.25).  ComplexF32:
+// bound by shared memory, four entries a thread.
+template <typename R>
+struct CgTile;
+template <>
+struct CgTile<double> {
+  static constexpr int BM = 8, BN = 16, BK = 32, TM = 1, TN = 1;
+};
+template <>
+struct CgTile<float> {
+  static constexpr int BM = 32, BN = 32, BK = 8, TM = 2, TN = 2;
+};
+template <typename R>
+constexpr int cg_threads = (CgTile<R>::BM / CgTile<R>::TM) * (CgTile<R>::BN / CgTile<R>::TN);
+
 template <typename R, int OA, int OB>
-__global__ void __launch_bounds__(256) cgemm_kernel(int64_t M, int64_t N, int64_t K, C<R> alpha,
-                                                    const C<R>* __restrict__ A, int64_t lda,
-                                                    const C<R>* __restrict__ B, int64_t ldb, C<R> beta,
-                                                    C<R>* __restrict__ Cm, int64_t ldc) {
-  constexpr int BM = 32, BN = 32, BK = 8;
+__global__ void __launch_bounds__(cg_threads<R>) cgemm_kernel(int64_t M, int64_t N, int64_t K, C<R> alpha,
+                                                              const C<R>* __restrict__ A, int64_t lda,
+                                                              const C<R>* __restrict__ B, int64_t ldb, C<R> beta,
+                                                              C<R>* __restrict__ Cm, int64_t ldc) {
+  using T = CgTile<R>;
+  constexpr int BM = T::BM, BN = T::BN, BK = T::BK, TM = T::TM, TN = T::TN, NT = cg_threads<R>;
+  constexpr int NX = BN / TN, NY = BM / TM, LA = BM * BK / NT, LB = BN * BK / NT;
   __shared__ C<R> As[BK][BM + 1];
   __shared__ C<R> Bs[BK][BN + 1];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  const int tid = threadIdx.x, tx = tid % NX, ty = tid / NX;
   const int64_t tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
   const bool zero_beta = beta.re == R(0) && beta.im == R(0);
   for (int64_t tile = blockIdx.x; tile < tiles_m * tiles_n; tile += gridDim.x) {
     const int64_t m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
-    C<R> acc[2][2] = {{C<R>(0), C<R>(0)}, {C<R>(0), C<R>(0)}};
-    for (int64_t k0 = 0; k0 < K; k0 += BK) {
-      {
-        const int i = tid % BM, k = tid / BM;
+    C<R> acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] = C<R>(0);
+    // the next slab of k waits in registers
+    C<R> ra[LA], rb[LB];
+    auto load = [&](int64_t k0) {
+#pragma unroll
+      for (int q = 0; q < LA; ++q) {
+        const int t = tid + q * NT, i = OA == 0 ? t % BM : t / BK, k = OA == 0 ? t / BM : t % BK;
         const int64_t gi = m0 + i, gk = k0 + k;
         C<R> v(0);
         if (gi < M && gk < K) v = OA == 0 ? A[gi + gk * lda] : A[gk + gi * lda];
-        if (OA == 2) v = conj(v);
-        As[k][i] = v;
+        ra[q] = OA == 2 ? conj(v) : v;
       }
-      {
-        const int k = tid % BK, j = tid / BK;
+#pragma unroll
+      for (int q = 0; q < LB; ++q) {
+        const int t = tid + q * NT, j = OB == 0 ? t / BK : t % BN, k = OB == 0 ? t % BK : t / BN;
         const int64_t gj = n0 + j, gk = k0 + k;
         C<R> v(0);
         if (gj < N && gk < K) v = OB == 0 ? B[gk + gj * ldb] : B[gj + gk * ldb];
-        if (OB == 2) v = conj(v);
-        Bs[k][j] = v;
+        rb[q] = OB == 2 ? conj(v) : v;
+      }
+    };
+    load(0);
+    for (int64_t k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+      for (int q = 0; q < LA; ++q) {
+        const int t = tid + q * NT;
+        As[OA == 0 ? t / BM : t % BK][OA == 0 ? t % BM : t / BK] = ra[q];
+      }
+#pragma unroll
+      for (int q = 0; q < LB; ++q) {
+        const int t = tid + q * NT;
+        Bs[OB == 0 ? t % BK : t / BN][OB == 0 ? t / BK : t % BN] = rb[q];
       }
       __syncthreads();
+      if (k0 + BK < K) load(k0 + BK);
 #pragma unroll
       for (int kk = 0; kk < BK; ++kk) {
-        const C<R> a0 = As[kk][ty], a1 = As[kk][ty + 16], b0 = Bs[kk][tx], b1 = Bs[kk][tx + 16];
-        acc[0][0] += a0 * b0;
-        acc[0][1] += a0 * b1;
-        acc[1][0] += a1 * b0;
-        acc[1][1] += a1 * b1;
+        C<R> a[TM], b[TN];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) a[i] = As[kk][ty + NY * i];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx + NX * j];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) {
+            if constexpr (sizeof(R) == 8) {
+              acc[i][j].re = fma(a[i].re, b[j].re, fma(-a[i].im, b[j].im, acc[i][j].re));
+              acc[i][j].im = fma(a[i].re, b[j].im, fma(a[i].im, b[j].re, acc[i][j].im));
+            } else {
+              acc[i][j] += a[i] * b[j];
+            }
+          }
       }
       __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int64_t gi = m0 + ty + 16 * i, gj = n0 + tx + 16 * j;
+      for (int j = 0; j < TN; ++j) {
+        const int64_t gi = m0 + ty + NY * i, gj = n0 + tx + NX * j;
         if (gi < M && gj < N) {
           C<R>* c = Cm + gi + gj * ldc;
           *c = zero_beta ? alpha * acc[i][j] : alpha * acc[i][j] + beta * *c;
@@ -751,11 +803,11 @@ void cgemm(lra_ctx* ctx, char ta, char tb, int64_t m, int64_t n, int64_t k, cx<R
            int64_t lda, const cx<R>* B, int64_t ldb, cx<R> beta, cx<R>* Cm, int64_t ldc) {
   if (m <= 0 || n <= 0) return;
   const int oa = ta == 'n' ? 0 : (ta == 't' ? 1 : 2), ob = tb == 'n' ? 0 : (tb == 't' ? 1 : 2);
-  const int64_t tiles = ((m + 31) / 32) * ((n + 31) / 32);
+  const int64_t tiles = ((m + CgTile<R>::BM - 1) / CgTile<R>::BM) * ((n + CgTile<R>::BN - 1) / CgTile<R>::BN);
   const unsigned g = (unsigned)std::min<int64_t>(tiles, (int64_t)ctx->num_sms * 8);
 #define CG(OA, OB)                                                                                             \
   if (oa == OA && ob == OB) {                                                                                  \
-    cgemm_kernel<R, OA, OB><<<g, 256, 0, ctx->stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, Cm, ldc);        \
+    cgemm_kernel<R, OA, OB><<<g, cg_threads<R>, 0, ctx->stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, Cm, ldc); \
     post_launch(ctx, "cgemm_kernel");                                                                          \
     return;                                                                                                    \
   }
