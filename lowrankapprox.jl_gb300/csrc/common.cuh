@@ -126,6 +126,32 @@ __device__ T block_max(T v, T* red) {
   return r;
 }
 
+// 16-byte words in global memory, read and written at once (sm_90 on)
+__device__ __forceinline__ void st_word(ulonglong2* p, unsigned long long x, unsigned long long y) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.release.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
+               : "memory");
+}
+__device__ __forceinline__ void st_word_relaxed(ulonglong2* p, unsigned long long x, unsigned long long y) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
+               : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_word_acquire(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("{\n .reg .b128 t;\n ld.acquire.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(v.x), "=l"(v.y)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ ulonglong2 ld_word(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(v.x), "=l"(v.y)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+
 // Grid barrier for cooperative launches (all CTAs co-resident).  The wait
 // is bounded: on time-out it records LRA_ETIMEDOUT (4) in `err` and every
 // CTA leaves; callers return when it yields false.

@@ -451,6 +451,379 @@ __global__ void __launch_bounds__(NT) cgeqp3_kernel(CQrParams<R> P) {
   if (b == 0 && threadIdx.x == 0) *P.k_out = kres;
 }
 
+// ---- the same with the columns in shared memory ---------------------------------
+//
+// Bound: FP64 latency and the exchange.  A block holds its columns in shared
+// memory for the whole factorization; columns never move, their positions do.
+// Each block stages its candidate beside the word that offers it, so a pivot costs
+// one trip through L2 (the general kernel: two grid barriers, one thread that
+// reads all partials, and the swap).  The reflector is scaled once a block,
+// and the norm downdates, whose divides and roots cost a warp as much for
+// one column as for 32, are done a lane per column.  The operations of each
+// column are the general kernel's, in its order: same bits.  ComplexF64,
+// n = 768, orders 40, 72 and 136, 211 pivots: 7.18 -> 2.83 ms.
+template <typename R>
+struct CQrBits;
+template <>
+struct CQrBits<double> {
+  // a norm as an integer of the same order, -1 for a NaN
+  static __device__ long long key(double v) {
+    const long long k = __double_as_longlong(v) & 0x7fffffffffffffffll;
+    return k > 0x7ff0000000000000ll ? -1 : k;
+  }
+  static __device__ double value(long long k) { return __longlong_as_double(k); }
+  // the leading bits of |v|, their exponent, whether its square and root are safe
+  static __device__ unsigned lead(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+  static __device__ int expo(unsigned h) { return (int)(h >> 20) - 1023; }
+  static __device__ bool safe(unsigned h) { return h >= (123u << 20) && h < (1923u << 20); }
+  static __device__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+};
+template <>
+struct CQrBits<float> {
+  static __device__ long long key(float v) {
+    const unsigned k = __float_as_uint(v) & 0x7fffffffu;
+    return k > 0x7f800000u ? -1 : (long long)k;
+  }
+  static __device__ float value(long long k) { return __uint_as_float((unsigned)k); }
+  static __device__ unsigned lead(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+  static __device__ int expo(unsigned h) { return (int)(h >> 23) - 127; }
+  static __device__ bool safe(unsigned h) { return h >= (27u << 23) && h < (227u << 23); }
+  static __device__ float pow2(int e) { return __int_as_float((e + 127) << 23); }
+};
+
+// block_cnrm2's sum in its order, the largest component by its exponent; the
+// result in warp 0 (elsewhere undefined).  `big` and `red`: NT / 32 entries each.
+template <typename R, int NT>
+__device__ __forceinline__ R block_cnrm2_bits(const C<R>* x, int len, unsigned* big, R* red) {
+  using B = CQrBits<R>;
+  constexpr int NW = NT / 32;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned h = 0;
+  for (int i = threadIdx.x; i < len; i += NT) h = max(h, max(B::lead(x[i].re), B::lead(x[i].im)));
+  h = __reduce_max_sync(0xffffffffu, h);
+  if (lane == 0) big[wid] = h;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < NW; ++w) h = max(h, big[w]);
+  if (!B::safe(h)) return len > 0 ? block_cnrm2(x, (int64_t)len, red) : R(0);
+  const int e = B::expo(h);
+  const R sc = B::pow2(-e);
+  R s = 0;
+  for (int i = threadIdx.x; i < len; i += NT) {
+    const R a = x[i].re * sc, b = x[i].im * sc;
+    s += fma(a, a, b * b);
+  }
+  s = warp_sum(s);
+  if (lane == 0) red[wid] = s;
+  __syncthreads();
+  if (wid != 0) return R(0);
+  s = lane < NW ? red[lane] : R(0);
+#pragma unroll
+  for (int o = NW / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return sqrt(__shfl_sync(0xffffffffu, s, 0)) * B::pow2(e);
+}
+
+// clarfg by a warp: divides that don't wait for one another are one instruction
+// stream of several lanes (with the norm on bits and one polling warp: 3.49 -> 2.83 ms)
+template <typename R>
+__device__ __forceinline__ void clarfg_warp(C<R> alpha, R xnorm, C<R>& tau, R& beta, C<R>& scal) {
+  const int lane = threadIdx.x & 31;
+  const R safmin = Real<R>::safmin / Real<R>::eps;
+  const R ax = fabs(alpha.re), ay = fabs(alpha.im), w = fmax(ax, fmax(ay, xnorm));
+  const R q = (lane == 0 ? ax : lane == 1 ? ay : xnorm) / w;
+  const R qa = __shfl_sync(0xffffffffu, q, 0), qb = __shfl_sync(0xffffffffu, q, 1), qc = __shfl_sync(0xffffffffu, q, 2);
+  beta = -copysign(w * sqrt(fma(qc, qc, fma(qa, qa, qb * qb))), alpha.re);
+  if ((xnorm == R(0) && alpha.im == R(0)) || !(fabs(beta) >= safmin) || !(fabs(beta) <= Real<R>::big)) {
+    clarfg(alpha, xnorm, tau, beta, scal);
+    return;
+  }
+  const R br = alpha.re - beta, bi = alpha.im;
+  const bool up = fabs(br) >= fabs(bi);  // cdiv's two cases, for 1 / (br, bi)
+  const R t = (lane == 0 ? beta - alpha.re : lane == 1 ? -bi : up ? bi : br) / (lane < 2 ? beta : up ? br : bi);
+  tau = C<R>(__shfl_sync(0xffffffffu, t, 0), __shfl_sync(0xffffffffu, t, 1));
+  const R r = __shfl_sync(0xffffffffu, t, 2);
+  const R d = up ? fma(bi, r, br) : fma(br, r, bi);
+  const R u = (up ? (lane == 0 ? R(1) : R(0) - r) : (lane == 0 ? r + R(0) : R(-1))) / d;
+  scal = C<R>(__shfl_sync(0xffffffffu, u, 0), __shfl_sync(0xffffffffu, u, 1));
+}
+
+// warp_sum of both parts: the first step leaves each half a warp one of them
+template <typename R>
+__device__ __forceinline__ C<R> warp_csum(C<R> w) {
+  const bool lo = (threadIdx.x & 16) == 0;
+  R s = lo ? w.re : w.im;
+  s += __shfl_xor_sync(0xffffffffu, lo ? w.im : w.re, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return C<R>(__shfl_sync(0xffffffffu, s, 0), __shfl_sync(0xffffffffu, s, 16));
+}
+
+template <typename R>
+constexpr size_t cqr_smem(int64_t m, int64_t nc) {  // nc columns a block
+  return (size_t)(nc * m + 2 * m) * sizeof(C<R>) + (size_t)nc * (2 * sizeof(R) + sizeof(int)) + 16;
+}
+
+// Complex products with the fused term written out, so that no surrounding code
+// decides which of the two is fused: as the general kernel has them.
+template <typename R>
+__device__ __forceinline__ C<R> cmul_fixed(C<R> a, C<R> b) {
+  return {fma(a.re, b.re, -(a.im * b.im)), fma(a.re, b.im, a.im * b.re)};
+}
+template <typename R>
+__device__ __forceinline__ C<R> cmul_fixed_scal(C<R> a, C<R> b) {
+  return {fma(a.re, b.re, -(a.im * b.im)), fma(a.im, b.re, a.re * b.im)};
+}
+template <typename R>
+__device__ __forceinline__ C<R> cmulc_fixed(C<R> a, C<R> b) {
+  return {fma(a.re, b.re, a.im * b.im), fma(a.re, b.im, -(a.im * b.re))};
+}
+
+template <typename R, int NT>
+__global__ void __launch_bounds__(NT, 1) cgeqp3_smem_kernel(CQrParams<R> P, ulonglong2* word, C<R>* stage) {
+  constexpr int NW = NT / 32;
+  using Bits = CQrBits<R>;
+  constexpr int PW = 256 / 32;  // words a lane of the polling warp
+  extern __shared__ __align__(16) unsigned char cq_smem[];
+  __shared__ R s_red[32];
+  __shared__ unsigned s_big[NW];
+  __shared__ long long s_key;
+  __shared__ int64_t s_pos;
+  __shared__ int s_q, s_owner, s_any, s_bad;
+  __shared__ C<R> s_tau, s_scal;
+  __shared__ R s_beta;
+  const int G = gridDim.x, b = blockIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t n = P.n, lda = P.lda;
+  const int m = (int)P.m;
+  const int64_t c0 = n * b / G;
+  const int nc = (int)((n + G - 1) / G), nloc = (int)(n * (b + 1) / G - c0);
+  const int64_t lastrk = m < n ? m : n;
+  const R tol3z = sqrt(Real<R>::eps);
+  C<R>* cols = reinterpret_cast<C<R>*>(cq_smem);  // [nc][m]
+  C<R>* sx = cols + (size_t)nc * m;               // the pivot column
+  C<R>* sv = sx + m;                              // the reflector
+  R* vn1 = reinterpret_cast<R*>(sv + m);
+  R* vn2 = vn1 + nc;
+  int* pos = reinterpret_cast<int*>(vn2 + nc);  // position, its complement once done or (between) flagged
+
+  for (int q = wid; q < nloc; q += NW) {
+    C<R>* a = cols + (size_t)q * m;
+    for (int i = lane; i < m; i += 32) a[i] = P.A[i + (c0 + q) * lda];
+    __syncwarp();
+    const R v = warp_cnrm2(a, (int64_t)m, lane);
+    if (lane == 0) {
+      vn1[q] = vn2[q] = v;
+      pos[q] = (int)(c0 + q);
+    }
+  }
+
+  // exchange e: the block's best column among the positions from `from` on
+  // (`only`: that position, whatever its norm) and its flag; then the best of all
+  int64_t pvt = n;
+  int owner = 0, anyflag = 0;
+  long long topkey = -1;
+  auto exchange = [&](int e, int from, bool only, int flag) -> bool {
+    __syncthreads();
+    if (wid == 0) {
+      long long v = -1;
+      int64_t i = n << 24;
+      for (int q = lane; q < nloc; q += 32)
+        if (pos[q] >= from && (!only || pos[q] == from))
+          argmax_merge<long long>(v, i, only ? 0 : Bits::key(vn1[q]), (int64_t)pos[q] << 24 | q);
+      warp_argmax(v, i);
+      if (lane == 0) {
+        s_q = v >= 0 ? (int)(i & 0xffffff) : -1;
+        s_key = v;
+        s_pos = v >= 0 ? i >> 24 : n;
+      }
+    }
+    __syncthreads();
+    C<R>* st = stage + ((size_t)(e & 1) * G + b) * m;
+    if (s_q >= 0) {
+      const C<R>* a = cols + (size_t)s_q * m;
+      for (int i = from + threadIdx.x; i < m; i += NT) st[i] = a[i];
+    }
+    __syncthreads();
+    if (wid == 0) {
+      ulonglong2* const wd = word + (size_t)(e & 1) * G;
+      if (lane == 0)
+        st_word(wd + b, (unsigned long long)s_key,
+                (unsigned long long)(e + 1) << 33 | (unsigned long long)s_pos << 1 | (unsigned long long)flag);
+      ulonglong2 w[PW];
+      uint64_t t0 = 0;
+      bool bad = false;
+      for (int it = 1;; ++it) {
+        bool all = true;
+#pragma unroll
+        for (int k = 0; k < PW; ++k)
+          if (k * 32 + lane < G) w[k] = ld_word(wd + k * 32 + lane);
+#pragma unroll
+        for (int k = 0; k < PW; ++k)
+          if (k * 32 + lane < G) all &= (w[k].y >> 33) == (unsigned long long)(e + 1);
+        if (__all_sync(0xffffffffu, all)) break;
+        if ((it & 63) == 0) {
+          const uint64_t t = globaltimer_ns();
+          if (t0 == 0) t0 = t;
+          if (t - t0 > wait_limit_ns()) atomicCAS(&P.bar->err, 0, 4);
+          bad = __any_sync(0xffffffffu, *((volatile int*)&P.bar->err) != 0);
+          if (bad) break;
+        }
+      }
+      __threadfence();
+      long long v = -1;
+      int64_t i = n << 16;
+      bool fl = false;
+#pragma unroll
+      for (int k = 0; k < PW; ++k)
+        if (k * 32 + lane < G) {
+          fl |= (w[k].y & 1) != 0;
+          argmax_merge<long long>(v, i, (long long)w[k].x, (int64_t)((w[k].y >> 1) & 0xffffffffull) << 16 | (k * 32 + lane));
+        }
+      warp_argmax(v, i);
+      fl = __any_sync(0xffffffffu, fl);
+      if (lane == 0) {
+        s_key = v;
+        s_pos = v >= 0 ? i >> 16 : n;
+        s_owner = (int)(i & 0xffff);
+        s_any = fl;
+        s_bad = bad;
+      }
+    }
+    __syncthreads();
+    topkey = s_key;
+    pvt = s_pos;
+    owner = s_owner;
+    anyflag = s_any;
+    return s_bad == 0;
+  };
+
+  int e = 0;
+  if (!exchange(e, 0, false, 0)) return;
+  const R maxnrm = topkey >= 0 ? Bits::value(topkey) : R(0);
+  const R ptol = (R)fmax(P.atol, P.rtol * (double)maxnrm);
+  int64_t kres = P.kmax;
+  int c = 0;
+  while (c < P.kmax) {
+    const int64_t jb = min(P.nb, P.kmax - c);
+    int64_t kk = 0, first_small = -1;
+    bool last_small = false, block_end = false;
+    while (kk < jb && !block_end) {
+      if (pvt >= n) {  // no norm is a number: the column at c, as it is
+        ++e;
+        if (!exchange(e, c, true, 0)) return;
+      }
+      {
+        const C<R>* st = stage + ((size_t)(e & 1) * G + owner) * m;
+        for (int i = c + threadIdx.x; i < m; i += NT) {
+          if constexpr (sizeof(R) == 8) {
+            const double2 t = __ldcg(reinterpret_cast<const double2*>(st + i));
+            sx[i] = C<R>(t.x, t.y);
+          } else {
+            const float2 t = __ldcg(reinterpret_cast<const float2*>(st + i));
+            sx[i] = C<R>(t.x, t.y);
+          }
+        }
+      }
+      __syncthreads();
+      const R xnorm = block_cnrm2_bits<R, NT>(sx + c + 1, m - c - 1, s_big, s_red);
+      if (wid == 0) {
+        C<R> t, sc;
+        R bt;
+        clarfg_warp(sx[c], xnorm, t, bt, sc);
+        if (lane == 0) {
+          s_tau = t;
+          s_scal = sc;
+          s_beta = bt;
+          if (b == 0) P.tau[c] = t;
+        }
+      }
+      __syncthreads();
+      const C<R> tau = s_tau, scal = s_scal;
+      const C<R> ctau = conj(tau);
+      const R beta = s_beta;
+      for (int i = c + 1 + threadIdx.x; i < m; i += NT) sv[i] = cmul_fixed_scal(scal, sx[i]);
+      // positions: the pivot's column is done, the one at c takes its place
+      for (int q = threadIdx.x; q < nloc; q += NT) {
+        const int p = pos[q];
+        if (p == pvt)
+          pos[q] = ~c;
+        else if (p == c)
+          pos[q] = (int)pvt;
+      }
+      __syncthreads();
+      for (int q = wid; q < nloc; q += NW) {
+        C<R>* a = cols + (size_t)q * m;
+        const int p = pos[q];
+        if (p == ~c) {  // beta and v in the column's place
+          for (int i = c + 1 + lane; i < m; i += 32) a[i] = sv[i];
+          if (lane == 0) a[c] = C<R>(beta, R(0));
+        }
+        if (p < 0) continue;
+        if (tau.re != R(0) || tau.im != R(0)) {
+          C<R> w(0);
+          for (int i = c + 1 + lane; i < m; i += 32) w += cmulc_fixed(sv[i], a[i]);
+          w = warp_csum(w);
+          w += a[c];
+          __syncwarp();
+          const C<R> f = cmul_fixed(ctau, w);
+          for (int i = c + 1 + lane; i < m; i += 32) a[i] -= cmul_fixed(f, sv[i]);
+          if (lane == 0) a[c] -= f;
+        }
+      }
+      __syncthreads();
+      int flag = 0;
+      if (c < lastrk - 1) {
+        for (int q0 = 0; q0 < nloc; q0 += NT) {
+          const int q = q0 + threadIdx.x;
+          bool recompute = false;
+          if (q < nloc && pos[q] >= 0) {
+            const R v1 = vn1[q];
+            if (v1 != R(0)) {
+              R temp = cabs(cols[(size_t)q * m + c]) / v1;
+              temp = fmax(R(0), (R(1) + temp) * (R(1) - temp));
+              const R r = v1 / vn2[q];
+              const R temp2 = temp * r * r;
+              if (temp2 <= tol3z)
+                recompute = true;
+              else
+                vn1[q] = v1 * sqrt(temp);
+            }
+          }
+          if (recompute) vn2[q] = R(-1);  // to be recomputed
+          flag |= __syncthreads_or(recompute);
+        }
+        if (flag) {
+          for (int q = wid; q < nloc; q += NW) {
+            if (pos[q] < 0 || vn2[q] != R(-1)) continue;
+            const R nr = warp_cnrm2(cols + (size_t)q * m + c + 1, (int64_t)m - c - 1, lane);
+            if (lane == 0) vn1[q] = vn2[q] = nr;
+          }
+        }
+      }
+      const bool small = fabs(beta) <= ptol;
+      if (small && first_small < 0) first_small = c;
+      last_small = small;
+      ++c;
+      ++kk;
+      ++e;
+      if (!exchange(e, c, false, flag ? 1 : 0)) return;
+      block_end = anyflag != 0;
+    }
+    if (last_small) {
+      kres = first_small;
+      break;
+    }
+  }
+  __syncthreads();
+  for (int q = wid; q < nloc; q += NW) {
+    const int p = pos[q] < 0 ? ~pos[q] : pos[q];
+    const C<R>* a = cols + (size_t)q * m;
+    for (int i = lane; i < m; i += 32) P.A[i + p * lda] = a[i];
+    if (lane == 0) P.jpvt[p] = c0 + q + 1;
+  }
+  if (b == 0 && threadIdx.x == 0) *P.k_out = kres;
+}
+
 // ---- Householder application, a warp per column of X ------------------------------
 // trans 0: X <- Q X = H_0 H_1 ... H_{k-1} X; trans 1: X <- Q^H X
 template <typename R>
@@ -878,10 +1251,32 @@ int64_t cgeqp3(lra_ctx* ctx, int64_t m, int64_t n, cx<R>* A, int64_t lda, int64_
     return 0;
   }
   if (!pivot) P.jpvt = ctx->arena.alloc_n<int64_t>(n);
-  void* args[] = {&P};
-  LRA_CUDA(cudaLaunchCooperativeKernel((const void*)cgeqp3_kernel<R, NT>, dim3(grid), dim3(NT), args, 0,
-                                       ctx->stream));
-  post_launch(ctx, "cgeqp3_kernel");
+  // the columns in shared memory where they fit: a warp's worth each at first
+  // (two a quarter of an SM, which costs the FP64 units no more than fewer
+  // would), over all SMs if that is too much for a block
+  const void* smk = (const void*)cgeqp3_smem_kernel<R, NT>;
+  cudaFuncAttributes fa;
+  LRA_CUDA(cudaFuncGetAttributes(&fa, smk));
+  int optin = 0;
+  LRA_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  const size_t cap = (size_t)optin - fa.sharedSizeBytes;
+  int G = std::min(grid, 256);
+  if (cqr_smem<R>(m, (n + G - 1) / G) > cap) G = (int)std::min<int64_t>(std::min(ctx->num_sms, 256), n);
+  const size_t smem = cqr_smem<R>(m, (n + G - 1) / G);
+  if (pivot && qr_smem_enabled() && m < (1 << 24) && n < (1 << 24) && smem <= cap) {
+    raise_smem_limit(ctx, smk);
+    ulonglong2* word = ctx->arena.alloc_n<ulonglong2>((size_t)2 * G);
+    cx<R>* stage = ctx->arena.alloc_n<cx<R>>((size_t)2 * G * m);
+    LRA_CUDA(cudaMemsetAsync(word, 0, (size_t)2 * G * sizeof(ulonglong2), ctx->stream));
+    void* args[] = {&P, &word, &stage};
+    LRA_CUDA(cudaLaunchCooperativeKernel(smk, dim3(G), dim3(NT), args, smem, ctx->stream));
+    post_launch(ctx, "cgeqp3_smem_kernel");
+  } else {
+    void* args[] = {&P};
+    LRA_CUDA(cudaLaunchCooperativeKernel((const void*)cgeqp3_kernel<R, NT>, dim3(grid), dim3(NT), args, 0,
+                                         ctx->stream));
+    post_launch(ctx, "cgeqp3_kernel");
+  }
   int64_t k = 0;
   GridBar hb;
   LRA_CUDA(cudaMemcpyAsync(&k, P.k_out, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));

@@ -183,6 +183,9 @@ void tc_sketch_batch(lra_ctx* ctx, int64_t count, const SketchItem* items, int64
 // host thread could undercut another thread's launch in between.
 void raise_smem_limit(lra_ctx* ctx, const void* kernel);
 
+// whether pivoted QRs may hold their columns in shared memory (LRA_QR_SMEM)
+bool qr_smem_enabled();
+
 // LRA_TRACE=1 in the environment: iteration counts of the iterative
 // kernels (Jacobi sweeps, pivots) on stderr.
 bool trace_on();

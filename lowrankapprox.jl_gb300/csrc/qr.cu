@@ -906,31 +906,6 @@ struct QrXw {
   float* prev;       // PG: [G][2][m] the previous reflector, each CTA its own
 };
 
-__device__ __forceinline__ void st_word(ulonglong2* p, unsigned long long x, unsigned long long y) {
-  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.release.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
-               : "memory");
-}
-__device__ __forceinline__ void st_word_relaxed(ulonglong2* p, unsigned long long x, unsigned long long y) {
-  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
-               : "memory");
-}
-__device__ __forceinline__ ulonglong2 ld_word_acquire(const ulonglong2* p) {
-  ulonglong2 v;
-  asm volatile("{\n .reg .b128 t;\n ld.acquire.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
-               : "=l"(v.x), "=l"(v.y)
-               : "l"(p)
-               : "memory");
-  return v;
-}
-__device__ __forceinline__ ulonglong2 ld_word(const ulonglong2* p) {
-  ulonglong2 v;
-  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
-               : "=l"(v.x), "=l"(v.y)
-               : "l"(p)
-               : "memory");
-  return v;
-}
-
 // PG: the previous reflector in global memory (sketches of more rows than two
 // reflectors fit shared memory)
 template <int NT, bool PG>
@@ -2834,7 +2809,7 @@ __global__ void col_norms_kernel(int64_t m, int64_t n, const T* __restrict__ A, 
 
 // LRA_QR_SMEM=0 keeps the double-float QR's columns in global memory
 // even where they would fit shared memory (both variants stay testable)
-static bool qr_smem_enabled() {
+bool qr_smem_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("LRA_QR_SMEM");
     return !(e && *e == '0');
