@@ -1,7 +1,7 @@
 // Column-major GEMM on CUDA cores, C = alpha op(A) op(B) + beta C, for the
-// input-precision ("native") path.  On GB300 the FP64 rate is the bound of
-// this kernel, which a register-tiled SIMT kernel reaches comfortably; the
-// split-precision tensor-core path lives in tc_sketch.cu.
+// input-precision ("native") path; the split-precision tensor-core path lives
+// in tc_sketch.cu.  An entry is summed over k in order whatever the tile, so
+// the tiles can follow the shape without a change of bits.
 
 #include <algorithm>
 
@@ -12,16 +12,29 @@ namespace lra {
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
-constexpr int NT = (BM / TM) * (BN / TN);  // 256
+// FP64: bound by the FP64 units, 64 cycles a warp instruction and quarter of an
+// SM, so one entry a thread and small blocks, a warp for each quarter, which
+// spread any shape evenly: 213 x 213 x 213 took 190 us on the 16 SMs that 64 x 64
+// tiles gave it, 20 us now; (40 + 72 + 136) x 1501, K = 2001: 2.71 ms, 1.26 ms now
+// (FP64 rate alone 1.3).  FP32: 16 entries a thread, 4 where the large tiles
+// would leave SMs idle (the 49 updates of a psvd of rank 370: 742 us, 433 us now).
+template <int BM_, int BN_, int BK_, int TM_, int TN_>
+struct Tile {
+  static constexpr int BM = BM_, BN = BN_, BK = BK_, TM = TM_, TN = TN_;
+  static constexpr int NT = (BM / TM) * (BN / TN);
+};
+using TileF64 = Tile<8, 16, 32, 1, 1>;
+using TileF32 = Tile<64, 64, 16, 4, 4>;
+using TileF32s = Tile<32, 32, 16, 2, 2>;
 
 // blockIdx.y selects a K slice of length kchunk; with gridDim.y > 1 each
 // slice writes its own partial product to C + y * ldc * N (split-K)
-template <typename T, bool TA, bool TB>
-__global__ void __launch_bounds__(NT) gemm_kernel(int64_t M, int64_t N, int64_t K, T alpha,
+template <typename T, typename Cfg, bool TA, bool TB>
+__global__ void __launch_bounds__(Cfg::NT) gemm_kernel(int64_t M, int64_t N, int64_t K, T alpha,
                                                   const T* __restrict__ A, int64_t lda,
                                                   const T* __restrict__ B, int64_t ldb, T beta,
                                                   T* __restrict__ C, int64_t ldc, int64_t kchunk) {
+  constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TM = Cfg::TM, TN = Cfg::TN, NT = Cfg::NT;
   {
     const int64_t k0 = (int64_t)blockIdx.y * kchunk;
     if (k0 >= K) return;
@@ -171,6 +184,17 @@ __global__ void scale_kernel(int64_t m, int64_t n, T beta, T* C, int64_t ldc) {
 
 }  // namespace
 
+template <typename T, typename Cfg>
+static void gemm_tiles(lra_ctx* ctx, bool TA, bool TB, int64_t nsplit, int64_t m, int64_t n, int64_t k, T alpha, const T* A,
+                       int64_t lda, const T* B, int64_t ldb, T beta, T* C, int64_t ldc, int64_t kchunk) {
+  const int64_t tiles = ((m + Cfg::BM - 1) / Cfg::BM) * ((n + Cfg::BN - 1) / Cfg::BN);
+  const dim3 grid((unsigned)std::min<int64_t>(tiles, (int64_t)ctx->num_sms * (Cfg::NT < 256 ? 16 : 4)), (unsigned)nsplit);
+  auto* f = TA ? (TB ? gemm_kernel<T, Cfg, true, true> : gemm_kernel<T, Cfg, true, false>)
+               : (TB ? gemm_kernel<T, Cfg, false, true> : gemm_kernel<T, Cfg, false, false>);
+  f<<<grid, Cfg::NT, 0, ctx->stream>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, kchunk);
+  post_launch(ctx, "gemm_kernel");
+}
+
 template <typename T>
 void gemm(lra_ctx* ctx, char ta, char tb, int64_t m, int64_t n, int64_t k, T alpha, const T* A,
           int64_t lda, const T* B, int64_t ldb, T beta, T* C, int64_t ldc) {
@@ -189,9 +213,9 @@ void gemm(lra_ctx* ctx, char ta, char tb, int64_t m, int64_t n, int64_t k, T alp
   }
   const bool TA = (ta == 't' || ta == 'T' || ta == 'c' || ta == 'C');
   const bool TB = (tb == 't' || tb == 'T' || tb == 'c' || tb == 'C');
-  const int64_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
-  const unsigned g = (unsigned)std::min<int64_t>(tiles, (int64_t)ctx->num_sms * 4);
-  // split K when the tiles alone leave most SMs idle
+  // split K when tiles of 64 x 64 would leave most SMs idle (a rule that the sums'
+  // order, not the speed of the tiles above, holds fast)
+  const int64_t tiles = ((m + 63) / 64) * ((n + 63) / 64);
   int64_t nsplit = 1;
   if (tiles < ctx->num_sms && k >= 1024)
     nsplit = std::min<int64_t>((2 * ctx->num_sms + tiles - 1) / tiles, k / 256);
@@ -207,24 +231,18 @@ void gemm(lra_ctx* ctx, char ta, char tb, int64_t m, int64_t n, int64_t k, T alp
     al = T(1);
     be = T(0);
   }
-  const dim3 grid(g, (unsigned)nsplit);
-  if (!TA && !TB)
-    gemm_kernel<T, false, false><<<grid, NT, 0, ctx->stream>>>(m, n, k, al, A, lda, B, ldb, be, out, ldo, kchunk);
-  else if (TA && !TB)
-    gemm_kernel<T, true, false><<<grid, NT, 0, ctx->stream>>>(m, n, k, al, A, lda, B, ldb, be, out, ldo, kchunk);
-  else if (!TA && TB)
-    gemm_kernel<T, false, true><<<grid, NT, 0, ctx->stream>>>(m, n, k, al, A, lda, B, ldb, be, out, ldo, kchunk);
+  if constexpr (sizeof(T) == 8)
+    gemm_tiles<T, TileF64>(ctx, TA, TB, nsplit, m, n, k, al, A, lda, B, ldb, be, out, ldo, kchunk);
+  else if (tiles * nsplit < ctx->num_sms)
+    gemm_tiles<T, TileF32s>(ctx, TA, TB, nsplit, m, n, k, al, A, lda, B, ldb, be, out, ldo, kchunk);
   else
-    gemm_kernel<T, true, true><<<grid, NT, 0, ctx->stream>>>(m, n, k, al, A, lda, B, ldb, be, out, ldo, kchunk);
+    gemm_tiles<T, TileF32>(ctx, TA, TB, nsplit, m, n, k, al, A, lda, B, ldb, be, out, ldo, kchunk);
   if (nsplit > 1) {
-    post_launch(ctx, "gemm_kernel");
     const unsigned gr = (unsigned)std::max<int64_t>(1, std::min<int64_t>((m * n + 255) / 256, ctx->num_sms * 8));
     splitk_reduce_kernel<T><<<gr, 256, 0, ctx->stream>>>(m, n, nsplit, out, alpha, beta, C, ldc);
     ctx->arena.release(mk);  // stream-ordered reuse
     post_launch(ctx, "splitk_reduce_kernel");
-    return;
   }
-  post_launch(ctx, "gemm_kernel");
 }
 
 template void gemm<float>(lra_ctx*, char, char, int64_t, int64_t, int64_t, float, const float*, int64_t,
