@@ -14,6 +14,7 @@
 #include "common.cuh"
 #include "cplx.cuh"
 #include "internal.hpp"
+#include "qr_cols.cuh"
 
 namespace lra {
 
@@ -462,40 +463,11 @@ __global__ void __launch_bounds__(NT) cgeqp3_kernel(CQrParams<R> P) {
 // one column as for 32, are done a lane per column.  The operations of each
 // column are the general kernel's, in its order: same bits.  ComplexF64,
 // n = 768, orders 40, 72 and 136, 211 pivots: 7.18 -> 2.83 ms.
-template <typename R>
-struct CQrBits;
-template <>
-struct CQrBits<double> {
-  // a norm as an integer of the same order, -1 for a NaN
-  static __device__ long long key(double v) {
-    const long long k = __double_as_longlong(v) & 0x7fffffffffffffffll;
-    return k > 0x7ff0000000000000ll ? -1 : k;
-  }
-  static __device__ double value(long long k) { return __longlong_as_double(k); }
-  // the leading bits of |v|, their exponent, whether its square and root are safe
-  static __device__ unsigned lead(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
-  static __device__ int expo(unsigned h) { return (int)(h >> 20) - 1023; }
-  static __device__ bool safe(unsigned h) { return h >= (123u << 20) && h < (1923u << 20); }
-  static __device__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
-};
-template <>
-struct CQrBits<float> {
-  static __device__ long long key(float v) {
-    const unsigned k = __float_as_uint(v) & 0x7fffffffu;
-    return k > 0x7f800000u ? -1 : (long long)k;
-  }
-  static __device__ float value(long long k) { return __uint_as_float((unsigned)k); }
-  static __device__ unsigned lead(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-  static __device__ int expo(unsigned h) { return (int)(h >> 23) - 127; }
-  static __device__ bool safe(unsigned h) { return h >= (27u << 23) && h < (227u << 23); }
-  static __device__ float pow2(int e) { return __int_as_float((e + 127) << 23); }
-};
-
 // block_cnrm2's sum in its order, the largest component by its exponent; the
 // result in warp 0 (elsewhere undefined).  `big` and `red`: NT / 32 entries each.
 template <typename R, int NT>
 __device__ __forceinline__ R block_cnrm2_bits(const C<R>* x, int len, unsigned* big, R* red) {
-  using B = CQrBits<R>;
+  using B = NormBits<R>;
   constexpr int NW = NT / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   unsigned h = 0;
@@ -579,16 +551,13 @@ __device__ __forceinline__ C<R> cmulc_fixed(C<R> a, C<R> b) {
 }
 
 template <typename R, int NT>
-__global__ void __launch_bounds__(NT, 1) cgeqp3_smem_kernel(CQrParams<R> P, ulonglong2* word, C<R>* stage) {
+__global__ void __launch_bounds__(NT, 1) cgeqp3_smem_kernel(CQrParams<R> P, ColXch<C<R>> X) {
   constexpr int NW = NT / 32;
-  using Bits = CQrBits<R>;
-  constexpr int PW = 256 / 32;  // words a lane of the polling warp
+  using Bits = NormBits<R>;
   extern __shared__ __align__(16) unsigned char cq_smem[];
   __shared__ R s_red[32];
   __shared__ unsigned s_big[NW];
-  __shared__ long long s_key;
-  __shared__ int64_t s_pos;
-  __shared__ int s_q, s_owner, s_any, s_bad;
+  __shared__ ColXchShared s_x;
   __shared__ C<R> s_tau, s_scal;
   __shared__ R s_beta;
   const int G = gridDim.x, b = blockIdx.x;
@@ -623,78 +592,16 @@ __global__ void __launch_bounds__(NT, 1) cgeqp3_smem_kernel(CQrParams<R> P, ulon
   int owner = 0, anyflag = 0;
   long long topkey = -1;
   auto exchange = [&](int e, int from, bool only, int flag) -> bool {
-    __syncthreads();
-    if (wid == 0) {
-      long long v = -1;
-      int64_t i = n << 24;
+    const bool ok = col_exchange<NT>(s_x, X, P.bar, e, from, m, n, cols, flag, [&](int lane, long long& v, int64_t& i) {
       for (int q = lane; q < nloc; q += 32)
         if (pos[q] >= from && (!only || pos[q] == from))
           argmax_merge<long long>(v, i, only ? 0 : Bits::key(vn1[q]), (int64_t)pos[q] << 24 | q);
-      warp_argmax(v, i);
-      if (lane == 0) {
-        s_q = v >= 0 ? (int)(i & 0xffffff) : -1;
-        s_key = v;
-        s_pos = v >= 0 ? i >> 24 : n;
-      }
-    }
-    __syncthreads();
-    C<R>* st = stage + ((size_t)(e & 1) * G + b) * m;
-    if (s_q >= 0) {
-      const C<R>* a = cols + (size_t)s_q * m;
-      for (int i = from + threadIdx.x; i < m; i += NT) st[i] = a[i];
-    }
-    __syncthreads();
-    if (wid == 0) {
-      ulonglong2* const wd = word + (size_t)(e & 1) * G;
-      if (lane == 0)
-        st_word(wd + b, (unsigned long long)s_key,
-                (unsigned long long)(e + 1) << 33 | (unsigned long long)s_pos << 1 | (unsigned long long)flag);
-      ulonglong2 w[PW];
-      uint64_t t0 = 0;
-      bool bad = false;
-      for (int it = 1;; ++it) {
-        bool all = true;
-#pragma unroll
-        for (int k = 0; k < PW; ++k)
-          if (k * 32 + lane < G) w[k] = ld_word(wd + k * 32 + lane);
-#pragma unroll
-        for (int k = 0; k < PW; ++k)
-          if (k * 32 + lane < G) all &= (w[k].y >> 33) == (unsigned long long)(e + 1);
-        if (__all_sync(0xffffffffu, all)) break;
-        if ((it & 63) == 0) {
-          const uint64_t t = globaltimer_ns();
-          if (t0 == 0) t0 = t;
-          if (t - t0 > wait_limit_ns()) atomicCAS(&P.bar->err, 0, 4);
-          bad = __any_sync(0xffffffffu, *((volatile int*)&P.bar->err) != 0);
-          if (bad) break;
-        }
-      }
-      __threadfence();
-      long long v = -1;
-      int64_t i = n << 16;
-      bool fl = false;
-#pragma unroll
-      for (int k = 0; k < PW; ++k)
-        if (k * 32 + lane < G) {
-          fl |= (w[k].y & 1) != 0;
-          argmax_merge<long long>(v, i, (long long)w[k].x, (int64_t)((w[k].y >> 1) & 0xffffffffull) << 16 | (k * 32 + lane));
-        }
-      warp_argmax(v, i);
-      fl = __any_sync(0xffffffffu, fl);
-      if (lane == 0) {
-        s_key = v;
-        s_pos = v >= 0 ? i >> 16 : n;
-        s_owner = (int)(i & 0xffff);
-        s_any = fl;
-        s_bad = bad;
-      }
-    }
-    __syncthreads();
-    topkey = s_key;
-    pvt = s_pos;
-    owner = s_owner;
-    anyflag = s_any;
-    return s_bad == 0;
+    }, [](int) { return 0; });
+    topkey = s_x.key;
+    pvt = s_x.id;
+    owner = s_x.owner;
+    anyflag = s_x.any;
+    return ok;
   };
 
   int e = 0;
@@ -713,7 +620,7 @@ __global__ void __launch_bounds__(NT, 1) cgeqp3_smem_kernel(CQrParams<R> P, ulon
         if (!exchange(e, c, true, 0)) return;
       }
       {
-        const C<R>* st = stage + ((size_t)(e & 1) * G + owner) * m;
+        const C<R>* st = X.stage + ((size_t)(e & 1) * G + owner) * m;
         for (int i = c + threadIdx.x; i < m; i += NT) {
           if constexpr (sizeof(R) == 8) {
             const double2 t = __ldcg(reinterpret_cast<const double2*>(st + i));
@@ -1304,10 +1211,11 @@ int64_t cgeqp3(lra_ctx* ctx, int64_t m, int64_t n, cx<R>* A, int64_t lda, int64_
   const size_t smem = cqr_smem<R>(m, (n + G - 1) / G);
   if (pivot && qr_smem_enabled() && m < (1 << 24) && n < (1 << 24) && smem <= cap) {
     raise_smem_limit(ctx, smk);
-    ulonglong2* word = ctx->arena.alloc_n<ulonglong2>((size_t)2 * G);
-    cx<R>* stage = ctx->arena.alloc_n<cx<R>>((size_t)2 * G * m);
-    LRA_CUDA(cudaMemsetAsync(word, 0, (size_t)2 * G * sizeof(ulonglong2), ctx->stream));
-    void* args[] = {&P, &word, &stage};
+    ColXch<cx<R>> X;
+    X.word = ctx->arena.alloc_n<ulonglong2>((size_t)2 * G);
+    X.stage = ctx->arena.alloc_n<cx<R>>((size_t)2 * G * m);
+    LRA_CUDA(cudaMemsetAsync(X.word, 0, (size_t)2 * G * sizeof(ulonglong2), ctx->stream));
+    void* args[] = {&P, &X};
     LRA_CUDA(cudaLaunchCooperativeKernel(smk, dim3(G), dim3(NT), args, smem, ctx->stream));
     post_launch(ctx, "cgeqp3_smem_kernel");
   } else {
