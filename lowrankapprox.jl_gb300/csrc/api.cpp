@@ -668,7 +668,7 @@ int sketchfact_steps(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, int
       int64_t k = 0;
       {
         Stage sq(ctx, 1);
-        k = geqp3_adap<T>(ctx, q.m, q.n, q.A, q.lda, q.jpvt, q.tau, q.kmax, o.nb, o.atol, o.rtol, true);
+        k = geqp3_adap<T>(ctx, q.m, q.n, q.A, q.lda, q.jpvt, q.tau, q.kmax, o.nb, o.atol, o.rtol, true, q.nt);
       }
       F.order = q.m;
       F.ld = q.lda;
@@ -761,11 +761,12 @@ Fact<T> sketchfact_dev(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, i
     }
     {
       Stage st(ctx, 1);
-      F.k = geqp3_adap<T>(ctx, order, N, F.B, F.ld, F.jpvt, F.tau, kmax, o.nb, o.atol, o.rtol, true);
+      F.k = geqp3_adap<T>(ctx, order, N, F.B, F.ld, F.jpvt, F.tau, kmax, o.nb, o.atol, o.rtol, true,
+                          adaptive ? nt : 0);
     }
     F.nsteps = step + 1;
     if (!adaptive || F.k < nt) break;
-    if (ahead) rank_hint = predict_rank<T>(ctx, F, kmax, o);
+    if (ahead) rank_hint = predict_rank<T>(ctx, F, F.k == nt ? nt : kmax, o);
     nt *= 2;
     ctx->arena.release(base);
   }
@@ -807,7 +808,7 @@ Fact<T> sketchfact_right_dev(lra_ctx* ctx, const lra_opts& o, char trans, int64_
     }
     {
       Stage st(ctx, 1);
-      F.k = geqp3_adap<T>(ctx, M, order, F.B, F.ld, F.jpvt, F.tau, kmax, o.nb, o.atol, o.rtol, true);
+      F.k = geqp3_adap<T>(ctx, M, order, F.B, F.ld, F.jpvt, F.tau, kmax, o.nb, o.atol, o.rtol, true, adaptive ? nt : 0);
     }
     F.nsteps = step + 1;
     if (!adaptive || F.k < nt) break;
@@ -1240,7 +1241,7 @@ void idfact_batched_grouped(lra_ctx* ctx, int64_t count, const lra_matdesc* mats
         RandSrc rs(ctx, nullptr, o.seed);
         sk.push_back(SketchItem{&split[(size_t)i], rs.lattice_src(s.order * d.m, false), s.B, s.order});
         s.ctr = ctx->rng_counter;
-        items.push_back(DfBatchItem{s.order, d.n, s.order, kmax, s.B, s.jpvt, s.tau});
+        items.push_back(DfBatchItem{s.order, d.n, s.order, kmax, s.B, s.jpvt, s.tau, adaptive ? s.nt : 0});
       }
       tc_sketch_batch(ctx, (int64_t)sk.size(), sk.data(), order, errs);
       std::vector<int64_t> map(act.begin(), act.end());
@@ -1542,7 +1543,7 @@ struct CFact {
 
 // geqp3_adap! of a dense rows x N device matrix B (ld), in place
 template <typename R>
-CFact<R> cpqr_backend(lra_ctx* ctx, const lra_opts& o, CX<R>* B, int64_t rows, int64_t N, int64_t ld) {
+CFact<R> cpqr_backend(lra_ctx* ctx, const lra_opts& o, CX<R>* B, int64_t rows, int64_t N, int64_t ld, int64_t stop_at = 0) {
   CFact<R> F;
   F.B = B;
   F.ld = ld;
@@ -1553,7 +1554,7 @@ CFact<R> cpqr_backend(lra_ctx* ctx, const lra_opts& o, CX<R>* B, int64_t rows, i
   F.jpvt = ctx->arena.alloc_n<int64_t>(std::max<int64_t>(N, 1));
   F.tau = ctx->arena.alloc_n<CX<R>>(std::max<int64_t>(l, 1));
   Stage st(ctx, 1);
-  F.k = cgeqp3<R>(ctx, rows, N, B, ld, F.jpvt, F.tau, kmax, o.nb, o.atol, o.rtol, true);
+  F.k = cgeqp3<R>(ctx, rows, N, B, ld, F.jpvt, F.tau, kmax, o.nb, o.atol, o.rtol, true, stop_at);
   return F;
 }
 
@@ -1576,7 +1577,7 @@ CFact<R> sketchfact_c(lra_ctx* ctx, const lra_opts& o, char trans, bool right, i
       make_sketch_c<R>(ctx, o, trans, M, N, A, lda, order, rs, B, right);
     }
     lra_opts oq = o;
-    F = cpqr_backend<R>(ctx, oq, B, rows, cols, std::max<int64_t>(rows, 1));
+    F = cpqr_backend<R>(ctx, oq, B, rows, cols, std::max<int64_t>(rows, 1), adaptive ? nt : 0);
     F.nsteps = step + 1;
     if (!adaptive || F.k < nt) break;
     nt *= 2;

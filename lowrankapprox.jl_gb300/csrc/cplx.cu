@@ -264,6 +264,7 @@ struct CQrParams {
   double atol, rtol;
   int pivot;
   int64_t* k_out;
+  int64_t stop_at;  // an adaptive step that has shown this rank ends there (0: never)
 };
 
 template <typename R, int NT>
@@ -715,9 +716,14 @@ __global__ void __launch_bounds__(NT, 1) cgeqp3_smem_kernel(CQrParams<R> P, ColX
       ++e;
       if (!exchange(e, c, false, flag ? 1 : 0)) return;
       block_end = anyflag != 0;
+      if (c == P.stop_at && first_small < 0) break;
     }
     if (last_small) {
       kres = first_small;
+      break;
+    }
+    if (c == P.stop_at && first_small < 0) {
+      kres = c;
       break;
     }
   }
@@ -1158,7 +1164,7 @@ void ccol_norms(lra_ctx* ctx, int64_t m, int64_t n, const cx<R>* A, int64_t lda,
 
 template <typename R>
 int64_t cgeqp3(lra_ctx* ctx, int64_t m, int64_t n, cx<R>* A, int64_t lda, int64_t* jpvt, cx<R>* tau, int64_t kmax,
-               int64_t nb, double atol, double rtol, bool pivot) {
+               int64_t nb, double atol, double rtol, bool pivot, int64_t stop_at) {
   constexpr int NT = 256;
   if (n <= 0) return 0;
   const ArenaMark mark = ctx->arena.mark();
@@ -1185,6 +1191,7 @@ int64_t cgeqp3(lra_ctx* ctx, int64_t m, int64_t n, cx<R>* A, int64_t lda, int64_
   P.atol = atol;
   P.rtol = rtol;
   P.pivot = pivot ? 1 : 0;
+  P.stop_at = stop_at;
   P.k_out = ctx->arena.alloc_n<int64_t>(1);
   LRA_CUDA(cudaMemsetAsync(P.bar, 0, sizeof(GridBar), ctx->stream));
   if (P.kmax <= 0) {
@@ -1388,7 +1395,7 @@ void ccluster_orth(lra_ctx* ctx, int64_t n, int64_t k, cx<R>* Z, int64_t ldz, co
   template void cconj<R>(lra_ctx*, int64_t, int64_t, cx<R>*, int64_t);                                         \
   template void ccol_norms<R>(lra_ctx*, int64_t, int64_t, const cx<R>*, int64_t, R*);                          \
   template int64_t cgeqp3<R>(lra_ctx*, int64_t, int64_t, cx<R>*, int64_t, int64_t*, cx<R>*, int64_t, int64_t,  \
-                             double, double, bool);                                                            \
+                             double, double, bool, int64_t);                                                   \
   template void capply_q<R>(lra_ctx*, char, int64_t, int64_t, const cx<R>*, int64_t, const cx<R>*, cx<R>*,     \
                             int64_t, int64_t);                                                                 \
   template void corgqr<R>(lra_ctx*, int64_t, int64_t, cx<R>*, int64_t, const cx<R>*);                          \

@@ -216,6 +216,7 @@ struct DfBatchItem {
   double* B;
   int64_t* jpvt;
   double* tau;
+  int64_t stop_at;  // as geqp3_adap's
 };
 bool geqp3_df_batch_fits(lra_ctx* ctx, int64_t m, int64_t n);
 // lra_idfact_batched's grouped path: whether the batch qualifies, and the run
@@ -229,7 +230,10 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
                     int64_t* k_dev);
 
 // Rank-adaptive column-pivoted Householder QR (geqp3_adap!), in place.
-// pivot == false runs the same Householder QR without pivoting.
+// pivot == false runs the same Householder QR without pivoting.  stop_at > 0: once
+// that many pivots are all above the tolerance the QR may end there with this
+// rank (an adaptive step that is going to be followed by a larger one, whose
+// factors nobody reads).
 // Several adaptive steps' sketches factored by one launch of the
 // shared-memory pivoted QR, each on CTAs of its own.  A step whose rank
 // comes out below its threshold (k < nt) stops the steps after it at their
@@ -257,7 +261,7 @@ int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* steps, int64_t nb
 
 template <typename T>
 int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_t* jpvt,
-                   T* tau, int64_t kmax, int64_t nb, double atol, double rtol, bool pivot);
+                   T* tau, int64_t kmax, int64_t nb, double atol, double rtol, bool pivot, int64_t stop_at = 0);
 
 // The same pivoted QR with its scratch in a fixed device array instead of
 // the context arena (no device allocation); n <= noalloc_max_cols().
@@ -500,7 +504,7 @@ void ccol_norms(lra_ctx* ctx, int64_t m, int64_t n, const cx<R>* A, int64_t lda,
 // geqp3_adap! with ZLAQPS / CLAQPS rules (pivot) or a plain Householder QR
 template <typename R>
 int64_t cgeqp3(lra_ctx* ctx, int64_t m, int64_t n, cx<R>* A, int64_t lda, int64_t* jpvt, cx<R>* tau, int64_t kmax,
-               int64_t nb, double atol, double rtol, bool pivot);
+               int64_t nb, double atol, double rtol, bool pivot, int64_t stop_at = 0);
 // X <- Q X ('n') or Q^H X ('c'), Q = H_1 ... H_k of the QR's reflectors
 template <typename R>
 void capply_q(lra_ctx* ctx, char trans, int64_t m, int64_t k, const cx<R>* V, int64_t ldv, const cx<R>* tau,

@@ -60,6 +60,9 @@ struct QrParams {
   // double-float QR: columns with at most this many rows below the pivot
   // row are summed by one thread each (the tuning table's qr_seq_len)
   int seq_len = 96;
+  // an adaptive step that has shown this rank is not the last one: its QR ends
+  // there (0: never; the shared-memory kernels)
+  int64_t stop_at = 0;
 };
 
 constexpr int CH = 16;  // rows per lane held in registers per column chunk
@@ -1098,9 +1101,14 @@ __global__ void __launch_bounds__(NT, 1) geqp3_f64_smem_kernel(QrParams<double> 
       ++e;
       if (!exchange(e, c, flag ? 1 : 0, true)) return;
       block_end = s_x.any != 0;
+      if (c == P.stop_at && first_small < 0) break;
     }
     if (last_small) {
       kres = first_small;
+      break;
+    }
+    if (c == P.stop_at && first_small < 0) {
+      kres = c;
       break;
     }
   }
@@ -2455,6 +2463,7 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
       stamp(c, 7);
       stop_block = s_stop != 0;
       ++kk;
+      if (j + kk == P.stop_at && first_small < 0) break;
     }
     const int64_t jn = j + kk;
     nfac = jn;
@@ -2462,6 +2471,10 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
     // is below ptol, the rank is the first i of this block with |R(i, i)| <= ptol
     if (last_small) {
       kres = first_small;
+      break;
+    }
+    if (jn == P.stop_at && first_small < 0) {
+      kres = jn;
       break;
     }
     j = jn;
@@ -3234,6 +3247,7 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
     J.P.rtol = rtol;
     J.P.pivot = 1;
     J.P.seq_len = ctx->tuning.qr_seq_len;
+    J.P.stop_at = it.stop_at;
     J.P.k_out = k_dev + i;
     J.X.piv = ctx->arena.alloc_n<int64_t>(std::max<int64_t>(J.P.kmax, 1));
     J.X.nfac = ctx->arena.alloc_n<int64_t>(1);
@@ -3657,6 +3671,7 @@ int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* st, int64_t nb, d
     q[i].job.S.success = success;
     q[i].job.S.job = i;
     q[i].job.S.nt = st[i].nt;
+    q[i].job.P.stop_at = st[i].nt;
     qp[i] = &q[i];
     smem = std::max(smem, q[i].smem);
   }
@@ -3686,7 +3701,7 @@ int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* st, int64_t nb, d
 
 template <typename T>
 int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_t* jpvt, T* tau,
-                   int64_t kmax, int64_t nb, double atol, double rtol, bool pivot) {
+                   int64_t kmax, int64_t nb, double atol, double rtol, bool pivot, int64_t stop_at) {
   constexpr int NT = 512;
   if (n <= 0) return 0;
   const ArenaMark mark = ctx->arena.mark();
@@ -3725,6 +3740,7 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
   P.k_out = ctx->arena.alloc_n<int64_t>(1);
   P.vcap = vcap;
   P.seq_len = ctx->tuning.qr_seq_len;
+  P.stop_at = stop_at;
   LRA_CUDA(cudaMemsetAsync(small, 0, 8 * sizeof(int), ctx->stream));
   LRA_CUDA(cudaMemsetAsync(P.bar, 0, sizeof(GridBar), ctx->stream));
   if (P.kmax <= 0) {
@@ -3755,6 +3771,7 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     if (need <= sm_capacity<Ar>(ctx) && sm_resident<Ar>(ctx, need)) {
       SmQr<T> q;
       sm_prepare<T>(ctx, q, m, n, A, lda, jpvt, tau, P.kmax, nb, atol, rtol, G);
+      q.job.P.stop_at = stop_at;
       SmQr<T>* qp = &q;
       sm_launch<T>(ctx, &qp, 1);
       sm_finish<T>(ctx, q);
@@ -4159,7 +4176,7 @@ template int64_t geqp3_adap_noalloc<double>(lra_ctx*, int64_t, int64_t, double*,
 
 #define INST(T)                                                                                   \
   template int64_t geqp3_adap<T>(lra_ctx*, int64_t, int64_t, T*, int64_t, int64_t*, T*, int64_t,  \
-                                 int64_t, double, double, bool);                                 \
+                                 int64_t, double, double, bool, int64_t);                        \
   template void trsm_upper<T>(lra_ctx*, int64_t, int64_t, const T*, int64_t, T*, int64_t, const T*); \
   template void apply_q<T>(lra_ctx*, char, int64_t, int64_t, const T*, int64_t, const T*, T*,    \
                            int64_t, int64_t);                                                    \
