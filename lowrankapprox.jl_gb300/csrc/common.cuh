@@ -162,7 +162,8 @@ struct GridBar {
   int pad;
 };
 
-__device__ __forceinline__ bool grid_sync(GridBar* gb) {
+// (of the first n CTAs that use `gb`)
+__device__ __forceinline__ bool group_sync(GridBar* gb, unsigned n) {
   __syncthreads();
   if (threadIdx.x == 0) {
     volatile unsigned int* vgen = &gb->gen;
@@ -170,7 +171,7 @@ __device__ __forceinline__ bool grid_sync(GridBar* gb) {
     const unsigned int g = *vgen;
     __threadfence();
     const unsigned int prev = atomicAdd(&gb->count, 1u);
-    if (prev == gridDim.x - 1) {
+    if (prev == n - 1) {
       atomicExch(&gb->count, 0u);
       __threadfence();
       atomicAdd(&gb->gen, 1u);
@@ -190,5 +191,6 @@ __device__ __forceinline__ bool grid_sync(GridBar* gb) {
   __syncthreads();
   return *((volatile int*)&gb->err) == 0;
 }
+__device__ __forceinline__ bool grid_sync(GridBar* gb) { return group_sync(gb, gridDim.x); }
 
 }  // namespace lra

@@ -1709,43 +1709,64 @@ namespace {
 
 constexpr int CB = 32;  // diagonal block size
 
-// upper Cholesky of the jb x jb diagonal block in place (one CTA); sets *bad
-// when the block is not positive definite
-// Right-looking Cholesky of one jb x jb diagonal block in shared memory, as
-// LAPACK xPOTF2 orders it: R(c, c) = sqrt(.), row c scaled by 1 / R(c, c),
-// then the trailing block updated in parallel.
+// Upper Cholesky of a jb x jb diagonal block in shared memory (256 threads), its
+// upper triangle in place; *bad set when the block is not positive definite.
+// LAPACK xPOTF2's order: R(c, c) = sqrt(.), row c times 1 / R(c, c), then the
+// trailing block.  Lane j of warp i mod 8 keeps entry (i, j); the warp of row c
+// updates it first, takes the root, the reciprocal and the scaling itself and
+// leaves the row in xs (two buffers): one barrier a column.  Bound: that chain, a
+// root and a divide.  With one thread for the scalars, three barriers and an
+// index division an entry, order 370 took 329 us in FP32 and 365 us of order 213
+// in FP64 (the whole factorization); 227 and 311 us with this block.
 template <typename T>
-__global__ void potrf_diag_kernel(int jb, T* G, int64_t ldg, int* bad) {
+__device__ void potrf_block(T (*a)[CB + 1], int jb, T (*xs)[CB], int* bad) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  T v[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) v[t] = wid + 8 * t < jb && lane < jb ? a[wid + 8 * t][lane] : T(0);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    for (int w = 0; w < 8; ++w) {
+      const int c = 8 * t + w;
+      if (c >= jb) break;
+      if (wid == w) {
+        T d = __shfl_sync(0xffffffffu, v[t], c);
+        if (!(d > T(0))) {
+          if (lane == 0) atomicExch(bad, 1);
+          d = T(1);
+        }
+        const T r = sqrt(d), inv = T(1) / r;
+        v[t] = lane == c ? r : v[t] * inv;
+        xs[c & 1][lane] = v[t];
+      }
+      __syncthreads();
+      const T xj = xs[c & 1][lane];
+      // rows of this group of eight first: the next pivot row is among them
+#pragma unroll
+      for (int u = t; u < 4; ++u) {
+        const int i = wid + 8 * u;
+        if (i > c && lane >= i) v[u] = fma(-xs[c & 1][i], xj, v[u]);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int i = wid + 8 * t;
+    if (i <= lane && lane < jb) a[i][lane] = v[t];
+  }
+  __syncthreads();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) potrf_diag_kernel(int jb, T* G, int64_t ldg, int* bad) {
   __shared__ T a[CB][CB + 1];
-  __shared__ T s_inv;
+  __shared__ T xs[2][CB];
   for (int t = threadIdx.x; t < jb * jb; t += blockDim.x) {
     const int i = t % jb, j = t / jb;
     a[i][j] = G[i + j * ldg];
   }
   __syncthreads();
-  for (int c = 0; c < jb; ++c) {
-    if (threadIdx.x == 0) {
-      T d = a[c][c];
-      if (!(d > T(0))) {
-        atomicExch(bad, 1);
-        d = T(1);
-      }
-      const T r = sqrt(d);
-      a[c][c] = r;
-      s_inv = T(1) / r;
-    }
-    __syncthreads();
-    const T inv = s_inv;
-    for (int j = c + 1 + threadIdx.x; j < jb; j += blockDim.x) a[c][j] *= inv;
-    __syncthreads();
-    // a[i][j] -= a[c][i] a[c][j] for c < i <= j < jb
-    const int w = jb - c - 1;
-    for (int t = threadIdx.x; t < w * w; t += blockDim.x) {
-      const int i = c + 1 + t % w, j = c + 1 + t / w;
-      if (i <= j) a[i][j] -= a[c][i] * a[c][j];
-    }
-    __syncthreads();
-  }
+  potrf_block<T>(a, jb, xs, bad);
   for (int t = threadIdx.x; t < jb * jb; t += blockDim.x) {
     const int i = t % jb, j = t / jb;
     G[i + j * ldg] = i <= j ? a[i][j] : T(0);
@@ -1753,13 +1774,13 @@ __global__ void potrf_diag_kernel(int jb, T* G, int64_t ldg, int* bad) {
 }
 
 // The whole blocked right-looking Cholesky in one cooperative launch, of
-// one matrix or two independent ones at once (their sequential diagonal
-// blocks then overlap): for each 32-wide diagonal block, CTA m factors
-// matrix m's block in shared memory (as potrf_diag_kernel), the grid solves
-// the block rows with a warp per column (lane i holds x_i; the columns of
-// both matrices dealt out over every warp, since the FP64 pipe of one SM
-// retires only a few FMAs a clock) and updates the upper trailing
-// triangles, with a bounded grid barrier between the phases.
+// one matrix or two independent ones at once, each on CTAs of its own: every
+// CTA factors each 32-wide diagonal block itself (the same operations, so the
+// same bits; no barrier and no trip through memory between the block and its
+// row), the CTAs solve the block row with a warp per column (lane i holds x_i)
+// and update the upper trailing triangle in tiles of 32 x 32, with a bounded
+// barrier of the matrix's CTAs after either.  Order 370 in FP32: 227 us with one CTA at
+// the block and an element a thread, 142 us now; 213 in FP64: 311 and 281 us.
 template <typename T>
 struct PotrfJobs {
   int n;           // 1 or 2
@@ -1770,111 +1791,84 @@ struct PotrfJobs {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(256) potrf_coop_kernel(PotrfJobs<T> J, GridBar* bar) {
-  __shared__ T a[2][CB][CB + 1];
-  __shared__ T rinv[2][CB];
-  __shared__ T s_inv;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t GT = (int64_t)gridDim.x * blockDim.x;
-  const int64_t kmax = J.n > 1 ? max(J.k[0], J.k[1]) : J.k[0];
-  for (int64_t j0 = 0; j0 < kmax; j0 += CB) {
-    // ---- 1. the diagonal blocks, CTA m for matrix m ----
-    for (int m = 0; m < J.n; ++m) {
-      if ((int)blockIdx.x != m % (int)gridDim.x || j0 >= J.k[m]) continue;
-      const int jb = (int)min((int64_t)CB, J.k[m] - j0);
-      const int64_t ldg = J.ldg[m];
-      T* Gjj = J.G[m] + j0 + j0 * ldg;
-      // every read of G goes around L1: other CTAs wrote it in earlier phases
-      for (int t = threadIdx.x; t < jb * jb; t += blockDim.x)
-        a[m][t % jb][t / jb] = __ldcg(Gjj + t % jb + (t / jb) * ldg);
-      __syncthreads();
-      for (int c = 0; c < jb; ++c) {
-        if (threadIdx.x == 0) {
-          T d = a[m][c][c];
-          if (!(d > T(0))) {
-            atomicExch(J.bad + m, 1);
-            d = T(1);
-          }
-          const T r = sqrt(d);
-          a[m][c][c] = r;
-          s_inv = T(1) / r;
-        }
-        __syncthreads();
-        const T inv = s_inv;
-        for (int j = c + 1 + threadIdx.x; j < jb; j += blockDim.x) a[m][c][j] *= inv;
-        __syncthreads();
-        const int w = jb - c - 1;
-        for (int t = threadIdx.x; t < w * w; t += blockDim.x) {
-          const int i = c + 1 + t % w, j = c + 1 + t / w;
-          if (i <= j) a[m][i][j] -= a[m][c][i] * a[m][c][j];
-        }
-        __syncthreads();
-      }
+__global__ void __launch_bounds__(256) potrf_coop_kernel(PotrfJobs<T> J, GridBar* bars) {
+  __shared__ T a[CB][CB + 1], pj[CB][CB + 1];
+  __shared__ T rinv[CB];
+  __shared__ T xs[2][CB];
+  const int m = (int)blockIdx.x % J.n, g = (int)blockIdx.x / J.n;
+  const int Gm = ((int)gridDim.x - m + J.n - 1) / J.n;  // CTAs of this matrix
+  GridBar* bar = bars + m;
+  const int64_t k = J.k[m], ldg = J.ldg[m];
+  T* const G = J.G[m];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int64_t j0 = 0; j0 < k; j0 += CB) {
+    // ---- 1. the diagonal block ----
+    // (every read of G goes around L1: other CTAs wrote it in earlier phases)
+    const int jb = (int)min((int64_t)CB, k - j0);
+    const int64_t rest = k - j0 - jb, o = j0 + jb;
+    if (rest <= 0 && g != 0) break;
+    T* Gjj = G + j0 + j0 * ldg;
+    for (int t = threadIdx.x; t < jb * jb; t += blockDim.x) a[t % jb][t / jb] = __ldcg(Gjj + t % jb + (t / jb) * ldg);
+    __syncthreads();
+    potrf_block<T>(a, jb, xs, J.bad + m);
+    // back to memory by one CTA, once every CTA has read the block as it was
+    auto store_block = [&]() {
       for (int t = threadIdx.x; t < jb * jb; t += blockDim.x) {
         const int i = t % jb, j = t / jb;
-        if (i <= j) Gjj[i + j * ldg] = a[m][i][j];
+        if (i <= j) Gjj[i + j * ldg] = a[i][j];
       }
+    };
+    if (rest <= 0) {
+      store_block();
+      break;
     }
-    if (!grid_sync(bar)) return;
-    int64_t rest[2] = {0, 0};
-    int jbm[2] = {0, 0};
-    for (int m = 0; m < J.n; ++m) {
-      if (j0 >= J.k[m]) continue;
-      jbm[m] = (int)min((int64_t)CB, J.k[m] - j0);
-      rest[m] = J.k[m] - j0 - jbm[m];
-    }
-    if (rest[0] + rest[1] <= 0) break;
-    // ---- 2. the block rows: R_{b,>b} = R_bb^{-T} G_{b,>b}, a warp per column ----
-    for (int m = 0; m < J.n; ++m) {
-      if (rest[m] <= 0) continue;
-      const int jb = jbm[m];
-      const T* Gjj = J.G[m] + j0 + j0 * J.ldg[m];
-      for (int t = threadIdx.x; t < jb * jb; t += blockDim.x)
-        a[m][t % jb][t / jb] = __ldcg(Gjj + t % jb + (t / jb) * J.ldg[m]);
-    }
+    // ---- 2. the block row: R_{b,>b} = R_bb^{-T} G_{b,>b}, a warp per column ----
+    if (threadIdx.x < jb) rinv[threadIdx.x] = T(1) / a[threadIdx.x][threadIdx.x];
     __syncthreads();
-    for (int m = 0; m < J.n; ++m)
-      if (rest[m] > 0 && threadIdx.x < jbm[m]) rinv[m][threadIdx.x] = T(1) / a[m][threadIdx.x][threadIdx.x];
-    __syncthreads();
-    {
-      const int lane = threadIdx.x & 31;
-      const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-      const int64_t GW = (int64_t)gridDim.x * (blockDim.x >> 5);
-      for (int64_t cc = gw; cc < rest[0] + rest[1]; cc += GW) {
-        const int m = cc < rest[0] ? 0 : 1;
-        const int64_t col = m == 0 ? cc : cc - rest[0];
-        const int jb = jbm[m];
-        T* p = J.G[m] + j0 + (j0 + jb + col) * J.ldg[m];
-        T x = lane < jb ? __ldcg(p + lane) : T(0);
-        // x_i = (g_i - sum_{q<i} R_qi x_q) / R_ii, the sums accumulated lane-wise
-        for (int i = 0; i < jb; ++i) {
-          const T xi = __shfl_sync(0xffffffffu, x, i) * rinv[m][i];
-          if (lane == i) x = xi;
-          if (lane > i && lane < jb) x -= a[m][i][lane] * xi;
-        }
-        if (lane < jb) p[lane] = x;
+    for (int64_t col = (int64_t)wid * Gm + g; col < rest; col += (int64_t)Gm * 8) {
+      T* p = G + j0 + (o + col) * ldg;
+      T x = lane < jb ? __ldcg(p + lane) : T(0);
+      // x_i = (g_i - sum_{q<i} R_qi x_q) / R_ii, the sums accumulated lane-wise
+      for (int i = 0; i < jb; ++i) {
+        const T xi = __shfl_sync(0xffffffffu, x, i) * rinv[i];
+        if (lane == i) x = xi;
+        if (lane > i && lane < jb) x -= a[i][lane] * xi;
       }
+      if (lane < jb) p[lane] = x;
     }
-    if (!grid_sync(bar)) return;
-    // ---- 3. trailing upper triangles: G(i, j) -= sum_q R(q, i) R(q, j), j0+jb <= i <= j ----
-    const int64_t n0 = rest[0] * rest[0];
-    for (int64_t t = gt; t < n0 + rest[1] * rest[1]; t += GT) {
-      const int m = t < n0 ? 0 : 1;
-      const int64_t tt = m == 0 ? t : t - n0, r = rest[m];
-      const int64_t i = tt % r, j = tt / r;
-      if (i > j) continue;
-      const int jb = jbm[m];
-      const int64_t ldg = J.ldg[m], o = j0 + jb;
-      T* G = J.G[m];
-      const T* ri = G + j0 + (o + i) * ldg;
-      const T* rj = G + j0 + (o + j) * ldg;
-      T s = 0;
+    if (!group_sync(bar, Gm)) return;
+    if (g == 0) {
+      store_block();
+      __syncthreads();
+    }
+    // ---- 3. trailing upper triangle: G(i, j) -= sum_q R(q, i) R(q, j), o <= i <= j ----
+    // (jb = 32 here)
+    const int64_t nt = (rest + CB - 1) / CB;
+    for (int64_t t = g; t < nt * nt; t += Gm) {
+      const int64_t ti = t % nt * CB, tj = t / nt * CB;
+      if (ti > tj) continue;
+      T gij[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int64_t ci = ti + wid + 8 * r, cj = tj + wid + 8 * r;
+        a[wid + 8 * r][lane] = ci < rest ? __ldcg(G + j0 + lane + (o + ci) * ldg) : T(0);
+        pj[wid + 8 * r][lane] = cj < rest ? __ldcg(G + j0 + lane + (o + cj) * ldg) : T(0);
+        gij[r] = ti + lane < rest && cj < rest && ti + lane <= cj ? __ldcg(G + o + ti + lane + (o + cj) * ldg) : T(0);
+      }
+      __syncthreads();
+      T s[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll 8
-      for (int q = 0; q < jb; ++q) s = fma(__ldcg(ri + q), __ldcg(rj + q), s);
-      T* gij = G + (o + i) + (o + j) * ldg;
-      *gij = __ldcg(gij) - s;
+      for (int q = 0; q < CB; ++q)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) s[r] = fma(a[lane][q], pj[wid + 8 * r][q], s[r]);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int64_t i = ti + lane, j = tj + wid + 8 * r;
+        if (i <= j && j < rest) G[o + i + (o + j) * ldg] = gij[r] - s[r];
+      }
+      __syncthreads();
     }
-    if (!grid_sync(bar)) return;
+    if (!group_sync(bar, Gm)) return;
   }
 }
 
@@ -2072,20 +2066,20 @@ void potrf_upper_batch(lra_ctx* ctx, int n, const int64_t* k, T* const* G, const
     int per_sm = 0;
     LRA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, potrf_coop_kernel<T>, 256, 0));
     const int grid = std::max(J.n, std::min(ctx->num_sms, ctx->num_sms * per_sm));
-    GridBar* bar = reinterpret_cast<GridBar*>(ctx->arena.alloc(sizeof(GridBar)));
-    LRA_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), ctx->stream));
+    GridBar* bar = reinterpret_cast<GridBar*>(ctx->arena.alloc(2 * sizeof(GridBar)));
+    LRA_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(GridBar), ctx->stream));
     void* args[] = {&J, &bar};
     LRA_CUDA(cudaLaunchCooperativeKernel((const void*)potrf_coop_kernel<T>, dim3(grid), dim3(256), args, 0,
                                          ctx->stream));
     post_launch(ctx, "potrf_coop_kernel");
     for (int m = 0; m < J.n; ++m) zero_lower(ctx, J.k[m], J.k[m], J.G[m], J.ldg[m]);
     int h[2] = {0, 0};
-    GridBar hb;
+    GridBar hb[2];
     LRA_CUDA(cudaMemcpyAsync(h, bad, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    LRA_CUDA(cudaMemcpyAsync(&hb, bar, sizeof(GridBar), cudaMemcpyDeviceToHost, ctx->stream));
+    LRA_CUDA(cudaMemcpyAsync(hb, bar, 2 * sizeof(GridBar), cudaMemcpyDeviceToHost, ctx->stream));
     LRA_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->arena.release(mk);
-    if (hb.err != 0) fail(LRA_ETIMEDOUT, "potrf: a grid barrier timed out");
+    if (hb[0].err != 0 || hb[1].err != 0) fail(LRA_ETIMEDOUT, "potrf: a grid barrier timed out");
     for (int m = 0; m < n; ++m)
       if (slot[m] >= 0) ok[m] = h[slot[m]] == 0;
     return;
@@ -2140,57 +2134,71 @@ namespace {
 // Y = R^-1 D with D = diag(R), the inverse of the unit upper triangular
 // D^-1 R (k x k, strictly lower part zero), a CTA per column: column j
 // solves R y = R_jj e_j by column-oriented back substitution -- y_j = 1,
-// then a_i -= R_iq y_q for i < q and y_q = a_q / R_qq from q = j down --
-// with the partial sums a_i in the registers of the thread owning row i
-// (rows tid + 128 u) and the finished y in shared memory; the column of R a
-// step needs is loaded one step ahead, and 1 / R_qq is computed for every q
-// first, so that no FP64 division sits on a step's critical path (a product
-// with the reciprocal instead, within an ulp of the quotient).  A graded R
+// then a_i -= R_iq y_q for i < q and y_q = a_q / R_qq from q = j down.  A graded R
 // (|R_iq| <= |R_ii|, as a
 // pivoted QR leaves it) has an inverse whose rows span its whole diagonal
 // range, which a GEMM that scales each row by its largest entry would
 // truncate; R^-1 D has entries of order one.
+//
+// Bound: the chain of FP64 operations.  Blocks of 32 rows from the bottom: warp 0
+// solves the block on its diagonal, a row a lane, its entries of R loaded while
+// the block before was applied; then all threads subtract the 32 columns from
+// the rows above, each entry in the order of q, with no barrier among them (a
+// barrier a column before: 200 us for order 460, 92 us now).  1 / R_qq is
+// computed for every q first, so that no FP64 division sits on the chain (a
+// product with the reciprocal instead, within an ulp of the quotient).
 constexpr int kTiNT = 128;
-constexpr int kTiRows = 16;   // rows a thread: k up to 2048
+constexpr int kTiMax = 2048;
 constexpr int kTiLeaf = 512;  // larger orders split in two on the tensor-core path
 
 template <typename T>
 __global__ void __launch_bounds__(kTiNT) tri_inv_upper_kernel(int64_t k, const T* __restrict__ R, int64_t ldr,
                                                               T* __restrict__ Y, int64_t ldy) {
-  extern __shared__ unsigned char ti_smem[];
-  T* ys = reinterpret_cast<T*>(ti_smem);  // k
-  T* rdi = ys + k;                        // 1 / R_qq, off the per-step critical path
-  const int tid = threadIdx.x;
-  const int U = (int)((k + kTiNT - 1) / kTiNT);
+  extern __shared__ __align__(16) unsigned char ti_smem[];
+  T* ys = reinterpret_cast<T*>(ti_smem);  // k: the partial sums a_i, then y
+  T* rdi = ys + k;                        // 1 / R_qq
+  const int tid = threadIdx.x, lane = tid & 31;
   for (int64_t q = tid; q < k; q += kTiNT) rdi[q] = T(1) / R[q + q * ldr];
-  __syncthreads();
   for (int64_t j = blockIdx.x; j < k; j += gridDim.x) {
-    T a[kTiRows], rc[kTiRows];
+    for (int64_t i = tid; i <= j; i += kTiNT) ys[i] = T(0);
+    T rr[32];  // warp 0: R(qb + lane, qb + t) of the next diagonal block
+    auto fetch = [&](int64_t qb) {
 #pragma unroll
-    for (int u = 0; u < kTiRows; ++u) {
-      const int64_t i = tid + (int64_t)kTiNT * u;
-      a[u] = T(0);
-      rc[u] = u < U && i < j ? R[i + j * ldr] : T(0);
-    }
-    if (tid == 0) ys[j] = T(1);
+      for (int t = 0; t < 32; ++t) rr[t] = lane < t && qb + t <= j ? __ldg(R + qb + lane + (qb + t) * ldr) : T(0);
+    };
+    int64_t qb = j / 32 * 32;
+    if (tid < 32) fetch(qb);
     __syncthreads();
-    for (int64_t q = j; q > 0; --q) {
-      const T yq = ys[q];
-      const T rqq = rdi[q - 1];
-      T rn[kTiRows];
+    for (; qb >= 0; qb -= 32) {
+      if (tid < 32) {
+        T a = qb + lane <= j ? ys[qb + lane] : T(0), y = T(0);
 #pragma unroll
-      for (int u = 0; u < kTiRows; ++u) {
-        const int64_t i = tid + (int64_t)kTiNT * u;
-        rn[u] = u < U && i < q - 1 ? R[i + (q - 1) * ldr] : T(0);
-      }
-#pragma unroll
-      for (int u = 0; u < kTiRows; ++u) {
-        const int64_t i = tid + (int64_t)kTiNT * u;
-        if (u < U && i < q) {
-          a[u] = fma(-rc[u], yq, a[u]);
-          if (i == q - 1) ys[q - 1] = a[u] * rqq;
+        for (int t = 31; t >= 0; --t) {
+          const int64_t q = qb + t;
+          if (q <= j) {
+            const T yq = q == j ? T(1) : __shfl_sync(0xffffffffu, a, t) * rdi[q];
+            if (lane == t) y = yq;
+            if (lane < t) a = fma(-rr[t], yq, a);
+          }
         }
-        rc[u] = rn[u];
+        if (qb + lane <= j) ys[qb + lane] = y;
+        if (qb > 0) fetch(qb - 32);
+      }
+      __syncthreads();
+      const int nq = (int)min((int64_t)32, j - qb + 1);
+      for (int64_t i = tid; i < qb; i += kTiNT) {
+        T a = ys[i];
+        const T* r = R + i + qb * ldr;
+        int t = nq - 1;
+        for (; t >= 7; t -= 8) {
+          T rv[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) rv[u] = __ldg(r + (t - u) * ldr);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) a = fma(-rv[u], ys[qb + t - u], a);
+        }
+        for (; t >= 0; --t) a = fma(-__ldg(r + t * ldr), ys[qb + t], a);
+        ys[i] = a;
       }
       __syncthreads();
     }
@@ -2230,7 +2238,7 @@ template void div_by_diag<double>(lra_ctx*, int64_t, int64_t, const double*, int
 template <typename T>
 bool tri_inv_upper(lra_ctx* ctx, int64_t k, const T* R, int64_t ldr, T* Y, int64_t ldy) {
   if (k <= 0) return true;
-  if (k > (int64_t)kTiNT * kTiRows) return false;
+  if (k > kTiMax) return false;
   if (sizeof(T) == 8 && ctx->gemm_tc && k > kTiLeaf) {
     // Recursive on the tensor-core path: with R = [A B; 0 C] and D = diag(R),
     // R^-1 D = [Ya, -Ya (Da^-1 B) Yc; 0, Yc] for Ya = A^-1 Da, Yc = C^-1 Dc.
@@ -2267,7 +2275,7 @@ template bool tri_inv_upper<double>(lra_ctx*, int64_t, const double*, int64_t, d
 template <typename T>
 bool trsm_by_inverse(const lra_ctx* ctx, int64_t k, int64_t other) {
   if (sizeof(T) != 8 || !ctx->gemm_tc || ctx->tuning.trsm_inv == 1) return false;
-  return k > 2 * CB && k <= (int64_t)kTiNT * kTiRows && tc_gemm_worthwhile(other, k, k);
+  return k > 2 * CB && k <= kTiMax && tc_gemm_worthwhile(other, k, k);
 }
 template bool trsm_by_inverse<float>(const lra_ctx*, int64_t, int64_t);
 template bool trsm_by_inverse<double>(const lra_ctx*, int64_t, int64_t);
