@@ -797,8 +797,16 @@ __global__ void __launch_bounds__(256) sketch_src_group_kernel(const SrcJob* __r
 // with t = ceil(log2(K chunks)) + 1 keeping |X| below 2^63.
 //
 // Same warp roles as the sketch kernel; one 144 KB stage (six 128 x 64 A
-// digit tiles, six 64 x 64 B digit tiles), so the loads of block k + 1
-// overlap the drain of block k.  blockIdx.y selects a range of K blocks;
+// digit tiles, six 64 x 64 B digit tiles).  Bound: the stage's loads from L2
+// (144 KB for 84 MMAs; 181 us a product on average in a psvd of rank 1800).  Two
+// stages do not fit, so the stage is handed on in thirds: the products with
+// digit 1 run first and free digits 1 and 6, those left with 2 and 5 free these,
+// then 3 and 4; each third is loaded for the next block while the others'
+// products run, and the next block begins with the products of the third that
+// came first.  The accumulators are handed over one diagonal at a time, in the
+// order the next chunk needs them.  The 69 products of that psvd: 14.35 ms with
+// the stage and the accumulators passed on whole, 12.5 ms now.
+// blockIdx.y selects a range of K blocks;
 // with several, each writes its unscaled partial product to a workspace.
 constexpr int G_TILE_M = 128, G_TILE_N = 64, G_NS = 6;
 constexpr int G_A_BYTES = G_TILE_M * KBLK * 2;               // 16 KB
@@ -827,11 +835,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* stA = base;
   unsigned char* stB = base + G_NS * G_A_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(base + G_STAGE);
-  uint64_t* empty = full + 1;
-  uint64_t* acc_ready = empty + 1;
-  uint64_t* acc_free = acc_ready + 1;
-  uint64_t* mma_done = acc_free + 1;
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + G_STAGE);  // [3]
+  uint64_t* empty = full + 3;                                    // [3]
+  uint64_t* acc_ready = empty + 3;
+  uint64_t* acc_free = acc_ready + 1;  // [G_NS], by diagonal
+  uint64_t* mma_done = acc_free + G_NS;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -842,10 +850,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const int t = P.tshift;
 
   if (threadIdx.x == 0) {
-    mbar_init(full, 1);
-    mbar_init(empty, 1);
+    for (int g = 0; g < 3; ++g) {
+      mbar_init(full + g, 1);
+      mbar_init(empty + g, 1);
+    }
     mbar_init(acc_ready, 1);
-    mbar_init(acc_free, 8);
+    for (int d = 0; d < G_NS; ++d) mbar_init(acc_free + d, 8);
     mbar_init(mma_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -861,46 +871,69 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      int issued = 0;
+      int issued = 0;  // thirds
       for (int it = 0; it < nloc; ++it) {
-        if (!mbar_wait(empty, (it & 1) ^ 1, P.err)) break;
-        ++issued;
         const int kx = (kb0 + it) * KBLK;
-        mbar_expect_tx(full, (uint32_t)G_STAGE);
-        for (int q = 0; q < G_NS; ++q) {
-          tma_load_3d(stA + q * G_A_BYTES, &tmA, kx, (int)(m_tile * G_TILE_M), q, full);
-          tma_load_3d(stB + q * G_B_BYTES, &tmB, kx, (int)(n_tile * G_TILE_N), q, full);
+        bool ok = true;
+        for (int g = 0; g < 3 && ok; ++g) {
+          ok = mbar_wait(empty + g, (it & 1) ^ 1, P.err);
+          if (!ok) break;
+          ++issued;
+          mbar_expect_tx(full + g, (uint32_t)(2 * (G_A_BYTES + G_B_BYTES)));
+          for (int h = 0; h < 2; ++h) {
+            const int q = h == 0 ? g : G_NS - 1 - g;
+            tma_load_3d(stA + q * G_A_BYTES, &tmA, kx, (int)(m_tile * G_TILE_M), q, full + g);
+            tma_load_3d(stB + q * G_B_BYTES, &tmB, kx, (int)(n_tile * G_TILE_N), q, full + g);
+          }
         }
+        if (!ok) break;
       }
+      // no copy is in flight when the CTA ends
       int dummy = 0;
-      if (issued > 0) mbar_wait(full, (issued - 1) & 1, &dummy);
+      for (int g = 0; g < 3; ++g) {
+        const int n = (issued + 2 - g) / 3;  // loads of third g
+        if (n > 0) mbar_wait(full + g, (n - 1) & 1, &dummy);
+      }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = idesc_bf16(G_TILE_M, G_TILE_N);
+      const uint32_t a0 = smem_u32(stA), b0 = smem_u32(stB);
+      unsigned fresh = 0;  // diagonals whose accumulator this chunk has not begun
+      auto product = [&](int su, int uu) {
+        const int d = su + uu;
+        const uint32_t acc = tmem + (uint32_t)(d * G_TILE_N);
+#pragma unroll
+        for (int k4 = 0; k4 < KBLK / 16; ++k4)
+          mma_bf16(acc, sw128_desc(a0 + su * G_A_BYTES + k4 * 32), sw128_desc(b0 + uu * G_B_BYTES + k4 * 32), idesc,
+                   (k4 == 0 && ((fresh >> d) & 1u)) ? 0u : 1u);
+        fresh &= ~(1u << d);
+      };
       for (int it = 0; it < nloc; ++it) {
         const int ch = it / G_CHUNK;  // drain chunk
         const bool first = (it % G_CHUNK) == 0;
-        if (first && ch > 0) {
-          if (!mbar_wait(acc_free, (ch - 1) & 1, P.err)) break;
+        if (first) fresh = (1u << G_NS) - 1;
+        // third g of the stage, and the diagonals g and 5 - g, which its products
+        // with digit 1 begin
+        auto ready = [&](int g) -> bool {
+          if (first && ch > 0)
+            if (!mbar_wait(acc_free + g, (ch - 1) & 1, P.err) || !mbar_wait(acc_free + G_NS - 1 - g, (ch - 1) & 1, P.err))
+              return false;
+          if (!mbar_wait(full + g, it & 1, P.err)) return false;
           tc_fence_after();
-        }
-        if (!mbar_wait(full, it & 1, P.err)) break;
-        tc_fence_after();
-        const uint32_t a0 = smem_u32(stA), b0 = smem_u32(stB);
-        for (int s = 0; s < G_NS; ++s) {
-          for (int u = 0; u + s < G_NS; ++u) {
-            const uint32_t acc = tmem + (uint32_t)((s + u) * G_TILE_N);
-#pragma unroll
-            for (int k4 = 0; k4 < KBLK / 16; ++k4) {
-              const uint64_t ad = sw128_desc(a0 + s * G_A_BYTES + k4 * 32);
-              const uint64_t bd = sw128_desc(b0 + u * G_B_BYTES + k4 * 32);
-              // each diagonal restarts with its (1, d + 1) product
-              mma_bf16(acc, ad, bd, idesc, (first && s == 0 && k4 == 0) ? 0u : 1u);
-            }
-          }
-        }
+          return true;
+        };
+        if (!ready(0)) break;
+        product(0, 0), product(0, 5), product(5, 0);
+        if (!ready(1)) break;
+        product(0, 1), product(1, 0), product(0, 4), product(4, 0);
+        if (!ready(2)) break;
+        product(0, 2), product(2, 0), product(0, 3), product(3, 0);
         mma_commit(empty);
+        product(1, 1), product(1, 2), product(2, 1), product(1, 3), product(3, 1), product(1, 4), product(4, 1);
+        mma_commit(empty + 1);
+        product(2, 2), product(2, 3), product(3, 2);
+        mma_commit(empty + 2);
         if ((it % G_CHUNK) == G_CHUNK - 1 || it == nloc - 1) mma_commit(acc_ready);
       }
       mma_commit(mma_done);
@@ -923,9 +956,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       tc_fence_after();
 #pragma unroll 1
-      for (int d = 0; d < G_NS; ++d) {
+      for (int t6 = 0; t6 < G_NS; ++t6) {
+        const int d = (t6 & 1) ? G_NS - 1 - t6 / 2 : t6 / 2;  // 0, 5, 1, 4, 2, 3
         uint32_t r[32];
         tmem_ld32(tmem + lane_base + (uint32_t)(d * G_TILE_N + half * G_COLS), r);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_free + d);
         const int w = 8 * (G_NS - 1 - d) - t;
         // |acc| <= 2^24: exact through a 32-bit conversion
         if (w >= 0) {
@@ -939,9 +976,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_free);
     }
     const int64_t i = m_tile * G_TILE_M + 32 * q4 + lane;
     if (ok && i < P.M) {
