@@ -149,7 +149,7 @@ struct TcSplit {
 bool tc_sketch_supported(int64_t order, int64_t M, int64_t N);
 template <typename T>
 void tc_split(lra_ctx* ctx, char trans, int64_t M, int64_t N, const T* A, int64_t lda, int ns,
-              TcSplit* out, bool balanced = false);
+              TcSplit* out);
 // where a sketch's lattice draws come from: an injected stream on the device, or
 // (g null) the generator of `seed` at counter `base`; `right`: drawn in the
 // layout of a right sketch (M x order), used transposed

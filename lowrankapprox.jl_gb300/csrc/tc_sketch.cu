@@ -466,6 +466,13 @@ __device__ __forceinline__ unsigned int abs_bits(float x) {
 }
 __device__ __forceinline__ double bits_value(unsigned long long b) { return __longlong_as_double((long long)b); }
 __device__ __forceinline__ double bits_value(unsigned int b) { return (double)__uint_as_float(b); }
+// colexp_of(bits_value(b)) by integer operations
+__device__ __forceinline__ int colexp_bits(unsigned long long b) {
+  const int ex = (int)(b >> 52);
+  if (ex >= 0x7FF) return kNonFinite;
+  if (ex > 0) return ex - 1022;
+  return b == 0 ? 0 : -1010 - __clzll((long long)b);
+}
 template <typename K>
 __device__ __forceinline__ K warp_max_bits(K v) {
 #pragma unroll
@@ -583,15 +590,14 @@ __device__ __forceinline__ void write_slices(long long F, int ns, int n_exact, i
 // 4096 Float32, 0.82 ms this way)
 template <typename T>
 __device__ __forceinline__ void split_n_run(int64_t K, int64_t N, const T* __restrict__ A, int64_t lda,
-                                            const int* __restrict__ e, int ns, int n_exact, int W,
-                                            __nv_bfloat16* __restrict__ S, int64_t Kp, int64_t j, int64_t run, int lane) {
+                                            int ej, int ns, int n_exact, int W, __nv_bfloat16* __restrict__ S,
+                                            int64_t Kp, int64_t j, int64_t run, int lane) {
   const int64_t plane = Kp * N, i = run * 128 + 4 * lane;
   if (i >= Kp) return;
   const T* a = A + j * lda + i;
   T x[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) x[q] = i + q < K ? a[q] : T(0);
-  const int ej = e[j];
   __nv_bfloat16 d[4][MAX_SLICES];
 #pragma unroll
   for (int q = 0; q < 4; ++q) write_slices<T>(i + q < K ? fixed_point(x[q], ej, W) : 0, ns, n_exact, W, d[q], 1);
@@ -616,7 +622,7 @@ __global__ void __launch_bounds__(256) split_n_kernel(int64_t K, int64_t N, cons
   const int64_t runs = (Kp + 127) / 128;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; u < runs * N; u += nw)
-    split_n_run(K, N, A, lda, e, ns, n_exact, W, S, Kp, u / runs, u % runs, lane);
+    split_n_run(K, N, A, lda, e[u / runs], ns, n_exact, W, S, Kp, u / runs, u % runs, lane);
 }
 
 // ---- the same for a batch: CTAs (matrix, part)
@@ -628,25 +634,28 @@ struct SplitJob {
   int* bad;  // set when an entry is NaN or infinite
 };
 
+__device__ __forceinline__ unsigned long long column_max(const double* __restrict__ a, int64_t K, int lane) {
+  unsigned long long mx = 0;
+  int64_t i = lane;
+  for (; i + 96 < K; i += 128) {
+    unsigned long long v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = abs_bits(a[i + 32 * q]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) mx = v[q] > mx ? v[q] : mx;
+  }
+  for (; i < K; i += 32) {
+    const unsigned long long v = abs_bits(a[i]);
+    mx = v > mx ? v : mx;
+  }
+  return warp_max_bits(mx);
+}
+
 __global__ void __launch_bounds__(256) colexp_group_kernel(const SplitJob* __restrict__ jobs) {
   const SplitJob J = jobs[blockIdx.x];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int64_t j = (int64_t)blockIdx.y * 8 + wid; j < J.N; j += (int64_t)gridDim.y * 8) {
-    const double* a = J.A + j * J.lda;
-    unsigned long long mx = 0;
-    int64_t i = lane;
-    for (; i + 96 < J.K; i += 128) {
-      unsigned long long v[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = abs_bits(a[i + 32 * q]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) mx = v[q] > mx ? v[q] : mx;
-    }
-    for (; i < J.K; i += 32) {
-      const unsigned long long v = abs_bits(a[i]);
-      mx = v > mx ? v : mx;
-    }
-    mx = warp_max_bits(mx);
+    const unsigned long long mx = column_max(J.A + j * J.lda, J.K, lane);
     if (lane == 0) {
       const int e = colexp_of(bits_value(mx));
       J.e[j] = e;
@@ -660,7 +669,7 @@ __global__ void __launch_bounds__(256) split_group_kernel(const SplitJob* __rest
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t runs = (J.Kp + 127) / 128;
   for (int64_t u = (int64_t)blockIdx.y * 8 + wid; u < runs * J.N; u += (int64_t)gridDim.y * 8)
-    split_n_run(J.K, J.N, J.A, J.lda, J.e, ns, n_exact, W, J.S, J.Kp, u / runs, u % runs, lane);
+    split_n_run(J.K, J.N, J.A, J.lda, J.e[u / runs], ns, n_exact, W, J.S, J.Kp, u / runs, u % runs, lane);
 }
 
 // op(A) = A^T through 32 x 32 shared-memory tiles
@@ -682,6 +691,95 @@ __global__ void split_c_kernel(int64_t K, int64_t N, const T* __restrict__ A, in
       if (i < Kp && j < N) {
         const long long F = fixed_point(tile[threadIdx.x][r], e[j], W);
         write_slices<T>(F, ns, n_exact, W, S + i + j * Kp, plane);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---- both operands of a digit product at once: blockIdx.y is the operand -----------
+// Bound: latency at the orders of the post-processing.  (A maximum, its exponent
+// and the digits in launches of their own for either operand: 1.1 ms for the 25
+// products of a psvd of rank 363, 0.46 ms so, and 70 launches fewer.)
+struct OpSplit {
+  int c;               // columns of the operand are rows of A
+  int64_t K, N, lda, Kp;
+  const double* A;
+  unsigned long long* mx;  // zeroed: the largest |entry| of each column
+  int* e;
+  __nv_bfloat16* S;
+};
+
+__global__ void __launch_bounds__(256) op_max_kernel(OpSplit a, OpSplit b) {
+  const OpSplit& J = blockIdx.y == 0 ? a : b;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (!J.c) {
+    for (int64_t j = (int64_t)blockIdx.x * 8 + wid; j < J.N; j += (int64_t)gridDim.x * 8) {
+      const unsigned long long mx = column_max(J.A + j * J.lda, J.K, lane);
+      if (lane == 0) J.mx[j] = mx;
+    }
+    return;
+  }
+  // tiles of 32 rows of A x 64 of its columns
+  const int64_t tn = (J.N + 31) / 32, tk = (J.K + 63) / 64;
+  for (int64_t t = blockIdx.x; t < tn * tk; t += gridDim.x) {
+    const int64_t j = (t % tn) * 32 + lane, i0 = (t / tn) * 64 + wid;
+    if (j >= J.N) continue;
+    unsigned long long v[8], m = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = i0 + 8 * q < J.K ? abs_bits(J.A[j + (i0 + 8 * q) * J.lda]) : 0ull;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) m = v[q] > m ? v[q] : m;
+    if (m > 0) atomicMax(J.mx + j, m);
+  }
+}
+
+__global__ void __launch_bounds__(256) op_split_kernel(OpSplit a, OpSplit b) {
+  __shared__ double tile[64][33];
+  __shared__ int se[32];
+  constexpr int NS = 6, W = 48;  // balanced digits
+  const OpSplit& J = blockIdx.y == 0 ? a : b;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (!J.c) {
+    const int64_t runs = (J.Kp + 127) / 128;
+    for (int64_t u = (int64_t)blockIdx.x * 8 + wid; u < runs * J.N; u += (int64_t)gridDim.x * 8) {
+      const int64_t j = u / runs;
+      const int ej = colexp_bits(J.mx[j]);
+      if (u % runs == 0 && lane == 0) J.e[j] = ej;
+      split_n_run(J.K, J.N, J.A, J.lda, ej, NS, 0, W, J.S, J.Kp, j, u % runs, lane);
+    }
+    return;
+  }
+  // tiles of 32 rows of A x 64 of its columns through shared memory, two entries a
+  // thread so that a warp writes 128 contiguous bytes a digit
+  const int64_t plane = J.Kp * J.N;
+  const int64_t ti = (J.Kp + 63) / 64, tj = (J.N + 31) / 32;
+  for (int64_t t = blockIdx.x; t < ti * tj; t += gridDim.x) {
+    const int64_t i0 = (t % ti) * 64, j0 = (t / ti) * 32;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = wid + 8 * q;
+      const int64_t j = j0 + lane, i = i0 + r;  // A(j, i) contiguous in j
+      tile[r][lane] = (i < J.K && j < J.N) ? J.A[j + i * J.lda] : 0.0;
+    }
+    if (threadIdx.x < 32 && j0 + lane < J.N) {
+      const int ej = colexp_bits(J.mx[j0 + lane]);
+      se[lane] = ej;
+      if (i0 == 0) J.e[j0 + lane] = ej;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = wid + 8 * q;
+      const int64_t i = i0 + 2 * lane, j = j0 + r;
+      if (i < J.Kp && j < J.N) {  // (Kp is even)
+        __nv_bfloat16 d[2][MAX_SLICES];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) write_slices<double>(fixed_point(tile[2 * lane + h][r], se[r], W), NS, 0, W, d[h], 1);
+#pragma unroll
+        for (int p = 0; p < NS; ++p)
+          *reinterpret_cast<ushort2*>(J.S + p * plane + i + j * J.Kp) =
+              make_ushort2(__bfloat16_as_ushort(d[0][p]), __bfloat16_as_ushort(d[1][p]));
       }
     }
     __syncthreads();
@@ -1056,10 +1154,9 @@ bool tc_sketch_supported(int64_t order, int64_t M, int64_t N) {
 }
 
 template <typename T>
-void tc_split(lra_ctx* ctx, char trans, int64_t M, int64_t N, const T* A, int64_t lda, int ns, TcSplit* out,
-              bool balanced) {
+void tc_split(lra_ctx* ctx, char trans, int64_t M, int64_t N, const T* A, int64_t lda, int ns, TcSplit* out) {
   const int W = 8 * ns;
-  const int n_exact = balanced ? 0 : std::min(ns, MAX_EXACT);
+  const int n_exact = std::min(ns, MAX_EXACT);
   const int64_t Kp = (M + 7) / 8 * 8;
   out->K = M;
   out->N = N;
@@ -1349,22 +1446,42 @@ void tc_gemm(lra_ctx* ctx, char ta, char tb, int64_t m, int64_t n, int64_t k, do
   const bool TB = (tb == 't' || tb == 'T' || tb == 'c' || tb == 'C');
   const ArenaMark mk = ctx->arena.mark();
   // X_A = op(A)^T (k x m) and X_B = op(B) (k x n), split by columns
-  TcSplit sa, sb;
-  tc_split<double>(ctx, TA ? 'n' : 'c', k, m, A, lda, G_NS, &sa, true);
-  tc_split<double>(ctx, TB ? 'c' : 'n', k, n, B, ldb, G_NS, &sb, true);
-  const int64_t Kp = sa.Kp;
+  const int64_t Kp = (k + 7) / 8 * 8;
+  OpSplit sa{TA ? 0 : 1, k, m, lda, Kp, A, nullptr, nullptr, nullptr}, sb{TB ? 1 : 0, k, n, ldb, Kp, B, nullptr, nullptr, nullptr};
+  sa.mx = ctx->arena.alloc_n<unsigned long long>((size_t)(m + n));
+  sb.mx = sa.mx + m;
+  sa.e = ctx->arena.alloc_n<int>((size_t)(m + n));
+  sb.e = sa.e + m;
+  sa.S = ctx->arena.alloc_n<__nv_bfloat16>((size_t)G_NS * Kp * m);
+  sb.S = ctx->arena.alloc_n<__nv_bfloat16>((size_t)G_NS * Kp * n);
+  LRA_CUDA(cudaMemsetAsync(sa.mx, 0, (size_t)(m + n) * sizeof(unsigned long long), ctx->stream));
+  {
+    // units of an operand: columns by eight or tiles; runs by eight or tiles
+    auto units = [](const OpSplit& o, bool split) {
+      const int64_t tn = (o.N + 31) / 32;
+      if (o.c) return tn * ((o.K + 63) / 64);
+      return split ? ((o.Kp + 127) / 128 * o.N + 7) / 8 : (o.N + 7) / 8;
+    };
+    const int64_t cap = (int64_t)ctx->num_sms * 8;
+    op_max_kernel<<<dim3((unsigned)std::min(cap, std::max(units(sa, false), units(sb, false))), 2), 256, 0, ctx->stream>>>(
+        sa, sb);
+    post_launch(ctx, "op_max_kernel");
+    op_split_kernel<<<dim3((unsigned)std::min(cap, std::max(units(sa, true), units(sb, true))), 2), 256, 0, ctx->stream>>>(
+        sa, sb);
+    post_launch(ctx, "op_split_kernel");
+  }
   CUtensorMap tmA, tmB;
   {
     cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)m, (cuuint64_t)G_NS};
     cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * m * 2};
     cuuint32_t box[3] = {KBLK, G_TILE_M, 1};
-    make_map(&tmA, sa.slices, 3, dims, strides, box);
+    make_map(&tmA, sa.S, 3, dims, strides, box);
   }
   {
     cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)n, (cuuint64_t)G_NS};
     cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)Kp * n * 2};
     cuuint32_t box[3] = {KBLK, G_TILE_N, 1};
-    make_map(&tmB, sb.slices, 3, dims, strides, box);
+    make_map(&tmB, sb.S, 3, dims, strides, box);
   }
   const int nkb = (int)((k + KBLK - 1) / KBLK);
   const int64_t tiles = ((m + G_TILE_M - 1) / G_TILE_M) * ((n + G_TILE_N - 1) / G_TILE_N);
@@ -1393,8 +1510,8 @@ void tc_gemm(lra_ctx* ctx, char ta, char tb, int64_t m, int64_t n, int64_t k, do
   P.nkb = nkb;
   P.kb_per = kb_per;
   P.tshift = tsh;
-  P.ea = sa.colexp;
-  P.eb = sb.colexp;
+  P.ea = sa.e;
+  P.eb = sb.e;
   P.alpha = alpha;
   P.beta = beta;
   P.err = err;
@@ -1421,8 +1538,8 @@ void tc_gemm(lra_ctx* ctx, char ta, char tb, int64_t m, int64_t n, int64_t k, do
   ctx->arena.release(mk);  // stream-ordered reuse
 }
 
-template void tc_split<float>(lra_ctx*, char, int64_t, int64_t, const float*, int64_t, int, TcSplit*, bool);
-template void tc_split<double>(lra_ctx*, char, int64_t, int64_t, const double*, int64_t, int, TcSplit*, bool);
+template void tc_split<float>(lra_ctx*, char, int64_t, int64_t, const float*, int64_t, int, TcSplit*);
+template void tc_split<double>(lra_ctx*, char, int64_t, int64_t, const double*, int64_t, int, TcSplit*);
 template void tc_sketch<float>(lra_ctx*, const TcSplit&, int, const SketchSrc*, const int64_t*, float*, int64_t);
 template void tc_sketch<double>(lra_ctx*, const TcSplit&, int, const SketchSrc*, const int64_t*, double*, int64_t);
 
