@@ -1973,7 +1973,161 @@ __global__ void trsm_left_diag_kernel(int jb, int64_t nrhs, const T* Rbb, int64_
   }
 }
 
+// ---- the whole Float32 solve in one launch ------------------------------------
+// trsm_upper's and trsm_right_upper's recursion (halves of multiples of 32, a
+// product between them, blocks of at most 32) on a few right-hand sides a CTA,
+// which wait in shared memory: kTfN columns of R^{-1} X, or rows of X R^{-1}.
+// Every entry sees the recursion's operations in its order: a product's sum
+// from 0 over its inner index, subtracted once; within a block its own chain.
+// Same bits as the recursion in launches, which cost one per block and product
+// (rank 363: 23 launches of 9 to 14 us).  Bound: the chain of the blocks and R's
+// way through L2, read once by every CTA; hence the limit on the right-hand sides.
+// Rank 757, 3339 columns: 0.61 ms in launches, 0.385 so; the five solves of a psvd of
+// rank 302: 1.0 and 0.39 ms.
+constexpr int kTfN = 8;      // right-hand sides a CTA, a warp each in a block
+constexpr int kTfMax = 1024;
+
+template <int NCT>
+__device__ __forceinline__ void tf_load(const float* x, float (&v)[NCT]) {
+  if constexpr (NCT >= 4) {
+#pragma unroll
+    for (int c = 0; c < NCT; c += 4) {
+      const float4 t = *reinterpret_cast<const float4*>(x + c);
+      v[c] = t.x, v[c + 1] = t.y, v[c + 2] = t.z, v[c + 3] = t.w;
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < NCT; ++c) v[c] = x[c];
+  }
+}
+
+template <bool RIGHT, int NCT>
+__device__ __forceinline__ void tf_update(const float* __restrict__ R, int64_t ldr, float* xs, int r0, int nr, int q0, int nq,
+                                          int tid, int nthreads) {
+  // rows r0..r0+nr (RIGHT: columns) of each right-hand side take those q0..q0+nq away
+  const int groups = kTfN / NCT, per = nthreads / groups;
+  const int g = tid / per;
+  for (int i = tid % per; i < nr; i += per) {
+    float acc[NCT];
+#pragma unroll
+    for (int c = 0; c < NCT; ++c) acc[c] = 0.f;
+    const float* r = RIGHT ? R + q0 + (int64_t)(r0 + i) * ldr : R + r0 + i + (int64_t)q0 * ldr;
+    const int64_t step = RIGHT ? 1 : ldr;
+    const float* x = xs + q0 * kTfN + g * NCT;
+    float rn[8];  // the next eight entries of R are on their way
+#pragma unroll
+    for (int u = 0; u < 8; ++u) rn[u] = u < nq ? __ldg(r + u * step) : 0.f;
+    for (int q = 0; q < nq; q += 8) {
+      float rv[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        rv[u] = rn[u];
+        rn[u] = q + 8 + u < nq ? __ldg(r + (q + 8 + u) * step) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (q + u < nq) {
+          float xv[NCT];
+          tf_load<NCT>(x + (q + u) * kTfN, xv);
+#pragma unroll
+          for (int c = 0; c < NCT; ++c) acc[c] = fmaf(rv[u], xv[c], acc[c]);
+        }
+    }
+    float* y = xs + (r0 + i) * kTfN + g * NCT;
+#pragma unroll
+    for (int c = 0; c < NCT; ++c) y[c] -= acc[c];
+  }
+}
+
+template <bool RIGHT>
+__global__ void __launch_bounds__(kTfN * 32) trsm_fused_kernel(int k, int64_t nrhs, const float* __restrict__ R, int64_t ldr,
+                                                               float* X, int64_t ldx) {
+  extern __shared__ __align__(16) float tf_x[];  // [k][kTfN]: a product reads all right-hand sides of an entry
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int64_t c0 = (int64_t)blockIdx.x * kTfN;
+  const int nc = (int)min((int64_t)kTfN, nrhs - c0);
+  for (int t = tid; t < k * kTfN; t += kTfN * 32) {
+    const int c = RIGHT ? t % kTfN : t / k, i = RIGHT ? t / kTfN : t % k;
+    tf_x[i * kTfN + c] = c < nc ? (RIGHT ? X[c0 + c + i * ldx] : X[i + (c0 + c) * ldx]) : 0.f;
+  }
+  __syncthreads();
+  // the recursion: (begin, length) still to be solved, or (begin, length) whose
+  // product is due (length negative)
+  int sb[24], sl[24], top = 0;
+  sb[0] = 0;
+  sl[0] = k;
+  top = 1;
+  while (top > 0) {
+    --top;
+    const int b = sb[top];
+    int len = sl[top];
+    if (len > 32) {
+      const int k1 = (len / 2 + 31) / 32 * 32;
+      // done last, pushed first
+      sb[top] = RIGHT ? b + k1 : b;
+      sl[top++] = RIGHT ? len - k1 : k1;
+      sb[top] = b;
+      sl[top++] = -len;
+      sb[top] = RIGHT ? b : b + k1;
+      sl[top++] = RIGHT ? k1 : len - k1;
+      continue;
+    }
+    if (len < 0) {
+      len = -len;
+      const int k1 = (len / 2 + 31) / 32 * 32, k2 = len - k1;
+      const int r0 = RIGHT ? b + k1 : b, nr = RIGHT ? k2 : k1, q0 = RIGHT ? b : b + k1, nq = RIGHT ? k1 : k2;
+      if (nr > 128)
+        tf_update<RIGHT, 8>(R, ldr, tf_x, r0, nr, q0, nq, tid, kTfN * 32);
+      else if (nr > 64)
+        tf_update<RIGHT, 4>(R, ldr, tf_x, r0, nr, q0, nq, tid, kTfN * 32);
+      else if (nr > 32)
+        tf_update<RIGHT, 2>(R, ldr, tf_x, r0, nr, q0, nq, tid, kTfN * 32);
+      else
+        tf_update<RIGHT, 1>(R, ldr, tf_x, r0, nr, q0, nq, tid, kTfN * 32);
+      __syncthreads();
+      continue;
+    }
+    // a block: warp = right-hand side, lane = entry
+    const float* Rb = R + b + (int64_t)b * ldr;
+    const float rinv = lane < len ? 1.0f / __ldg(Rb + lane + (int64_t)lane * ldr) : 0.f;
+    float s = lane < len ? tf_x[(b + lane) * kTfN + wid] : 0.f, y = 0.f;
+    float rr[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+      rr[q] = q < len && lane < len && (RIGHT ? q < lane : lane < q)
+                  ? __ldg(RIGHT ? Rb + q + (int64_t)lane * ldr : Rb + lane + (int64_t)q * ldr)
+                  : 0.f;
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+      const int q = RIGHT ? t : 31 - t;
+      if (q < len) {
+        const float xq = __shfl_sync(0xffffffffu, s * rinv, q);
+        if (lane == q) y = xq;
+        if (RIGHT ? lane > q : lane < q) s = fmaf(-rr[q], xq, s);
+      }
+    }
+    if (lane < len) tf_x[(b + lane) * kTfN + wid] = y;
+    __syncthreads();
+  }
+  for (int t = tid; t < k * kTfN; t += kTfN * 32) {
+    const int c = RIGHT ? t % kTfN : t / k, i = RIGHT ? t / kTfN : t % k;
+    if (c < nc) (RIGHT ? X[c0 + c + i * ldx] : X[i + (c0 + c) * ldx]) = tf_x[i * kTfN + c];
+  }
+}
+
 }  // namespace
+
+bool trsm_fused(lra_ctx* ctx, bool right, int64_t k, int64_t nrhs, const float* R, int64_t ldr, float* X, int64_t ldx) {
+  if (k > kTfMax || nrhs > (int64_t)ctx->num_sms * 4 * kTfN) return false;
+  const size_t smem = (size_t)kTfN * (size_t)k * sizeof(float);
+  const unsigned g = (unsigned)((nrhs + kTfN - 1) / kTfN);
+  if (right)
+    trsm_fused_kernel<true><<<g, kTfN * 32, smem, ctx->stream>>>((int)k, nrhs, R, ldr, X, ldx);
+  else
+    trsm_fused_kernel<false><<<g, kTfN * 32, smem, ctx->stream>>>((int)k, nrhs, R, ldr, X, ldx);
+  post_launch(ctx, "trsm_fused_kernel");
+  return true;
+}
 
 // one or two Cholesky factorizations G_m = R_m^T R_m in place (upper R,
 // lower part zeroed) in one cooperative launch; ok[m] false when G_m is not
@@ -2297,6 +2451,8 @@ void trsm_right_upper(lra_ctx* ctx, int64_t m, int64_t k, const T* R, int64_t ld
     ctx->arena.release(mk);  // stream-ordered reuse
     return;
   }
+  if constexpr (sizeof(T) == 4)
+    if (trsm_fused(ctx, true, k, m, R, ldr, X, ldx)) return;
   if (k <= CB) {
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((m + 127) / 128, ctx->num_sms * 8));
     trsm_right_diag_kernel<T><<<g, 128, 0, ctx->stream>>>(m, (int)k, R, ldr, X, ldx);

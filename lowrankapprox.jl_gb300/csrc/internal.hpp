@@ -273,6 +273,9 @@ int64_t noalloc_max_cols();
 // X (k x nrhs) <- triu(R)^{-1} X, R k x k (ldr).
 template <typename T>
 void trsm_left_diag(lra_ctx* ctx, int jb, int64_t nrhs, const T* R, int64_t ldr, T* X, int64_t ldx);
+// Float32: X <- triu(R)^{-1} X, or X triu(R)^{-1} (right; X nrhs x k), in one launch with the
+// bits of the recursive solves; false where there are too many right-hand sides
+bool trsm_fused(lra_ctx* ctx, bool right, int64_t k, int64_t nrhs, const float* R, int64_t ldr, float* X, int64_t ldx);
 // X <- triu(R)^{-1} X (k <= kBsMax) by back substitution, a thread per column
 constexpr int kBsMax = 128;
 template <typename T>

@@ -3963,6 +3963,8 @@ void trsm_upper(lra_ctx* ctx, int64_t k, int64_t nrhs, const T* R, int64_t ldr, 
     ctx->arena.release(mk);
     return;
   }
+  if constexpr (sizeof(T) == 4)
+    if (trsm_fused(ctx, false, k, nrhs, R, ldr, X, ldx)) return;
   if (k <= 32) {
     trsm_left_diag(ctx, (int)k, nrhs, R, ldr, X, ldx);
     return;
