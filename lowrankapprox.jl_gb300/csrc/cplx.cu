@@ -29,11 +29,11 @@ inline unsigned grid_for_c(lra_ctx* ctx, int64_t n, int t) {
 
 // ---- GEMM: C = alpha op(A) op(B) + beta C, op 0 = n, 1 = t, 2 = c ------------------
 // Each entry is summed over k in order, whatever the tile.  ComplexF64: bound by
-// the FP64 units, 4 instructions of 64 cycles a term and a quarter of an SM, so
+// the FP64 units, 6 instructions of 64 cycles a term and a quarter of an SM, so
 // an entry a thread and small blocks (8 x 16 entries, a warp for each quarter),
 // which deal a sketch's few rows out evenly and pad none of them (orders are
 // 32 2^t + 8): tiles of 32 x 32 left 40 x 768 on 48 SMs.  (40 + 72 + 136) x 768,
-// K = 1024: 5.42 ms so, 1.43 now (the instructions alone: 1.25).  ComplexF32:
+// K = 1024: 5.42 ms so, 2.39 now (the instructions alone: 2.0).  ComplexF32:
 // bound by shared memory, four entries a thread.
 template <typename R>
 struct CgTile;
@@ -114,8 +114,12 @@ __global__ void __launch_bounds__(cg_threads<R>) cgemm_kernel(int64_t M, int64_t
 #pragma unroll
           for (int j = 0; j < TN; ++j) {
             if constexpr (sizeof(R) == 8) {
-              acc[i][j].re = fma(a[i].re, b[j].re, fma(-a[i].im, b[j].im, acc[i][j].re));
-              acc[i][j].im = fma(a[i].re, b[j].im, fma(a[i].im, b[j].re, acc[i][j].im));
+              // the product rounded, then added, the fused terms written out: the
+              // bits of `acc += a * b` as it was first compiled, which an ID of a
+              // numerical rank near 1e6 carries into T (four fused operations a term:
+              // 1.43 ms, T 6e-10 away)
+              acc[i][j].re += fma(a[i].re, b[j].re, -(a[i].im * b[j].im));
+              acc[i][j].im += fma(a[i].im, b[j].re, a[i].re * b[j].im);
             } else {
               acc[i][j] += a[i] * b[j];
             }
