@@ -2815,8 +2815,8 @@ __global__ void __launch_bounds__(256) df_finish_group_kernel(const DfFinishJob*
 }
 // max |B| over an m x n matrix as the bits of a double, a warp per column
 template <typename T>
-__global__ void __launch_bounds__(256) absmax_cols_kernel(int64_t m, int64_t n, const T* __restrict__ B, int64_t ldb,
-                                                          unsigned long long* __restrict__ out) {
+__device__ __forceinline__ void absmax_cols(int64_t m, int64_t n, const T* __restrict__ B, int64_t ldb,
+                                            unsigned long long* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -2834,21 +2834,26 @@ __global__ void __launch_bounds__(256) absmax_cols_kernel(int64_t m, int64_t n, 
     if (lane == 0 && mx > 0) atomicMax(out, (unsigned long long)__double_as_longlong((double)mx));
   }
 }
-
-// scale = 2^-E with max |B| in [2^(E-1), 2^E)
-__global__ void df_scale_kernel(const unsigned long long* mx, double* scale) {
-  const double m = __longlong_as_double((long long)*mx);
-  *scale = m > 0 ? ldexp(1.0, -(ilogb(m) + 1)) : 1.0;
+template <typename T>
+__global__ void __launch_bounds__(256) absmax_cols_kernel(int64_t m, int64_t n, const T* __restrict__ B, int64_t ldb,
+                                                          unsigned long long* __restrict__ out) {
+  absmax_cols(m, n, B, ldb, out);
 }
 
-// (h, l) = split(B * scale) and each column's norm, a warp per four columns
-__global__ void __launch_bounds__(256) df_split_kernel(int64_t m, int64_t n, const double* __restrict__ B, int64_t ldb,
-                                                       const double* __restrict__ scale, float* __restrict__ Bh,
-                                                       float* __restrict__ Bl, int64_t ldh, double* __restrict__ vn0) {
+// scale = 2^-E with max |B| in [2^(E-1), 2^E)
+__device__ __forceinline__ double df_scale_of(const unsigned long long* mx) {
+  const double m = __longlong_as_double((long long)*mx);
+  return m > 0 ? ldexp(1.0, -(ilogb(m) + 1)) : 1.0;
+}
+__global__ void df_scale_kernel(const unsigned long long* mx, double* scale) { *scale = df_scale_of(mx); }
+
+// (h, l) = split(B * sc) and each column's norm, a warp per four columns
+__device__ __forceinline__ void df_split_cols(int64_t m, int64_t n, const double* __restrict__ B, int64_t ldb, double sc,
+                                              float* __restrict__ Bh, float* __restrict__ Bl, int64_t ldh,
+                                              double* __restrict__ vn0) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const double sc = *scale;
   const int k = ilogb(sc);
   for (int64_t j = 4 * w0; j < n; j += 4 * nw) {
     double acc[4] = {0, 0, 0, 0};
@@ -2876,6 +2881,12 @@ __global__ void __launch_bounds__(256) df_split_kernel(int64_t m, int64_t n, con
       __syncwarp();
     }
   }
+}
+
+__global__ void __launch_bounds__(256) df_split_kernel(int64_t m, int64_t n, const double* __restrict__ B, int64_t ldb,
+                                                       const double* __restrict__ scale, float* __restrict__ Bh,
+                                                       float* __restrict__ Bl, int64_t ldh, double* __restrict__ vn0) {
+  df_split_cols(m, n, B, ldb, *scale, Bh, Bl, ldh, vn0);
 }
 
 // the step at which each column became a pivot (n when it did not):
@@ -2912,16 +2923,14 @@ __global__ void __launch_bounds__(256) df_join_kernel(int64_t m, int64_t n, cons
   }
 }
 
-// the Float32 sketch's conversions for the shared-memory QR: max |B| (as
-// the bits of a double, for df_scale_kernel), B * scale (exact: a power of
-// two) with each column's norm, and back
-__global__ void __launch_bounds__(256) f32_split_kernel(int64_t m, int64_t n, const float* __restrict__ B, int64_t ldb,
-                                                        const double* __restrict__ scale, float* __restrict__ Bs,
-                                                        int64_t lds, double* __restrict__ vn0) {
+// the Float32 sketch's conversion for the shared-memory QR: B * scale (exact: a
+// power of two) with each column's norm
+__device__ __forceinline__ void f32_split_cols(int64_t m, int64_t n, const float* __restrict__ B, int64_t ldb, double scale,
+                                               float* __restrict__ Bs, int64_t lds, double* __restrict__ vn0) {
   const int lane = threadIdx.x & 31;
   const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const float sc = (float)*scale;
+  const float sc = (float)scale;
   for (int64_t j = 4 * w0; j < n; j += 4 * nw) {
     double acc[4] = {0, 0, 0, 0};
     for (int64_t i = lane; i < m; i += 32) {
@@ -3463,8 +3472,55 @@ struct SmQr {
   unsigned gm = 1;
 };
 
+// what a sketch's launch starts from zero, one block a sketch, so that one
+// memset clears all
+struct alignas(128) SmZero {
+  ulonglong2 slot[32];  // the exchange: four slots, a 128-byte line each
+  GridBar bar;
+  int64_t k_out, nfac;
+  unsigned long long mx;
+};
+
+// The sketches of a launch prepared together, blockIdx.y a sketch: the
+// permutations and the largest entries, then the conversions.  (A sketch's
+// five memsets and four launches of 2 us each: the ID of a 256 x 192 matrix 1.19 ms
+// so, 1.12 ms together.)
+struct SmPrep {
+  int64_t m, n, lda;
+  const void* A;
+  unsigned long long* mx;
+  double* scale;
+  float* Bh;
+  float* Bl;
+  double* vn0;
+  int64_t* col_at;
+  int64_t* pos;
+};
+struct SmPreps {
+  SmPrep j[kSmJobs];
+};
+
 template <typename T>
-void sm_prepare(lra_ctx* ctx, SmQr<T>& q, int64_t m, int64_t n, T* A, int64_t lda, int64_t* jpvt, T* tau,
+__global__ void __launch_bounds__(256) sm_prep_max_kernel(const SmPreps P) {
+  const SmPrep& J = P.j[blockIdx.y];
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < J.n; t += (int64_t)gridDim.x * blockDim.x)
+    J.col_at[t] = J.pos[t] = t;
+  absmax_cols<T>(J.m, J.n, static_cast<const T*>(J.A), J.lda, J.mx);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) sm_prep_split_kernel(const SmPreps P) {
+  const SmPrep& J = P.j[blockIdx.y];
+  const double sc = df_scale_of(J.mx);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *J.scale = sc;
+  if constexpr (sizeof(T) == 8)
+    df_split_cols(J.m, J.n, static_cast<const double*>(J.A), J.lda, sc, J.Bh, J.Bl, J.m, J.vn0);
+  else
+    f32_split_cols(J.m, J.n, static_cast<const float*>(J.A), J.lda, sc, J.Bh, J.m, J.vn0);
+}
+
+template <typename T>
+void sm_prepare(lra_ctx* ctx, SmQr<T>& q, SmZero* z, SmPrep& prep, int64_t m, int64_t n, T* A, int64_t lda, int64_t* jpvt, T* tau,
                 int64_t kmax, int64_t nb, double atol, double rtol, int G) {
   using Ar = SmA<T>;
   using E = typename Ar::E;
@@ -3484,56 +3540,30 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, int64_t m, int64_t n, T* A, int64_t ld
   P.jpvt = jpvt;
   P.tau = tau;
   P.part_d = ctx->arena.alloc_n<double>(G);
-  P.bar = reinterpret_cast<GridBar*>(ctx->arena.alloc(sizeof(GridBar)));
+  P.bar = &z->bar;
   P.kmax = std::min<int64_t>(kmax, std::min(m, n));
   P.nb = std::max<int64_t>(1, std::min<int64_t>(nb, std::max<int64_t>(P.kmax, 1)));
   P.atol = atol;
   P.rtol = rtol;
   P.pivot = 1;
-  P.k_out = ctx->arena.alloc_n<int64_t>(1);
+  P.k_out = &z->k_out;
   P.seq_len = ctx->tuning.qr_seq_len;
-  LRA_CUDA(cudaMemsetAsync(P.bar, 0, sizeof(GridBar), ctx->stream));
-  LRA_CUDA(cudaMemsetAsync(P.k_out, 0, sizeof(int64_t), ctx->stream));
   QrV2Extra& X = q.job.X;
   X.piv = ctx->arena.alloc_n<int64_t>(std::max<int64_t>(P.kmax, 1));
-  X.nfac = ctx->arena.alloc_n<int64_t>(1);
+  X.nfac = &z->nfac;
   X.part_k = ctx->arena.alloc_n<long long>(G);
   X.beta = ctx->arena.alloc_n<double>(std::max<int64_t>(P.kmax, 1));
-  LRA_CUDA(cudaMemsetAsync(X.nfac, 0, sizeof(int64_t), ctx->stream));
   q.col_at = ctx->arena.alloc_n<int64_t>(n);
   q.pos = ctx->arena.alloc_n<int64_t>(n);
-  const unsigned gi = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, ctx->num_sms * 4));
-  iota_kernel<<<gi, 256, 0, ctx->stream>>>(n, q.col_at, q.pos);
-  post_launch(ctx, "iota_kernel");
   // the sketch at a power-of-two scale in the kernel's arithmetic
   double* vn0 = ctx->arena.alloc_n<double>(n);
   q.scale = ctx->arena.alloc_n<double>(1);
-  unsigned long long* mx = ctx->arena.alloc_n<unsigned long long>(1);
-  LRA_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned long long), ctx->stream));
   q.gm = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, ctx->num_sms * 8));
-  const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 31) / 32, ctx->num_sms * 8));
   QrDf& D = q.job.D;
   D = QrDf{nullptr, nullptr, vn0, q.scale, nullptr};
-  if constexpr (sizeof(T) == 8) {
-    const double* Bd = reinterpret_cast<const double*>(A);
-    absmax_cols_kernel<double><<<q.gm, 256, 0, ctx->stream>>>(m, n, Bd, lda, mx);
-    post_launch(ctx, "absmax_cols_kernel");
-    df_scale_kernel<<<1, 1, 0, ctx->stream>>>(mx, q.scale);
-    post_launch(ctx, "df_scale_kernel");
-    D.Bh = ctx->arena.alloc_n<float>((size_t)m * n);
-    D.Bl = ctx->arena.alloc_n<float>((size_t)m * n);
-    df_split_kernel<<<gs, 256, 0, ctx->stream>>>(m, n, Bd, lda, q.scale, D.Bh, D.Bl, m, vn0);
-    post_launch(ctx, "df_split_kernel");
-  } else {
-    const float* Bf = reinterpret_cast<const float*>(A);
-    absmax_cols_kernel<float><<<q.gm, 256, 0, ctx->stream>>>(m, n, Bf, lda, mx);
-    post_launch(ctx, "absmax_cols_kernel");
-    df_scale_kernel<<<1, 1, 0, ctx->stream>>>(mx, q.scale);
-    post_launch(ctx, "df_scale_kernel");
-    D.Bh = ctx->arena.alloc_n<float>((size_t)m * n);
-    f32_split_kernel<<<gs, 256, 0, ctx->stream>>>(m, n, Bf, lda, q.scale, D.Bh, m, vn0);
-    post_launch(ctx, "f32_split_kernel");
-  }
+  D.Bh = ctx->arena.alloc_n<float>((size_t)m * n);
+  if constexpr (sizeof(T) == 8) D.Bl = ctx->arena.alloc_n<float>((size_t)m * n);
+  prep = SmPrep{m, n, lda, A, &z->mx, q.scale, D.Bh, D.Bl, vn0, q.col_at, q.pos};
   QrSm& S = q.job.S;
   S = QrSm{nullptr, nullptr};
   if (trace_on()) {
@@ -3543,12 +3573,26 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, int64_t m, int64_t n, T* A, int64_t ld
     S.pubt = ctx->arena.alloc_n<unsigned long long>((size_t)G * km);
     LRA_CUDA(cudaMemsetAsync(S.pubt, 0, (size_t)G * km * 8, ctx->stream));
   }
-  // the exchange: four slots, a 128-byte line each
-  S.slot = ctx->arena.alloc_n<ulonglong2>(32);
+  S.slot = z->slot;
   S.stage = ctx->arena.alloc_n<E>((size_t)2 * G * m);
-  LRA_CUDA(cudaMemsetAsync(S.slot, 0, 32 * sizeof(ulonglong2), ctx->stream));
   q.job.G = G;
   q.job.off = 0;
+}
+
+// the zeroed blocks of `count` sketches and, once all are prepared, their conversions
+inline SmZero* sm_zeros(lra_ctx* ctx, int count) {
+  SmZero* z = reinterpret_cast<SmZero*>(ctx->arena.alloc((size_t)count * sizeof(SmZero)));
+  LRA_CUDA(cudaMemsetAsync(z, 0, (size_t)count * sizeof(SmZero), ctx->stream));
+  return z;
+}
+template <typename T>
+void sm_convert(lra_ctx* ctx, const SmPreps& P, int count, int64_t n) {
+  const unsigned gm = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, ctx->num_sms * 8));
+  const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 31) / 32, ctx->num_sms * 8));
+  sm_prep_max_kernel<T><<<dim3(gm, (unsigned)count), 256, 0, ctx->stream>>>(P);
+  post_launch(ctx, "sm_prep_max_kernel");
+  sm_prep_split_kernel<T><<<dim3(gs, (unsigned)count), 256, 0, ctx->stream>>>(P);
+  post_launch(ctx, "sm_prep_split_kernel");
 }
 
 // one cooperative launch for nq prepared sketches (CTAs laid out in order)
@@ -3665,8 +3709,10 @@ int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* st, int64_t nb, d
   std::vector<SmQr<T>> q(count);
   std::vector<SmQr<T>*> qp(count);
   size_t smem = 0;
+  SmZero* z = sm_zeros(ctx, count);
+  SmPreps preps;
   for (int i = 0; i < count; ++i) {
-    sm_prepare<T>(ctx, q[i], st[i].m, st[i].n, st[i].A, st[i].lda, st[i].jpvt, st[i].tau, st[i].kmax, nb, atol,
+    sm_prepare<T>(ctx, q[i], z + i, preps.j[i], st[i].m, st[i].n, st[i].A, st[i].lda, st[i].jpvt, st[i].tau, st[i].kmax, nb, atol,
                   rtol, G[i]);
     q[i].job.S.success = success;
     q[i].job.S.job = i;
@@ -3675,6 +3721,7 @@ int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* st, int64_t nb, d
     qp[i] = &q[i];
     smem = std::max(smem, q[i].smem);
   }
+  sm_convert<T>(ctx, preps, count, st[0].n);
   if (smem > cap || !sm_resident<Ar>(ctx, smem)) fail(LRA_ECUDA, "geqp3_adap_steps: the launch cannot be resident");
   sm_launch<T>(ctx, qp.data(), count);
   std::vector<int64_t> kk(count);
@@ -3770,7 +3817,9 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     const size_t need = sm_smem<Ar>(m, (n + G - 1) / G);
     if (need <= sm_capacity<Ar>(ctx) && sm_resident<Ar>(ctx, need)) {
       SmQr<T> q;
-      sm_prepare<T>(ctx, q, m, n, A, lda, jpvt, tau, P.kmax, nb, atol, rtol, G);
+      SmPreps preps;
+      sm_prepare<T>(ctx, q, sm_zeros(ctx, 1), preps.j[0], m, n, A, lda, jpvt, tau, P.kmax, nb, atol, rtol, G);
+      sm_convert<T>(ctx, preps, 1, n);
       q.job.P.stop_at = stop_at;
       SmQr<T>* qp = &q;
       sm_launch<T>(ctx, &qp, 1);
