@@ -131,18 +131,6 @@ __device__ __forceinline__ void st_word(ulonglong2* p, unsigned long long x, uns
   asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.release.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
                : "memory");
 }
-__device__ __forceinline__ void st_word_relaxed(ulonglong2* p, unsigned long long x, unsigned long long y) {
-  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(x), "l"(y)
-               : "memory");
-}
-__device__ __forceinline__ ulonglong2 ld_word_acquire(const ulonglong2* p) {
-  ulonglong2 v;
-  asm volatile("{\n .reg .b128 t;\n ld.acquire.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
-               : "=l"(v.x), "=l"(v.y)
-               : "l"(p)
-               : "memory");
-  return v;
-}
 __device__ __forceinline__ ulonglong2 ld_word(const ulonglong2* p) {
   ulonglong2 v;
   asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
@@ -150,6 +138,16 @@ __device__ __forceinline__ ulonglong2 ld_word(const ulonglong2* p) {
                : "l"(p)
                : "memory");
   return v;
+}
+
+// two 64-bit words, each for itself and in no particular order
+__device__ __forceinline__ ulonglong2 ld_pair_acquire(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("ld.acquire.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_pair(ulonglong2* p, unsigned long long x, unsigned long long y) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
 }
 
 // Grid barrier for cooperative launches (all CTAs co-resident).  The wait

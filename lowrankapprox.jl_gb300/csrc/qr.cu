@@ -1624,11 +1624,15 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV
 // the winning candidate's column: each CTA stages its best candidate's
 // remaining rows in global memory, raises the exchange's maximum with its
 // word (norm key, column), and then arrives, counting its stop flag along.
-// Maximum and arrivals share 16 bytes, so the read that sees the last arrival
-// has the winner (a separate arrival counter cost a second L2 round trip, 0.7 us
-// of the 6.9 us a short pivot took; a fence of its own before the maximum 0.4
-// us); readers then load the winner's staged rows.  Slots rotate over four
-// exchanges and staged columns over two, so a CTA that runs ahead never
+// A read takes arrivals and maximum together, as a vector of two 64-bit words.
+// Such a read may take the maximum first, so the one that sees the last arrival
+// only says who has very likely won: the CTA goes on with that and loads the
+// staged rows, while a second read of the maximum, after the acquire and so
+// final, is under way; should it differ, the rows are loaded again from the CTA it
+// names.  (Waiting for it costs a second L2 round trip, 0.7 us of the 6.9 us a
+// short pivot took; one 64-bit word a CTA that every CTA reads: the ID of 65536 x
+// 4096 Float32 9.68 ms, 9.31 so.)  A word is only accessed by its 64 bits.
+// Slots rotate over four exchanges and staged columns over two, so a CTA that runs ahead never
 // overwrites what a slower CTA still reads.  The key keeps the 38
 // leading bits of the double-float norm (relative resolution 2^-30, far
 // below the error of the downdated norms); ties go to the smaller column
@@ -1636,7 +1640,7 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV
 struct QrSm {
   // the exchange, zeroed before the launch: exchange e in slot[(e % 4) * 8] (a
   // 128-byte line each), its largest word in x, in y the arrivals (low half) and
-  // how many of them stop (high half): one 16-byte read takes all three
+  // how many of them stop (high half)
   ulonglong2* slot;
   void* stage;               // [2][G][m] staged candidate columns (elements of the arithmetic)
   unsigned long long* pubt;  // LRA_TRACE: %globaltimer of each CTA's word per pivot, [kmax][G], or null
@@ -1791,7 +1795,8 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
   __shared__ V s_alpha, s_f, s_tau, s_beta;
   __shared__ double s_red[32];
   __shared__ unsigned long long s_win;
-  __shared__ int s_owner, s_stop, s_ok, s_cancel;
+  __shared__ int s_owner;
+  __shared__ unsigned char s_stop, s_ok, s_cancel, s_again;
   __shared__ double s_taud, s_betad;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t m = P.m, n = P.n, lda = P.lda;
@@ -1887,8 +1892,24 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
     }
     return done;
   };
-  // wait for all G arrivals of exchange e (bounded): the winning word, its
-  // CTA and the OR of the stop flags, in shared memory
+  // the pivot from the exchange's largest word (thread 0)
+  auto set_winner = [&](unsigned long long best, bool ok) {
+    // the winner's CTA: the one whose columns [n b / G, n (b + 1) / G)
+    // hold the winning column
+    const int64_t jw = (int64_t)(XW_IDX - (best & XW_IDX));
+    int own = 0;
+    if ((best & XW_LOW) != 0 && best != XW_CANCEL) {
+      own = (int)(((jw + 1) * (int64_t)G - 1) / n);
+      own = own < 0 ? 0 : (own >= G ? G - 1 : own);
+    }
+    s_win = best;
+    s_owner = own;
+    s_ok = ok && best != XW_CANCEL ? 1 : 0;
+  };
+  // wait for all G arrivals of exchange e (bounded): the winning word (to be
+  // confirmed by `sure`, thread 0's second read), its CTA and the OR of the stop
+  // flags, in shared memory
+  unsigned long long sure = 0;
   auto collect = [&](unsigned e, unsigned long long own_w, bool own_stop) -> bool {
     if (GCOL) {
       // one CTA: its own candidate is the pivot
@@ -1896,6 +1917,7 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
         s_owner = 0;
         s_win = own_w;
         s_stop = own_stop ? 1 : 0;
+        sure = own_w;
       }
       __syncthreads();
       return true;
@@ -1904,15 +1926,14 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
       // a lower step of the launch revealed its rank: this step stops at
       // the next exchange
       const int canc = S.success ? (*((volatile int*)S.success) < S.job ? 1 : 0) : 0;
-      // every CTA's arrival at exchange e, bounded; the read that sees the last
-      // one has the maximum with it (same 16 bytes, raised before the arrival)
+      // every CTA's arrival at exchange e, bounded
       ulonglong2* sl = S.slot + (e & 3) * 8;
       bool ok = true;
-      ulonglong2 v = ld_word_acquire(sl);
+      ulonglong2 v = ld_pair_acquire(sl);
       if ((unsigned)v.y != (unsigned)G) {
         const uint64_t t0 = globaltimer_ns(), lim = wait_limit_ns();
         for (unsigned it = 1;; ++it) {
-          v = ld_word_acquire(sl);
+          v = ld_pair_acquire(sl);
           if ((unsigned)v.y == (unsigned)G) break;
           // the error word and the clock every 16th poll
           if (it & 15) continue;
@@ -1927,24 +1948,14 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
           }
         }
       }
-      const unsigned long long best = v.x;
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(sure) : "l"(&sl->x) : "memory");
       const unsigned fl = (unsigned)(v.y >> 32);
       // every CTA has read exchange e - 1 (each read it before arriving at
       // e): its slot is cleared for exchange e + 3, before this CTA's next
       // arrival releases the clearing
-      if (b == 0 && ok) st_word_relaxed(S.slot + ((e + 3) & 3) * 8, 0ull, 0ull);
-      // the winner's CTA: the one whose columns [n b / G, n (b + 1) / G)
-      // hold the winning column
-      const int64_t jw = (int64_t)(XW_IDX - (best & XW_IDX));
-      int own = 0;
-      if ((best & XW_LOW) != 0 && best != XW_CANCEL) {
-        own = (int)(((jw + 1) * (int64_t)G - 1) / n);
-        own = own < 0 ? 0 : (own >= G ? G - 1 : own);
-      }
-      s_win = best;
-      s_owner = own;
+      if (b == 0 && ok) st_pair(S.slot + ((e + 3) & 3) * 8, 0ull, 0ull);
+      set_winner(v.x, ok);
       s_stop = fl ? 1 : 0;
-      s_ok = ok && best != XW_CANCEL ? 1 : 0;
       s_cancel = canc;
     }
     __syncthreads();
@@ -2005,19 +2016,21 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
     bool stop_block = false, last_small = false;
     while (kk < jb && !stop_block) {
       const int64_t c = j + kk;
-      const int64_t pvt = (int64_t)(XW_IDX - (s_win & XW_IDX));
-      const int owner = s_owner;
+      int64_t pvt;
+      int owner;
       stamp(c, 0);
-      // the pivot column is done; the previous step's deferred-update marks
-      // are cleared (a thread per slot, so each byte has one writer)
-      for (int s = threadIdx.x; s < nloc; s += NT) {
-        unsigned char st = (unsigned char)(s_st[s] & ~ST_UPD);
-        if (owner == b && s == pvt - c0) st |= ST_DONE;
-        s_st[s] = st;
-      }
-      // ---- the pivot column's rows c..m-1 from the winner's stage, and the
-      // per-warp partial sums of squares of rows c+1..m-1
-      {
+      while (true) {
+        pvt = (int64_t)(XW_IDX - (s_win & XW_IDX));
+        owner = s_owner;
+        // the pivot column is done; the previous step's deferred-update marks
+        // are cleared (a thread per slot, so each byte has one writer)
+        for (int s = threadIdx.x; s < nloc; s += NT) {
+          unsigned char st = (unsigned char)(s_st[s] & ~ST_UPD);
+          if (owner == b && s == pvt - c0) st |= ST_DONE;
+          s_st[s] = st;
+        }
+        // ---- the pivot column's rows c..m-1 from the winner's stage, and the
+        // per-warp partial sums of squares of rows c+1..m-1
         const E* src = GCOL ? C + (pvt - c0) * cs : static_cast<const E*>(S.stage) + ((size_t)(e & 1) * G + owner) * m;
         V acc = A::zero();
         for (int64_t i = c + threadIdx.x; i < m; i += NT) {
@@ -2030,8 +2043,17 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc = A::add(acc, A::shfl_xor(acc, o));
         if (lane == 0) s_part[wid] = acc;
+        if (!GCOL && threadIdx.x == 0) s_again = sure != s_win ? 1 : 0;
+        __syncthreads();
+        if (GCOL || !s_again) break;
+        // the maximum was read too early: the same with the final one
+        for (int s = threadIdx.x; s < nloc; s += NT)
+          if (owner == b && s == pvt - c0) s_st[s] &= (unsigned char)~ST_DONE;
+        __syncthreads();
+        if (threadIdx.x == 0) set_winner(sure, true);
+        __syncthreads();
+        if (!s_ok) return;
       }
-      __syncthreads();
       stamp(c, 1);
       const int64_t len = m - c - 1;
       if (wid == 0) {
