@@ -25,7 +25,8 @@
 // of its own two columns, so graded columns stay as accurate as their own
 // scale.  The diagonal blocks of the Gram matrix are carried from round to
 // round (32 x 32 inter-block entries are fresh each round) and formed anew in
-// a sweep's first round.
+// a sweep's first round: a group's CTAs have them in shared memory before they
+// meet, after which its first CTA writes them back rotated.
 
 #include <algorithm>
 #include <cmath>
@@ -209,8 +210,17 @@ __global__ void __launch_bounds__(JNT, 1) jacobi_gram_kernel(const JgParams P) {
       phase(-1);
       // a block paired with none has only its own column pairs to rotate
       if (b2 < nblk || first) {
-        // ---- partial Gram blocks of this CTA's rows
+        // ---- partial Gram blocks of this CTA's rows; the diagonal blocks, settled
+        // by the grid's barrier, are on their way meanwhile
         const int nprod = first ? 3 : 1;
+        float aa[JB * JB / JNT], bb[JB * JB / JNT];
+        if (!first) {
+#pragma unroll
+          for (int h = 0; h < JB * JB / JNT; ++h) {
+            aa[h] = __ldcg(P.diag + (size_t)b1 * JB * JB + threadIdx.x + h * JNT);
+            bb[h] = __ldcg(P.diag + (size_t)b2 * JB * JB + threadIdx.x + h * JNT);
+          }
+        }
         for (int pr = 0; pr < nprod; ++pr) {
           f2 acc[8][4];
 #pragma unroll
@@ -239,6 +249,16 @@ __global__ void __launch_bounds__(JNT, 1) jacobi_gram_kernel(const JgParams P) {
 #pragma unroll
             for (int w = 0; w < JNW; ++w) s += tile1[w * JB * JB + e];
             __stcg(dst + e, s);
+          }
+          // the diagonal blocks are in G before this CTA arrives at the meeting:
+          // after it rank 0 overwrites them
+          if (!first) {
+#pragma unroll
+            for (int h = 0; h < JB * JB / JNT; ++h) {
+              const int e = threadIdx.x + h * JNT, i = e / JB, j = e % JB;
+              G[i * JGS + j] = aa[h];
+              G[(JB + i) * JGS + JB + j] = bb[h];
+            }
           }
           __syncthreads();
         }
@@ -279,17 +299,14 @@ __global__ void __launch_bounds__(JNT, 1) jacobi_gram_kernel(const JgParams P) {
         // ---- G = [AA AB; AB' BB]
         {
           // every load in flight at once
-          float ab[JB * JB / JNT][JMAXC], aa[JB * JB / JNT], bb[JB * JB / JNT];
+          float ab[JB * JB / JNT][JMAXC];
 #pragma unroll
           for (int h = 0; h < JB * JB / JNT; ++h) {
             const int e = threadIdx.x + h * JNT;
             const float* src = P.part + (size_t)group * P.c * 3 * JB * JB + e;
 #pragma unroll
             for (int q = 0; q < JMAXC; ++q) ab[h][q] = q < P.c ? __ldcg(src + (size_t)q * 3 * JB * JB) : 0.f;
-            if (!first) {
-              aa[h] = __ldcg(P.diag + (size_t)b1 * JB * JB + e);
-              bb[h] = __ldcg(P.diag + (size_t)b2 * JB * JB + e);
-            } else {
+            if (first) {
               aa[h] = bb[h] = 0.f;
               for (int q = 0; q < P.c; ++q) {
                 aa[h] += __ldcg(src + ((size_t)q * 3 + 1) * JB * JB);
@@ -303,8 +320,10 @@ __global__ void __launch_bounds__(JNT, 1) jacobi_gram_kernel(const JgParams P) {
             float s = 0;
 #pragma unroll
             for (int q = 0; q < JMAXC; ++q) s += ab[h][q];
-            G[i * JGS + j] = aa[h];
-            G[(JB + i) * JGS + JB + j] = bb[h];
+            if (first) {
+              G[i * JGS + j] = aa[h];
+              G[(JB + i) * JGS + JB + j] = bb[h];
+            }
             G[i * JGS + JB + j] = s;
             G[(JB + j) * JGS + i] = s;
           }

@@ -56,3 +56,38 @@ def test_gram_sweeps_clusters(lra):
         assert np.abs(F.S - s).max() <= 1e-11
         defect.append(max(np.abs(Q.T @ Q - np.eye(90)).max() for Q in (np.asarray(F.U), np.asarray(F.Vt).T)))
     assert defect[0] <= 4 * defect[1] + 1e-10
+
+
+def test_gram_sweeps_beside_another_request(lra):
+    """Two requests at once, each with the other's kernels on its SMs: the CTAs of
+    a pair of blocks take the same rotations however far apart they run, so
+    both give the bits of a call alone."""
+    import threading
+    mats = [_matrix(k + 300, k + 150, k, k)[0] for k in (449, 640, 385)]
+
+    def run(A):
+        ctx = lra.Context(0)
+        F = lra.psvdfact(A, lra.LRAOptions(rtol=1e-10, precision="mixed", seed=3), ctx=ctx)
+        assert ctx.kernel_launches("jacobi_gram_kernel") == 1
+        out = [np.array(F.U), np.array(F.S), np.array(F.Vt)]
+        ctx.close()
+        return out
+
+    ref = [run(A) for A in mats]
+    bad = []
+
+    def work(t):
+        try:
+            for i in range(9):
+                q = (i + t) % len(mats)
+                if not all(np.array_equal(x, y) for x, y in zip(run(mats[q]), ref[q])):
+                    bad.append((t, i))
+        except Exception as e:  # noqa: BLE001
+            bad.append(repr(e))
+
+    ts = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad, bad
