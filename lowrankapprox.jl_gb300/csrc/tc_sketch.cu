@@ -127,6 +127,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   return true;
 }
 
+// A wait for copies or products that this CTA has issued, before it leaves: it
+// goes on when another wait has given up, and at least for the default limit,
+// since what is under way ends by itself in microseconds and must not land in
+// shared memory or TMEM that the CTA has given back.
+__device__ __forceinline__ void mbar_settle(uint64_t* bar, uint32_t parity, int* err) {
+  if (mbar_try_wait(bar, parity)) return;
+  const uint64_t t0 = globaltimer_ns(), lim = wait_limit_ns() > kWaitLimitNs ? wait_limit_ns() : kWaitLimitNs;
+  while (!mbar_try_wait(bar, parity))
+    if (globaltimer_ns() - t0 > lim) {
+      atomicCAS(err, 0, 4);
+      return;
+    }
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -273,9 +287,8 @@ __device__ __forceinline__ void tc_sketch_body(const CUtensorMap* tmA, const CUt
           tma_load_3d(st + S_BYTES + q * TILE_BYTES, tmA, (kb0 + kb) * KBLK, (int)(n_tile * TILE_M), q, full + s);
       }
       // no copy may still be landing in shared memory when the CTA exits
-      int dummy = 0;
       for (int kb = issued - NSTAGE; kb < issued; ++kb)
-        if (kb >= 0) mbar_wait(full + kb % NSTAGE, (kb / NSTAGE) & 1, &dummy);
+        if (kb >= 0) mbar_settle(full + kb % NSTAGE, (kb / NSTAGE) & 1, P.err);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -313,8 +326,7 @@ __device__ __forceinline__ void tc_sketch_body(const CUtensorMap* tmA, const CUt
       }
       // every issued MMA has completed before TMEM is released
       mma_commit(mma_done);
-      int dummy = 0;
-      mbar_wait(mma_done, 0, &dummy);
+      mbar_settle(mma_done, 0, P.err);
     }
   } else {
     // ---------------- drain / epilogue: warps 2..9 ----------------
@@ -987,10 +999,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (!ok) break;
       }
       // no copy is in flight when the CTA ends
-      int dummy = 0;
       for (int g = 0; g < 3; ++g) {
         const int n = (issued + 2 - g) / 3;  // loads of third g
-        if (n > 0) mbar_wait(full + g, (n - 1) & 1, &dummy);
+        if (n > 0) mbar_settle(full + g, (n - 1) & 1, P.err);
       }
     }
   } else if (warp == 1) {
@@ -1035,8 +1046,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if ((it % G_CHUNK) == G_CHUNK - 1 || it == nloc - 1) mma_commit(acc_ready);
       }
       mma_commit(mma_done);
-      int dummy = 0;
-      mbar_wait(mma_done, 0, &dummy);
+      mbar_settle(mma_done, 0, P.err);
     }
   } else {
     const int q4 = warp & 3;
