@@ -232,11 +232,13 @@ int lra_ctx_get_tuning(const lra_ctx* ctx, char* buf, int64_t len);
    device: it applies to every context on ctx's device.  Failure detection
    of this engine, no counterpart in the reference.                         */
 int lra_ctx_set_wait_limit(lra_ctx* ctx, int64_t ns);
-/* Self-test of the bounded waits: a two-CTA cooperative kernel meets at a
-   grid barrier whose arrival count starts at the grid size, so no arrival
-   completes it; both CTAs wait out the limit above and return.  Returns
-   LRA_ETIMEDOUT when that happened as designed; any other status means the
-   bounded-wait machinery misbehaved.                                       */
+/* Self-test of the bounded waits, in every part of the library that has its
+   own copy of the limit above: two-CTA cooperative kernels meet at a grid
+   barrier whose arrival count starts at the grid size, so no arrival
+   completes it, and wait for a word that nobody raises or (column exchange
+   of the pivoted QRs) for a CTA that never offers; all waits end by the
+   limit and both CTAs return.  Returns LRA_ETIMEDOUT when that happened as
+   designed; any other status means the bounded-wait machinery misbehaved.  */
 int lra_ctx_probe_wait(lra_ctx* ctx);
 
 /* LRAOptions(T) defaults (src/LowRankApprox.jl:96-119) */

@@ -5,6 +5,7 @@
 // the singular / eigen values that decide the truncation).
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -2294,6 +2295,33 @@ lra_psvd* ccur_middle(lra_ctx* ctx, int64_t m, int64_t n, const void* A, int64_t
 }  // namespace
 }  // namespace lra
 
+namespace {
+
+std::array<WaitUnit, 6> wait_units() {
+  return {wait_unit_qr(), wait_unit_cplx(), wait_unit_dense(), wait_unit_tc(), wait_unit_snorm(), wait_unit_jg()};
+}
+
+// runs a probe; its error word (4: the waits ran out) and how many CTAs returned
+int probe_wait(lra_ctx* ctx, const void* kernel, int* returned) {
+  const ArenaMark mark = ctx->arena.mark();
+  // a GridBar whose count starts at the grid size, 1 KB of zeros, the count of returns
+  int init[4 + 256 + 1] = {2};
+  int* d = ctx->arena.alloc_n<int>(4 + 256 + 4);
+  int *bar = d, *zeros = d + 4, *ret = d + 4 + 256;
+  LRA_CUDA(cudaMemcpyAsync(d, init, sizeof init, cudaMemcpyHostToDevice, ctx->stream));
+  void* args[] = {&bar, &zeros, &ret};
+  LRA_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(2), dim3(32), args, 0, ctx->stream));
+  post_launch(ctx, "probe_wait_kernel");
+  int hb[4] = {0, 0, 0, 0};
+  LRA_CUDA(cudaMemcpyAsync(hb, bar, sizeof hb, cudaMemcpyDeviceToHost, ctx->stream));
+  LRA_CUDA(cudaMemcpyAsync(returned, ret, sizeof *returned, cudaMemcpyDeviceToHost, ctx->stream));
+  LRA_CUDA(cudaStreamSynchronize(ctx->stream));
+  ctx->arena.release(mark);
+  return hb[2];
+}
+
+}  // namespace
+
 extern "C" {
 
 const char* lra_status_string(int s) {
@@ -2396,10 +2424,9 @@ int lra_ctx_set_wait_limit(lra_ctx* ctx, int64_t ns) {
     ctx->last_error = "wait limit < 0";
     return LRA_EINVAL;
   }
-  if (cudaSetDevice(ctx->device) != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess ||
-      set_wait_limit_qr((uint64_t)ns) != cudaSuccess || set_wait_limit_dense((uint64_t)ns) != cudaSuccess ||
-      set_wait_limit_tc((uint64_t)ns) != cudaSuccess || set_wait_limit_snorm((uint64_t)ns) != cudaSuccess ||
-      set_wait_limit_jg((uint64_t)ns) != cudaSuccess) {
+  bool ok = cudaSetDevice(ctx->device) == cudaSuccess && cudaStreamSynchronize(ctx->stream) == cudaSuccess;
+  for (const WaitUnit& u : wait_units()) ok = ok && u.set((uint64_t)ns) == cudaSuccess;
+  if (!ok) {
     ctx->last_error = cudaGetErrorString(cudaGetLastError());
     return LRA_ECUDA;
   }
@@ -2408,16 +2435,26 @@ int lra_ctx_set_wait_limit(lra_ctx* ctx, int64_t ns) {
 }
 
 int lra_ctx_probe_wait(lra_ctx* ctx) {
-  int returned = 0, err = 0;
-  const int st = guarded(ctx, [&] { err = probe_grid_wait(ctx, &returned); });
+  std::string bad;
+  const int st = guarded(ctx, [&] {
+    for (const WaitUnit& u : wait_units())
+      for (const void* kernel : u.probe) {
+        if (!kernel || !bad.empty()) continue;
+        int returned = 0;
+        const int err = probe_wait(ctx, kernel, &returned);
+        if (err != 4 || returned != 2) {
+          char msg[128];
+          std::snprintf(msg, sizeof msg, "probe: unexpected state in %s (err %d, %d CTAs returned)", u.name, err, returned);
+          bad = msg;
+        }
+      }
+  });
   if (st != LRA_OK) return st;
-  if (err == 4 && returned == 2) {
-    ctx->last_error = "probe: the grid barrier's bounded wait ran out and both CTAs returned";
+  if (bad.empty()) {
+    ctx->last_error = "probe: every unit's bounded waits ran out and both CTAs returned";
     return LRA_ETIMEDOUT;
   }
-  char msg[128];
-  std::snprintf(msg, sizeof msg, "probe: unexpected barrier state (err %d, %d CTAs returned)", err, returned);
-  ctx->last_error = msg;
+  ctx->last_error = bad;
   return LRA_ECUDA;
 }
 

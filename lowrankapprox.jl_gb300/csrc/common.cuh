@@ -150,6 +150,22 @@ __device__ __forceinline__ void st_pair(ulonglong2* p, unsigned long long x, uns
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
 }
 
+// waits until *word, which counts up, has reached `target`; bounded: on time-out it
+// records LRA_ETIMEDOUT (4) in `err`, and it gives up (false) once that is set
+__device__ __forceinline__ bool wait_reached(const unsigned* word, unsigned target, int* err) {
+  uint64_t t0 = 0;
+  for (unsigned it = 1;; ++it) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+    if ((int)(v - target) >= 0) return true;
+    if (it & 15) continue;  // the error word and the clock every 16th poll
+    const uint64_t t = globaltimer_ns();
+    if (t0 == 0) t0 = t;
+    if (t - t0 > wait_limit_ns()) atomicCAS(err, 0, 4);
+    if (*((volatile int*)err) != 0) return false;
+  }
+}
+
 // Grid barrier for cooperative launches (all CTAs co-resident).  The wait
 // is bounded: on time-out it records LRA_ETIMEDOUT (4) in `err` and every
 // CTA leaves; callers return when it yields false.

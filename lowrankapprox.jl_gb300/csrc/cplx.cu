@@ -15,6 +15,7 @@
 #include "cplx.cuh"
 #include "internal.hpp"
 #include "qr_cols.cuh"
+#include "waits.cuh"
 
 namespace lra {
 
@@ -1420,5 +1421,9 @@ void ccluster_orth(lra_ctx* ctx, int64_t n, int64_t k, cx<R>* Z, int64_t ldz, co
 INSTC(float)
 INSTC(double)
 #undef INSTC
+
+WaitUnit wait_unit_cplx() {
+  return this_wait_unit("cplx", (const void*)probe_col_exchange_kernel<C<double>>);
+}
 
 }  // namespace lra

@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "df64.cuh"
 #include "internal.hpp"
+#include "waits.cuh"
 
 namespace lra {
 
@@ -1247,18 +1248,7 @@ __global__ void __launch_bounds__(JBT * 64) jacobi_block_df_kernel(JacDf P) {
         if (st < 2) {
           const int b = st == 0 ? b1 : b2;
           if (b < nblk) {
-            uint64_t t0 = 0;
-            for (int it = 1;; ++it) {
-              unsigned v;
-              asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.done + b) : "memory");
-              if (v >= gen) break;
-              if ((it & 63) == 0) {
-                const uint64_t t = globaltimer_ns();
-                if (t0 == 0) t0 = t;
-                if (t - t0 > wait_limit_ns()) atomicCAS(&P.bar->err, 0, 4);
-                if (*((volatile int*)&P.bar->err) != 0) break;
-              }
-            }
+            wait_reached(P.done + b, gen, &P.bar->err);
           }
         }
         side_sync();
@@ -2671,6 +2661,6 @@ template void trsm_bs<double>(lra_ctx*, int64_t, int64_t, const double*, int64_t
 template void trsm_left_diag<float>(lra_ctx*, int, int64_t, const float*, int64_t, float*, int64_t);
 template void trsm_left_diag<double>(lra_ctx*, int, int64_t, const double*, int64_t, double*, int64_t);
 
-cudaError_t set_wait_limit_dense(uint64_t ns) { return set_unit_wait_limit(ns); }
+WaitUnit wait_unit_dense() { return this_wait_unit("dense"); }
 
 }  // namespace lra

@@ -474,15 +474,20 @@ double snorm_power(lra_ctx* ctx, int64_t m, int64_t n, const T* A, int64_t lda, 
 inline void count_launch(lra_ctx* ctx, int n = 1) { ctx->launches += n; }
 void post_launch(lra_ctx* ctx, const char* name);
 
-// the bounded-wait limit of each translation unit that waits (ns; 0: the
-// default), and the grid-barrier self-test: returns the barrier's error
-// word (4 when its wait ran out) and the number of CTAs that returned
-cudaError_t set_wait_limit_qr(uint64_t ns);
-cudaError_t set_wait_limit_dense(uint64_t ns);
-cudaError_t set_wait_limit_tc(uint64_t ns);
-cudaError_t set_wait_limit_snorm(uint64_t ns);
-cudaError_t set_wait_limit_jg(uint64_t ns);
-int probe_grid_wait(lra_ctx* ctx, int* returned);
+// the translation units that wait: the limit of each one's bounded waits (ns; 0:
+// the default) and its probes, kernels (GridBar*, 1 KB of zeros, int* returned) of
+// two CTAs whose waits nothing ends
+struct WaitUnit {
+  const char* name;
+  cudaError_t (*set)(uint64_t ns);
+  const void* probe[2];
+};
+WaitUnit wait_unit_qr();
+WaitUnit wait_unit_cplx();
+WaitUnit wait_unit_dense();
+WaitUnit wait_unit_tc();
+WaitUnit wait_unit_snorm();
+WaitUnit wait_unit_jg();
 
 // the tuning table: defaults, then the file named by LRA_TUNING or the
 // table beside liblra.so (tuning_gb300.txt); the source is recorded

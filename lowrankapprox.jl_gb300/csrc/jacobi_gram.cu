@@ -34,6 +34,7 @@
 
 #include "common.cuh"
 #include "internal.hpp"
+#include "waits.cuh"
 
 namespace lra {
 
@@ -270,21 +271,8 @@ __global__ void __launch_bounds__(JNT, 1) jacobi_gram_kernel(const JgParams P) {
           const unsigned target = meets * (unsigned)P.c;
           __threadfence();
           atomicAdd(cnt, 1u);
-          bool ok = true;
-          const uint64_t t0 = globaltimer_ns(), lim = wait_limit_ns();
-          for (unsigned it = 1;; ++it) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(cnt) : "memory");
-            if ((int)(v - target) >= 0) break;
-            if (it & 15) continue;
-            if (*((volatile int*)&P.bar->err) != 0 || globaltimer_ns() - t0 > lim) {
-              atomicCAS(&P.bar->err, 0, 4);
-              ok = false;
-              break;
-            }
-          }
+          s_ok = wait_reached(cnt, target, &P.bar->err);
           __threadfence();
-          s_ok = ok;
         }
         __syncthreads();
         if (!s_ok) return;
@@ -570,7 +558,7 @@ __global__ void __launch_bounds__(JNT, 1) jacobi_gram_kernel(const JgParams P) {
 
 }  // namespace
 
-cudaError_t set_wait_limit_jg(uint64_t ns) { return set_unit_wait_limit(ns); }
+WaitUnit wait_unit_jg() { return this_wait_unit("jacobi_gram"); }
 
 // X (n x n) and V (n x n, the identity on entry) with one leading dimension,
 // a multiple of 4, rows n .. ld zero; false when the shape does not fit

@@ -33,6 +33,7 @@
 #include "df64.cuh"
 #include "internal.hpp"
 #include "qr_cols.cuh"
+#include "waits.cuh"
 
 namespace lra {
 
@@ -4079,44 +4080,7 @@ void col_norms(lra_ctx* ctx, int64_t m, int64_t n, const T* A, int64_t lda, T* o
   post_launch(ctx, "col_norms_kernel");
 }
 
-// ---- bounded waits: the limit in force, and a self-test ----------------------------
-
-cudaError_t set_wait_limit_qr(uint64_t ns) { return set_unit_wait_limit(ns); }
-
-namespace {
-
-// Two CTAs meet at a grid barrier whose arrival count starts at the grid
-// size, so that no arrival completes it: both wait until the limit runs
-// out, the barrier records the time-out and every CTA returns.
-__global__ void probe_wait_kernel(GridBar* gb, int* returned) {
-  if (!grid_sync(gb)) {
-    if (threadIdx.x == 0) atomicAdd(returned, 1);
-    return;
-  }
-  if (threadIdx.x == 0) atomicAdd(returned, 1000);  // the barrier completed: not expected
-}
-
-}  // namespace
-
-int probe_grid_wait(lra_ctx* ctx, int* returned) {
-  const ArenaMark mark = ctx->arena.mark();
-  GridBar* gb = reinterpret_cast<GridBar*>(ctx->arena.alloc(sizeof(GridBar)));
-  int* ret = ctx->arena.alloc_n<int>(1);
-  static const GridBar init{2u, 0u, 0, 0};
-  LRA_CUDA(cudaMemcpyAsync(gb, &init, sizeof init, cudaMemcpyHostToDevice, ctx->stream));
-  LRA_CUDA(cudaMemsetAsync(ret, 0, sizeof(int), ctx->stream));
-  void* args[] = {&gb, &ret};
-  LRA_CUDA(cudaLaunchCooperativeKernel((const void*)probe_wait_kernel, dim3(2), dim3(32), args, 0, ctx->stream));
-  post_launch(ctx, "probe_wait_kernel");
-  GridBar hb;
-  int hr = 0;
-  LRA_CUDA(cudaMemcpyAsync(&hb, gb, sizeof hb, cudaMemcpyDeviceToHost, ctx->stream));
-  LRA_CUDA(cudaMemcpyAsync(&hr, ret, sizeof hr, cudaMemcpyDeviceToHost, ctx->stream));
-  LRA_CUDA(cudaStreamSynchronize(ctx->stream));
-  ctx->arena.release(mark);
-  *returned = hr;
-  return hb.err;
-}
+WaitUnit wait_unit_qr() { return this_wait_unit("qr", (const void*)probe_col_exchange_kernel<double>); }
 
 // ---- pivoted QR without any device allocation --------------------------------------
 //

@@ -138,4 +138,18 @@ __device__ __forceinline__ bool col_exchange(ColXchShared& s, const ColXch<E>& x
   return s.bad == 0;
 }
 
+// Of two blocks one offers and the other never does: the wait runs out.  (gb, zeros,
+// returned: as probe_wait_kernel's)
+template <typename E>
+__global__ void __launch_bounds__(32) probe_col_exchange_kernel(GridBar* gb, unsigned long long* zeros, int* returned) {
+  __shared__ ColXchShared s;
+  if (blockIdx.x == 0) {
+    const ColXch<E> x{reinterpret_cast<ulonglong2*>(zeros), reinterpret_cast<E*>(zeros + 64)};
+    const bool ok = col_exchange<32>(s, x, gb, 0, 0, 1, 1, static_cast<const E*>(nullptr), 0,
+                                     [](int, long long&, int64_t&) {}, [](int) { return 0; });
+    if (threadIdx.x == 0 && ok) atomicAdd(returned, 1000);
+  }
+  if (threadIdx.x == 0) atomicAdd(returned, 1);
+}
+
 }  // namespace lra

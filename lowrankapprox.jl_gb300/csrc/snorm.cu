@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "internal.hpp"
+#include "waits.cuh"
 
 namespace lra {
 
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(PNT, 2) snorm_power_kernel(const PowerArgs<T> 
 
 }  // namespace
 
-cudaError_t set_wait_limit_snorm(uint64_t ns) { return set_unit_wait_limit(ns); }
+WaitUnit wait_unit_snorm() { return this_wait_unit("snorm"); }
 
 template <typename T>
 double snorm_power(lra_ctx* ctx, int64_t m, int64_t n, const T* A, int64_t lda, const T* B, int64_t ldb, bool herm,

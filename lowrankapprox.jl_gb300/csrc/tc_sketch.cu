@@ -40,6 +40,7 @@
 #include "common.cuh"
 #include "draws.cuh"
 #include "internal.hpp"
+#include "waits.cuh"
 
 namespace lra {
 
@@ -1553,6 +1554,6 @@ template void tc_split<double>(lra_ctx*, char, int64_t, int64_t, const double*, 
 template void tc_sketch<float>(lra_ctx*, const TcSplit&, int, const SketchSrc*, const int64_t*, float*, int64_t);
 template void tc_sketch<double>(lra_ctx*, const TcSplit&, int, const SketchSrc*, const int64_t*, double*, int64_t);
 
-cudaError_t set_wait_limit_tc(uint64_t ns) { return set_unit_wait_limit(ns); }
+WaitUnit wait_unit_tc() { return this_wait_unit("tc_sketch"); }
 
 }  // namespace lra
