@@ -61,3 +61,18 @@ def test_same_bits(lra):
         assert a[7] == 1 and b[7] == 0, a
         # (the payload of a NaN is nobody's)
         assert a[:6] == b[:6] and ("nan" in a[2] or a[6] == b[6]), (a, b)
+
+
+def test_tall_sketches_spread_over_all_blocks(lra):
+    """Columns too long for eight a block: they are spread over every block, and
+    stay in shared memory."""
+    code = CODE.replace('("plain", "awkward", "small", "nan", "allnan")', '("plain", "awkward", "nan")')
+    got = []
+    for smem in ("1", "0"):
+        r = subprocess.run([sys.executable, "-c", code.format(root=ROOT, shapes=[(4000, 300, 90, 32), (3600, 200, 40, 32)])],
+                           env=dict(os.environ, LRA_QR_SMEM=smem), capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        got.append(json.loads([x for x in r.stdout.splitlines() if x.startswith("RESULT ")][0][7:]))
+    for a, b in zip(*got):
+        assert a[7] == 1 and b[7] == 0, a
+        assert a[:6] == b[:6] and ("nan" in a[2] or a[6] == b[6]), (a, b)
