@@ -2712,7 +2712,11 @@ __global__ void __launch_bounds__(512) df_prep_max_kernel(const DfPrepJob* __res
 // CTAs (matrix, part): the scaled float pairs and each column's norm, a warp
 // per four columns; a row-major workspace is written through a shared tile of
 // 32 columns (a column's rows are a row of the workspace apart: 8-byte stores
-// into 32 different sectors otherwise)
+// into 32 different sectors otherwise), but for sketches whose tile is larger than
+// shared memory (rows that only a raised qr_seq_len puts in this layout)
+constexpr int64_t kTileRows = 800;
+__host__ __device__ constexpr size_t tile_bytes(int64_t m) { return (size_t)32 * (m + 1) * sizeof(float2); }
+
 __global__ void __launch_bounds__(256) df_prep_split_kernel(const DfPrepJob* __restrict__ jobs) {
   extern __shared__ float2 prep_tile[];
   const DfPrepJob J = jobs[blockIdx.x];
@@ -2721,7 +2725,7 @@ __global__ void __launch_bounds__(256) df_prep_split_kernel(const DfPrepJob* __r
   const double sc = mx > 0 ? ldexp(1.0, -(ilogb(mx) + 1)) : 1.0;
   const int k = mx > 0 ? -(ilogb(mx) + 1) : 0;
   if (blockIdx.y == 0 && threadIdx.x == 0) *J.scale = sc;
-  const bool rowmaj = J.rs != 1;
+  const bool rowmaj = J.rs != 1 && J.m <= kTileRows;
   const int ts = (int)J.m + 1;
   for (int64_t j0 = (int64_t)blockIdx.y * 32; j0 < J.n; j0 += (int64_t)gridDim.y * 32) {
     const int64_t j = j0 + 4 * wid;
@@ -2739,7 +2743,7 @@ __global__ void __launch_bounds__(256) df_prep_split_kernel(const DfPrepJob* __r
           } else if (rowmaj)
             prep_tile[(4 * wid + g) * ts + i] = make_float2(h, l);
           else
-            J.work[(j + g) * J.cs + i] = make_float2(h, l);
+            J.work[(j + g) * J.cs + i * J.rs] = make_float2(h, l);
           acc[g] = fma(t, t, acc[g]);
         }
     }
@@ -2815,7 +2819,7 @@ __global__ void __launch_bounds__(256) df_finish_group_kernel(const DfFinishJob*
   const DfFinishJob J = jobs[blockIdx.x];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double inv = 1.0 / *J.scale;
-  const bool rowmaj = J.rs != 1;
+  const bool rowmaj = J.rs != 1 && J.m <= kTileRows;
   const int ts = (int)J.m + 1;
   for (int64_t j0 = (int64_t)blockIdx.y * 32; j0 < J.n; j0 += (int64_t)gridDim.y * 32) {
     if (rowmaj) {
@@ -2832,7 +2836,8 @@ __global__ void __launch_bounds__(256) df_finish_group_kernel(const DfFinishJob*
         continue;
       }
       const float2* w = rowmaj ? fin_tile + g * ts : J.work + (j0 + g) * J.cs;
-      for (int64_t i = lane; i < J.m; i += 32) o[i] = df_val(w[i].x, w[i].y) * inv;
+      const int64_t ws = rowmaj ? 1 : J.rs;
+      for (int64_t i = lane; i < J.m; i += 32) o[i] = df_val(w[i * ws].x, w[i * ws].y) * inv;
     }
   }
 }
@@ -3306,7 +3311,7 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
       S.G = G[(size_t)t];
       smem_gang = std::max(smem_gang, sm_smem<QrArithDf>(m, (n + S.G - 1) / S.G));
     }
-    if (rowmaj) smem_tile = std::max(smem_tile, (size_t)32 * (m + 1) * sizeof(float2));
+    if (rowmaj && m <= kTileRows) smem_tile = std::max(smem_tile, tile_bytes(m));
     smem_qr = std::max(smem_qr, (size_t)m * sizeof(float2) + (size_t)n * (5 * 8 + 1));
     smem_fin = std::max(smem_fin, (size_t)2 * n * sizeof(int));
   }

@@ -64,3 +64,30 @@ def test_batch_workspaces(lra):
         W = lra.idfact(A, o, ctx=one)
         one.close()
         assert np.array_equal(V.p, W.p) and np.array_equal(V.T, W.T)
+
+
+def test_batch_long_rows(lra):
+    """A raised qr_seq_len puts long sketches in the row-major workspace, also
+    those whose tile of 32 columns no shared memory holds (order 1032)."""
+    import torch
+    rng = np.random.default_rng(4)
+    mats = []
+    for m, n, k in [(700, 1100, 560), (300, 200, 20)]:
+        A = np.linalg.qr(rng.standard_normal((m, k)))[0] @ np.linalg.qr(rng.standard_normal((n, k)))[0].T
+        mats.append(torch.from_numpy(A).cuda().t().contiguous().t())
+    o = lra.LRAOptions(rtol=1e-9, precision="mixed", seed=3)
+
+    def context():
+        ctx = lra.Context(0)
+        ctx.set_tuning("qr_seq_len", 0, 1200)
+        return ctx
+
+    ctx = context()
+    batch = lra.idfact_batched(mats, o, ctx=ctx)
+    assert ctx.kernel_launches("geqp3_df_group_kernel") >= 1
+    ctx.close()
+    for A, V in zip(mats, batch):
+        one = context()
+        W = lra.idfact(A, o, ctx=one)
+        one.close()
+        assert V.k == W.k and np.array_equal(V.p, W.p) and np.array_equal(V.T, W.T)
