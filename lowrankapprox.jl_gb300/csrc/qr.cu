@@ -1645,6 +1645,7 @@ struct QrSm {
   ulonglong2* slot;
   void* stage;               // [2][G][m] staged candidate columns (elements of the arithmetic)
   unsigned long long* pubt;  // LRA_TRACE: %globaltimer of each CTA's word per pivot, [kmax][G], or null
+  int64_t cs = 0;            // column stride in shared memory
   // several adaptive steps factored by one launch: the lowest index of a
   // step whose rank came out below its threshold (k < nt), shared by the
   // launch's steps, or null; a step whose index is higher stops at its next
@@ -1753,10 +1754,11 @@ struct QrArithF32 {
   __device__ static unsigned long long key38(V v) { return v > 0.f ? (unsigned long long)__float_as_uint(v) << 6 : 0ull; }
 };
 
-// the column stride in shared memory: odd, so that a thread per column (short
-// columns) reads a row from 32 different banks (16-way conflicts at 40 and 72 rows
-// otherwise: 5.0 against 1.7 us of dot products at 72 rows, 338 columns a CTA)
-__host__ __device__ constexpr int64_t sm_stride(int64_t m) { return m | 1; }
+// the column stride in shared memory, where it fits: odd, so that a thread per
+// column (short columns) reads a row from 32 different banks (16-way conflicts at 40
+// and 72 rows otherwise: 5.0 against 1.7 us of dot products at 72 rows, 338
+// columns a CTA)
+constexpr int64_t sm_stride(int64_t m) { return m | 1; }
 
 template <class A>
 __device__ __forceinline__ unsigned long long xw_pack(typename A::V v, int64_t j) {
@@ -1811,7 +1813,7 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
   // element (row i, slot s) at C[s cs + i rs]: column-major in shared
   // memory; the workspace of GCOL may be row-major (coalesced thread-per-
   // column access)
-  const int64_t cs = GCOL ? gcs : sm_stride(m), rs = GCOL ? grs : 1;
+  const int64_t cs = GCOL ? gcs : S.cs, rs = GCOL ? grs : 1;
   V* s_vn1 = reinterpret_cast<V*>(GCOL ? Vc + m : C + ncap * cs);
   V* s_vn2 = s_vn1 + ncap;
   V* s_dot = s_vn2 + ncap;
@@ -3188,9 +3190,9 @@ static void print_qr_trace(lra_ctx* ctx, const unsigned long long* stamps, int64
 // largest first) and the replay into column order.  Each matrix comes out
 // as geqp3_adap leaves it when its shared-memory kernel runs, bit for bit.
 template <class A>
-size_t sm_smem(int64_t m, int64_t ncap);
+size_t sm_smem(int64_t m, int64_t ncap, int64_t cs);
 template <class A>
-int sm_min_ctas(size_t cap, int64_t m, int64_t n);
+int sm_min_ctas(size_t cap, int64_t m, int64_t n, int64_t cs);
 static int qr_sm_cap(const lra_ctx* ctx);
 static int sm_natural_ctas(lra_ctx* ctx, int64_t n);
 
@@ -3237,7 +3239,7 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
   int64_t sum_g = 0;
   for (int64_t t = 0; t < count && gang; ++t) {
     const DfBatchItem& it = items[ord[(size_t)t]];
-    sum_g += G[(size_t)t] = sm_min_ctas<QrArithDf>(cap, it.m, it.n);
+    sum_g += G[(size_t)t] = sm_min_ctas<QrArithDf>(cap, it.m, it.n, sm_stride(it.m));
     gang = G[(size_t)t] > 0 && G[(size_t)t] <= std::min(16, qr_sm_cap(ctx));
   }
   if (gang) {
@@ -3309,7 +3311,8 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
       S.S.slot = slots + 32 * t;
       S.S.stage = ctx->arena.alloc_n<float2>((size_t)2 * G[(size_t)t] * m);
       S.G = G[(size_t)t];
-      smem_gang = std::max(smem_gang, sm_smem<QrArithDf>(m, (n + S.G - 1) / S.G));
+      S.S.cs = sm_stride(m);
+      smem_gang = std::max(smem_gang, sm_smem<QrArithDf>(m, (n + S.G - 1) / S.G, S.S.cs));
     }
     if (rowmaj && m <= kTileRows) smem_tile = std::max(smem_tile, tile_bytes(m));
     smem_qr = std::max(smem_qr, (size_t)m * sizeof(float2) + (size_t)n * (5 * 8 + 1));
@@ -3435,14 +3438,14 @@ template <typename T>
 using SmA = typename std::conditional<sizeof(T) == 8, QrArithDf, QrArithF32>::type;
 constexpr int kSmNT = 512;  // warp 0 for the reflector, 15 column warps
 
-// dynamic shared memory of a CTA holding ncap columns of m rows: the pivot
-// column, the columns, four values, a stored element and a state byte per
+// dynamic shared memory of a CTA holding ncap columns of m rows, a stride of cs
+// entries apart: the pivot column, the columns, four values, a stored element and a state byte per
 // column
 template <class A>
-size_t sm_smem(int64_t m, int64_t ncap) {
+size_t sm_smem(int64_t m, int64_t ncap, int64_t cs) {
   using E = typename A::E;
   using V = typename A::V;
-  return (size_t)(m + ncap * sm_stride(m)) * sizeof(E) + (size_t)ncap * (4 * sizeof(V) + sizeof(E) + 1);
+  return (size_t)(m + ncap * cs) * sizeof(E) + (size_t)ncap * (4 * sizeof(V) + sizeof(E) + 1);
 }
 
 template <class A>
@@ -3476,11 +3479,11 @@ static int sm_natural_ctas(lra_ctx* ctx, int64_t n) {
 
 // the fewest CTAs whose shared memory holds an m x n sketch (0: not one column)
 template <class A>
-int sm_min_ctas(size_t cap, int64_t m, int64_t n) {
+int sm_min_ctas(size_t cap, int64_t m, int64_t n, int64_t cs) {
   using E = typename A::E;
   using V = typename A::V;
   const size_t fixed = (size_t)m * sizeof(E);
-  const size_t per = (size_t)sm_stride(m) * sizeof(E) + 4 * sizeof(V) + sizeof(E) + 1;
+  const size_t per = (size_t)cs * sizeof(E) + 4 * sizeof(V) + sizeof(E) + 1;
   if (cap < fixed + per) return 0;
   const int64_t ncap = (int64_t)((cap - fixed) / per);
   return (int)((n + ncap - 1) / ncap);
@@ -3549,7 +3552,7 @@ __global__ void __launch_bounds__(256) sm_prep_split_kernel(const SmPreps P) {
 
 template <typename T>
 void sm_prepare(lra_ctx* ctx, SmQr<T>& q, SmZero* z, SmPrep& prep, int64_t m, int64_t n, T* A, int64_t lda, int64_t* jpvt, T* tau,
-                int64_t kmax, int64_t nb, double atol, double rtol, int G) {
+                int64_t kmax, int64_t nb, double atol, double rtol, int G, size_t cap) {
   using Ar = SmA<T>;
   using E = typename Ar::E;
   q.m = m;
@@ -3558,7 +3561,9 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, SmZero* z, SmPrep& prep, int64_t m, in
   q.lda = lda;
   q.jpvt = jpvt;
   q.G = G;
-  q.smem = sm_smem<Ar>(m, (n + G - 1) / G);
+  const int64_t ncap = (n + G - 1) / G;
+  const int64_t cs = sm_smem<Ar>(m, ncap, sm_stride(m)) <= cap ? sm_stride(m) : m;
+  q.smem = sm_smem<Ar>(m, ncap, cs);
   QrParams<T>& P = q.job.P;
   P = QrParams<T>{};
   P.m = m;
@@ -3593,7 +3598,7 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, SmZero* z, SmPrep& prep, int64_t m, in
   if constexpr (sizeof(T) == 8) D.Bl = ctx->arena.alloc_n<float>((size_t)m * n);
   prep = SmPrep{m, n, lda, A, &z->mx, q.scale, D.Bh, D.Bl, vn0, q.col_at, q.pos};
   QrSm& S = q.job.S;
-  S = QrSm{nullptr, nullptr};
+  S = QrSm{nullptr, nullptr, nullptr, cs};
   if (trace_on()) {
     const int64_t km = std::max<int64_t>(P.kmax, 1);
     D.stamps = ctx->arena.alloc_n<unsigned long long>((size_t)16 * km);
@@ -3691,19 +3696,26 @@ static bool sm_applies(lra_ctx* ctx, int64_t m, int64_t n) {
   return m - 1 <= vcap;
 }
 
+// how many of `count` steps fit one launch, each on the fewest CTAs that hold it with
+// its columns an odd stride apart or not
 template <typename T>
-int geqp3_steps_fit(lra_ctx* ctx, int count, const int64_t* m, int64_t n) {
+static int sm_steps_fit(lra_ctx* ctx, int count, const int64_t* m, int64_t n, bool odd) {
   using Ar = SmA<T>;
   const size_t cap = sm_capacity<Ar>(ctx);
   int total = 0, fit = 0;
   for (int i = 0; i < count && i < kSmJobs; ++i) {
     if (!sm_applies<T>(ctx, m[i], n)) break;
-    const int g = sm_min_ctas<Ar>(cap, m[i], n);
+    const int g = sm_min_ctas<Ar>(cap, m[i], n, odd ? sm_stride(m[i]) : m[i]);
     if (g <= 0 || g > sm_natural_ctas(ctx, n) || total + g > qr_sm_cap(ctx)) break;
     total += g;
     fit = i + 1;
   }
   return fit;
+}
+
+template <typename T>
+int geqp3_steps_fit(lra_ctx* ctx, int count, const int64_t* m, int64_t n) {
+  return sm_steps_fit<T>(ctx, count, m, n, false);
 }
 
 template <typename T>
@@ -3724,7 +3736,9 @@ int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* st, int64_t nb, d
   // largest, with the most pivots) down
   std::vector<int> G(count);
   int spare = qr_sm_cap(ctx);
-  for (int i = 0; i < count; ++i) spare -= G[i] = sm_min_ctas<Ar>(cap, st[i].m, st[i].n);
+  const bool odd = sm_steps_fit<T>(ctx, count, ms.data(), st[0].n, true) == count;
+  for (int i = 0; i < count; ++i)
+    spare -= G[i] = sm_min_ctas<Ar>(cap, st[i].m, st[i].n, odd ? sm_stride(st[i].m) : st[i].m);
   auto widen = [&](int i) {
     const int more = std::max(0, std::min(spare, sm_natural_ctas(ctx, st[i].n) - G[i]));
     G[i] += more;
@@ -3741,7 +3755,7 @@ int geqp3_adap_steps(lra_ctx* ctx, int count, const QrStep<T>* st, int64_t nb, d
   SmPreps preps;
   for (int i = 0; i < count; ++i) {
     sm_prepare<T>(ctx, q[i], z + i, preps.j[i], st[i].m, st[i].n, st[i].A, st[i].lda, st[i].jpvt, st[i].tau, st[i].kmax, nb, atol,
-                  rtol, G[i]);
+                  rtol, G[i], cap);
     q[i].job.S.success = success;
     q[i].job.S.job = i;
     q[i].job.S.nt = st[i].nt;
@@ -3840,13 +3854,14 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     using Ar = SmA<T>;
     // the CTAs it may take, or the fewest that hold the sketch when those
     // are more
-    const int G = std::min(std::max(sm_natural_ctas(ctx, n), sm_min_ctas<Ar>(sm_capacity<Ar>(ctx), m, n)),
+    const size_t cap = sm_capacity<Ar>(ctx);
+    const int G = std::min(std::max(sm_natural_ctas(ctx, n), sm_min_ctas<Ar>(cap, m, n, sm_stride(m))),
                            std::min(ctx->num_sms, 256));
-    const size_t need = sm_smem<Ar>(m, (n + G - 1) / G);
-    if (need <= sm_capacity<Ar>(ctx) && sm_resident<Ar>(ctx, need)) {
+    const size_t need = sm_smem<Ar>(m, (n + G - 1) / G, m);
+    if (need <= cap && sm_resident<Ar>(ctx, need)) {
       SmQr<T> q;
       SmPreps preps;
-      sm_prepare<T>(ctx, q, sm_zeros(ctx, 1), preps.j[0], m, n, A, lda, jpvt, tau, P.kmax, nb, atol, rtol, G);
+      sm_prepare<T>(ctx, q, sm_zeros(ctx, 1), preps.j[0], m, n, A, lda, jpvt, tau, P.kmax, nb, atol, rtol, G, cap);
       sm_convert<T>(ctx, preps, 1, n);
       q.job.P.stop_at = stop_at;
       SmQr<T>* qp = &q;

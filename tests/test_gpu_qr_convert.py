@@ -91,3 +91,21 @@ def test_batch_long_rows(lra):
         W = lra.idfact(A, o, ctx=one)
         one.close()
         assert V.k == W.k and np.array_equal(V.p, W.p) and np.array_equal(V.T, W.T)
+
+
+def test_conversions_to_pairs(lra):
+    """The same for Float64 in pairs of floats (which a tolerance of zero does not
+    take: the QR is then in FP64)."""
+    eps = 60 * 2.0 ** -46
+    ctx = lra.Context(0)
+    for i, (name, A) in enumerate(_special(np.float64, 7).items()):
+        F = lra.pqrfact(A, lra.LRAOptions(rtol=1e-13, precision="mixed", sketch="none"), ctx=ctx)
+        assert ctx.kernel_launches("geqp3_df_smem_kernel") == i + 1, name
+        sc = 1.0 / np.abs(A).max()
+        A, R = A * sc, F.R * sc
+        assert F.k == 60, name
+        assert np.abs(A[:, F.p - 1] - F.Q @ R).max() <= eps * np.linalg.norm(A, axis=0).max(), name
+        for j in range(F.k):
+            left = np.linalg.norm(R[j:, j + 1:], axis=0)
+            assert left.size == 0 or left.max() <= abs(R[j, j]) * (1 + 1e-5) + eps * abs(R[0, 0]), (name, j)
+    ctx.close()

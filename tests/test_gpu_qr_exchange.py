@@ -61,3 +61,26 @@ def test_two_at_once(lra):
     for t in ts:
         t.join()
     assert not bad, bad
+
+
+def test_widest_sketches(lra):
+    """As many columns as shared memory holds back to back, more than it holds an odd
+    stride apart: the same factors, to the arithmetic, as with room to spare."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    m, n = 40, 630 * sms  # 640 columns a CTA fit at a stride of 40 rows, 626 at 41
+    rng = np.random.default_rng(2)
+    A = np.asfortranarray(rng.standard_normal((m, n)) * 10.0 ** (-2.0 * rng.random(n)))
+    ctx = lra.Context(0)
+    o = lra.LRAOptions(rtol=1e-9, precision="mixed", sketch="none")
+    F = lra.pqrfact(A, o, ctx=ctx)
+    assert ctx.kernel_launches("geqp3_df_smem_kernel") == 1
+    G = lra.pqrfact(np.asfortranarray(A[:, :600 * sms]), o, ctx=ctx)
+    assert ctx.kernel_launches("geqp3_df_smem_kernel") == 2
+    ctx.close()
+    # pairs of floats: 2^-46 an operation, a column sees 40 steps
+    for F, B in ((F, A), (G, A[:, :600 * sms])):
+        assert F.k == m
+        assert np.abs(B[:, F.p - 1] - F.Q @ F.R).max() <= m * 2.0 ** -46 * np.linalg.norm(A, axis=0).max()
+        d = np.abs(np.diag(F.R[:, :m]))
+        assert (d[1:] <= d[:-1] * (1 + 1e-6)).all()
