@@ -1160,6 +1160,7 @@ struct QrXw {
   ulonglong2* word;  // [2][G]
   float2* f;         // [2][G] the candidate's pending f
   float* prev;       // PG: [G][2][m] the previous reflector, each CTA its own
+  int far;           // row c of the columns is read back from memory: no room for s_arc
 };
 
 // PG: the previous reflector in global memory (sketches of more rows than two
@@ -1177,6 +1178,7 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV
   extern __shared__ unsigned char qr_dyn[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int G = (int)gridDim.x, cta = (int)blockIdx.x;
+  const bool far = PG && E.far;
   const int m = (int)P.m, n = (int)P.n;
   const int64_t lda = P.lda;
   auto stamp = [&](int64_t c, int ph) {
@@ -1196,7 +1198,7 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV
   Df* s_vn1 = reinterpret_cast<Df*>(PG ? vl + m : pl + m);
   Df* s_vn2 = s_vn1 + ncap;
   Df* s_arc = s_vn2 + ncap;  // row c of each column after step c
-  Df* s_fp = s_arc + ncap;   // f of the column's pending update (zero: none)
+  Df* s_fp = s_arc + (far ? 0 : ncap);  // f of the column's pending update (zero: none)
   unsigned char* s_st = reinterpret_cast<unsigned char*>(s_fp + ncap);
 
   // the CTA's candidate to all others, theirs back: the pivot (s_pvt) and the OR
@@ -1458,7 +1460,7 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV
           const Df arca = df_add(arcc, Df{-fa.h, -fa.l});
           ah[c] = arca.h;
           al[c] = arca.l;
-          s_arc[cur] = arca;
+          if (!far) s_arc[cur] = arca;
           s_fp[cur] = fa;
         }
       }
@@ -1479,7 +1481,7 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV
         Df v1 = s_vn1[s];
         if (c < lastrk - 1 && v1.h != 0.f) {
           // LAPACK's partial-norm downdate, in double-float
-          const Df a = s_arc[s];
+          const Df a = far ? Df{Bh[(int64_t)jj * lda + c], Bl[(int64_t)jj * lda + c]} : s_arc[s];
           Df temp = df_div(a.h < 0.f ? df_neg(a) : a, v1);
           temp = df_mul(df_add(Df{1.f, 0.f}, temp), df_add(Df{1.f, 0.f}, df_neg(temp)));
           if (temp.h < 0.f) temp = Df{0.f, 0.f};
@@ -3933,14 +3935,15 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     int64_t* step_of = nullptr;
     std::function<void()> join;  // the pairs back into A, in pivot order
     // the mixed-precision path factors Float64 sketches in double-float
-    // (two reflectors and four pairs per column in shared memory, one
-    // reflector when two do not fit; a million columns and more take the
-    // FP64 kernel, whose column state is smaller)
+    // (two reflectors and four pairs per column in shared memory; one reflector
+    // when two do not fit, three pairs when four do not beside it, from about 900
+    // thousand columns on, which always fits here)
     const int Gd = (int)std::min<int64_t>(qr_sm_cap(ctx), n);
-    const size_t cols_df = (size_t)((n + Gd - 1) / Gd) * 33;
-    const bool pg = (size_t)m * 16 + cols_df > 200 * 1024;
-    const size_t smem_df = (size_t)m * (pg ? 8 : 16) + cols_df;
-    const bool dfq = sizeof(T) == 8 && ctx->gemm_tc && pivot && smem_df <= 220 * 1024;
+    const size_t ncap_df = (size_t)((n + Gd - 1) / Gd);
+    const bool pg = (size_t)m * 16 + ncap_df * 33 > 200 * 1024;
+    const bool far = pg && (size_t)m * 8 + ncap_df * 33 > 200 * 1024;
+    const size_t smem_df = (size_t)m * (pg ? 8 : 16) + ncap_df * (far ? 25 : 33);
+    const bool dfq = sizeof(T) == 8 && ctx->gemm_tc && pivot;
     if (dfq) {
       float* Bh = ctx->arena.alloc_n<float>((size_t)m * n);
       float* Bl = ctx->arena.alloc_n<float>((size_t)m * n);
@@ -3981,6 +3984,7 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
         E.word = ctx->arena.alloc_n<ulonglong2>((size_t)2 * G);
         E.f = ctx->arena.alloc_n<float2>((size_t)2 * G);
         E.prev = pg ? ctx->arena.alloc_n<float>((size_t)G * 2 * m) : nullptr;
+        E.far = far ? 1 : 0;
         LRA_CUDA(cudaMemsetAsync(E.word, 0, (size_t)2 * G * sizeof(ulonglong2), ctx->stream));
         void* args[] = {&Pd, &X, &D, &E};
         LRA_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(NT), args, smem_df, ctx->stream));

@@ -54,3 +54,21 @@ def test_qr_global(lra):
         assert orth <= (m + k) * 2.0 ** -46, (m, n, orth)
         # pivoting: |R_ii| does not grow beyond the norms' downdating error
         assert step <= 1.0 + 1e-6, (m, n, step)
+
+
+def test_qr_global_many_columns(lra):
+    """So many columns a CTA that only three pairs of each fit shared memory (as
+    about a million do on all SMs): still in pairs of floats, with the factors
+    that all SMs give."""
+    code = CODE.replace("ctx = lra.Context(0)", "ctx = lra.Context(0); ctx.set_tuning('qr_sms', 0, sms)").replace(
+        "for m, n, k, rtol in", "for sms, m, n, k, rtol in")
+    cases = [(1, 40, 7000, 30, 1e-9), (1, 72, 8000, 40, 1e-9), (2, 300, 14000, 70, 1e-9)]
+    r = subprocess.run([sys.executable, "-c", code.format(root=ROOT, cases=cases)], env=dict(os.environ, LRA_QR_SMEM="0"),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    got = json.loads([x for x in r.stdout.splitlines() if x.startswith("RESULT ")][0][7:])
+    for (_, m, n, k, rtol), (used, kk, err, orth, step) in zip(cases, got):
+        assert used == 1, (m, n)
+        assert kk == k, (m, n, kk)
+        assert err <= (m + k) * 2.0 ** -46 and orth <= (m + k) * 2.0 ** -46, (m, n, err, orth)
+        assert step <= 1.0 + 1e-6, (m, n, step)
