@@ -207,7 +207,9 @@ int lra_ctx_stage_ms(const lra_ctx* ctx, double out[4]);
    from the table LRA_TUNING names or the one beside liblra.so
    (tuning_gb300.txt, written by lowrankapprox/autotune.py).  set overrides
    one entry of this context (keys "tc_tile_n" with index dtype * 16 +
-   ceil(log2 order), "qr_seq_len", "srft_wide" with index log2 l'; index 0
+   ceil(log2 order) (32, 64 or 96 sketch rows a tile; for Float32 also 128,
+   which is 128 rows where that means fewer tiles and 96 elsewhere),
+   "qr_seq_len", "srft_wide" with index log2 l'; index 0
    for the rest: "qr_steps" (adaptive steps a pivoted-QR launch may hold,
    1..8), "qr_sms" (SMs a QR launch may take, 0 all), "tc_split" (most K
    parts of the tensor-core sketch, 0 as many as fill the SMs),

@@ -150,7 +150,8 @@ bool trace_on() {
 // ---- tuning table -------------------------------------------------------------------
 //
 // Text, one entry per line ("#" starts a comment):
-//   tc_tile_n <f32|f64> <log2 order> <32|64|96>
+//   tc_tile_n <f32|f64> <log2 order> <32|64|96, Float32 also 128: 128 rows where that means fewer tiles than
+//     96, else 96>
 //   qr_seq_len <rows>
 //   srft_wide <log2 l'> <0|1>
 //   qr_steps <1..8>
@@ -166,8 +167,8 @@ bool trace_on() {
 // library.
 
 static void tuning_defaults(lra_tuning* t) {
-  for (auto& row : t->tc_tile_n)
-    for (int& v : row) v = 96;
+  for (int& v : t->tc_tile_n[0]) v = 128;
+  for (int& v : t->tc_tile_n[1]) v = 96;
   t->qr_seq_len = 96;
   for (int lb = 0; lb <= 10; ++lb) t->srft_wide[lb] = (lb >= 7 && lb <= 10) ? 1 : 0;
   t->qr_steps = 8;
@@ -181,7 +182,8 @@ static void tuning_defaults(lra_tuning* t) {
 
 bool set_tuning(lra_tuning* t, const char* key, int64_t index, int64_t value) {
   if (!std::strcmp(key, "tc_tile_n")) {
-    if (index < 0 || index >= 32 || (value != 32 && value != 64 && value != 96)) return false;
+    if (index < 0 || index >= 32) return false;
+    if (value != 32 && value != 64 && value != 96 && !(value == 128 && index < 16)) return false;
     t->tc_tile_n[index / 16][index % 16] = (int)value;
     return true;
   }

@@ -47,8 +47,9 @@ namespace lra {
 namespace {
 
 constexpr int TILE_M = 128;   // columns of op(A) per CTA
-// sketch rows per CTA (the MMA N): 32, 64 or 96, picked per element type and
-// sketch order by the tuning table; five accumulators of TN columns fit TMEM
+// sketch rows per CTA (the MMA N): 32, 64, 96 or, with three planes, 128, picked
+// per element type and sketch order by the tuning table; five accumulators of 96
+// columns fit TMEM, three of 128
 constexpr int KBLK = 64;      // K per stage (128 bytes of BF16: one SW128 row)
 constexpr int CHUNK_KB = 8;   // K-blocks per exact chunk (512)
 constexpr int MAX_NSTAGE = 4;  // ring stages, as many as shared memory holds (at least 2)
@@ -1203,11 +1204,14 @@ void tc_split(lra_ctx* ctx, char trans, int64_t M, int64_t N, const T* A, int64_
   }
 }
 
-// the tile N of the tuning table for this element type and sketch order
+// the tile N of the tuning table for this element type and sketch order.  Three
+// planes (Float32) leave TMEM for 128 rows a CTA: a quarter less plane traffic into
+// the SMs per row, the bound of this kernel, where that means fewer tiles
 static int tuned_tile_n(const lra_ctx* ctx, bool f64, int64_t order) {
   int lb = 0;
   while (lb < 15 && ((int64_t)1 << lb) < order) ++lb;
   const int v = ctx->tuning.tc_tile_n[f64 ? 1 : 0][lb];
+  if (v == 128 && !f64 && (order + 127) / 128 < (order + 95) / 96) return 128;
   return (v == 32 || v == 64) ? v : 96;
 }
 
@@ -1217,11 +1221,7 @@ void tc_sketch(lra_ctx* ctx, const TcSplit& sp, int nsrc, const SketchSrc* src, 
   const int ns = sp.ns;
   int64_t order = 0;
   for (int i = 0; i < nsrc; ++i) order += rows[i];
-  int TILE_N = tuned_tile_n(ctx, sizeof(T) == 8, order);
-  // three planes (Float32) leave TMEM for 128 rows a CTA: a quarter less plane
-  // traffic into the SMs per row, the bound of this kernel, where that means
-  // fewer tiles
-  if (TILE_N == 96 && ns <= 3 && (order + 127) / 128 < (order + 95) / 96) TILE_N = 128;
+  const int TILE_N = tuned_tile_n(ctx, sizeof(T) == 8, order);
   const int64_t Lp = (order + TILE_N - 1) / TILE_N * TILE_N;
   const ArenaMark mk = ctx->arena.mark();
   __nv_bfloat16* St = ctx->arena.alloc_n<__nv_bfloat16>((size_t)Kp * Lp);

@@ -7,9 +7,9 @@ writes the table liblra reads when a context is created
 What it tunes (the keys of lra_ctx_set_tuning):
 
 * ``tc_tile_n``: the tcgen05 sketch tile N (32, 64 or 96 sketch rows per
-  CTA) per element type and ceil(log2(sketch order)), timed on the Gaussian
-  sketch of the mixed path at the adaptive orders 40 ... 1032, on an
-  8192 x 8192 Float64 and a 65536 x 4096 Float32 matrix.  A small tile pads
+  CTA, for Float32 also 128 where that means fewer tiles than 96) per element type and ceil(log2(sketch order)), timed on the Gaussian
+  sketch of the mixed path at the adaptive orders and their sums, 40 ...
+  2024, on an 8192 x 8192 Float64 and a 65536 x 4096 Float32 matrix.  A small tile pads
   the order less; a large one reads the digit planes of op(A) fewer times.
 * ``qr_seq_len``: the row count below which the double-float pivoted QR
   sums a column with one thread instead of a warp per four columns, timed
@@ -35,7 +35,9 @@ import numpy as np
 from . import Context, LRAOptions, idfact, idfact_batched, sketch
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-ORDERS = [40, 72, 136, 264, 520, 1032]
+# the adaptive orders by themselves, and the sums that the steps sharing a launch
+# take as one product (72 + ... + 264, + 520, + 1032)
+ORDERS = [40, 72, 136, 264, 472, 520, 992, 1032, 2024]
 
 
 def _lb(order: int) -> int:
@@ -67,17 +69,24 @@ def sweep_tile_n(ctx: Context, reps: int, quick: bool):
         A = torch.randn((N, M), dtype=tdt, device="cuda").t()       # column-major M x N
         npdt = np.float64 if tdt == torch.float64 else np.float32
         o = LRAOptions(npdt, precision="mixed", rtol=1e-10 if npdt == np.float64 else 1e-6, seed=7)
+        tiles = (96, 64, 32) if tag == "f64" else (128, 96, 64, 32)
+        total = {}
         for order in ORDERS:
             B = torch.empty((N, order), dtype=tdt, device="cuda").t()
             times = {}
-            for tn in (32, 64, 96):
+            for tn in tiles:
                 ctx.set_tuning("tc_tile_n", (16 if tag == "f64" else 0) + _lb(order), tn)
                 times[tn] = _time(lambda: sketch("left", "n", A, order, o, ctx=ctx, out=B), reps)
-            best = min(times, key=times.get)
-            ctx.set_tuning("tc_tile_n", (16 if tag == "f64" else 0) + _lb(order), best)
-            out[(tag, _lb(order))] = best
+                t = total.setdefault(_lb(order), dict.fromkeys(tiles, 0.0))
+                t[tn] += times[tn]
             notes.append(f"# tc_tile_n {tag} order {order} ({M}x{N}): " +
                          ", ".join(f"N={k} {v:.3f} ms" for k, v in times.items()))
+        for lb, t in total.items():
+            best = min(t, key=t.get)
+            if best == 96 and t.get(128, math.inf) <= 1.01 * t[96]:
+                best = 128  # (runs as 96 where it saves no tile)
+            ctx.set_tuning("tc_tile_n", (16 if tag == "f64" else 0) + lb, best)
+            out[(tag, lb)] = best
         del A
     return out, notes
 

@@ -106,3 +106,26 @@ def test_jacobi_block_sizes(lra, jb):
     assert np.abs(F.S - s[:F.k]).max() <= 10 * rtol * s[0]
     for Q in (np.asarray(F.U), np.asarray(F.Vt).T):
         assert np.abs(Q.T @ Q - np.eye(F.k)).max() < 1e-10
+
+
+@pytest.mark.parametrize("order", [97, 128, 264, 520])
+def test_float32_tile_of_128_rows(lra, order):
+    """128 rows a tile is a value of its own for Float32 (97, 128 and 520 rows take
+    fewer tiles of it, 264 as many as of 96) and none for Float64; 96 stays 96; all
+    give the same bits."""
+    from lowrankapprox import _ffi
+    lib = _ffi.load()
+    rng = np.random.default_rng(order)
+    A = np.asfortranarray(rng.standard_normal((2000, 300)).astype(np.float32))
+    ctx = lra.Context(0)
+    g = lra.lattice_gauss(9, order * 2000 + 8)
+    o = lra.LRAOptions(np.float32, precision="mixed", rtol=1e-6)
+    lb = int(np.ceil(np.log2(order)))
+    outs = []
+    for tn in (32, 96, 128):
+        ctx.set_tuning("tc_tile_n", lb, tn)
+        assert f"tc_tile_n f32 {lb} {tn}" in ctx.tuning().splitlines()
+        outs.append(lra.sketch("left", "n", A, order, o, rand=lra.RandStream(gauss=g), ctx=ctx))
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
+    assert lib.lra_ctx_set_tuning(ctx.handle, b"tc_tile_n", 16 + lb, 128) == _ffi.LRA_EINVAL
+    ctx.close()
