@@ -368,7 +368,8 @@ int lra_cur_middle(lra_ctx* ctx, int dtype, int64_t m, int64_t n,
 
 /* ---- spectral norms (src/snorm.jl) ------------------------------------------ */
 
-/* snorm(A) (src/snorm.jl:14-45) */
+/* snorm(A) (src/snorm.jl:14-45); hermitian: 1 or 0 says whether A is, -1 lets
+   the call test it; without meaning unless m == n */
 int lra_snorm(lra_ctx* ctx, int dtype, int64_t m, int64_t n, const void* A,
               int64_t lda, int hermitian, const lra_opts* opts,
               const lra_rand* rand, double* out);

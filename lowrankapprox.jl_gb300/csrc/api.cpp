@@ -3733,7 +3733,7 @@ int lra_snorm(lra_ctx* ctx, int dtype, int64_t m, int64_t n, const void* A, int6
         using R = decltype(z);
         DMat<CX<R>> dA = stage_in<CX<R>>(ctx, A, m, n, lda);
         check_input_c<R>(ctx, *opts, m, n, dA);
-        const bool herm = hermitian < 0 ? (m == n && cis_hermitian<R>(ctx, n, dA.p, dA.ld)) : hermitian != 0;
+        const bool herm = m == n && (hermitian < 0 ? cis_hermitian<R>(ctx, n, dA.p, dA.ld) : hermitian != 0);
         RandSrc rs(ctx, rand, opts->seed);
         const CX<R> one(1), zero(0);
         *out = csnorm_loop<R>(
@@ -3747,7 +3747,7 @@ int lra_snorm(lra_ctx* ctx, int dtype, int64_t m, int64_t n, const void* A, int6
       using T = decltype(z);
       DMat<T> dA = stage_in<T>(ctx, A, m, n, lda);
       check_input(ctx, *opts, m, n, dA);
-      const bool herm = hermitian < 0 ? (m == n && is_symmetric(ctx, n, dA.p, dA.ld)) : hermitian != 0;
+      const bool herm = m == n && (hermitian < 0 ? is_symmetric(ctx, n, dA.p, dA.ld) : hermitian != 0);
       RandSrc rs(ctx, rand, opts->seed);
       if (!ctx->linop) {
         *out = snorm_dense<T>(ctx, *opts, m, n, dA.p, dA.ld, (const T*)nullptr, 0, herm, rs);

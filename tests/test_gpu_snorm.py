@@ -78,3 +78,32 @@ def test_snorm_scales(lra):
         ref = _power(A, x, False, 4, 0.0) * sc
         assert abs(s - ref) <= 1e-12 * ref
     assert lra.snorm(_dev(A * 0, 0), o, rand=lra.RandStream(gauss=x)) == 0.0
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
+@pytest.mark.parametrize("m,n", [(31, 33), (33, 31), (257, 1000), (5000, 67), (64, 40000), (1999, 1501)])
+def test_snorm_last_row_and_column(lra, dt, m, n):
+    """A matrix whose norm sits in its last row, and in its last column: none of
+    them is left out, in either type."""
+    rng = np.random.default_rng(m + n)
+    o = lra.LRAOptions(dt, rtol=0.0, snorm_niter=5)
+    for last in (np.s_[m - 1, :], np.s_[:, n - 1]):
+        A = 1e-3 * rng.standard_normal((m, n))
+        A[last] += rng.standard_normal(A[last].shape)
+        A = A.astype(dt)
+        x = rng.standard_normal(n)
+        ref = _power(A, x, False, 5, 0.0)
+        assert abs(lra.snorm(_dev(A, 1), o, rand=lra.RandStream(gauss=x)) - ref) <= 4 * (m + n) * np.finfo(dt).eps * ref
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.complex128])
+@pytest.mark.parametrize("m,n", [(40, 70), (70, 40), (3, 5000)])
+def test_snorm_hermitian_flag_needs_a_square_matrix(lra, dt, m, n):
+    """A rectangular matrix is not Hermitian, whatever the flag says."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((m, n)).astype(dt)
+    o = lra.LRAOptions(dt, rtol=0.0, snorm_niter=5, seed=3)
+    one, two = lra.Context(0), lra.Context(0)
+    assert lra.snorm(A, o, hermitian=True, ctx=one) == lra.snorm(A, o, hermitian=False, ctx=two)
+    one.close()
+    two.close()
