@@ -442,6 +442,12 @@ bool use_tc_gemm(const lra_opts& o, int dtype) {
   return o.precision == LRA_PREC_MIXED && dtype == LRA_F64 && o.rtol >= 1e-13;
 }
 
+// LRA_TRACE: the pivots an adaptive step's QR took (its threshold where it stopped there)
+void trace_step(int64_t order, int64_t nt, int64_t k) {
+  if (trace_on())
+    std::fprintf(stderr, "[lra] step of order %lld, threshold %lld: rank %lld\n", (long long)order, (long long)nt, (long long)k);
+}
+
 // right_layout: the Gaussian matrix is drawn as M x order (column-major), the
 // layout of a right sketch A S (src/sketch.jl:95-98), and used transposed
 template <typename T>
@@ -693,6 +699,7 @@ int sketchfact_steps(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, int
       if (st[(size_t)i].nt > rank_hint) likely = i;
     c = geqp3_adap_steps<T>(ctx, cnt, st.data(), o.nb, o.atol, o.rtol, ks.data(), likely);
   }
+  for (int i = 0; i <= (c < 0 ? cnt - 1 : c); ++i) trace_step(st[(size_t)i].m, st[(size_t)i].nt, ks[(size_t)i]);
   if (c < 0) {
     ctx->arena.release(base);
     return -cnt;
@@ -766,6 +773,7 @@ Fact<T> sketchfact_dev(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, i
                           adaptive ? nt : 0);
     }
     F.nsteps = step + 1;
+    if (adaptive) trace_step(order, nt, F.k);
     if (!adaptive || F.k < nt) break;
     if (ahead) rank_hint = predict_rank<T>(ctx, F, F.k == nt ? nt : kmax, o);
     nt *= 2;
@@ -812,6 +820,7 @@ Fact<T> sketchfact_right_dev(lra_ctx* ctx, const lra_opts& o, char trans, int64_
       F.k = geqp3_adap<T>(ctx, M, order, F.B, F.ld, F.jpvt, F.tau, kmax, o.nb, o.atol, o.rtol, true, adaptive ? nt : 0);
     }
     F.nsteps = step + 1;
+    if (adaptive) trace_step(order, nt, F.k);
     if (!adaptive || F.k < nt) break;
     nt *= 2;
     ctx->arena.release(base);
@@ -1260,6 +1269,7 @@ void idfact_batched_grouped(lra_ctx* ctx, int64_t count, const lra_matdesc* mats
         St& s = st[(size_t)map[t]];
         s.k = hk[t];
         s.nsteps = round + 1;
+        if (adaptive) trace_step(s.order, s.nt, s.k);
         if (!adaptive || s.k < s.nt)
           s.done = true;
         else
@@ -1580,6 +1590,7 @@ CFact<R> sketchfact_c(lra_ctx* ctx, const lra_opts& o, char trans, bool right, i
     lra_opts oq = o;
     F = cpqr_backend<R>(ctx, oq, B, rows, cols, std::max<int64_t>(rows, 1), adaptive ? nt : 0);
     F.nsteps = step + 1;
+    if (adaptive) trace_step(order, nt, F.k);
     if (!adaptive || F.k < nt) break;
     nt *= 2;
     ctx->arena.release(base);

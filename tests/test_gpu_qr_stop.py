@@ -33,3 +33,37 @@ def test_batch(lra):
     o = lra.LRAOptions(rtol=1e-4, precision="mixed", seed=7)
     for k, V in zip(ranks, lra.idfact_batched([_matrix(k, np.float64, k) for k in ranks], o)):
         assert V.k == k and V.nsteps == 1 + next(t for t in range(9) if k < 32 * 2 ** t)
+
+
+CODE = """
+import sys
+sys.path.insert(0, {root!r} + "/lowrankapprox.jl_gb300"); sys.path.insert(0, {root!r} + "/tests")
+import numpy as np
+import lowrankapprox as lra
+from test_gpu_qr_stop import _matrix
+dt = np.{dt}
+A = _matrix(100, dt, 100)
+o = lra.LRAOptions(dt, rtol=1e-4, precision={precision!r}, seed=7)
+V = lra.idfact_batched([A, A[:, :350].copy(order="F")], o)[0] if {batch} else lra.idfact(A, o)
+assert V.k == 100
+"""
+
+
+@pytest.mark.parametrize("dt,precision,batch", [("float64", "mixed", 0), ("float64", "native", 0), ("float32", "mixed", 0),
+                                                ("complex128", "native", 0), ("complex64", "native", 0),
+                                                ("float64", "mixed", 1)])
+def test_steps_end_at_their_thresholds(lra, dt, precision, batch):
+    """A matrix of rank 100: the QRs of orders 40 and 72 end with 32 and 64 pivots
+    (without the early end they would go on to 40 and 72), that of 136 reveals
+    the rank."""
+    import os
+    import re
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", CODE.format(root=root, dt=dt, precision=precision, batch=batch)],
+                       env=dict(os.environ, LRA_TRACE="1"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    steps = re.findall(r"step of order (\d+), threshold (\d+): rank (-?\d+)", r.stderr)
+    assert set(steps) == {("40", "32", "32"), ("72", "64", "64"), ("136", "128", "100")}, steps
+    assert len(steps) == 3 * (1 + batch)
