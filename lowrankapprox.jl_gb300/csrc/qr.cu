@@ -3257,6 +3257,9 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
   LRA_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), ctx->stream));
   ulonglong2* slots = gang ? ctx->arena.alloc_n<ulonglong2>((size_t)32 * count) : nullptr;
   if (gang) LRA_CUDA(cudaMemsetAsync(slots, 0, (size_t)32 * count * sizeof(ulonglong2), ctx->stream));
+  // (a QR whose wait runs out writes no pivot count: the replay then takes none)
+  int64_t* nfac = ctx->arena.alloc_n<int64_t>((size_t)count);
+  LRA_CUDA(cudaMemsetAsync(nfac, 0, (size_t)count * sizeof(int64_t), ctx->stream));
   unsigned long long* maxbits = ctx->arena.alloc_n<unsigned long long>((size_t)count);
   LRA_CUDA(cudaMemsetAsync(maxbits, 0, (size_t)count * sizeof(unsigned long long), ctx->stream));
   int64_t nmax = 1;
@@ -3291,7 +3294,7 @@ void geqp3_df_batch(lra_ctx* ctx, int64_t count, const DfBatchItem* items, int64
     J.P.stop_at = it.stop_at;
     J.P.k_out = k_dev + i;
     J.X.piv = ctx->arena.alloc_n<int64_t>(std::max<int64_t>(J.P.kmax, 1));
-    J.X.nfac = ctx->arena.alloc_n<int64_t>(1);
+    J.X.nfac = nfac + t;
     J.X.beta = ctx->arena.alloc_n<double>(std::max<int64_t>(J.P.kmax, 1));
     J.D.vn0 = vn0;
     J.D.scale = scale;
@@ -3925,6 +3928,7 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     QrV2Extra X;
     X.piv = ctx->arena.alloc_n<int64_t>(std::max<int64_t>(P.kmax, 1));
     X.nfac = ctx->arena.alloc_n<int64_t>(1);
+    LRA_CUDA(cudaMemsetAsync(X.nfac, 0, sizeof(int64_t), ctx->stream));
     X.part_k = ctx->arena.alloc_n<long long>(grid);
     X.beta = ctx->arena.alloc_n<double>(std::max<int64_t>(P.kmax, 1));
     int64_t* col_at = ctx->arena.alloc_n<int64_t>(n);
