@@ -371,16 +371,15 @@ __device__ __forceinline__ f2_t f2_mul(f2_t a, f2_t b) {
   return d;
 }
 // Block one-sided Jacobi for the FP32 sweeps: the columns are grouped in
-// blocks of JB; each grid-wide round pairs the blocks round-robin, and the
-// CTA holding a block pair loads its 2 JB columns of X and V into shared
-// memory and rotates every pair among them there (2 JB - 1 local rounds of
-// JB pairs, a warp per pair) before writing them back.  A sweep then costs
-// about n / JB grid barriers instead of n, and the local rotations also
+// blocks of JBT; each grid-wide round pairs the blocks round-robin, and the
+// CTA holding a block pair loads its 2 JBT columns of X and V into shared
+// memory and rotates every pair among them there (2 JBT - 1 local rounds of
+// JBT pairs, a warp per pair) before writing them back.  A sweep then costs
+// about n / JBT grid barriers instead of n, and the local rotations also
 // reach the pairs inside each block.  The local rotations are applied to X
-// one by one and gathered into a 2 JB x 2 JB orthogonal matrix, which is
+// one by one and gathered into a 2 JBT x 2 JBT orthogonal matrix, which is
 // applied to the block's columns of V once, a thread per row, after the
 // local rounds.
-constexpr int JB = 8;
 constexpr int JB_RPL = 16;  // rows per lane in registers (columns up to 512 long)
 constexpr int JB_QMAX = 16;  // 16-byte chunks a lane holds in the inter-block steps (columns up to 2048 long)
 
@@ -1159,8 +1158,6 @@ struct JdRot {
   float eps, sn;
   Df c, s;
 };
-
-__device__ __forceinline__ bool df_gt(Df x, Df y) { return x.h > y.h || (x.h == y.h && x.l > y.l); }
 
 __device__ __forceinline__ Df df_rot_a(Df c, Df s, Df u, Df w) { return df_add(df_mul(c, u), df_neg(df_mul(s, w))); }
 __device__ __forceinline__ Df df_rot_b(Df c, Df s, Df u, Df w) { return df_add(df_mul(s, u), df_mul(c, w)); }

@@ -3589,7 +3589,6 @@ void sm_prepare(lra_ctx* ctx, SmQr<T>& q, SmZero* z, SmPrep& prep, int64_t m, in
   QrV2Extra& X = q.job.X;
   X.piv = ctx->arena.alloc_n<int64_t>(std::max<int64_t>(P.kmax, 1));
   X.nfac = &z->nfac;
-  X.part_k = ctx->arena.alloc_n<long long>(G);
   X.beta = ctx->arena.alloc_n<double>(std::max<int64_t>(P.kmax, 1));
   q.col_at = ctx->arena.alloc_n<int64_t>(n);
   q.pos = ctx->arena.alloc_n<int64_t>(n);
@@ -3802,42 +3801,10 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
   // the reflector of each pivot is staged in shared memory when it fits
   const int64_t vcap = std::min<int64_t>(m, (int64_t)(160 * 1024 / sizeof(T)));
   const size_t dyn_smem = (size_t)vcap * sizeof(T);
-  raise_smem_limit(ctx, (const void*)geqp3_kernel<T, NT>);
-  int per_sm = 0;
-  LRA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, geqp3_kernel<T, NT>, NT, dyn_smem));
-  if (per_sm < 1) fail(LRA_ECUDA, "geqp3 kernel cannot be resident");
   const int64_t want = (n + (NT / 32) - 1) / (NT / 32);
-  int grid = (int)std::min<int64_t>((int64_t)qr_sm_cap(ctx) * std::min(per_sm, 1), want);
-  grid = std::max(grid, 1);
-
-  QrParams<T> P;
-  P.m = m;
-  P.n = n;
-  P.lda = lda;
-  P.A = A;
-  P.jpvt = jpvt;
-  P.tau = tau;
-  P.vn1 = ctx->arena.alloc_n<T>(n);
-  P.vn2 = ctx->arena.alloc_n<T>(n);
-  P.flag = ctx->arena.alloc_n<int>(n);
-  P.part_v = ctx->arena.alloc_n<T>(grid);
-  P.part_i = ctx->arena.alloc_n<int64_t>(grid);
-  P.part_d = ctx->arena.alloc_n<double>(std::max(grid, ctx->num_sms));
-  int* small = ctx->arena.alloc_n<int>(8);
-  P.lsticc = small;
-  P.bar = reinterpret_cast<GridBar*>(ctx->arena.alloc(sizeof(GridBar)));
-  P.kmax = std::min<int64_t>(kmax, std::min(m, n));
-  P.nb = std::max<int64_t>(1, std::min<int64_t>(nb, std::max<int64_t>(P.kmax, 1)));
-  P.atol = atol;
-  P.rtol = rtol;
-  P.pivot = pivot ? 1 : 0;
-  P.k_out = ctx->arena.alloc_n<int64_t>(1);
-  P.vcap = vcap;
-  P.seq_len = ctx->tuning.qr_seq_len;
-  P.stop_at = stop_at;
-  LRA_CUDA(cudaMemsetAsync(small, 0, 8 * sizeof(int), ctx->stream));
-  LRA_CUDA(cudaMemsetAsync(P.bar, 0, sizeof(GridBar), ctx->stream));
-  if (P.kmax <= 0) {
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)qr_sm_cap(ctx), want));
+  const int64_t top_k = std::min<int64_t>(kmax, std::min(m, n));
+  if (top_k <= 0) {
     // nothing to factor: identity permutation
     std::vector<int64_t> id(n);
     for (int64_t i = 0; i < n; ++i) id[i] = i + 1;
@@ -3866,7 +3833,7 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
     if (need <= cap && sm_resident<Ar>(ctx, need)) {
       SmQr<T> q;
       SmPreps preps;
-      sm_prepare<T>(ctx, q, sm_zeros(ctx, 1), preps.j[0], m, n, A, lda, jpvt, tau, P.kmax, nb, atol, rtol, G, cap);
+      sm_prepare<T>(ctx, q, sm_zeros(ctx, 1), preps.j[0], m, n, A, lda, jpvt, tau, top_k, nb, atol, rtol, G, cap);
       sm_convert<T>(ctx, preps, 1, n);
       q.job.P.stop_at = stop_at;
       SmQr<T>* qp = &q;
@@ -3882,6 +3849,24 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
       return k;
     }
   }
+  QrParams<T> P{};
+  P.m = m;
+  P.n = n;
+  P.lda = lda;
+  P.A = A;
+  P.jpvt = jpvt;
+  P.tau = tau;
+  P.kmax = top_k;
+  P.nb = std::max<int64_t>(1, std::min<int64_t>(nb, P.kmax));
+  P.atol = atol;
+  P.rtol = rtol;
+  P.pivot = pivot ? 1 : 0;
+  P.vcap = vcap;
+  P.seq_len = ctx->tuning.qr_seq_len;
+  P.stop_at = stop_at;
+  P.k_out = ctx->arena.alloc_n<int64_t>(1);
+  P.bar = reinterpret_cast<GridBar*>(ctx->arena.alloc(sizeof(GridBar)));
+  LRA_CUDA(cudaMemsetAsync(P.bar, 0, sizeof(GridBar), ctx->stream));
   if constexpr (sizeof(T) == 8) {
     // FP64 in shared memory: a warp's worth of columns a block at first, over all
     // the SMs it may take if that is too much for a block (100 pivots of 4000 x 300:
@@ -3918,6 +3903,14 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
       return k;
     }
   }
+  P.vn1 = ctx->arena.alloc_n<T>(n);
+  P.vn2 = ctx->arena.alloc_n<T>(n);
+  P.flag = ctx->arena.alloc_n<int>(n);
+  P.part_v = ctx->arena.alloc_n<T>(grid);
+  P.part_i = ctx->arena.alloc_n<int64_t>(grid);
+  P.part_d = ctx->arena.alloc_n<double>(std::max(grid, ctx->num_sms));
+  P.lsticc = ctx->arena.alloc_n<int>(2);
+  LRA_CUDA(cudaMemsetAsync(P.lsticc, 0, 2 * sizeof(int), ctx->stream));
   if (v2) {
     raise_smem_limit(ctx, (const void*)geqp3_v2_kernel<T, NT>);
     LRA_CUDA(cudaFuncSetAttribute(geqp3_v2_kernel<T, NT>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -4031,6 +4024,10 @@ int64_t geqp3_adap(lra_ctx* ctx, int64_t m, int64_t n, T* A, int64_t lda, int64_
       copy_matrix(ctx, m, n, tmp, m, A, lda);
     }
   } else {
+    raise_smem_limit(ctx, (const void*)geqp3_kernel<T, NT>);
+    int per_sm = 0;
+    LRA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, geqp3_kernel<T, NT>, NT, dyn_smem));
+    if (per_sm < 1) fail(LRA_ECUDA, "geqp3 kernel cannot be resident");
     void* args[] = {&P};
     LRA_CUDA(cudaLaunchCooperativeKernel((const void*)geqp3_kernel<T, NT>, dim3(grid), dim3(NT), args,
                                          dyn_smem, ctx->stream));
