@@ -1629,14 +1629,15 @@ __global__ void __launch_bounds__(NT, 1) geqp3_df_kernel(QrParams<double> P, QrV
 // word (norm key, column), and then arrives, counting its stop flag along.
 // A read takes arrivals and maximum together, as a vector of two 64-bit words.
 // Such a read may take the maximum first, so the one that sees the last arrival
-// only says who has very likely won: the CTA goes on with that and loads the
-// staged rows, while a second read of the maximum, after the acquire and so
-// final, is under way; should it differ, the rows are loaded again from the CTA it
-// names.  (Waiting for it costs a second L2 round trip, 0.7 us of the 6.9 us a
-// short pivot took; one 64-bit word a CTA that every CTA reads: the ID of 65536 x
-// 4096 Float32 9.68 ms, 9.31 so.)  A word is only accessed by its 64 bits.
-// Slots rotate over four exchanges and staged columns over two, so a CTA that runs ahead never
-// overwrites what a slower CTA still reads.  The key keeps the 38
+// only says who has very likely won: the CTA goes on with that, up to the dot
+// products, while a second read of the maximum, after the acquire and so
+// final, is under way; should it differ, that part of the step is done again with
+// the column it names.  (Waiting for it costs a second L2 round trip, 0.7 us of
+// the 6.9 us a short pivot took.  The ID of 65536 x 4096 Float32: 9.25 ms so, 9.31 with
+// the second read compared before the dot products, 9.68 with one 64-bit word a
+// CTA that every CTA reads.)  A word is only accessed by its 64 bits.  Slots
+// rotate over four exchanges and staged columns over two, so a CTA that runs
+// ahead never overwrites what a slower CTA still reads.  The key keeps the 38
 // leading bits of the double-float norm (relative resolution 2^-30, far
 // below the error of the downdated norms); ties go to the smaller column
 // index, as with xLAQPS's idamax.
@@ -2021,6 +2022,7 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
     bool stop_block = false, last_small = false;
     while (kk < jb && !stop_block) {
       const int64_t c = j + kk;
+      const int64_t len = m - c - 1;
       int64_t pvt;
       int owner;
       stamp(c, 0);
@@ -2048,10 +2050,161 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc = A::add(acc, A::shfl_xor(acc, o));
         if (lane == 0) s_part[wid] = acc;
-        if (!GCOL && threadIdx.x == 0) s_again = sure != s_win ? 1 : 0;
+        __syncthreads();
+        stamp(c, 1);
+        if (wid == 0) {
+          // xLARFG in double-float (the matrix is scaled to max |B| < 1, so
+          // neither the sum of squares nor beta can overflow, and no entry of
+          // a float pair is small enough for xLARFG's rescaling loop)
+          V acc = lane < NW ? s_part[lane] : A::zero();
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) acc = A::add(acc, A::shfl_xor(acc, o));
+          const V alpha = s_alpha;
+          V tau = A::zero(), beta = alpha, scal = A::one();
+          if (len > 0 && A::hi(acc) > 0.f) {
+            const V r = A::sqrt_(A::add(A::mul(alpha, alpha), acc));
+            beta = A::hi(alpha) >= 0.f ? A::neg(r) : r;
+            tau = A::div(A::add(beta, A::neg(alpha)), beta);
+            scal = A::div(A::one(), A::add(alpha, A::neg(beta)));
+          }
+          if (lane == 0) {
+            s_taud = A::val(tau);
+            s_betad = A::val(beta);
+            s_f = scal;
+            s_tau = tau;
+            s_beta = beta;
+            if (!GCOL) s_again = sure != s_win ? 1 : 0;
+            if (b == 0) {
+              P.tau[c] = (typename A::T)s_taud;
+              X.piv[c] = pvt;
+              X.beta[c] = s_betad;
+            }
+          }
+        } else if (len > 0 && len <= P.seq_len) {
+          // ---- short columns: a thread per column, the dot product summed
+          // row by row (a lane-strided sum and its reduction tree cost more
+          // than the products here).  The rule depends on len alone, so both
+          // forms of the kernel sum each column the same way.
+          for (int s = threadIdx.x - 32; s < nloc; s += NT - 32) {
+            if (s_st[s] & ST_DONE) continue;
+            const E* col = C + (int64_t)s * cs;
+            s_x0[s] = col[c * rs];
+            V d = A::zero();
+            // QSEQB rows loaded ahead, then added in row order (no masks in a whole
+            // chunk: a branch a row would keep the rows' products from overlapping)
+            int64_t i0 = c + 1;
+            for (; i0 + QSEQB <= m; i0 += QSEQB) {
+              E xb[QSEQB], vb[QSEQB];
+#pragma unroll
+              for (int r = 0; r < QSEQB; ++r) {
+                xb[r] = col[(i0 + r) * rs];
+                vb[r] = Vc[i0 + r];
+              }
+#pragma unroll
+              for (int r = 0; r < QSEQB; ++r) A::fma_acc(d, vb[r], xb[r]);
+            }
+            if (i0 < m) {
+              E xb[QSEQB];
+#pragma unroll
+              for (int r = 0; r < QSEQB; ++r) xb[r] = i0 + r < m ? col[(i0 + r) * rs] : A::ezero();
+#pragma unroll
+              for (int r = 0; r < QSEQB; ++r)
+                if (i0 + r < m) A::fma_acc(d, Vc[i0 + r], xb[r]);
+            }
+            s_dot[s] = A::norm(d);
+          }
+        } else if (len > 0) {
+          // ---- dot products x . a of the warp's live columns, GQ at a time
+          auto dots = [&](auto gqc) {
+            constexpr int GQ = decltype(gqc)::value;
+            constexpr int R = GQ == 4 ? QRPL : 8;  // rows per lane loaded ahead
+            constexpr int LG = 32 / GQ;            // lanes that end with one column's total
+            int s = wid - 1;
+            int q[GQ];
+            while (live_group<GQ>(s_st, nloc, NCW, s, q)) {
+              const E* cg[GQ];
+#pragma unroll
+              for (int g = 0; g < GQ; ++g) cg[g] = C + (int64_t)(q[g] >= 0 ? q[g] : q[0]) * cs;
+              int qg = q[0];  // this lane's column once the sums are reduced
+#pragma unroll
+              for (int g = 1; g < GQ; ++g) qg = lane / LG == g ? q[g] : qg;
+              // row c of the column, for the update that follows the dots
+              if (lane % LG == 0 && qg >= 0) s_x0[qg] = C[(int64_t)qg * cs + c * rs];
+              // R rows per lane are loaded before they are used, so that a
+              // group has GQ R loads in flight (the global-memory form waits
+              // an L2 round trip per chunk); each lane still adds its rows in
+              // increasing order
+              V d[GQ];
+#pragma unroll
+              for (int g = 0; g < GQ; ++g) d[g] = A::zero();
+              int64_t b0 = c + 1;
+              for (; b0 + 32 * R <= m; b0 += 32 * R) {  // whole chunks: no row to mask
+                E xv[R], xc[GQ][R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  const int64_t i = b0 + lane + 32 * r;
+                  xv[r] = Vc[i];
+#pragma unroll
+                  for (int g = 0; g < GQ; ++g) xc[g][r] = cg[g][i * rs];
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                  for (int g = 0; g < GQ; ++g) A::fma_acc(d[g], xv[r], xc[g][r]);
+              }
+              if (b0 < m) {
+                E xv[R], xc[GQ][R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  const int64_t i = b0 + lane + 32 * r;
+                  const bool in = i < m;
+                  xv[r] = in ? Vc[i] : A::ezero();
+#pragma unroll
+                  for (int g = 0; g < GQ; ++g) xc[g][r] = in ? cg[g][i * rs] : A::ezero();
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                  if (b0 + lane + 32 * r < m) {
+#pragma unroll
+                    for (int g = 0; g < GQ; ++g) A::fma_acc(d[g], xv[r], xc[g][r]);
+                  }
+              }
+#pragma unroll
+              for (int g = 0; g < GQ; ++g) d[g] = A::norm(d[g]);
+              // transposed butterfly: a level that halves the columns a lane holds
+              // as it adds, then the rest; lanes LG g .. LG g + LG - 1 end with
+              // column g's total
+              V t;
+              if constexpr (GQ == 4) {
+                const bool up = lane & 16;
+                const V k0 = up ? d[2] : d[0], k1 = up ? d[3] : d[1];
+                const V e0 = A::add(k0, A::shfl_xor(up ? d[0] : d[2], 16));
+                const V e1 = A::add(k1, A::shfl_xor(up ? d[1] : d[3], 16));
+                const bool hi = lane & 8;
+                t = A::add(hi ? e1 : e0, A::shfl_xor(hi ? e0 : e1, 8));
+              } else if constexpr (GQ == 2) {
+                const bool up = lane & 16;
+                t = A::add(up ? d[1] : d[0], A::shfl_xor(up ? d[0] : d[1], 16));
+                t = A::add(t, A::shfl_xor(t, 8));
+              } else {
+                t = A::add(d[0], A::shfl_xor(d[0], 16));
+                t = A::add(t, A::shfl_xor(t, 8));
+              }
+#pragma unroll
+              for (int o = 4; o > 0; o >>= 1) t = A::add(t, A::shfl_xor(t, o));
+              if (lane % LG == 0 && qg >= 0) s_dot[qg] = t;
+            }
+          };
+          if (per_warp >= 3)
+            dots(std::integral_constant<int, 4>{});
+          else if (per_warp == 2)
+            dots(std::integral_constant<int, 2>{});
+          else
+            dots(std::integral_constant<int, 1>{});
+        }
         __syncthreads();
         if (GCOL || !s_again) break;
-        // the maximum was read too early: the same with the final one
+        // the maximum was read too early: the step so far again with the final one
         for (int s = threadIdx.x; s < nloc; s += NT)
           if (owner == b && s == pvt - c0) s_st[s] &= (unsigned char)~ST_DONE;
         __syncthreads();
@@ -2059,158 +2212,6 @@ __device__ __forceinline__ void geqp3_df_body(const QrParams<typename A::T>& P, 
         __syncthreads();
         if (!s_ok) return;
       }
-      stamp(c, 1);
-      const int64_t len = m - c - 1;
-      if (wid == 0) {
-        // xLARFG in double-float (the matrix is scaled to max |B| < 1, so
-        // neither the sum of squares nor beta can overflow, and no entry of
-        // a float pair is small enough for xLARFG's rescaling loop)
-        V acc = lane < NW ? s_part[lane] : A::zero();
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc = A::add(acc, A::shfl_xor(acc, o));
-        const V alpha = s_alpha;
-        V tau = A::zero(), beta = alpha, scal = A::one();
-        if (len > 0 && A::hi(acc) > 0.f) {
-          const V r = A::sqrt_(A::add(A::mul(alpha, alpha), acc));
-          beta = A::hi(alpha) >= 0.f ? A::neg(r) : r;
-          tau = A::div(A::add(beta, A::neg(alpha)), beta);
-          scal = A::div(A::one(), A::add(alpha, A::neg(beta)));
-        }
-        if (lane == 0) {
-          s_taud = A::val(tau);
-          s_betad = A::val(beta);
-          s_f = scal;
-          s_tau = tau;
-          s_beta = beta;
-          if (b == 0) {
-            P.tau[c] = (typename A::T)s_taud;
-            X.piv[c] = pvt;
-            X.beta[c] = s_betad;
-          }
-        }
-      } else if (len > 0 && len <= P.seq_len) {
-        // ---- short columns: a thread per column, the dot product summed
-        // row by row (a lane-strided sum and its reduction tree cost more
-        // than the products here).  The rule depends on len alone, so both
-        // forms of the kernel sum each column the same way.
-        for (int s = threadIdx.x - 32; s < nloc; s += NT - 32) {
-          if (s_st[s] & ST_DONE) continue;
-          const E* col = C + (int64_t)s * cs;
-          s_x0[s] = col[c * rs];
-          V d = A::zero();
-          // QSEQB rows loaded ahead, then added in row order (no masks in a whole
-          // chunk: a branch a row would keep the rows' products from overlapping)
-          int64_t i0 = c + 1;
-          for (; i0 + QSEQB <= m; i0 += QSEQB) {
-            E xb[QSEQB], vb[QSEQB];
-#pragma unroll
-            for (int r = 0; r < QSEQB; ++r) {
-              xb[r] = col[(i0 + r) * rs];
-              vb[r] = Vc[i0 + r];
-            }
-#pragma unroll
-            for (int r = 0; r < QSEQB; ++r) A::fma_acc(d, vb[r], xb[r]);
-          }
-          if (i0 < m) {
-            E xb[QSEQB];
-#pragma unroll
-            for (int r = 0; r < QSEQB; ++r) xb[r] = i0 + r < m ? col[(i0 + r) * rs] : A::ezero();
-#pragma unroll
-            for (int r = 0; r < QSEQB; ++r)
-              if (i0 + r < m) A::fma_acc(d, Vc[i0 + r], xb[r]);
-          }
-          s_dot[s] = A::norm(d);
-        }
-      } else if (len > 0) {
-        // ---- dot products x . a of the warp's live columns, GQ at a time
-        auto dots = [&](auto gqc) {
-          constexpr int GQ = decltype(gqc)::value;
-          constexpr int R = GQ == 4 ? QRPL : 8;  // rows per lane loaded ahead
-          constexpr int LG = 32 / GQ;            // lanes that end with one column's total
-          int s = wid - 1;
-          int q[GQ];
-          while (live_group<GQ>(s_st, nloc, NCW, s, q)) {
-            const E* cg[GQ];
-#pragma unroll
-            for (int g = 0; g < GQ; ++g) cg[g] = C + (int64_t)(q[g] >= 0 ? q[g] : q[0]) * cs;
-            int qg = q[0];  // this lane's column once the sums are reduced
-#pragma unroll
-            for (int g = 1; g < GQ; ++g) qg = lane / LG == g ? q[g] : qg;
-            // row c of the column, for the update that follows the dots
-            if (lane % LG == 0 && qg >= 0) s_x0[qg] = C[(int64_t)qg * cs + c * rs];
-            // R rows per lane are loaded before they are used, so that a
-            // group has GQ R loads in flight (the global-memory form waits
-            // an L2 round trip per chunk); each lane still adds its rows in
-            // increasing order
-            V d[GQ];
-#pragma unroll
-            for (int g = 0; g < GQ; ++g) d[g] = A::zero();
-            int64_t b0 = c + 1;
-            for (; b0 + 32 * R <= m; b0 += 32 * R) {  // whole chunks: no row to mask
-              E xv[R], xc[GQ][R];
-#pragma unroll
-              for (int r = 0; r < R; ++r) {
-                const int64_t i = b0 + lane + 32 * r;
-                xv[r] = Vc[i];
-#pragma unroll
-                for (int g = 0; g < GQ; ++g) xc[g][r] = cg[g][i * rs];
-              }
-#pragma unroll
-              for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int g = 0; g < GQ; ++g) A::fma_acc(d[g], xv[r], xc[g][r]);
-            }
-            if (b0 < m) {
-              E xv[R], xc[GQ][R];
-#pragma unroll
-              for (int r = 0; r < R; ++r) {
-                const int64_t i = b0 + lane + 32 * r;
-                const bool in = i < m;
-                xv[r] = in ? Vc[i] : A::ezero();
-#pragma unroll
-                for (int g = 0; g < GQ; ++g) xc[g][r] = in ? cg[g][i * rs] : A::ezero();
-              }
-#pragma unroll
-              for (int r = 0; r < R; ++r)
-                if (b0 + lane + 32 * r < m) {
-#pragma unroll
-                  for (int g = 0; g < GQ; ++g) A::fma_acc(d[g], xv[r], xc[g][r]);
-                }
-            }
-#pragma unroll
-            for (int g = 0; g < GQ; ++g) d[g] = A::norm(d[g]);
-            // transposed butterfly: a level that halves the columns a lane holds
-            // as it adds, then the rest; lanes LG g .. LG g + LG - 1 end with
-            // column g's total
-            V t;
-            if constexpr (GQ == 4) {
-              const bool up = lane & 16;
-              const V k0 = up ? d[2] : d[0], k1 = up ? d[3] : d[1];
-              const V e0 = A::add(k0, A::shfl_xor(up ? d[0] : d[2], 16));
-              const V e1 = A::add(k1, A::shfl_xor(up ? d[1] : d[3], 16));
-              const bool hi = lane & 8;
-              t = A::add(hi ? e1 : e0, A::shfl_xor(hi ? e0 : e1, 8));
-            } else if constexpr (GQ == 2) {
-              const bool up = lane & 16;
-              t = A::add(up ? d[1] : d[0], A::shfl_xor(up ? d[0] : d[1], 16));
-              t = A::add(t, A::shfl_xor(t, 8));
-            } else {
-              t = A::add(d[0], A::shfl_xor(d[0], 16));
-              t = A::add(t, A::shfl_xor(t, 8));
-            }
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) t = A::add(t, A::shfl_xor(t, o));
-            if (lane % LG == 0 && qg >= 0) s_dot[qg] = t;
-          }
-        };
-        if (per_warp >= 3)
-          dots(std::integral_constant<int, 4>{});
-        else if (per_warp == 2)
-          dots(std::integral_constant<int, 2>{});
-        else
-          dots(std::integral_constant<int, 1>{});
-      }
-      __syncthreads();
       stamp(c, 2);
       const double tau = s_taud;
       const V scal = s_f;
