@@ -171,7 +171,8 @@ def main(argv=None):
              f"# ({'quick' if args.quick else 'full'} sweep, {time.time() - t0:.0f} s; best of {args.reps})"]
     lines += n1 + n2 + n3
     for (tag, lb), v in sorted(tiles.items()):
-        lines.append(f"tc_tile_n {tag} {lb} {v}")
+        # (128 is what the library takes where the table has no entry)
+        lines.append(f"tc_tile_n {tag} {lb} {v}" if v != 128 else f"# tc_tile_n {tag} {lb}: {v}, the default")
     lines.append(f"qr_seq_len {seq}")
     for lb, v in sorted(wide.items()):
         lines.append(f"srft_wide {lb} {v}")
