@@ -16,7 +16,7 @@ namespace {
 // SM, so one entry a thread and small blocks, a warp for each quarter, which
 // spread any shape evenly: 213 x 213 x 213 took 190 us on the 16 SMs that 64 x 64
 // tiles gave it, 20 us now; (40 + 72 + 136) x 1501, K = 2001: 2.71 ms, 1.26 ms now
-// (FP64 rate alone 1.3).  FP32: 16 entries a thread, 4 where the large tiles
+// (1.19 at 1.25 TFLOP/s).  FP32: 16 entries a thread, 4 where the large tiles
 // would leave SMs idle (the 49 updates of a psvd of rank 370: 742 us, 433 us now).
 template <int BM_, int BN_, int BK_, int TM_, int TN_>
 struct Tile {

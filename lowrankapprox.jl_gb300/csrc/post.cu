@@ -580,7 +580,7 @@ void jacobi_svd_fast(lra_ctx* ctx, int64_t n, T* X, int64_t ldx, T* V, int64_t l
   // from cosines below that gap: the start level falls with n)
   const double start = ctx->tuning.gram_start > 0 ? 1e-4 * ctx->tuning.gram_start : std::min(kGramStart, 12.0 / (double)n);
   // Gram-product sweeps (jacobi_gram.cu) at every order they take (64 on): 3.5
-  // -> 2.3 ms against the in-cluster kernel at n = 363, 70 -> 26 ms against the
+  // -> 2.4 ms against the in-cluster kernel at n = 363, 70 -> 26 ms against the
   // block-pair kernel at n = 1803; the tuning keys of those two ask for them
   // instead.  A shifted eigenproblem stays with the column rotations: its norms
   // lie together, the pairwise sweeps have to finish it, and they start
