@@ -1522,7 +1522,8 @@ void make_sketch_c(lra_ctx* ctx, const lra_opts& o, char trans, int64_t M, int64
       CX<R>* g = ctx->arena.alloc_n<CX<R>>(std::max<int64_t>(K, 1));
       cgauss<R>(rs, K, g);
       std::vector<int64_t> start(order + 1, 0);
-      for (int64_t i = 1; i <= order; ++i) start[i] = start[i - 1] + (K - i) / order + 1;
+      // fld(K - i, order) + 1 rows in group i: none from i = K + 1 on
+      for (int64_t i = 1; i <= order; ++i) start[i] = start[i - 1] + (i <= K ? (K - i) / order + 1 : 0);
       int64_t* dst = ctx->arena.alloc_n<int64_t>(order + 1);
       LRA_CUDA(cudaMemcpyAsync(dst, start.data(), (order + 1) * sizeof(int64_t), cudaMemcpyHostToDevice,
                                ctx->stream));

@@ -157,3 +157,21 @@ def test_complex_curfact_and_snorm(lra, oracle, dt):
     d = lra.snormdiff(B, C, rand=lra.RandStream(gauss=g))
     dref = oracle.snormdiff_dense(B, C, oracle.Opts(), oracle.RandStream(gauss=g))
     assert abs(d - dref) <= 1e-3 * dref
+
+
+@pytest.mark.parametrize("dt", CDT)
+@pytest.mark.parametrize("m,n,order", [(6, 2, 32), (1, 5, 9), (33, 40, 41), (40, 33, 40)])
+def test_complex_sparse_sketch_of_few_rows(lra, oracle, dt, m, n, order):
+    """A sparse Gaussian sketch with more rows than the matrix: those beyond are
+    empty, and nothing past the permutation is read."""
+    rng = np.random.default_rng(m)
+    A = np.asfortranarray((rng.standard_normal((m, n)) + 1j * rng.standard_normal((m, n))).astype(dt))
+    tol = 1e-12 if dt == np.complex128 else 1e-5
+    for side, trans in (("left", "n"), ("left", "c"), ("right", "n"), ("right", "c")):
+        ors, grs = streams(lra, oracle, 12)
+        B = lra.sketch(side, trans, A, order, lra.LRAOptions(dt, sketch="sprn"), rand=grs)
+        R = oracle.sketch(side, trans, A, order, oracle.Opts(sketch="sprn"), ors)
+        assert np.abs(B - R).max() <= tol * max(1.0, np.abs(R).max()), (side, trans)
+    V = lra.idfact(A, lra.LRAOptions(dt, rtol=1e-4, sketch="sprn", seed=3))
+    E = A[:, V.rd - 1] - A[:, V.sk - 1] @ V.T
+    assert V.k == min(m, n) and (E.size == 0 or np.abs(E).max() <= 1e-3 * np.abs(A).max())
